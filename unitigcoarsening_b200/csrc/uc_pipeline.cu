@@ -25,7 +25,6 @@
 #include "uc_pipeline.h"
 
 #include <cuda_pipeline.h>
-#include <cub/device/device_radix_sort.cuh>
 
 namespace uc {
 
@@ -2490,12 +2489,6 @@ static int grid_for(const Env& e, uint64_t work, int block) {
   return int(std::max<uint64_t>(1, std::min(want, cap)));
 }
 
-#define UC_CK(call)                                                                                  \
-  do {                                                                                               \
-    cudaError_t _e = (call);                                                                         \
-    if (_e != cudaSuccess) return e.fail(UC_ECUDA, std::string(#call) + ": " + cudaGetErrorString(_e)); \
-  } while (0)
-
 int Env::fail(int code, const std::string& msg) {
   err = msg;
   return code;
@@ -2978,19 +2971,6 @@ static int bucket_offsets(Env& e, const Front& f, const uint32_t* counts, uint64
 }
 static int bucket_offsets(Env& e, const Front& f, uint64_t M, uint64_t& copies) {
   return bucket_offsets(e, f, f.counts, M, f.boff, copies);
-}
-
-// Let a kernel take all the dynamic shared memory an SM offers a block.  The
-// attribute is process-wide, so it is always set to the same maximum: a
-// per-call size would let one host thread lower it under another thread's
-// launch (concurrent contexts and server lanes).
-template <class K>
-static int allow_max_smem(Env& e, K kernel) {
-  cudaFuncAttributes a{};
-  UC_CK(cudaFuncGetAttributes(&a, kernel));
-  UC_CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             e.smem_optin - int(a.sharedSizeBytes)));
-  return UC_OK;
 }
 
 // Level split of the scatter: 2^mcb coarse partitions of 2^fb buckets.
@@ -4427,246 +4407,6 @@ int compact_device(Env& e, const char* d_text, size_t bytes, int k, int l, char*
   out_bytes = len;
   if (r == UC_OK && e.sorted && len) r = sort_lines(e, out, len, k);
   return r;
-}
-
-// ============================================================ sorted output
-
-// 0x80 in every byte of w that is a line break.
-__device__ __forceinline__ uint32_t nl_bytes(uint32_t w) {
-  const uint32_t z = w ^ 0x0A0A0A0Au;
-  return ~(((z & 0x7F7F7F7Fu) + 0x7F7F7F7Fu) | z) & 0x80808080u;
-}
-
-// Line breaks in each 64 KiB chunk of out[0, n), 16-byte loads (out is
-// 16-byte aligned; the tail of a chunk that ends inside a word is read
-// byte by byte).
-constexpr uint32_t NL_CHUNK = 1u << 16;
-__global__ void __launch_bounds__(256) k_nl_count16(const char* __restrict__ out, uint64_t n,
-                                                    uint32_t* __restrict__ cnt) {
-  const uint64_t c0 = uint64_t(blockIdx.x) * NL_CHUNK;
-  uint32_t acc = 0;
-#pragma unroll 4
-  for (uint32_t j = 0; j < NL_CHUNK / (16 * 256); ++j) {
-    const uint64_t off = c0 + 16ull * (threadIdx.x + 256u * j);
-    if (off + 16 <= n) {
-      const uint4 v = __ldcs(reinterpret_cast<const uint4*>(out + off));
-      acc += __popc(nl_bytes(v.x)) + __popc(nl_bytes(v.y)) + __popc(nl_bytes(v.z)) + __popc(nl_bytes(v.w));
-    } else {
-      for (uint64_t i = off; i < n && i < off + 16; ++i) acc += (out[i] == '\n');
-    }
-  }
-  acc = __reduce_add_sync(0xFFFFFFFFu, acc);
-  __shared__ uint32_t sh[8];
-  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = acc;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    uint32_t t = 0;
-    for (int w = 0; w < 8; ++w) t += sh[w];
-    cnt[blockIdx.x] = t;
-  }
-}
-
-// Line starts: starts[0] = 0 and starts[r + 1] = 1 + the position of the
-// r-th line break in out[0, n).  Each thread owns 256 contiguous bytes of its
-// block's chunk: a count pass, a block scan, then a pass that writes.
-__global__ void __launch_bounds__(256) k_nl_starts16(const char* __restrict__ out, uint64_t n,
-                                                     const unsigned long long* __restrict__ coff,
-                                                     unsigned long long* __restrict__ starts, uint64_t nlines) {
-  const uint64_t t0 = uint64_t(blockIdx.x) * NL_CHUNK + 256ull * threadIdx.x;
-  if (blockIdx.x == 0 && threadIdx.x == 0) starts[0] = 0;
-  uint32_t mine = 0;
-  for (uint32_t j = 0; j < 16; ++j) {
-    const uint64_t off = t0 + 16ull * j;
-    if (off + 16 <= n) {
-      const uint4 v = *reinterpret_cast<const uint4*>(out + off);
-      mine += __popc(nl_bytes(v.x)) + __popc(nl_bytes(v.y)) + __popc(nl_bytes(v.z)) + __popc(nl_bytes(v.w));
-    } else {
-      for (uint64_t i = off; i < n && i < off + 16; ++i) mine += (out[i] == '\n');
-    }
-  }
-  __shared__ uint32_t sc[33];
-  uint32_t tot;
-  uint64_t r = coff[blockIdx.x] + block_excl_scan(mine, sc, &tot);
-  for (uint32_t j = 0; j < 16; ++j) {
-    const uint64_t off = t0 + 16ull * j;
-    if (off + 16 <= n) {
-      const uint4 v = *reinterpret_cast<const uint4*>(out + off);
-      const uint32_t wv[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        uint32_t m = nl_bytes(wv[q]);
-        while (m) {
-          const int b = (__ffs(m) - 1) >> 3;
-          m &= m - 1;
-          ++r;
-          if (r < nlines) starts[r] = off + 4u * q + b + 1;
-        }
-      }
-    } else {
-      for (uint64_t i = off; i < n && i < off + 16; ++i) {
-        if (out[i] == '\n') {
-          ++r;
-          if (r < nlines) starts[r] = i + 1;
-        }
-      }
-    }
-  }
-}
-
-// Line keys: each line's first k chars, packed big-endian (first char in the
-// top bits of hi, chars 32.. in lo), so that numeric order is byte order.
-// Every k-mer begins at most one line, so these keys order the lines
-// completely.  The k chars are read as 4-byte words
-// (funnel-shifted to the line's byte offset) and converted 4 codes at a time;
-// the little-endian codes are then reversed into big-endian keys.  Reads up
-// to 12 bytes past a line's k chars (inside the output buffer's bound).
-__global__ void k_line_keys4(const char* __restrict__ out, const unsigned long long* __restrict__ starts,
-                             uint64_t L, int k, unsigned long long* __restrict__ khi,
-                             unsigned long long* __restrict__ klo, uint32_t* __restrict__ idx) {
-  const int nw = (k + 3) / 4;
-  const uint64_t m0 = (k >= 32) ? ~0ull : ((1ull << (2 * k)) - 1ull);
-  const uint64_t m1 = (k <= 32) ? 0ull : ((k - 32 >= 32) ? ~0ull : ((1ull << (2 * (k - 32))) - 1ull));
-  for (uint64_t j = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; j < L; j += uint64_t(gridDim.x) * blockDim.x) {
-    const uintptr_t a = reinterpret_cast<uintptr_t>(out + starts[j]);
-    const uint32_t* w = reinterpret_cast<const uint32_t*>(a & ~uintptr_t(3));
-    const uint32_t sh = 8u * uint32_t(a & 3u);
-    uint64_t w0 = 0, w1 = 0;
-    uint32_t cur = w[0];
-    for (int q = 0; q < nw; ++q) {
-      const uint32_t nxt = w[q + 1];
-      const uint32_t x = __funnelshift_r(cur, nxt, sh);
-      cur = nxt;
-      const uint64_t g = gather_codes(((x >> 1) ^ (x >> 2)) & 0x03030303u);
-      if (q < 8) w0 |= g << (8 * q);
-      else w1 |= g << (8 * (q - 8));
-    }
-    khi[j] = rev2(w0 & m0);
-    klo[j] = rev2(w1 & m1);
-    idx[j] = uint32_t(j);
-  }
-}
-
-__global__ void k_gather_u64(const unsigned long long* __restrict__ src, const uint32_t* __restrict__ idx,
-                             uint64_t L, unsigned long long* __restrict__ dst) {
-  for (uint64_t j = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; j < L; j += uint64_t(gridDim.x) * blockDim.x)
-    dst[j] = src[idx[j]];
-}
-
-__global__ void k_sorted_len(const unsigned long long* __restrict__ starts, const uint32_t* __restrict__ idx,
-                             uint64_t L, uint32_t* __restrict__ len) {
-  for (uint64_t j = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; j < L; j += uint64_t(gridDim.x) * blockDim.x) {
-    const uint32_t i = idx[j];
-    len[j] = uint32_t(starts[i + 1] - starts[i]);
-  }
-}
-
-// Lines to their sorted places: a warp resolves 32 lines, then copies them.
-__global__ void k_line_copy(const char* __restrict__ src, const unsigned long long* __restrict__ starts,
-                            const uint32_t* __restrict__ idx, const unsigned long long* __restrict__ dsto,
-                            uint64_t L, char* __restrict__ dst) {
-  const int lane = threadIdx.x & 31;
-  const uint64_t warp = (uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-  const uint64_t nwarps = (uint64_t(gridDim.x) * blockDim.x) >> 5;
-  for (uint64_t base = warp * 32u; base < L; base += nwarps * 32u) {
-    const uint64_t j = base + uint64_t(lane);
-    uint64_t so = 0, d = 0;
-    uint32_t m = 0;
-    if (j < L) {
-      const uint32_t i = idx[j];
-      so = starts[i];
-      m = uint32_t(starts[i + 1] - so);
-      d = dsto[j];
-    }
-    uint32_t todo = __ballot_sync(0xFFFFFFFFu, j < L);
-    while (todo) {
-      const int q = __ffs(todo) - 1;
-      todo &= todo - 1;
-      const uint64_t a = __shfl_sync(0xFFFFFFFFu, so, q);
-      const uint64_t b = __shfl_sync(0xFFFFFFFFu, d, q);
-      const uint32_t n = __shfl_sync(0xFFFFFFFFu, m, q);
-      for (uint32_t x = lane; x < n; x += 32) dst[b + x] = src[a + x];
-    }
-  }
-}
-
-int sort_lines(Env& e, char* out, uint64_t bytes, int k) {
-  if (bytes == 0) return UC_OK;
-  e.reset();
-  const uint32_t chunk = NL_CHUNK;
-  const uint64_t nchunks = std::max<uint64_t>(1, (bytes - 1 + chunk - 1) / chunk);
-  const bool aligned = (reinterpret_cast<uintptr_t>(out) & 15u) == 0;  // else byte-wise line scan
-  // lines end with '\n'; the last one at bytes - 1
-  const uint64_t Lmax = bytes / uint64_t(k + 1) + 1;
-  size_t cub_bytes = 0;
-  cub::DeviceRadixSort::SortPairs(nullptr, cub_bytes, static_cast<const unsigned long long*>(nullptr),
-                                  static_cast<unsigned long long*>(nullptr), static_cast<const uint32_t*>(nullptr),
-                                  static_cast<uint32_t*>(nullptr), int(Lmax), 0, 64, e.stream);
-  size_t need = 0;
-  auto add = [&](size_t b) { need += (b + 255) & ~size_t(255); };
-  add(bytes); add(nchunks * 4); add((nchunks + 1) * 8); add(scan_tmp_elems(nchunks) * 8);
-  add((Lmax + 1) * 8);                         // starts
-  add(Lmax * 8); add(Lmax * 8); add(Lmax * 8); // khi, klo, sorted keys
-  add(Lmax * 4); add(Lmax * 4);                // idx, sorted idx
-  add(Lmax * 4); add((Lmax + 1) * 8); add(scan_tmp_elems(Lmax) * 8);
-  add(cub_bytes);
-  int r = e.reserve(1, need);
-  if (r) return r;
-  char* tmp = static_cast<char*>(e.take(1, bytes));
-  uint32_t* cnt = static_cast<uint32_t*>(e.take(1, nchunks * 4));
-  auto T64 = [&](uint64_t c) { return static_cast<unsigned long long*>(e.take(1, c * 8)); };
-  auto T32 = [&](uint64_t c) { return static_cast<uint32_t*>(e.take(1, c * 4)); };
-  unsigned long long* coff = T64(nchunks + 1);
-  unsigned long long* ctmp = T64(scan_tmp_elems(nchunks));
-  unsigned long long* starts = T64(Lmax + 1);
-  unsigned long long* khi = T64(Lmax);
-  unsigned long long* klo = T64(Lmax);
-  unsigned long long* ks = T64(Lmax);
-  uint32_t* idx = T32(Lmax);
-  uint32_t* idx2 = T32(Lmax);
-  uint32_t* len = T32(Lmax);
-  unsigned long long* dsto = T64(Lmax + 1);
-  unsigned long long* stmp = T64(scan_tmp_elems(Lmax));
-  void* cub_tmp = e.take(1, cub_bytes);
-  if (!cub_tmp) return e.fail(UC_EBUDGET, "arena overflow (sorted output)");
-  const uint8_t* ob = reinterpret_cast<const uint8_t*>(out);
-  e.launches += 1 + 6 + 1;
-  if (aligned) k_nl_count16<<<unsigned(nchunks), 256, 0, e.stream>>>(out, bytes - 1, cnt);
-  else k_count_nl<<<unsigned(nchunks), 256, 0, e.stream>>>(ob, 0, bytes - 1, cnt, chunk);
-  scan_excl<uint32_t, unsigned long long>(cnt, nchunks, coff, ctmp, e.stream);
-  unsigned long long nl = 0;
-  UC_CK(cudaMemcpyAsync(&nl, coff + nchunks, 8, cudaMemcpyDeviceToHost, e.stream));
-  UC_CK(cudaStreamSynchronize(e.stream));
-  const uint64_t L = nl + 1;
-  if (L > Lmax || L >= 0x7FFFFFFFull) return e.fail(UC_EINTERNAL, "line count of the output out of range");
-  if (aligned) k_nl_starts16<<<unsigned(nchunks), 256, 0, e.stream>>>(out, bytes - 1, coff, starts, L);
-  else k_write_starts<<<unsigned(nchunks), 256, 0, e.stream>>>(ob, 0, bytes - 1, coff, chunk, starts, L);
-  UC_CK(cudaMemcpyAsync(starts + L, &bytes, 8, cudaMemcpyHostToDevice, e.stream));
-  const int g = grid_for(e, L, 256);
-  e.launches += 1;
-  k_line_keys4<<<g, 256, 0, e.stream>>>(out, starts, L, k, khi, klo, idx);
-  // least significant part first; radix sort is stable
-  uint32_t* order = idx;
-  if (k > 32) {
-    UC_CK(cub::DeviceRadixSort::SortPairs(cub_tmp, cub_bytes, klo, ks, idx, idx2, int(L), 128 - 2 * k, 64,
-                                          e.stream));
-    ++e.launches;
-    k_gather_u64<<<g, 256, 0, e.stream>>>(khi, idx2, L, klo);
-    UC_CK(cub::DeviceRadixSort::SortPairs(cub_tmp, cub_bytes, klo, ks, idx2, idx, int(L), 0, 64, e.stream));
-    order = idx;
-  } else {
-    UC_CK(cub::DeviceRadixSort::SortPairs(cub_tmp, cub_bytes, khi, ks, idx, idx2, int(L), 64 - 2 * k, 64,
-                                          e.stream));
-    order = idx2;
-  }
-  e.launches += 2 + 6;
-  k_sorted_len<<<g, 256, 0, e.stream>>>(starts, order, L, len);
-  scan_excl<uint32_t, unsigned long long>(len, L, dsto, stmp, e.stream);
-  k_line_copy<<<g, 256, 0, e.stream>>>(out, starts, order, dsto, L, tmp);
-  UC_CK(cudaGetLastError());
-  UC_CK(cudaMemcpyAsync(out, tmp, bytes, cudaMemcpyDeviceToDevice, e.stream));
-  UC_CK(cudaStreamSynchronize(e.stream));
-  e.reset();
-  return UC_OK;
 }
 
 }  // namespace uc

@@ -73,6 +73,25 @@ struct Env {
   int check_err(const Counters* h);
 };
 
+#define UC_CK(call)                                                                                  \
+  do {                                                                                               \
+    cudaError_t _e = (call);                                                                         \
+    if (_e != cudaSuccess) return e.fail(UC_ECUDA, std::string(#call) + ": " + cudaGetErrorString(_e)); \
+  } while (0)
+
+// Let a kernel take all the dynamic shared memory an SM offers a block.  The
+// attribute is process-wide, so it is always set to the same maximum: a
+// per-call size would let one host thread lower it under another thread's
+// launch (concurrent contexts and server lanes).
+template <class K>
+int allow_max_smem(Env& e, K kernel) {
+  cudaFuncAttributes a{};
+  UC_CK(cudaFuncGetAttributes(&a, kernel));
+  UC_CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             e.smem_optin - int(a.sharedSizeBytes)));
+  return UC_OK;
+}
+
 int parse_header(Env& e, const char* d_text, size_t bytes, uint64_t& n, uint64_t& body);
 int pack(Env& e, const char* d_text, size_t bytes, int k, uint64_t* d_keys, uint64_t& n_out);
 int minimizers(Env& e, const uint64_t* d_keys, uint64_t n, int k, int l, uint64_t seed,

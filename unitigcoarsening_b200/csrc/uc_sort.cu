@@ -1,0 +1,978 @@
+// uc_sort.cu — the lines of a finished job in byte order (sorted output).
+//
+// Every line begins with a distinct k-mer, so its first k chars order it, and
+// most lines are that k-mer plus a few chars.  A line is therefore sorted as
+// a record that holds all of it in 2-bit codes (one or two key words and a
+// tail word), and the sorted text is spelled from the records:
+//   k_line_recs    text -> records, and a count per bin of leading key bits
+//   k_line_plan    bins -> tiles of about TILE_WINDOW records
+//   k_line_group   records -> their tiles (by groups of tiles first)
+//   k_line_tiles   one block per tile: order in shared memory, the tile's
+//                  place in the output by look-back, lines spelled and stored
+// Nothing returns to the host in between.  The text is read once and written
+// once.  Lines with more than TAIL_MAX chars after the k-mer keep their chars
+// in a copy of the text and are copied.
+//
+// 256 Mbp, k = 31 (107M lines, 3.6 GB) on a B200: 1.9 + 2.2 + 3.0 ms (records,
+// groups, tiles), where a radix sort of (key, line index) pairs with a gather
+// of the lines (seven passes over pairs or lines) took 28 ms.
+#include <algorithm>
+#include <cstring>
+
+#include "uc_kernels.cuh"
+#include "uc_lookback.cuh"
+#include "uc_pipeline.h"
+
+namespace uc {
+
+namespace {
+
+constexpr int TAIL_MAX = 28;                         // chars after the k-mer that a tail word holds
+constexpr uint64_t TAIL_LONG = 1ull << 63;           // tail word: index of a LongLine
+constexpr int TAIL_LEN_SHIFT = 58;                   // else: char count above the codes (first char lowest)
+constexpr unsigned long long HUGE_LINE = 1ull << 16; // bytes from which a line is copied by the whole grid
+
+constexpr uint32_t LR_CHUNK = 16384;  // text bytes whose line starts one block pass takes
+constexpr uint32_t LR_PRE = 16;       // bytes before them (the line break before the first start)
+constexpr uint32_t LR_HALO = 112;     // bytes after them: k + TAIL_MAX + 1 <= 92, read in words
+constexpr uint32_t LR_PIECES = (LR_PRE + LR_CHUNK + LR_HALO) / 16;
+
+constexpr uint32_t TILE_THREADS = 256;
+constexpr uint32_t TILE_SUB = 2048;  // sub-bins of a tile
+// records a tile sorts in shared memory: four blocks per SM (three with two
+// key words) fit
+template <int RW>
+__host__ __device__ constexpr uint32_t tile_cap() {
+  return RW == 2 ? 2048u : 1536u;
+}
+constexpr uint32_t PLAN_ITEMS = 16;  // bins per thread of the plan
+// Cursors lie 32 bytes apart: atomics on words of one L2 line queue up (about
+// 2 ns each).
+constexpr uint32_t CUR_STRIDE = 8;
+constexpr int MAX_BIN_BITS = 23;     // counts stay in L2 (32 MiB)
+
+struct LongLine {
+  unsigned long long at;   // offset in the text
+  unsigned long long len;  // bytes, line break included
+  unsigned long long to;   // of a huge line: offset in the sorted text
+};
+
+struct SortCtr {
+  uint32_t nrec, nlong, nhuge, ntiles;
+  uint32_t plan_ticket, tile_ticket, fail, pad;
+};
+
+// One record: keys big-endian (first char in the top bits), so that numeric
+// order is byte order.  RW words: (key, tail) for k <= 31, (key, key, tail)
+// otherwise; the first two words lie together.
+template <int RW>
+struct Rec {
+  uint64_t hi, lo, tail;
+};
+template <int RW>
+struct RecArr {
+  ulonglong2* a;
+  unsigned long long* t;  // tails (RW == 3)
+};
+template <int RW>
+__device__ __forceinline__ Rec<RW> ld_rec(const RecArr<RW>& r, uint64_t i) {
+  const ulonglong2 v = r.a[i];
+  if constexpr (RW == 2) return Rec<RW>{v.x, 0ull, v.y};
+  else return Rec<RW>{v.x, v.y, r.t[i]};
+}
+template <int RW>
+__device__ __forceinline__ void st_rec(const RecArr<RW>& r, uint64_t i, const Rec<RW>& x) {
+  if constexpr (RW == 2) {
+    r.a[i] = make_ulonglong2(x.hi, x.tail);
+  } else {
+    r.a[i] = make_ulonglong2(x.hi, x.lo);
+    r.t[i] = x.tail;
+  }
+}
+
+__device__ __forceinline__ unsigned long long line_bytes_of(uint64_t tail, int k, const LongLine* longs) {
+  return (tail & TAIL_LONG) ? longs[uint32_t(tail)].len : uint64_t(k) + 1u + ((tail >> TAIL_LEN_SHIFT) & 31u);
+}
+
+// Text -> records.  A block reads a chunk of text with 16-byte loads and keeps
+// its 2-bit codes and a bit per line break in shared memory (the text itself
+// is not staged: a line's key and tail are then a few funnel shifts of code
+// words), lists the chunk's line starts from the bits (two words per thread,
+// one block scan), and makes one line's record per thread.
+// The records come in no particular order: a block reserves the places of its
+// lines with one atomic.  256 Mbp, k = 31: 1.9 ms for 5.3 GB, bound by issue
+// (60%) and barriers; converting each line from staged text instead took 2.3.
+template <int RW>
+__global__ void __launch_bounds__(256, 5) k_line_recs(const char* __restrict__ out, uint64_t n, int k, int bits,
+                                                   RecArr<RW> rec, uint32_t* __restrict__ counts,
+                                                   LongLine* __restrict__ longs, uint32_t* __restrict__ huge,
+                                                   SortCtr* sc) {
+  __shared__ uint32_t code[LR_PIECES];  // 16 chars each
+  __shared__ __align__(16) uint32_t nlw[LR_PIECES / 2 + 1];
+  __shared__ uint32_t scan[33];
+  __shared__ uint32_t s_base, s_open;
+  __shared__ unsigned long long s_end;
+  extern __shared__ uint16_t starts[];  // LR_CHUNK / (k + 1) + 2
+  uint16_t* nl16 = reinterpret_cast<uint16_t*>(nlw);
+  const uint32_t tid = threadIdx.x;
+  // positions are relative to the 16-byte boundary at or below out
+  const char* A = reinterpret_cast<const char*>(reinterpret_cast<uintptr_t>(out) & ~uintptr_t(15));
+  const uint64_t off0 = uint64_t(out - A), end = off0 + n;
+  const uint64_t nchunks = (end + LR_CHUNK - 1) / LR_CHUNK;
+  const uint64_t m0 = (2 * k >= 64) ? ~0ull : ((1ull << (2 * k)) - 1ull);
+  for (uint64_t c = blockIdx.x; c < nchunks; c += gridDim.x) {
+    const uint64_t c0 = c * LR_CHUNK;
+    // (all loads of the chunk in flight together; a chunk inside the text
+    // needs no checks)
+    const bool inside = c0 >= off0 + LR_PRE && c0 + LR_CHUNK + LR_HALO <= end;
+    constexpr uint32_t PP = (LR_PIECES + 255) / 256;
+    uint4 v[PP];
+#pragma unroll
+    for (uint32_t q = 0; q < PP; ++q) {
+      const uint32_t p = q * 256 + tid;
+      const int64_t x = int64_t(c0) - int64_t(LR_PRE) + 16 * int64_t(p);
+      v[q] = make_uint4(0x41414141u, 0x41414141u, 0x41414141u, 0x41414141u);
+      if (p < LR_PIECES && (inside || (x >= int64_t(off0) && x + 16 <= int64_t(end))))
+        v[q] = __ldcs(reinterpret_cast<const uint4*>(A + x));
+    }
+#pragma unroll
+    for (uint32_t q = 0; q < PP; ++q) {
+      const uint32_t p = q * 256 + tid;
+      if (p >= LR_PIECES) break;
+      const int64_t x = int64_t(c0) - int64_t(LR_PRE) + 16 * int64_t(p);
+      if (!inside && (x < int64_t(off0) || x + 16 > int64_t(end)) && x + 16 > int64_t(off0) && x < int64_t(end)) {
+        uint32_t w[4] = {0x41414141u, 0x41414141u, 0x41414141u, 0x41414141u};  // a piece at an end of the text
+#pragma unroll
+        for (int b = 0; b < 16; ++b)
+          if (x + b >= int64_t(off0) && x + b < int64_t(end))
+            w[b >> 2] ^= (uint32_t(static_cast<unsigned char>(A[x + b])) ^ 0x41u) << (8 * (b & 3));
+        v[q] = make_uint4(w[0], w[1], w[2], w[3]);
+      }
+      code[p] = codes16(v[q]);
+      nl16[p] = uint16_t(breaks16(v[q]));
+    }
+    if (tid == 0) {
+      s_open = 0;
+      nlw[LR_PIECES / 2] = 0;
+    }
+    __syncthreads();
+    // a line starts after each line break, and at the text's first byte
+    uint32_t sb[2];
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      const uint32_t w = 2 * tid + q;
+      uint32_t b = __funnelshift_r(nlw[w], nlw[w + 1], LR_PRE - 1);
+      const uint64_t x0 = c0 + 32ull * w;
+      if (x0 == 0) b |= 1u << off0;
+      if (x0 + 32 > end) b &= (x0 >= end) ? 0u : (0xFFFFFFFFu >> (32u - uint32_t(end - x0)));
+      sb[q] = b;
+    }
+    uint32_t nl;
+    uint32_t at = block_excl_scan(uint32_t(__popc(sb[0]) + __popc(sb[1])), scan, &nl);
+    const uint32_t cap = LR_CHUNK / (uint32_t(k) + 1u) + 2u;
+    if (nl > cap) {  // a line shorter than k: not this library's output
+      if (tid == 0) atomicOr(&sc->fail, 2u);
+      nl = 0;
+    }
+    if (nl) {
+#pragma unroll
+      for (int q = 0; q < 2; ++q)
+        for (uint32_t b = sb[q]; b; b &= b - 1) starts[at++] = uint16_t(64 * tid + 32 * q + (__ffs(b) - 1));
+    }
+    if (tid == 0) s_base = nl ? atomicAdd(&sc->nrec, nl) : 0u;
+    __syncthreads();
+    auto emit = [&](uint32_t j, uint32_t s, unsigned long long len) {  // len: chars of the line
+      const bool is_long = len > uint64_t(k + TAIL_MAX);
+      const uint32_t t = is_long ? 0u : uint32_t(len) - uint32_t(k);
+      // the line's code stream from its first char (words past the halo are
+      // not reached: k + TAIL_MAX chars at most count)
+      const uint32_t wi = (LR_PRE + s) >> 4, sh = 2u * ((LR_PRE + s) & 15u);
+      constexpr int NC = RW == 2 ? 4 : 6;
+      uint32_t c[NC + 1], x[NC];
+#pragma unroll
+      for (int q = 0; q <= NC; ++q) c[q] = code[wi + q];
+#pragma unroll
+      for (int q = 0; q < NC; ++q) x[q] = __funnelshift_r(c[q], c[q + 1], sh);
+      const uint64_t s0 = x[0] | (uint64_t(x[1]) << 32), s1 = x[2] | (uint64_t(x[3]) << 32);
+      uint64_t tl;
+      Rec<RW> r;
+      if constexpr (RW == 2) {
+        r.hi = rev2(s0 & m0);
+        r.lo = 0;
+        tl = (s0 >> (2 * k)) | (s1 << (64 - 2 * k));
+      } else {
+        const uint64_t s2 = x[NC - 2] | (uint64_t(x[NC - 1]) << 32);
+        const int u = 2 * k - 64;
+        r.hi = rev2(s0);
+        r.lo = rev2(s1 & ((1ull << u) - 1ull));
+        tl = u ? ((s1 >> u) | (s2 << (64 - u))) : s1;
+      }
+      if (is_long) {
+        const uint32_t i = atomicAdd(&sc->nlong, 1u);
+        longs[i] = LongLine{c0 + s - off0, len + 1, 0ull};
+        if (len + 1 >= HUGE_LINE) huge[atomicAdd(&sc->nhuge, 1u)] = i;
+        r.tail = TAIL_LONG | i;
+      } else {
+        r.tail = (uint64_t(t) << TAIL_LEN_SHIFT) | (tl & ((1ull << (2 * t)) - 1ull));
+      }
+      atomicAdd(counts + (r.hi >> (64 - bits)), 1u);
+      st_rec<RW>(rec, s_base + j, r);
+    };
+    for (uint32_t j = tid; j < nl; j += 256) {
+      const uint32_t s = starts[j];
+      uint32_t len;
+      if (j + 1 < nl) {
+        len = uint32_t(starts[j + 1]) - s - 1u;
+      } else {
+        // the chunk's last line: its break in the bits, or past the halo
+        const uint32_t i0 = LR_PRE + s + uint32_t(k);
+        uint32_t w = i0 >> 5, m = nlw[w] & (0xFFFFFFFFu << (i0 & 31u));
+        while (!m && ++w < LR_PIECES / 2) m = nlw[w];
+        len = m ? 32u * w + uint32_t(__ffs(m) - 1) - LR_PRE - s : 0u;
+        if (!m) s_open = j + 1u;
+      }
+      if (len >= uint32_t(k)) emit(j, s, len);
+      else if (len || j + 1 < nl) atomicOr(&sc->fail, 2u);
+    }
+    __syncthreads();
+    if (s_open) {
+      // the last line goes on past the halo: the whole block looks for its break
+      const uint32_t j = s_open - 1u, s = starts[j];
+      if (tid == 0) s_end = end;
+      __syncthreads();
+      for (uint64_t x0 = c0 + LR_CHUNK + LR_HALO; x0 < end; x0 += 8u * 16u * 256u) {
+        unsigned long long found = end;
+#pragma unroll
+        for (int q = 7; q >= 0; --q) {
+          const uint64_t x = x0 + 16u * (uint32_t(q) * 256u + tid);
+          if (x + 16 <= end) {
+            const uint4 v = __ldcs(reinterpret_cast<const uint4*>(A + x));
+            const uint32_t m = breaks16(v);
+            if (m) found = x + uint32_t(__ffs(m) - 1);
+          } else {
+            for (uint64_t y = end; y > x;) {
+              --y;
+              if (A[y] == '\n') found = y;
+            }
+          }
+        }
+        if (found < end) atomicMin(&s_end, found);
+        __syncthreads();
+        const bool stop = s_end < end;
+        __syncthreads();
+        if (stop) break;
+      }
+      if (tid == 0) emit(j, s, s_end - (c0 + s));
+    }
+    __syncthreads();  // code, nlw, starts are reused
+  }
+}
+
+// Bins -> tiles.  Tile t takes the bins whose first record's rank lies in
+// [t * win, (t + 1) * win), so a tile holds at most one window and the rest of
+// its last bin.  One pass: prefix sums by look-back, each bin's tile in place
+// of its count, each tile's first record and first bin, and the cursors of
+// the tiles and of the groups of 2^gsh tiles.
+__global__ void __launch_bounds__(256) k_line_plan(uint32_t* __restrict__ counts, uint32_t m, uint32_t win,
+                                                   uint2* __restrict__ tile, uint32_t* __restrict__ cur,
+                                                   uint32_t* __restrict__ gcur, uint32_t gsh, unsigned long long* st,
+                                                   SortCtr* sc) {
+  __shared__ uint32_t scan[33];
+  __shared__ uint32_t s_t, s_base;
+  if (threadIdx.x == 0) s_t = atomicAdd(&sc->plan_ticket, 1u);
+  __syncthreads();
+  const uint32_t b = s_t;
+  const uint32_t i0 = (b * 256u + threadIdx.x) * PLAN_ITEMS;
+  uint32_t c[PLAN_ITEMS];
+  uint32_t sum = 0;
+  uint4* src = reinterpret_cast<uint4*>(counts + i0);
+#pragma unroll
+  for (uint32_t q = 0; q < PLAN_ITEMS / 4; ++q) {
+    const uint4 v = i0 < m ? src[q] : make_uint4(0u, 0u, 0u, 0u);
+    c[4 * q] = v.x;
+    c[4 * q + 1] = v.y;
+    c[4 * q + 2] = v.z;
+    c[4 * q + 3] = v.w;
+    sum += v.x + v.y + v.z + v.w;
+  }
+  uint32_t tot;
+  const uint32_t pre = block_excl_scan(sum, scan, &tot);
+  if (threadIdx.x < 32) {
+    if (threadIdx.x == 0) lb_publish(st, b, LB_SUM, tot);
+    __syncwarp();
+    const uint32_t e = uint32_t(lb_exclusive(st, b, tot, &sc->fail));
+    if (threadIdx.x == 0) s_base = e;
+  }
+  __syncthreads();
+  uint32_t p = s_base + pre;
+  if (i0 >= m) return;
+  if (i0 == 0) {
+    tile[0] = make_uint2(0u, 0u);
+    cur[0] = gcur[0] = 0;
+  }
+  uint32_t tp = p / win;
+#pragma unroll
+  for (uint32_t q = 0; q < PLAN_ITEMS; ++q) {
+    const uint32_t nx = p + c[q], tn = nx / win;
+    c[q] = tp;
+    for (uint32_t t = tp + 1; t <= tn; ++t) {
+      tile[t] = make_uint2(nx, i0 + q + 1);
+      cur[t * CUR_STRIDE] = nx;
+      if (!(t & ((1u << gsh) - 1u))) gcur[(t >> gsh) * CUR_STRIDE] = nx;
+    }
+    p = nx;
+    tp = tn;
+  }
+#pragma unroll
+  for (uint32_t q = 0; q < PLAN_ITEMS / 4; ++q)
+    src[q] = make_uint4(c[4 * q], c[4 * q + 1], c[4 * q + 2], c[4 * q + 3]);
+  if (i0 + PLAN_ITEMS >= m) {
+    tile[tp + 1] = make_uint2(p, m);
+    sc->ntiles = tp + 1;
+  }
+}
+
+// n bytes from src to dst (any alignment) by `size` threads: 16-byte stores
+// of the destination, each from five source words.  Reads up to 3 bytes on
+// either side of the source bytes' words.
+__device__ __forceinline__ void copy_bytes(char* dst, const char* src, unsigned long long n, uint32_t rank,
+                                           uint32_t size) {
+  const uint32_t head = uint32_t(min((unsigned long long)((16u - uint32_t(reinterpret_cast<uintptr_t>(dst) & 15u)) & 15u), n));
+  if (rank < head) dst[rank] = src[rank];
+  dst += head;
+  src += head;
+  n -= head;
+  const uint32_t sh = 8u * uint32_t(reinterpret_cast<uintptr_t>(src) & 3u);
+  const uint32_t* w = reinterpret_cast<const uint32_t*>(reinterpret_cast<uintptr_t>(src) & ~uintptr_t(3));
+  const unsigned long long np = n >> 4;
+  for (unsigned long long p = rank; p < np; p += size) {
+    const uint32_t a = w[4 * p], b = w[4 * p + 1], c = w[4 * p + 2], d = w[4 * p + 3];
+    const uint32_t e = sh ? w[4 * p + 4] : 0u;
+    reinterpret_cast<uint4*>(dst)[p] = make_uint4(__funnelshift_r(a, b, sh), __funnelshift_r(b, c, sh),
+                                                  __funnelshift_r(c, d, sh), __funnelshift_r(d, e, sh));
+  }
+  const uint32_t rest = uint32_t(n & 15u);
+  for (uint32_t q = rank; q < rest; q += size) dst[16 * np + q] = src[16 * np + q];
+}
+
+// Records -> groups of 2^sh tiles (sh = 0: their tiles), in any order inside a
+// group.  A block takes a chunk of records, counts them per group in shared
+// memory, reserves one run per group present (cursors at cur) and writes the
+// runs out.  Groups are counted from the chunk's lowest one; a record past
+// the counted ones reserves its own place (a chunk that spans many groups:
+// few records among bins that overflow their tiles).
+//
+// Records scattered one by one, each with its own atomic, ran at 32 to 45 G
+// records/s whatever the occupancy (3.3 ms at 256 Mbp); as runs, two levels
+// take 2.2 ms.  With at most GRP_BINS tiles one level does.
+constexpr uint32_t GRP_THREADS = 512, GRP_BINS = 1024;
+template <int RW>
+__host__ __device__ constexpr uint32_t grp_chunk() {
+  return RW == 2 ? 4096u : 2048u;
+}
+template <int RW>
+__host__ __device__ constexpr size_t grp_smem() {
+  return size_t(grp_chunk<RW>()) * (8 * RW + 2) + GRP_BINS * 8 + 16;
+}
+template <int RW>
+__global__ void __launch_bounds__(GRP_THREADS, 2) k_line_group(RecArr<RW> in, RecArr<RW> to,
+                                                               const uint32_t* __restrict__ tmap, int bits, uint32_t sh,
+                                                               uint32_t* __restrict__ cur, const SortCtr* sc) {
+  extern __shared__ __align__(16) unsigned char sm[];
+  constexpr uint32_t CH = grp_chunk<RW>(), PER = CH / GRP_THREADS, BPT = GRP_BINS / GRP_THREADS;
+  static_assert(BPT == 2 && CH <= 4096, "a record's bin (10 bits) and its place in it share a word");
+  ulonglong2* sa = reinterpret_cast<ulonglong2*>(sm);
+  unsigned long long* stl = reinterpret_cast<unsigned long long*>(sa + CH);  // RW == 3
+  uint32_t* lofs = reinterpret_cast<uint32_t*>(sm + size_t(CH) * 8 * RW);    // [GRP_BINS] counts, then offsets
+  uint32_t* gofs = lofs + GRP_BINS;                                          // [GRP_BINS] global place of slot 0
+  uint16_t* sbin = reinterpret_cast<uint16_t*>(gofs + GRP_BINS);             // [CH]
+  __shared__ uint32_t scan[33], s_min;
+  const uint32_t tid = threadIdx.x;
+  if (sc->fail) return;
+  const uint32_t n = sc->nrec;
+  for (uint64_t c0 = uint64_t(blockIdx.x) * CH; c0 < n; c0 += uint64_t(gridDim.x) * CH) {
+    const uint32_t cn = uint32_t(min(uint64_t(n) - c0, uint64_t(CH)));
+    Rec<RW> r[PER];
+    uint32_t g[PER], low = 0xFFFFFFFFu;
+#pragma unroll
+    for (uint32_t q = 0; q < PER; ++q)
+      if (q * GRP_THREADS + tid < cn) r[q] = ld_rec<RW>(in, c0 + q * GRP_THREADS + tid);
+#pragma unroll
+    for (uint32_t q = 0; q < PER; ++q) {
+      g[q] = 0xFFFFFFFFu;
+      if (q * GRP_THREADS + tid < cn) g[q] = tmap[r[q].hi >> (64 - bits)] >> sh;
+      low = min(low, g[q]);
+    }
+    if (tid == 0) s_min = 0xFFFFFFFFu;
+    lofs[2 * tid] = lofs[2 * tid + 1] = 0;
+    __syncthreads();
+    low = __reduce_min_sync(0xFFFFFFFFu, low);
+    if ((tid & 31u) == 0) atomicMin(&s_min, low);
+    __syncthreads();
+    low = s_min;
+#pragma unroll
+    for (uint32_t q = 0; q < PER; ++q) {
+      if (q * GRP_THREADS + tid >= cn) continue;
+      const uint32_t b = g[q] - low;
+      if (b < GRP_BINS) {
+        g[q] = (atomicAdd(lofs + b, 1u) << 10) | b;
+      } else {
+        const uint32_t pos = atomicAdd(cur + g[q] * CUR_STRIDE, 1u);
+        if (pos < n) st_rec<RW>(to, pos, r[q]);
+        g[q] = 0xFFFFFFFFu;
+      }
+    }
+    __syncthreads();
+    uint32_t placed;
+    {
+      const uint32_t h0 = lofs[2 * tid], h1 = lofs[2 * tid + 1];
+      const uint32_t pre = block_excl_scan(h0 + h1, scan, &placed);
+      uint32_t* cc = cur + (low + 2 * tid) * CUR_STRIDE;
+      lofs[2 * tid] = pre;
+      lofs[2 * tid + 1] = pre + h0;
+      if (h0) gofs[2 * tid] = atomicAdd(cc, h0) - pre;
+      if (h1) gofs[2 * tid + 1] = atomicAdd(cc + CUR_STRIDE, h1) - (pre + h0);
+    }
+    __syncthreads();
+#pragma unroll
+    for (uint32_t q = 0; q < PER; ++q) {
+      if (q * GRP_THREADS + tid >= cn || g[q] == 0xFFFFFFFFu) continue;
+      const uint32_t b = g[q] & (GRP_BINS - 1u), sl = lofs[b] + (g[q] >> 10);
+      if constexpr (RW == 2) {
+        sa[sl] = make_ulonglong2(r[q].hi, r[q].tail);
+      } else {
+        sa[sl] = make_ulonglong2(r[q].hi, r[q].lo);
+        stl[sl] = r[q].tail;
+      }
+      sbin[sl] = uint16_t(b);
+    }
+    __syncthreads();
+    for (uint32_t sl = tid; sl < placed; sl += GRP_THREADS) {
+      const uint32_t pos = gofs[sbin[sl]] + sl;
+      if (pos >= n) continue;  // (counts that disagree: nothing out of bounds)
+      to.a[pos] = sa[sl];
+      if constexpr (RW == 3) to.t[pos] = stl[sl];
+    }
+    __syncthreads();  // the shared arrays are reused
+  }
+}
+
+// The chars of the long lines are kept: the sorted text overwrites them.
+__global__ void __launch_bounds__(256) k_line_keep(const char* __restrict__ out, char* __restrict__ keep,
+                                                   const LongLine* __restrict__ longs,
+                                                   const uint32_t* __restrict__ huge, const SortCtr* sc) {
+  const uint32_t nlong = sc->nlong, nhuge = sc->nhuge;
+  const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nwarps = (gridDim.x * blockDim.x) >> 5;
+  for (uint32_t i = warp; i < nlong; i += nwarps) {
+    const LongLine L = longs[i];
+    if (L.len < HUGE_LINE) copy_bytes(keep + L.at, out + L.at, L.len, threadIdx.x & 31u, 32u);
+  }
+  for (uint32_t h = 0; h < nhuge; ++h) {
+    const LongLine L = longs[huge[h]];
+    for (unsigned long long x = blockIdx.x * HUGE_LINE; x < L.len; x += gridDim.x * HUGE_LINE)
+      copy_bytes(keep + L.at + x, out + L.at + x, min(HUGE_LINE, L.len - x), threadIdx.x, blockDim.x);
+  }
+}
+
+// The line's bytes (k-mer, tail, line break) at shared-memory position pos of
+// buf: whole words where the line owns them, halves and bytes at its two ends
+// (shared with the neighbouring lines).
+template <int RW>
+__device__ __forceinline__ void spell_line(uint32_t* buf, uint32_t pos, const Rec<RW>& r, int k) {
+  const uint32_t t = uint32_t(r.tail >> TAIL_LEN_SHIFT) & 31u;
+  const uint64_t codes = r.tail & ((1ull << TAIL_LEN_SHIFT) - 1ull);
+  // the code stream, first char lowest, moved up by the chars before the
+  // line in its first word
+  const uint32_t a = pos & 3u;
+  constexpr int NC = RW == 2 ? 4 : 6;
+  uint32_t c[NC];
+  {
+    uint64_t w[3];
+    w[0] = rev2(r.hi);
+    w[1] = w[2] = 0;
+    if constexpr (RW == 2) {
+      w[0] |= codes << (2 * k);
+      w[1] = codes >> (64 - 2 * k);
+    } else {
+      const int u = 2 * k - 64;
+      w[1] = rev2(r.lo) | (codes << u);
+      w[2] = u ? codes >> (64 - u) : 0ull;
+    }
+    uint32_t x[NC];
+#pragma unroll
+    for (int q = 0; q < NC; ++q) x[q] = uint32_t(w[q >> 1] >> (32 * (q & 1)));
+    c[0] = x[0] << (2 * a);
+#pragma unroll
+    for (int q = 1; q < NC; ++q) c[q] = __funnelshift_l(x[q - 1], x[q], 2 * a);
+  }
+  const uint32_t last = a + uint32_t(k) + t;        // place of the break, from the first word's start
+  const uint32_t nw = last >> 2, rem = last & 3u;   // its word, and the chars before it there
+  uint32_t* d = buf + (pos >> 2);
+  uint32_t first = 0, tailw = 0;
+#pragma unroll
+  for (int g = 0; g < NC; ++g) {
+    if (4u * g > nw) break;
+    uint32_t w[4];
+    letters16(c[g], w);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const uint32_t j = 4u * g + q;
+      if (j == nw) tailw = w[q];
+      if (j < nw && (j > 0 || a == 0)) d[j] = w[q];
+    }
+    if (g == 0) first = w[0];
+  }
+  const uint32_t v = (tailw & ((1u << (8 * rem)) - 1u)) | (uint32_t('\n') << (8 * rem));
+  char* e = reinterpret_cast<char*>(d + nw);
+  if (nw == 0 && a) {  // a line inside one word (k < 3)
+    for (uint32_t q = a; q <= rem; ++q) e[q] = char(v >> (8 * q));
+    return;
+  }
+  if (rem == 3) {
+    d[nw] = v;
+  } else {
+    if (rem) *reinterpret_cast<uint16_t*>(e) = uint16_t(v);
+    if (rem != 1) e[rem] = '\n';
+  }
+  if (a) {
+    char* f = reinterpret_cast<char*>(d);
+    if (a & 1u) f[a] = char(first >> (8 * a));
+    if (a < 3) *reinterpret_cast<uint16_t*>(f + 2) = uint16_t(first >> 16);
+  }
+}
+
+// Stores the lines of ranks [r0, r1) of one warp, the first at byte `at` of
+// the sorted text: 32 lines at a time are spelled into the warp's buffer and
+// leave as 16-byte stores; the up to 15 bytes after the last one stay for the
+// next 32 lines.  get(r) gives the record of rank r.
+template <int RW, class Get>
+__device__ __forceinline__ void store_lines(char* out, uint64_t at, uint32_t r0, uint32_t r1, int k, uint32_t* buf,
+                                            LongLine* longs, const char* keep, Get get) {
+  const uint32_t lane = threadIdx.x & 31u;
+  char* bb = reinterpret_cast<char*>(buf);
+  char* dst = out + at;                       // next byte of the sorted text
+  uint32_t fill = uint32_t(reinterpret_cast<uintptr_t>(dst) & 15u);  // bytes of buf before it
+  uint32_t head = fill;                       // of which another warp's
+  auto flush_rest = [&] {
+    if (lane >= head && lane < fill) (dst - fill)[lane] = bb[lane];
+    __syncwarp();
+  };
+  for (uint32_t base = r0; base < r1; base += 32) {
+    const bool live = base + lane < r1;
+    Rec<RW> r{0ull, 0ull, 0ull};
+    if (live) r = get(base + lane);
+    const bool is_long = live && (r.tail & TAIL_LONG);
+    const unsigned long long len = live ? line_bytes_of(r.tail, k, longs) : 0ull;
+    if (__any_sync(0xFFFFFFFFu, is_long)) {
+      flush_rest();
+      unsigned long long inc = len;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const unsigned long long v = __shfl_up_sync(0xFFFFFFFFu, inc, o);
+        if (lane >= uint32_t(o)) inc += v;
+      }
+      const unsigned long long total = __shfl_sync(0xFFFFFFFFu, inc, 31);
+      if (live && !is_long) {
+        // into the lane's own part of the buffer, then byte by byte
+        char* p = dst + (inc - len);
+        uint32_t* mine = buf + lane * ((uint32_t(k) + TAIL_MAX + 4u) >> 2);
+        spell_line<RW>(mine, 0u, r, k);
+        for (uint32_t q = 0; q < uint32_t(len); ++q) p[q] = reinterpret_cast<char*>(mine)[q];
+      }
+      uint32_t todo = __ballot_sync(0xFFFFFFFFu, is_long);
+      while (todo) {
+        const int q = __ffs(todo) - 1;
+        todo &= todo - 1;
+        const uint32_t i = uint32_t(__shfl_sync(0xFFFFFFFFu, r.tail, q));
+        const unsigned long long n = __shfl_sync(0xFFFFFFFFu, len, q);
+        const unsigned long long o = __shfl_sync(0xFFFFFFFFu, inc - len, q);
+        char* p = dst + o;
+        const unsigned long long src = longs[i].at;
+        if (n < HUGE_LINE) copy_bytes(p, keep + src, n, lane, 32u);
+        else if (lane == 0) longs[i].to = uint64_t(p - out);  // copied by k_huge_lines
+      }
+      __syncwarp();
+      dst += total;
+      fill = head = uint32_t(reinterpret_cast<uintptr_t>(dst) & 15u);
+      continue;
+    }
+    uint32_t inc = uint32_t(len);
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t v = __shfl_up_sync(0xFFFFFFFFu, inc, o);
+      if (lane >= uint32_t(o)) inc += v;
+    }
+    const uint32_t total = __shfl_sync(0xFFFFFFFFu, inc, 31);
+    if (live) spell_line<RW>(buf, fill + inc - uint32_t(len), r, k);
+    __syncwarp();
+    const uint32_t full = (fill + total) >> 4, rem = (fill + total) & 15u;
+    char* w = dst - fill;
+    for (uint32_t p = lane; p < full; p += 32) {
+      if (p == 0 && head) {
+        for (uint32_t q = head; q < 16; ++q) w[q] = bb[q];
+      } else {
+        reinterpret_cast<uint4*>(w)[p] = reinterpret_cast<const uint4*>(buf)[p];
+      }
+    }
+    __syncwarp();
+    if (full) {
+      if (lane < 4) buf[lane] = buf[4 * full + lane];
+      head = 0;
+    }
+    __syncwarp();
+    dst += total;
+    fill = rem;
+  }
+  flush_rest();
+}
+
+// Stable order of n records of one tile too large for shared memory, by one
+// block: 8 bits of the key per pass, least significant first, between two
+// buffers.  Returns 1 where the result lies in y.  (A bin of more than a
+// tile's records: thousands of lines that share their first chars.)
+template <int RW>
+__device__ int order_in_memory(RecArr<RW> x, RecArr<RW> y, uint64_t beg, uint32_t n, int k, uint32_t* hist,
+                               uint32_t* wcnt) {
+  constexpr uint32_t W = TILE_THREADS / 32;
+  const uint32_t tid = threadIdx.x, lane = tid & 31u, wid = tid >> 5;
+  __shared__ uint32_t sc[33];
+  int in_y = 0;
+  for (int pass = 0; pass < (RW == 3 ? 16 : 8); ++pass) {
+    const bool low = RW == 3 && pass < 8;
+    const int sh = 8 * (pass & 7);
+    // bytes below the k-mer's last char hold nothing
+    if (low ? (sh + 8 <= 128 - 2 * k) : (sh + 8 <= 64 - 2 * k)) continue;
+    const RecArr<RW> a = in_y ? y : x, b = in_y ? x : y;
+    auto digit = [&](const Rec<RW>& r) { return uint32_t((low ? r.lo : r.hi) >> sh) & 255u; };
+    hist[tid] = 0;  // (TILE_THREADS = 256 digits)
+    __syncthreads();
+    for (uint32_t i = tid; i < n; i += TILE_THREADS) atomicAdd(hist + digit(ld_rec<RW>(a, beg + i)), 1u);
+    __syncthreads();
+    uint32_t tot;
+    const uint32_t pre = block_excl_scan(hist[tid], sc, &tot);
+    hist[tid] = pre;
+    for (uint32_t i0 = 0; i0 < n; i0 += TILE_THREADS) {
+      for (uint32_t q = tid; q < W * 256u; q += TILE_THREADS) wcnt[q] = 0;
+      __syncthreads();
+      const bool live = i0 + tid < n;
+      Rec<RW> r{0ull, 0ull, 0ull};
+      if (live) r = ld_rec<RW>(a, beg + i0 + tid);
+      const uint32_t d = live ? digit(r) : 256u;
+      const uint32_t same = __match_any_sync(0xFFFFFFFFu, d);
+      const uint32_t rank = __popc(same & ((1u << lane) - 1u));
+      if (live && rank == 0) wcnt[wid * 256u + d] = __popc(same);
+      __syncthreads();
+      uint32_t run = hist[tid];
+      for (uint32_t w = 0; w < W; ++w) {
+        const uint32_t c = wcnt[w * 256u + tid];
+        wcnt[w * 256u + tid] = run;
+        run += c;
+      }
+      hist[tid] = run;
+      __syncthreads();
+      if (live) st_rec<RW>(b, beg + wcnt[wid * 256u + d] + rank, r);
+      __syncthreads();
+    }
+    in_y ^= 1;
+  }
+  return in_y;
+}
+
+template <int RW>
+__host__ __device__ constexpr uint32_t tile_buf_words(int k) {
+  // a warp's buffer: 15 bytes kept, 32 lines, word stores
+  return (16u + 32u * ((uint32_t(k) + TAIL_MAX + 4u) & ~3u) + 16u) / 4u;
+}
+// Shared memory of a tile: the records; the sub-bins and the first index
+// list, whose place the warps' buffers take; the final index list.
+template <int RW>
+__host__ __device__ constexpr size_t tile_area_words(int k) {
+  const size_t a = TILE_SUB + 2 + tile_cap<RW>() / 2;
+  const size_t b = size_t(TILE_THREADS / 32) * tile_buf_words<RW>(k);
+  const size_t c = (TILE_THREADS / 32 + 1) * 256;  // order_in_memory
+  return ((a > b ? (a > c ? a : c) : (b > c ? b : c)) + 3) & ~size_t(3);
+}
+template <int RW>
+__host__ __device__ constexpr size_t tile_smem(int k) {
+  return size_t(tile_cap<RW>()) * (8 * RW + 2) + tile_area_words<RW>(k) * 4;
+}
+
+// One block per tile.  The records' keys are spread over TILE_SUB sub-bins of
+// the tile's key range (about one record each), counted and placed with
+// shared-memory atomics, and each record's final rank is its sub-bin's start
+// plus the smaller records in the sub-bin.  The tile's first byte comes from
+// the look-back over the tiles' byte counts.  Then each warp stores a run of
+// ranks (store_lines).  256 Mbp, k = 31: 3.0 ms for 5.3 GB, issue-bound (about
+// 650 instructions per line, spelling the most of them); 3.5 ms with three
+// blocks per SM instead of four.
+template <int RW>
+__global__ void __launch_bounds__(TILE_THREADS, RW == 2 ? 4 : 3) k_line_tiles(RecArr<RW> rec, RecArr<RW> spare,
+                                                             const uint2* __restrict__ tile, int bits, char* out, int k,
+                                                             LongLine* longs, const char* keep,
+                                                             unsigned long long* st, SortCtr* sc) {
+  extern __shared__ __align__(16) unsigned char sm[];
+  constexpr uint32_t TILE_CAP = tile_cap<RW>();
+  uint64_t* khi = reinterpret_cast<uint64_t*>(sm);
+  uint64_t* klo = khi + TILE_CAP;                      // RW == 3
+  uint64_t* tl = khi + size_t(TILE_CAP) * (RW - 1);
+  uint32_t* area = reinterpret_cast<uint32_t*>(khi + size_t(TILE_CAP) * RW);
+  uint32_t* sub = area;                                // [TILE_SUB + 1]
+  uint16_t* ord = reinterpret_cast<uint16_t*>(area + TILE_SUB + 2);
+  uint16_t* fin = reinterpret_cast<uint16_t*>(area + tile_area_words<RW>(k));
+  __shared__ uint32_t scan[33], s_t;
+  __shared__ unsigned long long s_sum[TILE_THREADS / 32], s_at, s_w[TILE_THREADS / 32];
+  const uint32_t tid = threadIdx.x, lane = tid & 31u, wid = tid >> 5;
+  constexpr uint32_t W = TILE_THREADS / 32, PER = TILE_CAP / TILE_THREADS;
+  if (sc->fail) return;  // (of the kernels before; uniform)
+  const uint32_t ntiles = sc->ntiles;
+  for (;;) {
+    if (tid == 0) s_t = atomicAdd(&sc->tile_ticket, 1u);
+    __syncthreads();
+    const uint32_t t = s_t;
+    if (t >= ntiles) break;
+    const uint2 T0 = tile[t], T1 = tile[t + 1];
+    const uint32_t beg = T0.x, n = T1.x - beg;
+    const bool fits = n <= TILE_CAP;
+    // the tile's key range, spread over the sub-bins
+    const uint64_t kmin = T0.y ? uint64_t(T0.y) << (64 - bits) : 0ull;
+    const int sh = max(0, 53 - bits + (T1.y - T0.y > 1u ? 32 - __clz(T1.y - T0.y - 1u) : 0));
+    unsigned long long bytes = 0;
+    uint32_t rk[PER];
+    for (uint32_t j = tid; j < TILE_SUB; j += TILE_THREADS) sub[j] = 0;
+    __syncthreads();
+    if (fits) {
+#pragma unroll
+      for (uint32_t q = 0; q < PER; ++q) {
+        if (q * TILE_THREADS >= n) break;
+        const uint32_t i = q * TILE_THREADS + tid;
+        if (i < n) {
+          const Rec<RW> r = ld_rec<RW>(rec, uint64_t(beg) + i);
+          khi[i] = r.hi;
+          if constexpr (RW == 3) klo[i] = r.lo;
+          tl[i] = r.tail;
+          bytes += line_bytes_of(r.tail, k, longs);
+          // the sub-bin and the record's place in it
+          const uint32_t b = min(uint32_t((r.hi - kmin) >> sh), TILE_SUB - 1u);
+          rk[q] = (atomicAdd(sub + b, 1u) << 11) | b;
+        }
+      }
+    } else {
+      for (uint32_t i = tid; i < n; i += TILE_THREADS)
+        bytes += line_bytes_of(ld_rec<RW>(rec, uint64_t(beg) + i).tail, k, longs);
+    }
+#pragma unroll
+    for (int o = 16; o; o >>= 1) bytes += __shfl_xor_sync(0xFFFFFFFFu, bytes, o);
+    if (lane == 0) s_sum[wid] = bytes;
+    __syncthreads();
+    bytes = 0;
+#pragma unroll
+    for (uint32_t w = 0; w < W; ++w) bytes += s_sum[w];
+    if (tid == 0) lb_publish(st, t, LB_SUM, bytes);
+    int in_spare = 0;
+    if (fits) {
+      {
+        constexpr uint32_t C = TILE_SUB / TILE_THREADS;
+        uint32_t c[C], sum = 0;
+#pragma unroll
+        for (uint32_t q = 0; q < C; ++q) {
+          c[q] = sub[tid * C + q];
+          sum += c[q];
+        }
+        uint32_t tot;
+        uint32_t pre = block_excl_scan(sum, scan, &tot);
+#pragma unroll
+        for (uint32_t q = 0; q < C; ++q) {
+          sub[tid * C + q] = pre;
+          pre += c[q];
+        }
+        if (tid == 0) sub[TILE_SUB] = n;
+      }
+      __syncthreads();
+#pragma unroll
+      for (uint32_t q = 0; q < PER; ++q) {
+        if (q * TILE_THREADS >= n) break;
+        const uint32_t i = q * TILE_THREADS + tid;
+        if (i < n) ord[sub[rk[q] & (TILE_SUB - 1u)] + (rk[q] >> 11)] = uint16_t(i);
+      }
+      __syncthreads();
+      for (uint32_t j = tid; j < n; j += TILE_THREADS) {
+        const uint32_t i = ord[j];
+        const uint64_t h = khi[i];
+        const uint32_t b = min(uint32_t((h - kmin) >> sh), TILE_SUB - 1u);
+        const uint32_t lo = sub[b], hi = sub[b + 1];
+        uint32_t rank = lo;
+        for (uint32_t m = lo; m < hi; ++m) {
+          const uint32_t o = ord[m];
+          const uint64_t x = khi[o];
+          bool less = x < h;
+          if (x == h) {
+            if constexpr (RW == 3) less = klo[o] < klo[i] || (klo[o] == klo[i] && o < i);
+            else less = o < i;
+          }
+          rank += less ? 1u : 0u;
+        }
+        fin[rank] = uint16_t(i);
+      }
+    } else {
+      in_spare = order_in_memory<RW>(rec, spare, beg, n, k, area, area + 256);
+    }
+    __syncthreads();
+    const RecArr<RW> sorted = in_spare ? spare : rec;
+    auto get = [&](uint32_t r) {
+      if (!fits) return ld_rec<RW>(sorted, uint64_t(beg) + r);
+      const uint32_t i = fin[r];
+      Rec<RW> x;
+      x.hi = khi[i];
+      if constexpr (RW == 3) x.lo = klo[i];
+      else x.lo = 0;
+      x.tail = tl[i];
+      return x;
+    };
+    // each warp's run of ranks and its bytes, and the tile's first byte
+    const uint32_t per = ((n + W - 1) / W + 31u) & ~31u;
+    const uint32_t r0 = min(n, wid * per), r1 = min(n, r0 + per);
+    unsigned long long wb = 0;
+    for (uint32_t r = r0 + lane; r < r1; r += 32)
+      wb += line_bytes_of(fits ? tl[fin[r]] : get(r).tail, k, longs);
+#pragma unroll
+    for (int o = 16; o; o >>= 1) wb += __shfl_xor_sync(0xFFFFFFFFu, wb, o);
+    if (lane == 0) s_w[wid] = wb;
+    if (wid == 0) {
+      const unsigned long long e = lb_exclusive(st, t, bytes, &sc->fail);
+      if (lane == 0) s_at = e;
+    }
+    __syncthreads();
+    unsigned long long at = s_at;
+    for (uint32_t w = 0; w < wid; ++w) at += s_w[w];
+    // (a failed wait leaves the text as it is)
+    if (r0 < r1 && !*reinterpret_cast<volatile uint32_t*>(&sc->fail))
+      store_lines<RW>(out, at, r0, r1, k, area + wid * tile_buf_words<RW>(k), longs, keep, get);
+    __syncthreads();  // the tile's shared memory is reused
+  }
+}
+
+// Lines of HUGE_LINE bytes or more, each by the whole grid: from the kept
+// copy to the place k_line_tiles noted.
+__global__ void __launch_bounds__(256) k_huge_lines(char* out, const char* keep, const LongLine* longs,
+                                                    const uint32_t* huge, const SortCtr* sc) {
+  const uint32_t nhuge = sc->nhuge;
+  for (uint32_t h = 0; h < nhuge; ++h) {
+    const LongLine L = longs[huge[h]];
+    for (unsigned long long x = blockIdx.x * HUGE_LINE; x < L.len; x += gridDim.x * HUGE_LINE)
+      copy_bytes(out + L.to + x, keep + L.at + x, min(HUGE_LINE, L.len - x), threadIdx.x, blockDim.x);
+  }
+}
+
+// The launch sequence for one key width.
+template <int RW>
+int sort_lines_rw(Env& e, char* out, uint64_t bytes, int k) {
+  const uint64_t lmax = bytes / uint64_t(k + 1) + 1;
+  if (lmax >= 0xFFFFFFF0ull) return e.fail(UC_EINTERNAL, "line count of the output out of range");
+  // about 32 records per bin: a tile then is a window and a fraction of one,
+  // and a bin can be 32 times as dense before its tile outgrows shared memory
+  int bits = 4;
+  while (bits < std::min(MAX_BIN_BITS, 2 * k) && (lmax >> bits) > 32) ++bits;
+  const uint32_t m = 1u << bits;
+  // windows of 1000 records; shorter ones while there are fewer than two
+  // tiles per SM.  (Not a power of two: the tiles fill at one pace, and with
+  // windows of 1024 their write frontiers lay 16 KB apart, in few of L2's
+  // slices and sets.)
+  uint32_t win = 1000;
+  while (win > 250 && lmax / win < 2ull * e.sm_count) win /= 2;
+  const uint64_t ntmax = lmax / win + 2;
+  const uint64_t nplan = (uint64_t(m) + 256 * PLAN_ITEMS - 1) / (256 * PLAN_ITEMS);
+  const uint64_t nlongs = bytes / uint64_t(k + TAIL_MAX + 2) + 1, nhuges = bytes / HUGE_LINE + 1;
+  // more tiles than k_line_group counts at once: groups of 2^gsh first
+  uint32_t gsh = 0;
+  if (ntmax > GRP_BINS)
+    for (gsh = 5; (ntmax >> gsh) > GRP_BINS / 2; ) ++gsh;
+  // cleared: the counters, the look-back words, the bin counts
+  const size_t zero = 256 + (nplan + ntmax) * 8 + m * 4ull + 256;
+  size_t need = 0;
+  auto add = [&](size_t b) { need += (b + 255) & ~size_t(255); };
+  add(zero);
+  for (int q = 0; q < 2; ++q) {
+    add(lmax * 16);
+    if (RW == 3) add(lmax * 8);
+  }
+  add((ntmax + 1) * 8);
+  add((ntmax + GRP_BINS) * CUR_STRIDE * 4);
+  add(((ntmax >> gsh) + 1 + GRP_BINS) * CUR_STRIDE * 4);
+  add(nlongs * sizeof(LongLine));
+  add(nhuges * 4);
+  add(bytes + 16);
+  int r = e.reserve(1, need);
+  if (r) return r;
+  char* z = static_cast<char*>(e.take(1, zero));
+  RecArr<RW> ra{}, rb{};
+  for (RecArr<RW>* q : {&ra, &rb}) {
+    q->a = static_cast<ulonglong2*>(e.take(1, lmax * 16));
+    if (RW == 3) q->t = static_cast<unsigned long long*>(e.take(1, lmax * 8));
+  }
+  uint2* tile = static_cast<uint2*>(e.take(1, (ntmax + 1) * 8));
+  uint32_t* cur = static_cast<uint32_t*>(e.take(1, (ntmax + GRP_BINS) * CUR_STRIDE * 4));
+  uint32_t* gcur = static_cast<uint32_t*>(e.take(1, ((ntmax >> gsh) + 1 + GRP_BINS) * CUR_STRIDE * 4));
+  LongLine* longs = static_cast<LongLine*>(e.take(1, nlongs * sizeof(LongLine)));
+  uint32_t* huge = static_cast<uint32_t*>(e.take(1, nhuges * 4));
+  char* keep = static_cast<char*>(e.take(1, bytes + 16));
+  if (!keep) return e.fail(UC_EBUDGET, "arena overflow (sorted output)");
+  SortCtr* sc = reinterpret_cast<SortCtr*>(z);
+  unsigned long long* st_plan = reinterpret_cast<unsigned long long*>(z + 256);
+  unsigned long long* st_tile = st_plan + nplan;
+  uint32_t* counts = reinterpret_cast<uint32_t*>((reinterpret_cast<uintptr_t>(st_tile + ntmax) + 255) & ~uintptr_t(255));
+  UC_CK(cudaMemsetAsync(z, 0, zero, e.stream));
+  auto grid = [&](uint64_t want, int occ) {
+    return unsigned(std::max<uint64_t>(1, std::min<uint64_t>(want, uint64_t(e.sm_count) * uint64_t(std::max(1, occ)))));
+  };
+  const uint64_t nchunks = (bytes + 15 + LR_CHUNK - 1) / LR_CHUNK;
+  const size_t sm_recs = (LR_CHUNK / (uint32_t(k) + 1u) + 2u) * 2u;
+  const size_t sm_tile = tile_smem<RW>(k);
+  int occ = 0;
+  UC_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_line_recs<RW>, 256, sm_recs));
+  e.launches += 4;
+  k_line_recs<RW><<<grid(nchunks, occ), 256, sm_recs, e.stream>>>(out, bytes, k, bits, ra, counts, longs, huge, sc);
+  k_line_plan<<<unsigned(nplan), 256, 0, e.stream>>>(counts, m, win, tile, cur, gcur, gsh, st_plan, sc);
+  if (nlongs > 1) {
+    ++e.launches;
+    k_line_keep<<<grid((nlongs + 7) / 8, 4), 256, 0, e.stream>>>(out, keep, longs, huge, sc);
+  }
+  r = allow_max_smem(e, k_line_group<RW>);
+  if (r) return r;
+  RecArr<RW> from = ra, to = rb;
+  for (uint32_t level = gsh ? 0u : 1u; level < 2; ++level) {
+    ++e.launches;
+    k_line_group<RW><<<grid((lmax + grp_chunk<RW>() - 1) / grp_chunk<RW>(), 2), GRP_THREADS, grp_smem<RW>(),
+                       e.stream>>>(from, to, counts, bits, level ? 0u : gsh, level ? cur : gcur, sc);
+    std::swap(from, to);
+  }
+  r = allow_max_smem(e, k_line_tiles<RW>);
+  if (r) return r;
+  UC_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_line_tiles<RW>, int(TILE_THREADS), sm_tile));
+  if (occ < 1) return e.fail(UC_EINTERNAL, "line tile kernel does not fit an SM");
+  k_line_tiles<RW><<<grid(ntmax, occ), TILE_THREADS, sm_tile, e.stream>>>(from, to, tile, bits, out, k, longs, keep,
+                                                                         st_tile, sc);
+  UC_CK(cudaGetLastError());
+  SortCtr h;
+  UC_CK(cudaMemcpyAsync(&h, sc, sizeof h, cudaMemcpyDeviceToHost, e.stream));
+  UC_CK(cudaStreamSynchronize(e.stream));
+  if (h.fail & 1u) return e.fail(UC_ETIMEOUT, "a bounded device wait ran out (sorted output)");
+  if (h.fail) return e.fail(UC_EINTERNAL, "a line of the output is shorter than k");
+  if (h.nhuge) {
+    ++e.launches;
+    k_huge_lines<<<unsigned(e.sm_count) * 4u, 256, 0, e.stream>>>(out, keep, longs, huge, sc);
+    UC_CK(cudaGetLastError());
+    UC_CK(cudaStreamSynchronize(e.stream));
+  }
+  e.reset();
+  return UC_OK;
+}
+
+}  // namespace
+
+int sort_lines(Env& e, char* out, uint64_t bytes, int k) {
+  if (bytes == 0) return UC_OK;
+  e.reset();
+  return k <= 31 ? sort_lines_rw<2>(e, out, bytes, k) : sort_lines_rw<3>(e, out, bytes, k);
+}
+
+}  // namespace uc
