@@ -176,19 +176,17 @@ __device__ __forceinline__ uint32_t ascii4(uint32_t c) {
   return __byte_perm(0x54474341u, 0u, x);
 }
 
-// 4 ACGT bytes (first char lowest) -> their codes in byte 3, first char
-// lowest: ((b >> 1) ^ (b >> 2)) & 3 of each byte, gathered by one multiply
-// (the partial products below bit 24 do not meet, so nothing carries).
-__device__ __forceinline__ uint32_t code_byte3(uint32_t x) {
-  return (((x >> 1) ^ (x >> 2)) & 0x03030303u) * 0x01041040u;
+// Bits 1 and 2 of 16 letters, first letter lowest: A 0, C 1, T 2, G 3 (a line
+// break reads as 1).  Each 4 letters' pairs are gathered into a byte by one
+// multiply (the partial products below bit 24 do not meet, so nothing carries).
+__device__ __forceinline__ uint32_t letter_bits16(const uint4& v) {
+  auto g = [](uint32_t x) { return (x & 0x06060606u) * 0x00820820u; };  // in byte 3
+  return __byte_perm(__byte_perm(g(v.x), g(v.y), 0x0073), __byte_perm(g(v.z), g(v.w), 0x0073), 0x5410);
 }
-
-// 16 bytes of letters and line breaks -> 16 codes, first byte lowest (a line
-// break reads as 3).
-__device__ __forceinline__ uint32_t codes16(const uint4& v) {
-  return __byte_perm(__byte_perm(code_byte3(v.x), code_byte3(v.y), 0x0073),
-                     __byte_perm(code_byte3(v.z), code_byte3(v.w), 0x0073), 0x5410);
-}
+// Those bits -> codes (A 0, C 1, G 2, T 3).
+__device__ __forceinline__ uint32_t codes_of_bits(uint32_t r) { return r ^ ((r >> 1) & 0x55555555u); }
+// 16 bytes of letters and line breaks -> 16 codes, first byte lowest.
+__device__ __forceinline__ uint32_t codes16(const uint4& v) { return codes_of_bits(letter_bits16(v)); }
 // Of 16 bytes of ACGT and line breaks, a bit per line break (bit 6 is clear
 // in '\n' and set in the letters), the first byte's lowest.  Two words share
 // one byte of a product; the partial products do not meet.
@@ -197,17 +195,18 @@ __device__ __forceinline__ uint32_t breaks16(const uint4& v) {
   const uint32_t c = (~v.z >> 6) & 0x01010101u, d = (~v.w >> 6) & 0x01010101u;
   return __byte_perm(a * 0x01020408u + b * 0x10204080u, c * 0x01020408u + d * 0x10204080u, 0x4473) & 0xFFFFu;
 }
-// 16 codes (first lowest) -> their letters: the letters of the even and of
-// the odd chars, then their bytes interleaved.
-__device__ __forceinline__ void letters16(uint32_t c, uint32_t w[4]) {
+// 16 two-bit values (first lowest) -> their letters by a table of four: the
+// letters of the even and of the odd chars, then their bytes interleaved.
+__device__ __forceinline__ void spread16(uint32_t table, uint32_t c, uint32_t w[4]) {
   const uint32_t e = c & 0x33333333u, o = (c >> 2) & 0x33333333u;
-  const uint32_t e0 = __byte_perm(0x54474341u, 0u, e), e1 = __byte_perm(0x54474341u, 0u, e >> 16);
-  const uint32_t o0 = __byte_perm(0x54474341u, 0u, o), o1 = __byte_perm(0x54474341u, 0u, o >> 16);
+  const uint32_t e0 = __byte_perm(table, 0u, e), e1 = __byte_perm(table, 0u, e >> 16);
+  const uint32_t o0 = __byte_perm(table, 0u, o), o1 = __byte_perm(table, 0u, o >> 16);
   w[0] = __byte_perm(e0, o0, 0x5140);
   w[1] = __byte_perm(e0, o0, 0x7362);
   w[2] = __byte_perm(e1, o1, 0x5140);
   w[3] = __byte_perm(e1, o1, 0x7362);
 }
+__device__ __forceinline__ void letters16(uint32_t codes, uint32_t w[4]) { spread16(0x54474341u, codes, w); }
 
 // codes of chars ch..ch+3 of a packed key in the low 8 bits (chars past the
 // key read as 0)

@@ -51,7 +51,7 @@ constexpr unsigned long long SEG_OFF_MASK = (1ull << SEG_OFF_BITS) - 1ull;
 // indices).
 struct JobTab {
   const uint8_t* text;
-  unsigned long long tbytes, body, end, n, koff, lb0;  // lb0: first 256-line block
+  unsigned long long tbytes, body, end, n, koff, lb0;  // lb0: first block of lines (k_pack)
   unsigned long long obase, ocap;
   uint32_t seg_base, seg_cap;
   uint32_t fixed;  // every line is k chars + '\n'

@@ -106,38 +106,67 @@ __device__ __forceinline__ uint32_t base_code(uint32_t c) {
   return (c == 'C') ? 1u : (c == 'G') ? 2u : (c == 'T') ? 3u : 0u;
 }
 
-// SWAR conversion of 4 text bytes (little-endian in x) to 2-bit codes.
-// A=0x41 C=0x43 G=0x47 T=0x54 give ((b>>1)^(b>>2))&3 = 0,1,2,3; a byte is
-// kept only if rebuilding its letter from that code gives the byte back, so
-// every other byte packs as A (the zeroed char_map of compact_kmers,
-// driver.cpp:228-232).  Returns the codes of the 4 bytes in bytes 0..3 of the
-// result (values 0..3); *nl gets 0x80 in each byte equal to '\n'.
-__device__ __forceinline__ uint32_t swar_codes(uint32_t x, uint32_t* nl) {
-  const uint32_t t = ((x >> 1) ^ (x >> 2)) & 0x03030303u;
-  const uint32_t f = (t << 1) + (((t >> 1) & 0x01010101u) << 1) + (t & (t >> 1) & 0x01010101u) * 11u;
-  const uint32_t eq = ~((0x41414141u + f) ^ x);
-  const uint32_t ok = ((eq & 0x7F7F7F7Fu) + 0x01010101u) & eq & 0x80808080u;  // 0x80 where byte matches
-  const uint32_t z = x ^ 0x0A0A0A0Au;
-  *nl = ~(((z & 0x7F7F7F7Fu) + 0x7F7F7F7Fu) | z) & 0x80808080u;
-  return t & ((ok >> 7) * 3u);
+// A block packs 512 consecutive lines per pass.  Their text comes in by
+// asynchronous copies while the pass before is packed; each 16 bytes become
+// one word of 2-bit codes in shared memory, and a thread's line is then a few
+// funnel shifts of code words.
+//
+// Lines of k chars and a break (k >= 15): a 16-byte piece holds at most one
+// line break, at a place that follows from its offset, so it is checked by
+// spelling its codes again and comparing, with the break expected at its
+// place.  A pass where every piece agrees needs no other check.
+//
+// Any other pass (another layout, the count line's and the last piece, a
+// byte that is not ACGT) keeps, per piece, a bit per line break and a bit per
+// byte that is neither ACGT nor a break, and checks each line's bits; a byte
+// that is not ACGT packs as A (the zeroed char_map of compact_kmers,
+// driver.cpp:228-232), so its code is cleared.
+//
+// With FUSE the prefix/suffix minimizer buckets of every key are computed and
+// counted in the same pass (lmin_buckets.h:299-318).
+//
+// Bound by instruction issue (79% at 30 Mbp, k = 31).  256 Mbp, k = 31:
+// 3.6 ms (8.2 GB of text); 6.3 ms when each thread converted its own line
+// from staged text, 3.8 ms with bits per byte for every piece.
+constexpr int PACK_LINES = 512;
+constexpr int PACK_SPAN = 36864;  // text bytes staged per pass at most (wider lines: byte by byte)
+
+// 16-byte pieces a pass stages: those of its lines at fixed width, or
+// PACK_SPAN where the lines' starts are given.  Even, as two share a mask word.
+static uint32_t pack_pieces(bool fixed, int k) {
+  const uint32_t bytes = fixed ? uint32_t(PACK_LINES) * uint32_t(k + 1) + 16u : uint32_t(PACK_SPAN);
+  return ((std::min<uint32_t>(bytes, PACK_SPAN) + 31u) / 32u) * 2u;
 }
-// 4 byte-wise codes -> one byte c0 | c1<<2 | c2<<4 | c3<<6
-__device__ __forceinline__ uint32_t gather_codes(uint32_t t) { return ((t * 0x41041u) >> 18) & 0xFFu; }
+// raw text, codes, two masks (a line's last words reach past the pieces)
+static size_t pack_smem(uint32_t pieces) { return size_t(pieces) * 16 + (size_t(pieces) + 8) * 8; }
 
-// A block packs 256 consecutive lines per pass.  It first stages the text
-// span of those lines in shared memory with 16-byte loads from every thread
-// (the whole span in flight at once), inserting a 4-byte gap after every 32
-// bytes so that lines 32 bytes apart fall in different banks.  Then each
-// thread packs one line, 4 chars per 32-bit SWAR step.  With FUSE the
-// prefix/suffix minimizer buckets of every key are computed and counted in the
-// same pass (lmin_buckets.h:299-318).
-constexpr int PACK_LINES = 256;
-constexpr int PACK_SPAN = 18432;                    // staged text bytes per pass
-// + 32 words: a (short) line starting at the end of the span reads up to
-// k + 4 bytes past its start
-constexpr int PACK_WORDS = PACK_SPAN / 4 + PACK_SPAN / 32 + 32;
-
-__device__ __forceinline__ uint32_t pad_word(uint32_t byte_off) { return (byte_off >> 2) + (byte_off >> 5); }
+// The piece v of 16 text bytes: codes (of bytes that are ACGT), possible line
+// breaks (nl: a break where the code is 1, which is checked per line) and
+// other bytes (bad), a bit per byte.  Bits 1 and 2 of a letter are free, the
+// others follow from them (T has bit 2 without bit 1, bit 4 and no bit 0); a
+// byte with bit 3 set has to agree with 0x0A in the others.
+__device__ __forceinline__ uint32_t text_piece(const uint4& v, uint32_t& nl, uint32_t& bad) {
+  const uint32_t x[4] = {v.x, v.y, v.z, v.w};
+  uint32_t f[4], d[4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    f[q] = (x[q] >> 3) & 0x01010101u;
+    const uint32_t t = (x[q] >> 2) & ~(x[q] >> 1) & 0x01010101u;
+    const uint32_t want = 0x41414141u + t * 0x0Fu - f[q] * 0x39u;  // (no byte borrows: 0x41 or 0x50, less 0x39)
+    d[q] = (x[q] & 0xF9F9F9F9u) ^ want;
+  }
+  nl = __byte_perm(f[0] * 0x01020408u + f[1] * 0x10204080u, f[2] * 0x01020408u + f[3] * 0x10204080u, 0x4473) & 0xFFFFu;
+  bad = 0;
+  if (d[0] | d[1] | d[2] | d[3]) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const uint32_t z = (((d[q] & 0x7F7F7F7Fu) + 0x7F7F7F7Fu) | d[q]) & 0x80808080u;  // bytes that differ
+      bad |= (((z >> 7) * 0x01020408u) >> 24) << (4 * q);
+    }
+    nl &= ~bad;
+  }
+  return codes16(v);
+}
 
 __device__ __forceinline__ uint32_t job_of_block(const JobTab* __restrict__ jobs, uint32_t njobs, uint64_t g) {
   uint32_t lo = 0, hi = njobs;  // last job with lb0 <= g
@@ -180,173 +209,281 @@ __global__ void k_count_buckets(const uint32_t* __restrict__ b1, const uint32_t*
   }
 }
 
+// What regular_piece expects of a piece whose line break is byte p (none for
+// p >= 16).
+struct Break16 {
+  uint32_t e[4];  // per word, the break's difference from the letter its bits read as
+  uint32_t lo, at;  // the break's two bits as read, and their place
+};
+__device__ __forceinline__ Break16 break_at(uint32_t p) {
+  Break16 x;
+  const uint32_t d = uint32_t('C' ^ '\n') << (8 * (p & 3u));
+#pragma unroll
+  for (uint32_t q = 0; q < 4; ++q) x.e[q] = (p >> 2) == q ? d : 0u;
+  x.lo = p < 16u ? 1u << (2 * (p & 15u)) : 0u;
+  x.at = 3u * x.lo;
+  return x;
+}
+// The codes of the 16 text bytes v where they are letters, but for a line
+// break where x says; bad becomes nonzero where they are not.  (The letters
+// that bits 1 and 2 of each byte read as are compared with the bytes; the
+// break reads as C, and no other byte that does differs from C as it does.)
+__device__ __forceinline__ uint32_t regular_piece(const uint4& v, const Break16& x, uint32_t& bad) {
+  const uint32_t r = letter_bits16(v);
+  uint32_t w[4];
+  spread16(0x47544341u, r, w);  // A C T G
+  bad |= (w[0] ^ v.x ^ x.e[0]) | (w[1] ^ v.y ^ x.e[1]);
+  bad |= (w[2] ^ v.z ^ x.e[2]) | (w[3] ^ v.w ^ x.e[3]);
+  bad |= (r ^ x.lo) & x.at;
+  return codes_of_bits(r);
+}
+
+// Prefix and suffix minimizer buckets of a packed key in the fused path.  An
+// l-mer's id is its 2l bits of the key as they lie (first char lowest), so
+// each costs a funnel shift by a constant, a multiply-add and a min, with no
+// reversal of the key: chars right of the l-mer are in the id's upper bits and
+// drop out of the product (lmins, with (id * m + a) << (32 - 2l) as there).
+// The priority order is free (find_edges and uc_minimizers use lmins' order).
+template <int NW, int KC>
+__device__ __forceinline__ void key_buckets(const Key<NW>& key, int k, int l, uint64_t seed, uint32_t bits, uint32_t& b1,
+                                            uint32_t& b2) {
+  const uint32_t ps = 32u - 2u * uint32_t(l);
+  const uint32_t m = lmer_mult(seed) << ps, a = static_cast<uint32_t>(seed >> 32) << ps;
+  uint32_t x[2 * NW + 1];
+#pragma unroll
+  for (int q = 0; q < 2 * NW; ++q) x[q] = uint32_t(key.w[q >> 1] >> (32 * (q & 1)));
+  x[2 * NW] = 0;
+  const int last = k - l;  // l-mers 0 .. last
+  uint32_t mid = 0xFFFFFFFFu;
+  auto pri = [&](int p) { return __funnelshift_r(x[p >> 4], x[(p >> 4) + 1], 2 * (p & 15)) * m + a; };
+#pragma unroll
+  for (int p = 1; p < 32 * NW - 2; p += 2) {  // 1 .. last - 1 (l <= 16: KC - 17 of them at least)
+    if ((KC == 0 || p >= KC - 16) && p >= last) break;
+    const uint32_t u = pri(p), v = pri(p + 1);
+    mid = __vimin3_u32(mid, u, ((KC == 0 || p + 1 >= KC - 16) && p + 1 >= last) ? u : v);
+  }
+  const int s = 2 * last;
+  uint32_t e;
+  if constexpr (NW == 1) e = uint32_t(key.w[0] >> s);
+  else e = s >= 64 ? uint32_t(key.w[NW - 1] >> (s - 64)) : uint32_t((key.w[0] >> s) | (s ? key.w[NW - 1] << (64 - s) : 0ull));
+  b1 = bucket_of(min(mid, x[0] * m + a) >> ps, bits);
+  b2 = bucket_of(min(mid, e * m + a) >> ps, bits);
+}
+
 // MULTI: the block's job comes from the job table (batches); otherwise the
 // one job is a kernel parameter, read from the constant bank.
-// KC, LC: k and l fixed at compile time (0: taken from the arguments), so
-// that the per-word and per-l-mer loops of the common shapes unroll with
-// constant shifts.
-template <int NW, bool FUSE, bool MULTI, int KC = 0, int LC = 0>
-__global__ void __launch_bounds__(256) k_pack(const JobTab* __restrict__ jobs, const JobTab one, uint32_t njobs,
+// KC: k fixed at compile time (0: taken from the argument).
+template <int NW, bool FUSE, bool MULTI, int KC = 0>
+__global__ void __launch_bounds__(256, NW == 1 && KC ? 6 : 5) k_pack(const JobTab* __restrict__ jobs, const JobTab one, uint32_t njobs,
                                               uint64_t nblocks,
                                               const unsigned long long* __restrict__ starts, int k_arg,
-                                              uint64_t* __restrict__ keys, uint32_t* err, int l_arg, uint64_t seed,
+                                              uint64_t* __restrict__ keys, uint32_t* err, int l, uint64_t seed,
                                               uint32_t jb, uint32_t* __restrict__ b1, uint32_t* __restrict__ b2,
                                               uint32_t* __restrict__ counts, uint32_t cshift,
-                                              uint32_t* __restrict__ jcross) {
-  __shared__ uint32_t buf[PACK_WORDS];
+                                              uint32_t* __restrict__ jcross, uint32_t pcap) {
+  extern __shared__ __align__(16) unsigned char sm_pack[];
+  uint4* raw = reinterpret_cast<uint4*>(sm_pack);                        // [pcap] text of the next pass
+  uint32_t* code = reinterpret_cast<uint32_t*>(raw + pcap);              // [pcap + 8]
+  uint32_t* nlw = code + pcap + 8;                                       // [(pcap + 8) / 2]
+  uint32_t* badw = nlw + (pcap + 8) / 2;                                 // [(pcap + 8) / 2]
+  uint16_t* nl16 = reinterpret_cast<uint16_t*>(nlw);
+  uint16_t* bad16 = reinterpret_cast<uint16_t*>(badw);
   __shared__ uint32_t s_cross;
   const int k = KC ? KC : k_arg;
-  const int l = LC ? LC : l_arg;
-  uint32_t bad = 0;
+  uint32_t bad = 0, mycross = 0;
   const uint32_t stride = uint32_t(k) + 1;
-  uint64_t kmask_hi;
-  if constexpr (NW == 1) kmask_hi = (k >= 32) ? ~0ull : ((1ull << (2 * k)) - 1ull);
-  else kmask_hi = (2 * k - 64 >= 64) ? ~0ull : ((1ull << ((2 * k - 64) & 63)) - 1ull);
-  for (uint64_t g = blockIdx.x; g < nblocks; g += gridDim.x) {
-    const uint32_t j = MULTI ? job_of_block(jobs, njobs, g) : 0u;
-    const uint8_t* text = MULTI ? jobs[j].text : one.text;
-    const uint64_t tbytes = MULTI ? jobs[j].tbytes : one.tbytes;
-    const uint64_t body = MULTI ? jobs[j].body : one.body;
-    const uint64_t end = MULTI ? jobs[j].end : one.end;
-    const uint64_t n = MULTI ? jobs[j].n : one.n;
-    const uint64_t koff = MULTI ? jobs[j].koff : one.koff;
-    const uint64_t b0 = (g - (MULTI ? jobs[j].lb0 : one.lb0)) * PACK_LINES;
-    const uintptr_t tb = reinterpret_cast<uintptr_t>(text);
-    const uint32_t cnt = uint32_t((n - b0) < PACK_LINES ? (n - b0) : PACK_LINES);
-    const uint64_t s0 = starts ? uint64_t(starts[b0]) : body + b0 * stride;
-    const uint64_t s1 = (b0 + cnt < n) ? (starts ? uint64_t(starts[b0 + cnt]) : body + (b0 + cnt) * stride) : end;
-    const uintptr_t A0 = (tb + s0) & ~uintptr_t(15);
-    const uint64_t span = (tb + s1) - A0;
-    const bool staged = span + 16 <= PACK_SPAN;
-    if (threadIdx.x == 0) s_cross = 0;
-    if (staged) {
-      const uint32_t nch = uint32_t((span + 15) / 16);
-      for (uint32_t c = threadIdx.x; c < nch; c += blockDim.x) {
-        const uintptr_t a = A0 + 16u * c;
-        uint4 v;
-        if (a >= tb && a + 16 <= tb + tbytes) {
-          v = __ldcs(reinterpret_cast<const uint4*>(a));  // read once: evict first
-        } else {
-          uint32_t w[4] = {0x0A0A0A0Au, 0x0A0A0A0Au, 0x0A0A0A0Au, 0x0A0A0A0Au};
-          for (int q = 0; q < 16; ++q) {
-            const uintptr_t x = a + q;
-            if (x >= tb && x < tb + tbytes) {
-              const uint32_t byte = *reinterpret_cast<const uint8_t*>(x);
-              w[q >> 2] = (w[q >> 2] & ~(0xFFu << (8 * (q & 3)))) | (byte << (8 * (q & 3)));
-            }
-          }
-          v = make_uint4(w[0], w[1], w[2], w[3]);
+  const uint64_t kmask_hi = (1ull << (2 * k - 64 * (NW - 1))) - 1ull;  // (at most 62 bits)
+  // a bit per char of a line, and the place of the break after it (k <= 31 or 63)
+  using Mask = typename std::conditional<NW == 1, uint32_t, uint64_t>::type;
+  const Mask term = Mask(1) << k, chars = term - 1;
+  // one pass: its lines and their text
+  struct Pass {
+    const uint8_t* text;
+    uint64_t end, b0, s0, span, koff;
+    uint32_t j, cnt, first, nterm;
+  };
+  // The pass's text on its way into raw (each thread its own pieces, which it
+  // converts itself: no barrier between the copy and the conversion).
+  auto fetch = [&](uint64_t g) {
+    Pass P;
+    P.j = MULTI ? job_of_block(jobs, njobs, g) : 0u;
+    P.text = MULTI ? jobs[P.j].text : one.text;
+    const uint64_t tbytes = MULTI ? jobs[P.j].tbytes : one.tbytes;
+    const uint64_t body = MULTI ? jobs[P.j].body : one.body;
+    P.end = MULTI ? jobs[P.j].end : one.end;
+    const uint64_t n = MULTI ? jobs[P.j].n : one.n;
+    P.koff = MULTI ? jobs[P.j].koff : one.koff;
+    P.b0 = (g - (MULTI ? jobs[P.j].lb0 : one.lb0)) * PACK_LINES;
+    const uintptr_t tb = reinterpret_cast<uintptr_t>(P.text);
+    P.cnt = uint32_t((n - P.b0) < PACK_LINES ? (n - P.b0) : PACK_LINES);
+    P.s0 = starts ? uint64_t(starts[P.b0]) : body + P.b0 * stride;
+    const bool more = P.b0 + P.cnt < n;
+    const uint64_t s1 = more ? (starts ? uint64_t(starts[P.b0 + P.cnt]) : body + (P.b0 + P.cnt) * stride) : P.end;
+    P.first = uint32_t((tb + P.s0) & 15u);  // first line's start in the staged span
+    P.span = s1 - P.s0 + P.first;
+    P.nterm = starts ? 0u : (more ? P.cnt : P.cnt - 1u);  // lines whose break is checked
+    if (P.span <= uint64_t(pcap) * 16) {
+      const uintptr_t A0 = tb + P.s0 - P.first;
+      const uint32_t nch = uint32_t(P.span + 15) / 16;
+      const bool inside = A0 >= tb && A0 + 16u * nch <= tb + tbytes;
+      uint32_t c = threadIdx.x;
+      if (inside) {
+        const uint4* src = reinterpret_cast<const uint4*>(A0);
+        for (; c + 768 < nch; c += 1024) {
+#pragma unroll
+          for (int q = 0; q < 4; ++q) __pipeline_memcpy_async(raw + c + 256 * q, src + c + 256 * q, 16);
         }
-        const uint32_t wi = pad_word(16u * c);  // 4 words, never split by a gap
-        buf[wi] = v.x;
-        buf[wi + 1] = v.y;
-        buf[wi + 2] = v.z;
-        buf[wi + 3] = v.w;
+      }
+      for (; c < nch; c += 256) {
+        const uintptr_t a = A0 + 16u * c;
+        if (inside || (a >= tb && a + 16 <= tb + tbytes)) {
+          __pipeline_memcpy_async(raw + c, reinterpret_cast<const void*>(a), 16);
+        } else {
+          for (int b = 0; b < 16; ++b) {
+            const uintptr_t x = a + b;
+            reinterpret_cast<uint8_t*>(raw + c)[b] =
+                (x >= tb && x < tb + tbytes) ? *reinterpret_cast<const uint8_t*>(x) : uint8_t('\n');
+          }
+        }
       }
     }
-    __syncthreads();
-    const uint32_t t = threadIdx.x;
-    uint32_t mycross = 0;
-    if (t < cnt) {
-      const uint64_t line = b0 + t;
-      const uint64_t s = starts ? uint64_t(starts[line]) : body + line * stride;
-      Key<NW> key;
+    __pipeline_commit();
+    return P;
+  };
+  if (blockIdx.x >= nblocks) return;
+  Pass next = fetch(blockIdx.x);
+  for (uint64_t g = blockIdx.x; g < nblocks; g += gridDim.x) {
+    const Pass P = next;
+    const uint64_t end = P.end, b0 = P.b0, s0 = P.s0;
+    const uint8_t* text = P.text;
+    const uint32_t cnt = P.cnt, j = P.j;
+    const bool staged = P.span <= uint64_t(pcap) * 16;
+    uint64_t* kout = keys + (P.koff + b0) * NW;
+    uint32_t* o1 = FUSE ? b1 + P.koff + b0 : nullptr;
+    uint32_t* o2 = FUSE ? b2 + P.koff + b0 : nullptr;
+    if (MULTI && threadIdx.x == 0) s_cross = 0;
+    __pipeline_wait_prior(0);
+    const uint32_t nch = uint32_t(P.span + 15) / 16;
+    bool regular = staged && !starts && stride >= 16;
+    if (regular) {
+      uint32_t odd = 0, c = threadIdx.x;
+      // the piece's offset from a line's start, in [0, stride)
+      uint32_t r = (16u * threadIdx.x + stride - P.first % stride) % stride;
+      Break16 x = break_at(uint32_t(k) - r);
+      auto step = [&] {
+        if constexpr (KC == 0 || 4096 % (KC + 1) != 0) {
+          r += 4096u % stride;
+          r -= r >= stride ? stride : 0u;
+          x = break_at(uint32_t(k) - r);
+        }
+      };
+      for (; c + 768 < nch; c += 1024) {
+        uint4 v[4];
 #pragma unroll
-      for (int w = 0; w < NW; ++w) key.w[w] = 0;
-      bool lbad = false;
-      const bool check_term = !starts && line + 1 < n;
-      bool fast = false;
-      if (staged) {
-        const uint32_t off = uint32_t((tb + s) - A0);     // line start in the staged span
-        const uint32_t lim = uint32_t((tb + s1) - A0);    // end of the staged lines
-        lbad |= (off + uint32_t(k) > lim);
-        const uint32_t sh = 8u * (off & 3u);
-        const uint32_t base = off & ~3u;
-        // fast form: codes of 4 bytes in 3 operations, then one check that
-        // every byte is the letter its code spells ("ACGT"[code]); a line
-        // with any other byte among its k chars (a non-ACGT letter or a line
-        // break) is packed again by the exact form below
-        {
-          uint32_t cur = buf[pad_word(base)];
-          uint32_t mism = 0;
-          const int nfull = k / 4;
-#pragma unroll 4
-          for (int jw = 0; jw <= nfull; ++jw) {
-            const uint32_t nxt = buf[pad_word(base + 4u * (jw + 1))];
-            const uint32_t x = __funnelshift_r(cur, nxt, sh);
-            cur = nxt;
-            const int c0 = 4 * jw;
-            // the last word holds k % 4 chars and the line break
-            const uint32_t inmask = (jw < nfull) ? 0xFFFFFFFFu : ((1u << (8 * (k - c0))) - 1u);
-            const uint32_t g = gather_codes(((x >> 1) ^ (x >> 2)) & 0x03030303u);
-            mism |= (ascii4(g) ^ x) & inmask;
-            if (check_term && jw == nfull) lbad |= ((x >> (8 * (k - c0))) & 0xFFu) != '\n';
-            // codes past char k-1 fall under kmask_hi below; a word never
-            // straddles the two key words (32 is a multiple of 4)
-            const uint64_t gc = uint64_t(g);
-            if (NW == 1 || c0 < 32) key.w[0] |= gc << (2 * c0);
-            else key.w[NW - 1] |= gc << (2 * (c0 - 32));
-          }
-          fast = (mism == 0);
+        for (int q = 0; q < 4; ++q) v[q] = raw[c + 256 * q];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          code[c + 256 * q] = regular_piece(v[q], x, odd);
+          step();
         }
       }
-      if (staged && !fast) {
+      for (; c < nch; c += 256) {
+        code[c] = regular_piece(raw[c], x, odd);
+        step();
+      }
+      regular = !__syncthreads_or(odd != 0);
+    }
+    if (!regular) {
+      if (staged) {
+        for (uint32_t c = threadIdx.x; c < nch; c += 256) {
+          uint32_t nl, bd;
+          code[c] = text_piece(raw[c], nl, bd);
+          nl16[c] = uint16_t(nl);
+          bad16[c] = uint16_t(bd);
+        }
+      }
+      __syncthreads();
+    }
+    if (g + gridDim.x < nblocks) next = fetch(g + gridDim.x);
+    for (uint32_t t = threadIdx.x; t < cnt; t += 256) {
+      Key<NW> key;
+      bool lbad = false;
+      const bool check_term = t < P.nterm;
+      if (regular) {
+        const uint32_t off = P.first + t * stride, wi = off >> 4, sh = 2u * (off & 15u);
+        uint32_t c[2 * NW + 1];
+#pragma unroll
+        for (int w = 0; w <= 2 * NW; ++w) c[w] = code[wi + w];
+#pragma unroll
+        for (int w = 0; w < NW; ++w)
+          key.w[w] = __funnelshift_r(c[2 * w], c[2 * w + 1], sh) |
+                     (uint64_t(__funnelshift_r(c[2 * w + 1], c[2 * w + 2], sh)) << 32);
+        key.w[NW - 1] &= kmask_hi;
+      } else if (staged) {
+        // (a line past the staged ones is an error: it reads the first line's place)
+        uint32_t off = P.first + (starts ? uint32_t(uint64_t(starts[b0 + t]) - s0) : t * stride);
+        lbad = off + uint32_t(k) > uint32_t(P.span);
+        if (lbad) off = 0;
+        const uint32_t wi = off >> 4, sh = 2u * (off & 15u), mi = off >> 5, ms = off & 31u;
+        uint32_t c[2 * NW + 1];
+#pragma unroll
+        for (int w = 0; w <= 2 * NW; ++w) c[w] = code[wi + w];
+#pragma unroll
+        for (int w = 0; w < NW; ++w)
+          key.w[w] = __funnelshift_r(c[2 * w], c[2 * w + 1], sh) |
+                     (uint64_t(__funnelshift_r(c[2 * w + 1], c[2 * w + 2], sh)) << 32);
+        // possible line breaks and other bytes among the k chars, and the
+        // break after them
+        Mask nm = __funnelshift_r(nlw[mi], nlw[mi + 1], ms), bm = __funnelshift_r(badw[mi], badw[mi + 1], ms);
+        if constexpr (NW == 2) {
+          nm |= uint64_t(__funnelshift_r(nlw[mi + 1], nlw[mi + 2], ms)) << 32;
+          bm |= uint64_t(__funnelshift_r(badw[mi + 1], badw[mi + 2], ms)) << 32;
+        }
+        const uint32_t after = uint32_t((NW == 1 || k < 32) ? key.w[0] >> (2 * k) : key.w[NW - 1] >> (2 * k - 64)) & 3u;
+        lbad |= check_term && (!(nm & term) || after != 1u);
+        key.w[NW - 1] &= kmask_hi;
+        if ((nm | bm) & chars) {
+          for (Mask m = (nm | bm) & chars; m; m &= m - 1) {
+            const int i = __ffsll((long long)m) - 1;
+            const bool low = NW == 1 || i < 32;
+            const uint64_t at = 3ull << (2 * (i & 31)), w = low ? key.w[0] : key.w[NW - 1];
+            if (((nm >> i) & 1u) && ((w >> (2 * (i & 31))) & 3u) == 1u) lbad = true;  // a line break
+            if (low) key.w[0] &= ~at;
+            else key.w[NW - 1] &= ~at;
+          }
+        }
+      } else {
 #pragma unroll
         for (int w = 0; w < NW; ++w) key.w[w] = 0;
-        const uint32_t off = uint32_t((tb + s) - A0);
-        const uint32_t lim = uint32_t((tb + s1) - A0);
-        lbad |= (off + uint32_t(k) > lim);
-        const uint32_t sh = 8u * (off & 3u);
-        const uint32_t base = off & ~3u;
-        uint32_t cur = buf[pad_word(base)];
-        const int nwords = (k + 4) / 4;  // covers chars 0..k (k chars + terminator)
-#pragma unroll 4
-        for (int jw = 0; jw < nwords; ++jw) {
-          const uint32_t nxt = buf[pad_word(base + 4u * (jw + 1))];
-          const uint32_t x = __funnelshift_r(cur, nxt, sh);
-          cur = nxt;
-          uint32_t nl;
-          const uint32_t tc = swar_codes(x, &nl);
-          const int c0 = 4 * jw;
-          const uint32_t inmask = (c0 + 4 <= k) ? 0xFFFFFFFFu : (c0 >= k ? 0u : (0xFFFFFFFFu >> (8 * (c0 + 4 - k))));
-          lbad |= (nl & inmask) != 0;
-          if (check_term && c0 <= k && k < c0 + 4) {
-            const uint32_t tbyte = (x >> (8 * (k - c0))) & 0xFFu;
-            lbad |= (tbyte != '\n');
-          }
-          const uint64_t gc = uint64_t(gather_codes(tc & inmask));
-          if (NW == 1 || c0 < 32) key.w[0] |= gc << (2 * c0);
-          else key.w[NW - 1] |= gc << (2 * (c0 - 32));
-        }
-      } else if (!staged) {
+        const uint64_t s = starts ? uint64_t(starts[b0 + t]) : s0 + uint64_t(t) * stride;
         for (int c = 0; c <= k; ++c) {
           const uint64_t pos = s + c;
           const uint32_t ch = (pos < end) ? uint32_t(__ldg(text + pos)) : uint32_t('\n');
           if (c < k) {
             lbad |= (ch == '\n') || (pos >= end);
-            const uint64_t code = base_code(ch);
-            if (c < 32) key.w[0] |= code << (2 * c);
-            else key.w[NW - 1] |= code << (2 * (c - 32));
+            const uint64_t cd = base_code(ch);
+            if (c < 32) key.w[0] |= cd << (2 * c);
+            else key.w[NW - 1] |= cd << (2 * (c - 32));
           } else if (check_term && ch != '\n') {
             lbad = true;
           }
         }
       }
-      key.w[NW - 1] &= kmask_hi;
       if (lbad) bad = 1;
       // keys and bucket ids stream out with evict-first stores, so that the
       // text and them do not push the bucket counts out of L2
-      if constexpr (NW == 1) __stcs(reinterpret_cast<unsigned long long*>(keys) + koff + line,
+      if constexpr (NW == 1) __stcs(reinterpret_cast<unsigned long long*>(kout) + t,
                                     static_cast<unsigned long long>(key.w[0]));
-      else st_key<NW>(keys, koff + line, key);
+      else st_key<NW>(kout, t, key);
       if constexpr (FUSE) {
         uint32_t a, b;
-        lmins<NW>(key, k, l, seed, nullptr, a, b);
-        const uint32_t jp = j << jb;
-        a = jp | bucket_of(a, jb);
-        b = jp | bucket_of(b, jb);
-        __stcs(b1 + koff + line, a);
-        __stcs(b2 + koff + line, b);
+        key_buckets<NW, KC>(key, k, l, seed, jb, a, b);
+        if (MULTI) {
+          a |= j << jb;
+          b |= j << jb;
+        }
+        __stcs(o1 + t, a);
+        __stcs(o2 + t, b);
         if (counts) {  // (the streamed path's second pass only needs the buckets)
           if (cshift == CNT16) {
             count16(counts, a);
@@ -356,16 +493,21 @@ __global__ void __launch_bounds__(256) k_pack(const JobTab* __restrict__ jobs, c
             atomicAdd(counts + (a >> cshift), 1u);
             if (a != b) atomicAdd(counts + (b >> cshift), 1u);
           }
-          mycross = (a != b) ? 1u : 0u;
+          mycross += (a != b) ? 1u : 0u;
         }
       }
     }
-    if constexpr (FUSE) {
+    if (FUSE && MULTI) {  // (one job: counted over all passes)
       mycross = __reduce_add_sync(0xFFFFFFFFu, mycross);
       if ((threadIdx.x & 31) == 0 && mycross) atomicAdd(&s_cross, mycross);
+      mycross = 0;
     }
     __syncthreads();
-    if (FUSE && threadIdx.x == 0 && s_cross && jcross) atomicAdd(jcross + j, s_cross);
+    if (FUSE && MULTI && threadIdx.x == 0 && s_cross && jcross) atomicAdd(jcross + j, s_cross);
+  }
+  if (FUSE && !MULTI) {
+    mycross = __reduce_add_sync(0xFFFFFFFFu, mycross);
+    if ((threadIdx.x & 31) == 0 && mycross && jcross) atomicAdd(jcross, mycross);
   }
   if (__syncthreads_or(bad) && threadIdx.x == 0) atomicOr(err, starts ? ERR_LINE : ERR_LAYOUT);
 }
@@ -2620,46 +2762,21 @@ struct FuseArgs {
   uint64_t M = 0;
 };
 
-template <int NW, bool FUSE, bool MULTI, int KC = 0, int LC = 0>
-static int pack_occupancy() {
-  static int o = 0;  // resident CTAs per SM (per template instance)
-  if (!o) {
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, k_pack<NW, FUSE, MULTI, KC, LC>, 256, 0);
-    if (o < 1) o = 1;
-  }
-  return o;
-}
-
-// The single-job fused pack with k and l fixed at compile time: k = 31 or
-// 63 with l in [8, 16] (the bucket count raises l to at least 13 for large
-// jobs).  Returns false for other shapes.
-template <int NW, int KC, int LC>
-static bool launch_pack_fixed_l(Env& e, const JobTab* jobs, const JobTab& J, uint64_t nblocks, uint64_t* keys,
-                                const FuseArgs* fz) {
-  const int o = pack_occupancy<NW, true, false, KC, LC>();
-  const int grid = int(std::max<uint64_t>(1, std::min<uint64_t>(nblocks, uint64_t(e.sm_count) * o)));
+// One wave of resident CTAs: blocks stride over equal-sized line blocks, so a
+// partial second wave would double the time.
+template <int NW, bool FUSE, bool MULTI, int KC>
+static void launch_pack_as(Env& e, const JobTab* jobs, const JobTab& J, uint32_t njobs, uint64_t nblocks,
+                           const unsigned long long* starts, int k, uint64_t* keys, const FuseArgs& fz) {
+  const uint32_t pcap = pack_pieces(starts == nullptr, k);
+  const size_t sm = pack_smem(pcap);
+  if (sm > 48 * 1024) allow_max_smem(e, k_pack<NW, FUSE, MULTI, KC>);
+  int occ = 0;
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_pack<NW, FUSE, MULTI, KC>, 256, sm);
+  const int grid = int(std::max<uint64_t>(1, std::min<uint64_t>(nblocks, uint64_t(e.sm_count) * std::max(1, occ))));
   ++e.launches;
-  k_pack<NW, true, false, KC, LC><<<grid, 256, 0, e.stream>>>(jobs, J, 1, nblocks, nullptr, KC, keys, &e.ctr->err,
-                                                               LC, fz->seed, fz->jb, fz->b1, fz->b2, fz->counts,
-                                                               fz->cshift, fz->jcross);
-  return true;
-}
-
-template <int NW, int KC>
-static bool launch_pack_fixed(Env& e, const JobTab* jobs, const JobTab& J, uint64_t nblocks, uint64_t* keys,
-                              const FuseArgs* fz) {
-  switch (fz->l) {
-    case 8: return launch_pack_fixed_l<NW, KC, 8>(e, jobs, J, nblocks, keys, fz);
-    case 9: return launch_pack_fixed_l<NW, KC, 9>(e, jobs, J, nblocks, keys, fz);
-    case 10: return launch_pack_fixed_l<NW, KC, 10>(e, jobs, J, nblocks, keys, fz);
-    case 11: return launch_pack_fixed_l<NW, KC, 11>(e, jobs, J, nblocks, keys, fz);
-    case 12: return launch_pack_fixed_l<NW, KC, 12>(e, jobs, J, nblocks, keys, fz);
-    case 13: return launch_pack_fixed_l<NW, KC, 13>(e, jobs, J, nblocks, keys, fz);
-    case 14: return launch_pack_fixed_l<NW, KC, 14>(e, jobs, J, nblocks, keys, fz);
-    case 15: return launch_pack_fixed_l<NW, KC, 15>(e, jobs, J, nblocks, keys, fz);
-    case 16: return launch_pack_fixed_l<NW, KC, 16>(e, jobs, J, nblocks, keys, fz);
-    default: return false;
-  }
+  k_pack<NW, FUSE, MULTI, KC><<<grid, 256, sm, e.stream>>>(jobs, J, njobs, nblocks, starts, k, keys, &e.ctr->err, fz.l,
+                                                           fz.seed, fz.jb, fz.b1, fz.b2, fz.counts, fz.cshift,
+                                                           fz.jcross, pcap);
 }
 
 // one: the job of a single-job launch (host copy), or NULL for a batch
@@ -2667,31 +2784,18 @@ static bool launch_pack_fixed(Env& e, const JobTab* jobs, const JobTab& J, uint6
 template <int NW>
 static void launch_pack(Env& e, const JobTab* jobs, const JobTab* one, uint32_t njobs, uint64_t nblocks,
                         const unsigned long long* starts, int k, uint64_t* keys, const FuseArgs* fz) {
-  // one wave of resident CTAs: blocks stride over equal-sized line blocks,
-  // so a partial second wave would double the time
-  const int o = fz ? (one ? pack_occupancy<NW, true, false>() : pack_occupancy<NW, true, true>())
-                   : (one ? pack_occupancy<NW, false, false>() : pack_occupancy<NW, false, true>());
-  const int grid = int(std::max<uint64_t>(1, std::min<uint64_t>(nblocks, uint64_t(e.sm_count) * o)));
+  constexpr int KC = NW == 1 ? 31 : 63;
   const JobTab J = one ? *one : JobTab{};
-  if (fz && one && !starts) {
-    if (NW == 1 && k == 31 && launch_pack_fixed<NW, 31>(e, jobs, J, nblocks, keys, fz)) return;
-    if (NW == 2 && k == 63 && launch_pack_fixed<NW, 63>(e, jobs, J, nblocks, keys, fz)) return;
+  if (!fz) {
+    if (k == KC) launch_pack_as<NW, false, false, KC>(e, jobs, J, njobs, nblocks, starts, k, keys, FuseArgs{});
+    else launch_pack_as<NW, false, false, 0>(e, jobs, J, njobs, nblocks, starts, k, keys, FuseArgs{});
+  } else if (one) {
+    if (k == KC) launch_pack_as<NW, true, false, KC>(e, jobs, J, njobs, nblocks, starts, k, keys, *fz);
+    else launch_pack_as<NW, true, false, 0>(e, jobs, J, njobs, nblocks, starts, k, keys, *fz);
+  } else {
+    if (k == KC) launch_pack_as<NW, true, true, KC>(e, jobs, J, njobs, nblocks, starts, k, keys, *fz);
+    else launch_pack_as<NW, true, true, 0>(e, jobs, J, njobs, nblocks, starts, k, keys, *fz);
   }
-  ++e.launches;
-  if (fz && one)
-    k_pack<NW, true, false><<<grid, 256, 0, e.stream>>>(jobs, J, njobs, nblocks, starts, k, keys, &e.ctr->err,
-                                                        fz->l, fz->seed, fz->jb, fz->b1, fz->b2, fz->counts,
-                                                        fz->cshift, fz->jcross);
-  else if (fz)
-    k_pack<NW, true, true><<<grid, 256, 0, e.stream>>>(jobs, J, njobs, nblocks, starts, k, keys, &e.ctr->err,
-                                                       fz->l, fz->seed, fz->jb, fz->b1, fz->b2, fz->counts,
-                                                       fz->cshift, fz->jcross);
-  else if (one)
-    k_pack<NW, false, false><<<grid, 256, 0, e.stream>>>(jobs, J, njobs, nblocks, starts, k, keys, &e.ctr->err, 0,
-                                                         0, 0, nullptr, nullptr, nullptr, CNT16, nullptr);
-  else
-    k_pack<NW, false, true><<<grid, 256, 0, e.stream>>>(jobs, J, njobs, nblocks, starts, k, keys, &e.ctr->err, 0,
-                                                        0, 0, nullptr, nullptr, nullptr, CNT16, nullptr);
 }
 
 // Grow-only device buffers for the job table and the per-job counters.
