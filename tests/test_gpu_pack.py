@@ -69,3 +69,18 @@ def test_break_inside_a_line_is_an_error(comp, k):
     with pytest.raises(api.UCError) as e:
         comp.load_kmers(dev(bytes(text)), k)
     assert e.value.status == 1
+
+
+@pytest.mark.parametrize("k", [5, 21, 63])
+@pytest.mark.parametrize("n", [1, 2, 500, 9000])
+@pytest.mark.parametrize("end", ["\n", "", "\r\n\n\n"])
+def test_line_index(comp, oracle, k, n, end):
+    """Lines of different widths (columns after the k-mer), among them one
+    wider than a chunk of the index and breaks on both sides of its edges."""
+    r = random.Random(n * k)
+    rows = [x + "\t" + "7" * r.randrange(0, 40) for x in lines(n, k, n)]
+    rows[n // 2] += "9" * 40_000
+    for pad in (0, 5, 11):
+        keys_equal(comp, oracle, (" " * pad + f"{n}\n" + "\n".join(rows) + end).encode(), k)
+    with pytest.raises(api.UCError):
+        comp.load_kmers(dev((f"{n + 1}\n" + "\n".join(rows) + end).encode()), k)
