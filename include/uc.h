@@ -61,10 +61,10 @@ typedef struct uc_tuning {
     uint32_t tile_capacity;   /* copies per shared-memory tile (max 8192) */
     uint32_t tile_threads;    /* threads per tile CTA (256 or 512) */
     uint32_t bucket_bits;     /* log2 of the bucket count */
-    uint32_t load_factor_pct; /* tile hash slots per 100 copies (150..800; 200) */
+    uint32_t load_factor_pct; /* tile hash slots per 100 copies (150..800; 300 warp, 200 block) */
     uint32_t contract_method; /* UC_CONTRACT_* for the segment stitch */
     uint32_t warp_capacity;   /* copies per warp tile (32..1024; 1 = no warp tier) */
-    uint32_t bucket_fill;     /* buckets per tile when bucket_bits is 0 (1..64; 8) */
+    uint32_t bucket_fill;     /* buckets per tile when bucket_bits is 0 (1..64; 4) */
 } uc_tuning;
 
 /* ---- context --------------------------------------------------------- */

@@ -459,10 +459,10 @@ uc_status uc_autotune(uc_ctx* c, const char* d_text, size_t bytes, int k, int l,
   uc_tuning cur{};
   cur.tile_capacity = 4096;
   cur.tile_threads = 512;
-  cur.load_factor_pct = 200;
+  cur.load_factor_pct = 0;  // (300 for warp tiles, 200 for block tiles)
   cur.contract_method = UC_CONTRACT_POINTER_JUMP;
   cur.warp_capacity = 256;
-  cur.bucket_fill = 8;
+  cur.bucket_fill = 4;
   float cur_ms = 0.f;
   int r = time_one(cur, cur_ms);
   if (r) {

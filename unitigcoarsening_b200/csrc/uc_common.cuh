@@ -208,6 +208,96 @@ __device__ __forceinline__ void spread16(uint32_t table, uint32_t c, uint32_t w[
 }
 __device__ __forceinline__ void letters16(uint32_t codes, uint32_t w[4]) { spread16(0x54474341u, codes, w); }
 
+// Text of n chars (codes x, first char lowest) and, with brk = 1, a line break
+// at byte pos of a shared-memory buffer: whole words where the text owns them,
+// halves and bytes at its two ends (shared with its neighbours).
+template <int NC>
+__device__ __forceinline__ void spell_text(uint32_t* buf, uint32_t pos, const uint32_t x[NC], uint32_t n, uint32_t brk) {
+  const uint32_t a = pos & 3u;
+  // the code stream, moved up by the chars before the text in its first word
+  uint32_t c[NC];
+  c[0] = x[0] << (2 * a);
+#pragma unroll
+  for (int q = 1; q < NC; ++q) c[q] = __funnelshift_l(x[q - 1], x[q], 2 * a);
+  const uint32_t last = a + n;                      // one past the last char, from the first word's start
+  const uint32_t nw = last >> 2, rem = last & 3u;   // its word, and the chars before it there
+  uint32_t* d = buf + (pos >> 2);
+  uint32_t first = 0, tail = 0;
+#pragma unroll
+  for (int g = 0; g < NC; ++g) {
+    if (4u * g > nw) break;
+    uint32_t w[4];
+    letters16(c[g], w);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const uint32_t j = 4u * g + q;
+      if (j == nw) tail = w[q];
+      if (j < nw && (j > 0 || a == 0)) d[j] = w[q];
+    }
+    if (g == 0) first = w[0];
+  }
+  if (brk) tail = (tail & ((1u << (8 * rem)) - 1u)) | (uint32_t('\n') << (8 * rem));
+  const uint32_t nb = rem + brk;  // bytes of the last word
+  char* e = reinterpret_cast<char*>(d + nw);
+  if (nw == 0 && a) {  // inside one word
+    for (uint32_t q = a; q < nb; ++q) e[q] = char(tail >> (8 * q));
+    return;
+  }
+  if (nb == 4) {
+    d[nw] = tail;
+  } else {
+    if (nb & 2u) *reinterpret_cast<uint16_t*>(e) = uint16_t(tail);
+    if (nb & 1u) e[nb & 2u] = char(tail >> (8 * (nb & 2u)));
+  }
+  if (a) {
+    char* f = reinterpret_cast<char*>(d);
+    if (a & 1u) f[a] = char(first >> (8 * a));
+    if (a < 3) *reinterpret_cast<uint16_t*>(f + 2) = uint16_t(first >> 16);
+  }
+}
+
+// A stream of text to global memory by one warp: texts are spelled one after
+// another into the warp's shared-memory buffer and leave as 16-byte stores.
+// The bytes after the last whole piece stay in the buffer for the next
+// texts; the first and the last piece, shared with other streams, go byte by
+// byte.
+struct WarpText {
+  char* dst;      // next byte of the stream
+  uint32_t fill;  // bytes of buf before it, from the 16-byte boundary below dst
+  uint32_t head;  // of which another stream's
+  __device__ __forceinline__ void begin(char* at) {
+    dst = at;
+    fill = head = uint32_t(reinterpret_cast<uintptr_t>(at) & 15u);
+  }
+  // total bytes were spelled into buf from byte fill on (every lane calls,
+  // after a __syncwarp).  Reads buf up to 16 bytes past them.
+  __device__ __forceinline__ void flush(uint32_t* buf, uint32_t total) {
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t full = (fill + total) >> 4;
+    char* w = dst - fill;
+    for (uint32_t p = lane; p < full; p += 32) {
+      if (p == 0 && head) {
+        for (uint32_t q = head; q < 16; ++q) w[q] = reinterpret_cast<const char*>(buf)[q];
+      } else {
+        reinterpret_cast<uint4*>(w)[p] = reinterpret_cast<const uint4*>(buf)[p];
+      }
+    }
+    __syncwarp();
+    if (full) {
+      if (lane < 4) buf[lane] = buf[4 * full + lane];
+      head = 0;
+    }
+    __syncwarp();
+    fill = (fill + total) & 15u;
+    dst += total;
+  }
+  __device__ __forceinline__ void end(const uint32_t* buf) const {
+    const uint32_t lane = threadIdx.x & 31u;
+    if (lane >= head && lane < fill) (dst - fill)[lane] = reinterpret_cast<const char*>(buf)[lane];
+    __syncwarp();
+  }
+};
+
 // codes of chars ch..ch+3 of a packed key in the low 8 bits (chars past the
 // key read as 0)
 template <int NW>

@@ -76,7 +76,7 @@ struct TileParams {
   int k;
   uint32_t cap;                 // shared-memory tile capacity (copies)
   uint32_t tslots;              // shared-memory hash slots (power of two >= 2*cap)
-  uint32_t lf;                  // hash slots per 100 copies of a tile (150..800)
+  uint32_t lf, wlf;             // hash slots per 100 copies of a block / warp tile (150..800)
   int mode;                     // 0 = edges by id, 1 = fused emission
   uint32_t* succ;
   uint32_t* pred;

@@ -1428,6 +1428,209 @@ __device__ void jump_rounds(uint32_t c, IT* px, IT* rx, IT* py, IT* ry, IT*& ptr
   rnk = rx;
 }
 
+// Segments and lines of a warp tile whose kept edges are known (A: local
+// successor or NONE, P: local predecessor or NONE).  In-tile paths are short
+// (the consecutive k-mers that share one minimizer, and half of the edges of
+// canonical k-mers drop), so a lane takes a segment's end and walks back to
+// its start, gathering the chars the later copies add as 2-bit codes; the
+// text of 32 segments at a time is spelled into shared memory from those codes
+// and leaves as 16-byte stores.  Against ranking the copies by pointer jumping
+// and storing each copy's char by itself: 64 Mbp, k = 63, the kernel takes
+// 2.36 instead of 3.01 ms; at k = 31 it is as long (8.7 ms at 256 Mbp), with
+// half as many stores.
+constexpr uint32_t TAIL_CODES = 28;  // later chars a lane keeps as codes; longer segments store byte by byte
+template <int NW, int KC>
+__device__ __forceinline__ void emit_warp_tile(const TileParams& p, const TileMem<NW, uint16_t>& m, uint64_t beg,
+                                               uint32_t c, uint32_t job) {
+  constexpr uint32_t NONE_I = Ix<uint16_t>::NONE;
+  const int k = KC ? KC : p.k;
+  const uint32_t lane = threadIdx.x & 31u, below = (1u << lane) - 1u;
+  // segment ends, in B (the in-counts are used up)
+  uint32_t nend = 0;
+  for (uint32_t base = 0; base < c; base += 32) {
+    const uint32_t i = base + lane;
+    const bool e = i < c && m.A[i] == NONE_I;
+    const uint32_t mask = __ballot_sync(0xFFFFFFFFu, e);
+    if (e) m.B[nend + __popc(mask & below)] = uint16_t(i);
+    nend += uint32_t(__popc(mask));
+  }
+  __syncwarp();
+  // sizes; the closed segments' ends to the front of A, the open ones' to its
+  // back (the successors are used up: cycles are found from P)
+  uint32_t nclosed, nopen, heads, cbytes, obytes;
+  for (bool cut = false;; cut = true) {
+    nclosed = nopen = 0;
+    uint32_t h = 0, cb = 0, ob = 0, covered = 0;
+    for (uint32_t base = 0; base < nend; base += 32) {
+      const bool live = base + lane < nend;
+      uint32_t i = 0, s = 0, len = 0;
+      bool starts_p = false, closed = false;
+      if (live) {
+        i = s = m.B[base + lane];
+        len = 1;
+        for (uint32_t q = m.P[s]; q != NONE_I && len < c; q = m.P[s]) {
+          s = q;
+          ++len;
+        }
+        starts_p = (roles(skey(m, s)) & ROLE_P) != 0;
+        closed = starts_p && (roles(skey(m, i)) & ROLE_S);
+        covered += len;
+        if (closed) {
+          cb += uint32_t(k) + len;
+        } else {
+          ob += starts_p ? uint32_t(k) - 1u + len : len - 1u;
+          h += starts_p ? 1u : 0u;
+        }
+      }
+      const uint32_t cm = __ballot_sync(0xFFFFFFFFu, closed), om = __ballot_sync(0xFFFFFFFFu, live && !closed);
+      if (closed) m.A[nclosed + __popc(cm & below)] = uint16_t(i);
+      else if (live) m.A[c - 1u - nopen - __popc(om & below)] = uint16_t(i);
+      nclosed += uint32_t(__popc(cm));
+      nopen += uint32_t(__popc(om));
+    }
+    covered = __reduce_add_sync(0xFFFFFFFFu, covered);
+    heads = __reduce_add_sync(0xFFFFFFFFu, h);
+    cbytes = __reduce_add_sync(0xFFFFFFFFu, cb);
+    obytes = __reduce_add_sync(0xFFFFFFFFu, ob);
+    if (covered == c || cut) break;
+    // local cycles hold the copies no end reaches (rare): one lane cuts each
+    // before its smallest key, which then starts a segment
+    for (uint32_t i = lane; i < c; i += 32) m.Q[i] = 0;
+    __syncwarp();
+    for (uint32_t j = lane; j < nend; j += 32)
+      for (uint32_t s = m.B[j], n = 0; s != NONE_I && n < c; s = m.P[s], ++n) m.Q[s] = 1;
+    __syncwarp();
+    if (lane == 0) {
+      for (uint32_t i = 0; i < c; ++i) {
+        if (m.Q[i]) continue;
+        uint32_t best = i;
+        m.Q[i] = 1;
+        for (uint32_t s = m.P[i], n = 0; s != i && s != NONE_I && n < c; s = m.P[s], ++n) {
+          m.Q[s] = 1;
+          if (key_lt(skey(m, s), skey(m, best))) best = s;
+        }
+        m.B[nend++] = m.P[best];
+        m.P[best] = uint16_t(NONE_I);
+      }
+    }
+    nend = __shfl_sync(0xFFFFFFFFu, nend, 0);
+    __syncwarp();
+  }
+  unsigned long long at[3];
+  if (!WarpGroup::reserve(p, job, U3{cbytes, obytes, heads}, at)) return;
+  __syncwarp();
+  // text buffer: the arrays Q and T, less the piece that WarpText::flush may
+  // read past the text (room for one line is left in the smallest tile: 32
+  // copies have 192 bytes there)
+  const uintptr_t q0 = reinterpret_cast<uintptr_t>(m.Q);
+  uint32_t* buf = reinterpret_cast<uint32_t*>((q0 + 15) & ~uintptr_t(15));
+  const uint32_t room =
+      (uint32_t(reinterpret_cast<uintptr_t>(m.T + m.ts) - reinterpret_cast<uintptr_t>(buf)) & ~15u) - 16u;
+  uint32_t head0 = p.xcount + uint32_t(at[2]);  // id of the next segment that starts a line
+  constexpr int NC = NW == 1 ? 4 : 6;
+#pragma unroll 1
+  for (uint32_t open = 0; open < 2; ++open) {
+    const uint32_t nseg = open ? nopen : nclosed;
+    WarpText T;
+    T.begin(open ? p.segchars + at[1] : p.out + at[0]);
+    for (uint32_t base = 0; base < nseg;) {
+      const bool live = base + lane < nseg;
+      uint32_t i = 0, s = 0, len = 0;
+      uint64_t tail = 0;
+      Key<NW> ks;
+#pragma unroll
+      for (int w = 0; w < NW; ++w) ks.w[w] = 0;
+      bool starts_p = false;
+      uint32_t xs = NONE, xe = NONE;
+      if (live) {
+        i = s = open ? m.A[c - 1u - base - lane] : m.A[base + lane];
+        len = 1;
+        for (uint32_t q = m.P[s]; q != NONE_I && len < c; q = m.P[s]) {
+          tail = (tail << 2) | key_char(skey(m, s), k - 1);
+          s = q;
+          ++len;
+        }
+        ks = skey(m, s);
+        starts_p = (roles(ks) & ROLE_P) != 0;
+        if (open) {
+          // this segment's id (S-only start), the next one's (P-only end)
+          if (!starts_p) xs = p.plink[beg + s];
+          if (!(roles(skey(m, i)) & ROLE_S)) xe = p.plink[beg + i];
+        }
+      }
+      // chars: the first k-mer in full, unless it ends the segment before
+      const uint32_t nch = live ? (starts_p ? uint32_t(k) - 1u + len : len - 1u) : 0u;
+      const uint32_t nb = live ? nch + (open ? 0u : 1u) : 0u;
+      uint32_t inc = nb;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t v = __shfl_up_sync(0xFFFFFFFFu, inc, o);
+        if (lane >= uint32_t(o)) inc += v;
+      }
+      const bool direct = __any_sync(0xFFFFFFFFu, len > TAIL_CODES + 1u);
+      // the lanes whose text fits the buffer (all of them when it is not used)
+      const bool take = live && (direct || T.fill + inc <= room);
+      const uint32_t taken = __ballot_sync(0xFFFFFFFFu, take);
+      const uint32_t cnt = uint32_t(__popc(taken));  // a prefix of the lanes
+      const uint32_t total = __shfl_sync(0xFFFFFFFFu, inc, int(cnt) - 1);
+      char* const first = T.dst + (inc - nb);
+      if (!direct) {
+        if (take) {
+          uint64_t w[3];
+          const uint64_t codes = len > 1u ? tail : 0ull;
+          w[0] = w[1] = w[2] = 0;
+          const Key<NW> x = strip(ks);
+          if (!starts_p) {
+            w[0] = codes;
+          } else if constexpr (NW == 1) {
+            w[0] = x.w[0] | (codes << (2 * k));
+            w[1] = codes >> (64 - 2 * k);
+          } else {
+            const int u = 2 * k - 64;
+            w[0] = x.w[0];
+            w[1] = x.w[1] | (codes << u);
+            w[2] = u ? codes >> (64 - u) : 0ull;
+          }
+          uint32_t xx[NC];
+#pragma unroll
+          for (int q = 0; q < NC; ++q) xx[q] = uint32_t(w[q >> 1] >> (32 * (q & 1)));
+          spell_text<NC>(buf, T.fill + inc - nb, xx, nch, open ? 0u : 1u);
+        }
+        __syncwarp();
+        T.flush(buf, total);
+      } else {
+        T.end(buf);
+        if (live) {
+          if (starts_p) spell_key<NW>(first, ks, k);
+          char* d = first + nch;  // the chars of the later copies, last first
+          if (!open) *d = '\n';
+          uint32_t t = i;
+          for (uint32_t r = 1; r < len; ++r) {
+            *--d = acgt(key_char(skey(m, t), k - 1));
+            t = m.P[t];
+          }
+        }
+        __syncwarp();
+        T.begin(T.dst + total);
+      }
+      if (open) {
+        const uint32_t hm = __ballot_sync(0xFFFFFFFFu, take && starts_p);
+        if (take) {
+          // the segment's record under its id; it continues in segment xe
+          SegRec rec;
+          rec.off_job = uint64_t(first - p.segchars) | (static_cast<unsigned long long>(job) << SEG_OFF_BITS);
+          rec.len = len;
+          rec.next = xe;
+          p.seg[starts_p ? head0 + __popc(hm & below) : xs] = rec;
+        }
+        head0 += uint32_t(__popc(hm));
+      }
+      base += cnt;
+    }
+    T.end(buf);
+  }
+}
+
 // KC: k fixed at compile time (0: p.k), so that the masks, shifts and
 // spelling loops of the common shapes are constants.
 template <int NW, typename IT, typename G, int KC = 0>
@@ -1435,13 +1638,15 @@ __device__ void process_tile(const TileParams& p, const TileMem<NW, IT>& m, uint
                              uint32_t job) {
   constexpr uint32_t NONE_I = Ix<IT>::NONE, DUP_I = Ix<IT>::DUP, CNONE_I = Ix<IT>::CNONE;
   constexpr uint32_t OPEN_S = NONE_I - 1u;  // an open segment that starts at an S-only copy
+  constexpr bool WARP = std::is_same<G, WarpGroup>::value;
   const int k = KC ? KC : p.k;
   const PrefMask pm = pref_mask(k);
   // this tile's hash slots: the power of two above c * lf / 100, at most the
   // carved table (32-bit arithmetic for shared-memory tiles, c <= 8192)
   uint32_t ts;
   {
-    const uint32_t want = (sizeof(IT) == 2) ? (c * p.lf) / 100u : uint32_t((uint64_t(c) * p.lf) / 100u);
+    const uint32_t lf = WARP ? p.wlf : p.lf;
+    const uint32_t want = (sizeof(IT) == 2) ? (c * lf) / 100u : uint32_t((uint64_t(c) * lf) / 100u);
     const uint32_t x = want > c ? want : c + 1u;
     ts = 1u << (32 - __clz(x - 1u));
     ts = ts < m.ts ? ts : m.ts;
@@ -1489,6 +1694,38 @@ __device__ void process_tile(const TileParams& p, const TileMem<NW, IT>& m, uint
   // ---- prefix table of the P copies (generate_hashmap, assembler.h:120-150):
   // one slot per distinct (k-1)-prefix; a prefix held by two copies marks the
   // slot's copy DUP ("nullified")
+  if constexpr (WARP) {
+    // one warp works the table, so a free slot is taken by a plain store and
+    // a look at who won it (16-bit compare-and-swaps are several times as long)
+    for (uint32_t base = 0; base < c; base += 32) {
+      const uint32_t i = base + G::rank();
+      bool open = i < c;
+      Key<NW> pf;
+      uint32_t h = 0;
+      if (open) {
+        const Key<NW> x = skey(m, i);
+        open = (roles(x) & ROLE_P) != 0;
+        pf = prefix_of(x, pm);
+        h = key_hash(pf) & tmask;
+      }
+      while (__any_sync(0xFFFFFFFFu, open)) {
+        if (open && m.T[h] == NONE_I) m.T[h] = IT(i);
+        __syncwarp();
+        if (open) {
+          const uint32_t cur = m.T[h];
+          if (cur == i) {
+            open = false;
+          } else if (key_eq(prefix_of(skey(m, cur), pm), pf)) {
+            m.A[cur] = IT(CNONE_I | DUP_I);
+            open = false;
+          } else {
+            h = (h + 1) & tmask;
+          }
+        }
+        __syncwarp();
+      }
+    }
+  } else {
   for (uint32_t i = G::rank(); i < c; i += G::size()) {
     const Key<NW> x = skey(m, i);
     if (!(roles(x) & ROLE_P)) continue;
@@ -1503,6 +1740,7 @@ __device__ void process_tile(const TileParams& p, const TileMem<NW, IT>& m, uint
       }
       h = (h + 1) & tmask;
     }
+  }
   }
   G::sync();
   // ---- suffix lookups of the S copies (find_vtx_from_edge, assembler.h:89-111)
@@ -1537,8 +1775,10 @@ __device__ void process_tile(const TileParams& p, const TileMem<NW, IT>& m, uint
     const uint32_t q = (m.B[i] == 1u) ? uint32_t(m.P[i]) : NONE_I;
     m.A[i] = IT(s);
     m.P[i] = IT(q);
-    m.Q[i] = IT(q == NONE_I ? i : q);
-    m.T[i] = IT(q == NONE_I ? 0u : 1u);
+    if constexpr (!WARP) {
+      m.Q[i] = IT(q == NONE_I ? i : q);
+      m.T[i] = IT(q == NONE_I ? 0u : 1u);
+    }
   }
   G::sync();
   if (p.mode == 0) {
@@ -1550,6 +1790,10 @@ __device__ void process_tile(const TileParams& p, const TileMem<NW, IT>& m, uint
     }
     return;
   }
+  if constexpr (WARP) {
+    emit_warp_tile<NW, KC>(p, m, beg, c, job);
+    return;
+  } else {
   // ---- local segments: list ranking by pointer jumping
   IT *ptr, *rnk;
   jump_rounds<G, IT>(c, m.Q, m.T, m.B, m.T + c, ptr, rnk);
@@ -1615,35 +1859,11 @@ __device__ void process_tile(const TileParams& p, const TileMem<NW, IT>& m, uint
   // whole unitigs; the others are stitched across tiles.  Open segments that
   // start at a P-role copy start a stitched line: they take head-pool ids;
   // the others start at an S-only copy and take its cross index.
-  // A warp tile first packs its segment ends into a list (in A, which only
-  // marked the ends from here on), so that the per-segment loops keep every
-  // lane busy; a block tile walks its copies and skips the others.  Each
-  // thread's lines are contiguous in the tile's output, in the order the
+  // Each thread's lines are contiguous in the tile's output, in the order the
   // thread visits them (the order of lines is free).
-  constexpr bool WARP = std::is_same<G, WarpGroup>::value;
-  uint32_t nend = c;
-  if constexpr (WARP) {
-    const uint32_t lane = G::rank();
-    nend = 0;
-    for (uint32_t base = 0; base < c; base += 32) {
-      const uint32_t i = base + lane;
-      const bool e = i < c && m.A[i] == NONE_I;
-      const uint32_t mask = __ballot_sync(0xFFFFFFFFu, e);
-      __syncwarp();  // the reads of this chunk before any write into it
-      if (e) m.A[nend + __popc(mask & ((1u << lane) - 1u))] = IT(i);
-      nend += uint32_t(__popc(mask));
-    }
-    __syncwarp();
-  }
-  // the segment end visited at step j (NONE_I: not an end)
-  auto end_at = [&](uint32_t j) -> uint32_t {
-    if constexpr (WARP) return m.A[j];
-    else return m.A[j] == NONE_I ? j : NONE_I;
-  };
   U3 mine{0, 0, 0};
-  for (uint32_t j = G::rank(); j < nend; j += G::size()) {
-    const uint32_t i = end_at(j);
-    if (i == NONE_I) continue;
+  for (uint32_t i = G::rank(); i < c; i += G::size()) {
+    if (m.A[i] != NONE_I) continue;  // not a segment's end
     const uint32_t s = ptr[i];
     const uint32_t len = uint32_t(rnk[i]) + 1;
     const bool starts_p = (roles(skey(m, s)) & ROLE_P) != 0;
@@ -1662,9 +1882,8 @@ __device__ void process_tile(const TileParams& p, const TileMem<NW, IT>& m, uint
   // the segment before), then its line break or, for an open segment, its
   // record.  The cross indices the record needs are loaded first, so that
   // they arrive while the rest is worked out.
-  for (uint32_t j = G::rank(); j < nend; j += G::size()) {
-    const uint32_t i = end_at(j);
-    if (i == NONE_I) continue;
+  for (uint32_t i = G::rank(); i < c; i += G::size()) {
+    if (m.A[i] != NONE_I) continue;  // not a segment's end
     const uint32_t s = ptr[i];
     const Key<NW> ks = skey(m, s);
     const uint64_t re = roles(skey(m, i));
@@ -1721,6 +1940,7 @@ __device__ void process_tile(const TileParams& p, const TileMem<NW, IT>& m, uint
     char* dst = (sid == NONE_I) ? (p.out + cbase + loc) : (p.segchars + obase + loc);
     dst[(sid == OPEN_S ? 0u : uint32_t(k)) + r - 1] = acgt(key_char(skey(m, i), k - 1));
   }
+  }  // (block tiles)
 }
 
 // Persistent tile kernels.  Warp tiles (<= warp capacity copies): every warp
@@ -1729,7 +1949,7 @@ __device__ void process_tile(const TileParams& p, const TileMem<NW, IT>& m, uint
 // the tile capacity): the whole CTA works one tile.  Larger tiles go to
 // k_tile_big.
 template <int NW, int KC>
-__global__ void __launch_bounds__(256) k_tile_warp(TileParams p) {
+__global__ void __launch_bounds__(256, NW == 1 ? 4 : 3) k_tile_warp(TileParams p) {
   extern __shared__ __align__(16) char smem[];
   const uint32_t wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const TileMem<NW, uint16_t> m = carve<NW, uint16_t>(smem + size_t(wid) * p.wbytes, p.wcap, p.wts);
@@ -2978,7 +3198,7 @@ int minimizers(Env& e, const uint64_t* d_keys, uint64_t n, int k, int l, uint64_
 // sizes jb, and njobs << jb buckets in all (rounded up to a power of two,
 // bits = log2 of that).
 struct Plan {
-  uint32_t bits, jb, cap, pack, tslots, wcap, wts, wbytes, lf;
+  uint32_t bits, jb, cap, pack, tslots, wcap, wts, wbytes, lf, wlf;
   uint32_t cg;  // the pack's count groups: 2^cg buckets each
   int l_used;
   uint64_t M;
@@ -3016,15 +3236,30 @@ static Plan plan_buckets(const Env& e, uint64_t nmax, uint32_t njobs, int k, int
   } else {
     // about bucket_fill buckets per tile: small enough that tiles pack well,
     // large enough that each bucket gathers several l-mers
-    const uint32_t fill = e.tune.bucket_fill ? e.tune.bucket_fill : 8;
+    // (256 Mbp, k = 31: 4 per tile of 256 copies takes the bucket phase from
+    // 7.85 to 7.5 ms against 8, with 2% more tiles; 200 Mbp stays below the
+    // count groups that way)
+    const uint32_t fill = e.tune.bucket_fill ? e.tune.bucket_fill : 4;
     while ((copies >> jb) > std::max<uint32_t>(1, pack_cap / fill) && jb < 25) ++jb;
   }
   jb = std::min(jb, jbits_max);
-  // enough l-mers that each bucket gathers several of them
-  const int lmin = int((jb + 2 + 1) / 2);
+  // enough l-mers that each bucket gathers several of them, and that the most
+  // taken l-mer (the lowest priority: every k-mer that holds it) brings at
+  // most about 20 k-mers in a uniform genome, some hundreds at 30% GC, so that
+  // few buckets outgrow a warp tile.  Longer ones only add cross k-mers.
+  // Tile kernels at the l of the first rule and of both: 13M k-mers, k = 47,
+  // 30% GC, l = 11 and 14: 0.83 and 0.61 ms; 66M, k = 63, l = 12 and 14: 3.66
+  // and 3.32; 257M, k = 31, l = 13 and 14: 9.27 and 8.86 (15: the whole job is
+  // as long as at 13).
+  int lmin = int((jb + 2 + 1) / 2);
+  while (lmin < std::min(16, k - 1) && 20.0 * std::ldexp(1.0, 2 * lmin) < double(nmax) * double(k - lmin)) ++lmin;
   int lu = std::max(l, lmin);
   lu = std::min(lu, std::min(16, k - 1));
+  // hash slots per 100 copies: 300 for warp tiles (a table of 1024 slots at 218
+  // copies; a warp's probes end with its longest one: 257M k-mers, k = 31, 8.7
+  // ms at 200 and 7.5 at 300), 200 for block tiles (two of them per SM)
   const uint32_t lf = e.tune.load_factor_pct ? e.tune.load_factor_pct : 200;
+  const uint32_t wlf = e.tune.load_factor_pct ? e.tune.load_factor_pct : 300;
   uint32_t ts = big_slots(cap, lf);
   while (ts > pow2_at_least(2ull * cap) && tile_bytes(nw, cap, ts) > size_t(e.smem_optin)) ts >>= 1;
   P.jb = jb;
@@ -3033,12 +3268,13 @@ static Plan plan_buckets(const Env& e, uint64_t nmax, uint32_t njobs, int k, int
   P.pack = pack_cap;
   P.tslots = ts;
   P.wcap = warp_tier ? wcap : 0;
-  uint32_t wts = warp_tier ? big_slots(wcap, lf) : 0;
+  uint32_t wts = warp_tier ? big_slots(wcap, wlf) : 0;
   // eight warp tiles share a CTA's shared memory
   while (warp_tier && wts > pow2_at_least(2ull * wcap) && 8 * tile_bytes(nw, wcap, wts) > size_t(e.smem_optin))
     wts >>= 1;
   P.wts = wts;
   P.lf = lf;
+  P.wlf = wlf;
   P.wbytes = warp_tier ? uint32_t((tile_bytes(nw, wcap, P.wts) + 15) & ~size_t(15)) : 0;
   P.l_used = lu;
   P.M = 1ull << P.bits;
@@ -3449,6 +3685,7 @@ int find_edges(Env& e, const uint64_t* d_keys, uint64_t n, int k, int l, uint64_
   tp.cap = P.cap;
   tp.tslots = P.tslots;
   tp.lf = P.lf;
+  tp.wlf = P.wlf;
   tp.wcap = P.wcap;
   tp.wts = P.wts;
   tp.wbytes = P.wbytes;
@@ -4155,6 +4392,7 @@ int compact_batch(Env& e, uint32_t njobs, const char* const* texts, const size_t
   tp.cap = P.cap;
   tp.tslots = P.tslots;
   tp.lf = P.lf;
+  tp.wlf = P.wlf;
   tp.wcap = P.wcap;
   tp.wts = P.wts;
   tp.wbytes = P.wbytes;
@@ -4444,6 +4682,7 @@ int compact_streamed(Env& e, const char* h_text, size_t bytes, int k, int l, cha
   tp.cap = P.cap;
   tp.tslots = P.tslots;
   tp.lf = P.lf;
+  tp.wlf = P.wlf;
   tp.wcap = P.wcap;
   tp.wts = P.wts;
   tp.wbytes = P.wbytes;

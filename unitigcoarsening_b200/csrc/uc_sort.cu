@@ -474,89 +474,37 @@ __global__ void __launch_bounds__(256) k_line_keep(const char* __restrict__ out,
   }
 }
 
-// The line's bytes (k-mer, tail, line break) at shared-memory position pos of
-// buf: whole words where the line owns them, halves and bytes at its two ends
-// (shared with the neighbouring lines).
+// The line (k-mer, tail, break) at shared-memory position pos of buf.
 template <int RW>
 __device__ __forceinline__ void spell_line(uint32_t* buf, uint32_t pos, const Rec<RW>& r, int k) {
   const uint32_t t = uint32_t(r.tail >> TAIL_LEN_SHIFT) & 31u;
   const uint64_t codes = r.tail & ((1ull << TAIL_LEN_SHIFT) - 1ull);
-  // the code stream, first char lowest, moved up by the chars before the
-  // line in its first word
-  const uint32_t a = pos & 3u;
   constexpr int NC = RW == 2 ? 4 : 6;
-  uint32_t c[NC];
-  {
-    uint64_t w[3];
-    w[0] = rev2(r.hi);
-    w[1] = w[2] = 0;
-    if constexpr (RW == 2) {
-      w[0] |= codes << (2 * k);
-      w[1] = codes >> (64 - 2 * k);
-    } else {
-      const int u = 2 * k - 64;
-      w[1] = rev2(r.lo) | (codes << u);
-      w[2] = u ? codes >> (64 - u) : 0ull;
-    }
-    uint32_t x[NC];
-#pragma unroll
-    for (int q = 0; q < NC; ++q) x[q] = uint32_t(w[q >> 1] >> (32 * (q & 1)));
-    c[0] = x[0] << (2 * a);
-#pragma unroll
-    for (int q = 1; q < NC; ++q) c[q] = __funnelshift_l(x[q - 1], x[q], 2 * a);
-  }
-  const uint32_t last = a + uint32_t(k) + t;        // place of the break, from the first word's start
-  const uint32_t nw = last >> 2, rem = last & 3u;   // its word, and the chars before it there
-  uint32_t* d = buf + (pos >> 2);
-  uint32_t first = 0, tailw = 0;
-#pragma unroll
-  for (int g = 0; g < NC; ++g) {
-    if (4u * g > nw) break;
-    uint32_t w[4];
-    letters16(c[g], w);
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const uint32_t j = 4u * g + q;
-      if (j == nw) tailw = w[q];
-      if (j < nw && (j > 0 || a == 0)) d[j] = w[q];
-    }
-    if (g == 0) first = w[0];
-  }
-  const uint32_t v = (tailw & ((1u << (8 * rem)) - 1u)) | (uint32_t('\n') << (8 * rem));
-  char* e = reinterpret_cast<char*>(d + nw);
-  if (nw == 0 && a) {  // a line inside one word (k < 3)
-    for (uint32_t q = a; q <= rem; ++q) e[q] = char(v >> (8 * q));
-    return;
-  }
-  if (rem == 3) {
-    d[nw] = v;
+  uint64_t w[3];
+  w[0] = rev2(r.hi);
+  w[1] = w[2] = 0;
+  if constexpr (RW == 2) {
+    w[0] |= codes << (2 * k);
+    w[1] = codes >> (64 - 2 * k);
   } else {
-    if (rem) *reinterpret_cast<uint16_t*>(e) = uint16_t(v);
-    if (rem != 1) e[rem] = '\n';
+    const int u = 2 * k - 64;
+    w[1] = rev2(r.lo) | (codes << u);
+    w[2] = u ? codes >> (64 - u) : 0ull;
   }
-  if (a) {
-    char* f = reinterpret_cast<char*>(d);
-    if (a & 1u) f[a] = char(first >> (8 * a));
-    if (a < 3) *reinterpret_cast<uint16_t*>(f + 2) = uint16_t(first >> 16);
-  }
+  uint32_t x[NC];
+#pragma unroll
+  for (int q = 0; q < NC; ++q) x[q] = uint32_t(w[q >> 1] >> (32 * (q & 1)));
+  spell_text<NC>(buf, pos, x, uint32_t(k) + t, 1u);
 }
 
 // Stores the lines of ranks [r0, r1) of one warp, the first at byte `at` of
-// the sorted text: 32 lines at a time are spelled into the warp's buffer and
-// leave as 16-byte stores; the up to 15 bytes after the last one stay for the
-// next 32 lines.  get(r) gives the record of rank r.
+// the sorted text, 32 lines at a time.  get(r) gives the record of rank r.
 template <int RW, class Get>
 __device__ __forceinline__ void store_lines(char* out, uint64_t at, uint32_t r0, uint32_t r1, int k, uint32_t* buf,
                                             LongLine* longs, const char* keep, Get get) {
   const uint32_t lane = threadIdx.x & 31u;
-  char* bb = reinterpret_cast<char*>(buf);
-  char* dst = out + at;                       // next byte of the sorted text
-  uint32_t fill = uint32_t(reinterpret_cast<uintptr_t>(dst) & 15u);  // bytes of buf before it
-  uint32_t head = fill;                       // of which another warp's
-  auto flush_rest = [&] {
-    if (lane >= head && lane < fill) (dst - fill)[lane] = bb[lane];
-    __syncwarp();
-  };
+  WarpText T;
+  T.begin(out + at);
   for (uint32_t base = r0; base < r1; base += 32) {
     const bool live = base + lane < r1;
     Rec<RW> r{0ull, 0ull, 0ull};
@@ -564,7 +512,7 @@ __device__ __forceinline__ void store_lines(char* out, uint64_t at, uint32_t r0,
     const bool is_long = live && (r.tail & TAIL_LONG);
     const unsigned long long len = live ? line_bytes_of(r.tail, k, longs) : 0ull;
     if (__any_sync(0xFFFFFFFFu, is_long)) {
-      flush_rest();
+      T.end(buf);
       unsigned long long inc = len;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
@@ -574,7 +522,7 @@ __device__ __forceinline__ void store_lines(char* out, uint64_t at, uint32_t r0,
       const unsigned long long total = __shfl_sync(0xFFFFFFFFu, inc, 31);
       if (live && !is_long) {
         // into the lane's own part of the buffer, then byte by byte
-        char* p = dst + (inc - len);
+        char* p = T.dst + (inc - len);
         uint32_t* mine = buf + lane * ((uint32_t(k) + TAIL_MAX + 4u) >> 2);
         spell_line<RW>(mine, 0u, r, k);
         for (uint32_t q = 0; q < uint32_t(len); ++q) p[q] = reinterpret_cast<char*>(mine)[q];
@@ -586,14 +534,13 @@ __device__ __forceinline__ void store_lines(char* out, uint64_t at, uint32_t r0,
         const uint32_t i = uint32_t(__shfl_sync(0xFFFFFFFFu, r.tail, q));
         const unsigned long long n = __shfl_sync(0xFFFFFFFFu, len, q);
         const unsigned long long o = __shfl_sync(0xFFFFFFFFu, inc - len, q);
-        char* p = dst + o;
+        char* p = T.dst + o;
         const unsigned long long src = longs[i].at;
         if (n < HUGE_LINE) copy_bytes(p, keep + src, n, lane, 32u);
         else if (lane == 0) longs[i].to = uint64_t(p - out);  // copied by k_huge_lines
       }
       __syncwarp();
-      dst += total;
-      fill = head = uint32_t(reinterpret_cast<uintptr_t>(dst) & 15u);
+      T.begin(T.dst + total);
       continue;
     }
     uint32_t inc = uint32_t(len);
@@ -603,27 +550,11 @@ __device__ __forceinline__ void store_lines(char* out, uint64_t at, uint32_t r0,
       if (lane >= uint32_t(o)) inc += v;
     }
     const uint32_t total = __shfl_sync(0xFFFFFFFFu, inc, 31);
-    if (live) spell_line<RW>(buf, fill + inc - uint32_t(len), r, k);
+    if (live) spell_line<RW>(buf, T.fill + inc - uint32_t(len), r, k);
     __syncwarp();
-    const uint32_t full = (fill + total) >> 4, rem = (fill + total) & 15u;
-    char* w = dst - fill;
-    for (uint32_t p = lane; p < full; p += 32) {
-      if (p == 0 && head) {
-        for (uint32_t q = head; q < 16; ++q) w[q] = bb[q];
-      } else {
-        reinterpret_cast<uint4*>(w)[p] = reinterpret_cast<const uint4*>(buf)[p];
-      }
-    }
-    __syncwarp();
-    if (full) {
-      if (lane < 4) buf[lane] = buf[4 * full + lane];
-      head = 0;
-    }
-    __syncwarp();
-    dst += total;
-    fill = rem;
+    T.flush(buf, total);
   }
-  flush_rest();
+  T.end(buf);
 }
 
 // Stable order of n records of one tile too large for shared memory, by one
