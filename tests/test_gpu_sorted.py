@@ -69,3 +69,22 @@ def test_line_lengths(comp, oracle, k, lengths):
 def test_small_k(comp, oracle, k):
     kmers = sorted(set(walk_kmers(random_seq(40 * 4 ** min(k, 5) // 10 + k, 9), k)))
     check(comp, oracle, text_of(shuffled(kmers, 1)), k, shift=1)
+
+
+@pytest.mark.parametrize("k", [31, 63])
+@pytest.mark.parametrize("tuning", [dict(warp_capacity=1), dict(warp_capacity=32), dict(warp_capacity=1024),
+                                    dict(tile_capacity=256, bucket_fill=1), dict(load_factor_pct=150),
+                                    dict(contract_method=1)])
+def test_lines_from_every_tier(comp, oracle, k, tuning):
+    """Lines that come as records (warp tiles), as text (block and oversized
+    tiles, stitched lines) and both, with cycles among them."""
+    from tests.cases import cyclic_kmers
+    kmers = []
+    for i, m in enumerate([k, k + 1, k + 3, k + 28, k + 29, k + 30, 400] * 300):
+        kmers += walk_kmers(random_seq(m, 5000 * k + i), k)
+    kmers += cyclic_kmers(k + 40, k, seed=2) + cyclic_kmers(300, k, seed=8)
+    comp.set_tuning(**tuning)
+    try:
+        check(comp, oracle, text_of(shuffled(kmers, 4)), k, shift=9)
+    finally:
+        comp.set_tuning(**{f: 0 for f in tuning})

@@ -9,22 +9,70 @@
 namespace uc {
 
 // Device-side counters of one pipeline run (one allocation, zeroed per run).
+// Atomics on words of one 128-byte line queue up in L2 (about 2 ns each), so
+// the counters that every tile adds to have lines of their own: with all of
+// them in one line, 1.24M warp tiles with four atomics each took 9.7 ms.
 struct Counters {
-  unsigned long long out_cursor;     // bytes of finished lines written
-  unsigned long long seg_char_cursor;
-  unsigned long long n_copies;
+  alignas(128) unsigned long long seg_char_cursor;
+  // lines the tiles left as records (low half) and head-pool ids taken (high
+  // half), in sorted output
+  alignas(128) unsigned long long rec_slots;
+  alignas(128) uint32_t wtile_next;
+  alignas(128) unsigned long long rec_bytes;  // the records' lines
   unsigned long long cycles;
-  uint32_t seg_count;
   uint32_t cross_count;
   uint32_t ntiles;
   uint32_t tile_next;
   uint32_t nbig;
-  uint32_t active;                   // stitch: active list length
-  uint32_t active_next;
   uint32_t err;
-  uint32_t work_next;                // level-2 scatter work counter
+  uint32_t work_next;                // scatter work counter
   uint32_t nwarp, nblock;            // tiles per tier
-  uint32_t wtile_next;
+};
+
+// A line as a record (sorted output): its k-mer big-endian (first char in the
+// top bits of hi, chars 32.. in lo), so that numeric order is byte order, and a
+// tail word: the chars after the k-mer as codes (first one lowest) under their
+// count, or, with TAIL_LONG, the index of a line kept as text.  Two words (hi,
+// tail) for k <= 31, three otherwise; the first two lie together.
+constexpr int TAIL_MAX = 28;
+constexpr uint64_t TAIL_LONG = 1ull << 63;
+constexpr int TAIL_LEN_SHIFT = 58;
+template <int RW>
+struct Rec {
+  uint64_t hi, lo, tail;
+};
+template <int RW>
+struct RecArr {
+  ulonglong2* a;
+  unsigned long long* t;  // tails (RW == 3)
+};
+template <int RW>
+__device__ __forceinline__ Rec<RW> ld_rec(const RecArr<RW>& r, uint64_t i) {
+  const ulonglong2 v = r.a[i];
+  if constexpr (RW == 2) return Rec<RW>{v.x, 0ull, v.y};
+  else return Rec<RW>{v.x, v.y, r.t[i]};
+}
+template <int RW>
+__device__ __forceinline__ void st_rec(const RecArr<RW>& r, uint64_t i, const Rec<RW>& x) {
+  if constexpr (RW == 2) {
+    r.a[i] = make_ulonglong2(x.hi, x.tail);
+  } else {
+    r.a[i] = make_ulonglong2(x.hi, x.lo);
+    r.t[i] = x.tail;
+  }
+}
+
+// Lines the tiles left as records: the records (rec_bytes bytes of lines), a
+// second array as large, and a count per bin of the key's leading bits.  The
+// arrays lie in the back arena below `used`.
+struct LineRecs {
+  char *a = nullptr, *b = nullptr;
+  uint64_t cap = 0;  // records either array holds
+  uint32_t* counts = nullptr;
+  int bits = 0;
+  uint32_t n = 0;
+  uint64_t bytes = 0;
+  size_t used = 0;
 };
 
 // One open segment of the fused path (written by the tile that finds it): the
@@ -87,6 +135,12 @@ struct TileParams {
   uint32_t seg_cap;
   SegRec* seg;                  // open segments by id
   uint32_t xcount;              // cross k-mers (the head pool starts there)
+  // sorted output: closed lines of warp tiles leave as records (rec_a null:
+  // all lines as text)
+  ulonglong2* rec_a;
+  unsigned long long* rec_t;
+  uint32_t* rec_counts;
+  int rec_bits;
 };
 
 // Shared memory of one tile: keys plus four 16-bit arrays per copy (sized

@@ -1335,7 +1335,9 @@ __device__ __forceinline__ int reserve_space(const TileParams& p, uint32_t job, 
   const JobTab& J = p.jobs[job];
   b[0] = tot.a ? atomicAdd(p.jout + job, tot.a) : 0ull;
   b[1] = tot.b ? atomicAdd(&p.ctr->seg_char_cursor, tot.b) : 0ull;
-  b[2] = tot.c ? atomicAdd(p.jseg + job, uint32_t(tot.c)) : 0u;
+  b[2] = !tot.c ? 0u
+         : p.rec_a ? atomicAdd(&p.ctr->rec_slots, tot.c << 32) >> 32
+                   : (unsigned long long)atomicAdd(p.jseg + job, uint32_t(tot.c));
   if (b[0] + tot.a > J.ocap || b[1] + tot.b > p.segchars_cap || b[2] + tot.c > J.seg_cap) {
     atomicOr(&p.ctr->err, ERR_CAPACITY);
     return 0;
@@ -1437,11 +1439,11 @@ __device__ void jump_rounds(uint32_t c, IT* px, IT* rx, IT* py, IT* ry, IT*& ptr
 // and leaves as 16-byte stores.  Against ranking the copies by pointer jumping
 // and storing each copy's char by itself: 64 Mbp, k = 63, the kernel takes
 // 2.36 instead of 3.01 ms; at k = 31 it is as long (8.7 ms at 256 Mbp), with
-// half as many stores.
-constexpr uint32_t TAIL_CODES = 28;  // later chars a lane keeps as codes; longer segments store byte by byte
+// half as many stores.  Segments with more than TAIL_MAX later chars store
+// them byte by byte.
 template <int NW, int KC>
 __device__ __forceinline__ void emit_warp_tile(const TileParams& p, const TileMem<NW, uint16_t>& m, uint64_t beg,
-                                               uint32_t c, uint32_t job) {
+                                               uint32_t c, uint32_t job, unsigned long long& rec_bytes) {
   constexpr uint32_t NONE_I = Ix<uint16_t>::NONE;
   const int k = KC ? KC : p.k;
   const uint32_t lane = threadIdx.x & 31u, below = (1u << lane) - 1u;
@@ -1458,9 +1460,10 @@ __device__ __forceinline__ void emit_warp_tile(const TileParams& p, const TileMe
   // sizes; the closed segments' ends to the front of A, the open ones' to its
   // back (the successors are used up: cycles are found from P)
   uint32_t nclosed, nopen, heads, cbytes, obytes;
+  bool longer;  // a closed line with more later chars than a record holds
   for (bool cut = false;; cut = true) {
     nclosed = nopen = 0;
-    uint32_t h = 0, cb = 0, ob = 0, covered = 0;
+    uint32_t h = 0, cb = 0, ob = 0, covered = 0, lmax = 0;
     for (uint32_t base = 0; base < nend; base += 32) {
       const bool live = base + lane < nend;
       uint32_t i = 0, s = 0, len = 0;
@@ -1477,6 +1480,7 @@ __device__ __forceinline__ void emit_warp_tile(const TileParams& p, const TileMe
         covered += len;
         if (closed) {
           cb += uint32_t(k) + len;
+          lmax = max(lmax, len);
         } else {
           ob += starts_p ? uint32_t(k) - 1u + len : len - 1u;
           h += starts_p ? 1u : 0u;
@@ -1492,6 +1496,7 @@ __device__ __forceinline__ void emit_warp_tile(const TileParams& p, const TileMe
     heads = __reduce_add_sync(0xFFFFFFFFu, h);
     cbytes = __reduce_add_sync(0xFFFFFFFFu, cb);
     obytes = __reduce_add_sync(0xFFFFFFFFu, ob);
+    longer = __any_sync(0xFFFFFFFFu, lmax > uint32_t(TAIL_MAX) + 1u);
     if (covered == c || cut) break;
     // local cycles hold the copies no end reaches (rare): one lane cuts each
     // before its smallest key, which then starts a segment
@@ -1516,9 +1521,53 @@ __device__ __forceinline__ void emit_warp_tile(const TileParams& p, const TileMe
     nend = __shfl_sync(0xFFFFFFFFu, nend, 0);
     __syncwarp();
   }
-  unsigned long long at[3];
-  if (!WarpGroup::reserve(p, job, U3{cbytes, obytes, heads}, at)) return;
-  __syncwarp();
+  // sorted output: the closed lines leave as records (unless one is too long)
+  const bool recs = p.rec_a != nullptr && !longer;
+  unsigned long long at[3] = {0, 0, 0};
+  if (recs) {
+    unsigned long long v = 0;
+    uint32_t ok = 1;
+    if (lane == 0) {
+      if (nclosed | heads) v = atomicAdd(&p.ctr->rec_slots, (static_cast<unsigned long long>(heads) << 32) | nclosed);
+      if (obytes) at[1] = atomicAdd(&p.ctr->seg_char_cursor, (unsigned long long)obytes);
+      if (at[1] + obytes > p.segchars_cap || (v >> 32) + heads > p.jobs[job].seg_cap) {
+        atomicOr(&p.ctr->err, ERR_CAPACITY);
+        ok = 0;
+      }
+    }
+    v = __shfl_sync(0xFFFFFFFFu, v, 0);
+    at[1] = __shfl_sync(0xFFFFFFFFu, at[1], 0);
+    if (!__shfl_sync(0xFFFFFFFFu, ok, 0)) return;
+    at[2] = (v >> 32) + p.jobs[job].seg_base;
+    rec_bytes += cbytes;
+    const uint32_t slot = uint32_t(v);
+    __syncwarp();
+    const RecArr<NW + 1> out{p.rec_a, p.rec_t};
+    for (uint32_t j = lane; j < nclosed; j += 32) {
+      uint32_t s = m.A[j], len = 1;
+      uint64_t tail = 0;
+      for (uint32_t q = m.P[s]; q != NONE_I && len < c; q = m.P[s]) {
+        tail = (tail << 2) | key_char(skey(m, s), k - 1);
+        s = q;
+        ++len;
+      }
+      const Key<NW> x = strip(skey(m, s));
+      Rec<NW + 1> r;
+      if constexpr (NW == 1) {
+        r.hi = rev2(x.w[0]);
+        r.lo = 0;
+      } else {
+        r.hi = rev2(x.w[0]);
+        r.lo = rev2(x.w[1]);
+      }
+      r.tail = (uint64_t(len - 1u) << TAIL_LEN_SHIFT) | tail;
+      atomicAdd(p.rec_counts + (r.hi >> (64 - p.rec_bits)), 1u);
+      st_rec<NW + 1>(out, uint64_t(slot) + j, r);
+    }
+  } else {
+    if (!WarpGroup::reserve(p, job, U3{cbytes, obytes, heads}, at)) return;
+    __syncwarp();
+  }
   // text buffer: the arrays Q and T, less the piece that WarpText::flush may
   // read past the text (room for one line is left in the smallest tile: 32
   // copies have 192 bytes there)
@@ -1529,7 +1578,7 @@ __device__ __forceinline__ void emit_warp_tile(const TileParams& p, const TileMe
   uint32_t head0 = p.xcount + uint32_t(at[2]);  // id of the next segment that starts a line
   constexpr int NC = NW == 1 ? 4 : 6;
 #pragma unroll 1
-  for (uint32_t open = 0; open < 2; ++open) {
+  for (uint32_t open = recs ? 1u : 0u; open < 2; ++open) {
     const uint32_t nseg = open ? nopen : nclosed;
     WarpText T;
     T.begin(open ? p.segchars + at[1] : p.out + at[0]);
@@ -1567,7 +1616,7 @@ __device__ __forceinline__ void emit_warp_tile(const TileParams& p, const TileMe
         const uint32_t v = __shfl_up_sync(0xFFFFFFFFu, inc, o);
         if (lane >= uint32_t(o)) inc += v;
       }
-      const bool direct = __any_sync(0xFFFFFFFFu, len > TAIL_CODES + 1u);
+      const bool direct = __any_sync(0xFFFFFFFFu, len > uint32_t(TAIL_MAX) + 1u);
       // the lanes whose text fits the buffer (all of them when it is not used)
       const bool take = live && (direct || T.fill + inc <= room);
       const uint32_t taken = __ballot_sync(0xFFFFFFFFu, take);
@@ -1635,7 +1684,7 @@ __device__ __forceinline__ void emit_warp_tile(const TileParams& p, const TileMe
 // spelling loops of the common shapes are constants.
 template <int NW, typename IT, typename G, int KC = 0>
 __device__ void process_tile(const TileParams& p, const TileMem<NW, IT>& m, uint64_t beg, uint32_t c,
-                             uint32_t job) {
+                             uint32_t job, unsigned long long& rec_bytes) {
   constexpr uint32_t NONE_I = Ix<IT>::NONE, DUP_I = Ix<IT>::DUP, CNONE_I = Ix<IT>::CNONE;
   constexpr uint32_t OPEN_S = NONE_I - 1u;  // an open segment that starts at an S-only copy
   constexpr bool WARP = std::is_same<G, WarpGroup>::value;
@@ -1791,7 +1840,7 @@ __device__ void process_tile(const TileParams& p, const TileMem<NW, IT>& m, uint
     return;
   }
   if constexpr (WARP) {
-    emit_warp_tile<NW, KC>(p, m, beg, c, job);
+    emit_warp_tile<NW, KC>(p, m, beg, c, job, rec_bytes);
     return;
   } else {
   // ---- local segments: list ranking by pointer jumping
@@ -1953,20 +2002,20 @@ __global__ void __launch_bounds__(256, NW == 1 ? 4 : 3) k_tile_warp(TileParams p
   extern __shared__ __align__(16) char smem[];
   const uint32_t wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const TileMem<NW, uint16_t> m = carve<NW, uint16_t>(smem + size_t(wid) * p.wbytes, p.wcap, p.wts);
-  const uint32_t nt = p.ctr->nwarp;
-  uint32_t j = 0;
-  if (lane == 0) j = atomicAdd(&p.ctr->wtile_next, 1u);
-  j = __shfl_sync(0xFFFFFFFFu, j, 0);
+  const uint32_t nt = p.ctr->nwarp, nw = gridDim.x * (blockDim.x >> 5);
+  unsigned long long rec_bytes = 0;
+  uint32_t j = blockIdx.x * (blockDim.x >> 5) + wid;  // the first tile needs no counter
   while (j < nt) {
     uint32_t jn = 0;  // the next tile's index is in flight while this tile is worked
-    if (lane == 0) jn = atomicAdd(&p.ctr->wtile_next, 1u);
+    if (lane == 0) jn = nw + atomicAdd(&p.ctr->wtile_next, 1u);
     const uint32_t t = p.wlist[j];
     const uint64_t beg = p.tile_begin[t];
     const uint32_t c = uint32_t(p.tile_begin[t + 1] - beg);
-    process_tile<NW, uint16_t, WarpGroup, KC>(p, m, beg, c, p.tile_job[t]);
+    process_tile<NW, uint16_t, WarpGroup, KC>(p, m, beg, c, p.tile_job[t], rec_bytes);
     __syncwarp();
     j = __shfl_sync(0xFFFFFFFFu, jn, 0);
   }
+  if (lane == 0 && rec_bytes) atomicAdd(&p.ctr->rec_bytes, rec_bytes);
 }
 
 template <int NW, int KC>
@@ -1984,7 +2033,8 @@ __global__ void __launch_bounds__(512) k_tile(TileParams p) {
     const uint32_t t = p.blist[j];
     const uint64_t beg = p.tile_begin[t];
     const uint32_t c = uint32_t(p.tile_begin[t + 1] - beg);
-    process_tile<NW, uint16_t, BlockGroup, KC>(p, m, beg, c, p.tile_job[t]);
+    unsigned long long none = 0;
+    process_tile<NW, uint16_t, BlockGroup, KC>(p, m, beg, c, p.tile_job[t], none);
     __syncthreads();
   }
 }
@@ -1997,7 +2047,8 @@ __global__ void __launch_bounds__(1024) k_tile_big(TileParams p) {
   const uint64_t c = p.tile_begin[t + 1] - beg;
   const uint32_t ts = big_slots(c, p.lf);
   const TileMem<NW, uint32_t> m = carve<NW, uint32_t>(p.big_scratch + p.big_off[blockIdx.x], uint32_t(c), ts);
-  process_tile<NW, uint32_t, BlockGroup>(p, m, beg, uint32_t(c), p.tile_job[t]);
+  unsigned long long none = 0;
+  process_tile<NW, uint32_t, BlockGroup>(p, m, beg, uint32_t(c), p.tile_job[t], none);
 }
 
 // ================================================================= stitch
@@ -2039,10 +2090,10 @@ __device__ __forceinline__ uint32_t block_append(uint32_t* count, uint32_t c, ui
 
 // X[v] = (start pointer, weight distance); heads point at themselves.
 __global__ void __launch_bounds__(256) k_rank_init(const uint32_t* __restrict__ prev, const uint32_t* __restrict__ w,
-                            uint64_t n, const Counters* ctr, unsigned long long* __restrict__ X,
+                            uint64_t n, unsigned long long* __restrict__ X,
                             uint32_t* __restrict__ act, uint32_t* act_count) {
   __shared__ uint32_t sc[33];
-  const uint64_t N = ctr ? uint64_t(ctr->seg_count) : n;
+  const uint64_t N = n;
   const uint64_t stride = uint64_t(gridDim.x) * blockDim.x;
   // whole blocks iterate together (block_append needs every thread)
   for (uint64_t s0 = uint64_t(blockIdx.x) * blockDim.x; s0 < N; s0 += stride) {
@@ -2576,8 +2627,8 @@ struct HecPool {
 };
 
 __global__ void k_hec_level0(HecPool h, const uint32_t* __restrict__ prev, const uint32_t* __restrict__ next,
-                             const uint32_t* __restrict__ w, uint64_t n, const Counters* nctr) {
-  const uint64_t N = nctr ? uint64_t(nctr->seg_count) : n;
+                             const uint32_t* __restrict__ w, uint64_t n) {
+  const uint64_t N = n;
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     h.lb[0] = 0;
     h.ln[0] = uint32_t(N);
@@ -2782,9 +2833,9 @@ __global__ void k_hec_emit(HecPool h, unsigned long long* __restrict__ X, uint8_
   }
 }
 
-__global__ void k_cycle_list(const uint8_t* __restrict__ oncycle, uint64_t n, const Counters* nctr,
+__global__ void k_cycle_list(const uint8_t* __restrict__ oncycle, uint64_t n,
                              uint32_t* __restrict__ act, uint32_t* __restrict__ cnt) {
-  const uint64_t N = nctr ? uint64_t(nctr->seg_count) : n;
+  const uint64_t N = n;
   for (uint64_t s = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; s < N; s += uint64_t(gridDim.x) * blockDim.x)
     if (oncycle[s]) act[atomicAdd(cnt, 1u)] = uint32_t(s);
 }
@@ -2926,6 +2977,26 @@ int Env::reserve(int w, size_t bytes) {
     return fail(UC_ENOMEM, "cudaMalloc of " + std::to_string(bytes >> 20) + " MiB failed");
   }
   a.cap = bytes;
+  return UC_OK;
+}
+
+int Env::big_scratch(size_t bytes, char*& p, const char* what) {
+  if (bytes > big_cap) {
+    if (big_buf) {
+      cudaStreamSynchronize(stream);
+      cudaFree(big_buf);
+    }
+    big_buf = nullptr;
+    big_cap = 0;
+    if (bytes > budget) return fail(UC_EBUDGET, what);
+    if (dev_malloc(reinterpret_cast<void**>(&big_buf), bytes) != cudaSuccess) {
+      cudaGetLastError();
+      big_buf = nullptr;
+      return fail(UC_ENOMEM, what);
+    }
+    big_cap = bytes;
+  }
+  p = big_buf;
   return UC_OK;
 }
 
@@ -3076,10 +3147,12 @@ static JobDev job_dev(Env& e, uint32_t njobs) {
   JobDev d;
   d.tab = reinterpret_cast<JobTab*>(e.jbuf);
   char* q = e.jbuf + ((size_t(njobs) * sizeof(JobTab) + 255) & ~size_t(255));
+  // (jout and jseg, which every tile adds to, in L2 lines of their own)
+  auto line = [](void* p) { return reinterpret_cast<char*>((reinterpret_cast<uintptr_t>(p) + 127) & ~uintptr_t(127)); };
   d.jout = reinterpret_cast<unsigned long long*>(q);
-  d.jclosed = d.jout + njobs;
+  d.jseg = reinterpret_cast<uint32_t*>(line(d.jout + njobs));
+  d.jclosed = reinterpret_cast<unsigned long long*>(line(d.jseg + njobs));
   d.jcross = reinterpret_cast<uint32_t*>(d.jclosed + njobs);
-  d.jseg = d.jcross + njobs;
   return d;
 }
 
@@ -3606,22 +3679,10 @@ static int run_tiles(Env& e, TileParams& tp, const Front& f, uint32_t threads) {
     if (e.pool) {
       big = static_cast<char*>(e.take(1, want));
       if (!big) return e.fail(UC_EBUDGET, "scratch for oversized buckets exceeds the pool slice");
-    } else if (want > e.big_cap) {
-      if (e.big_buf) {
-        cudaStreamSynchronize(e.stream);
-        cudaFree(e.big_buf);
-      }
-      e.big_buf = nullptr;
-      e.big_cap = 0;
-      if (want > e.budget) return e.fail(UC_EBUDGET, "scratch for oversized buckets");
-      if (e.dev_malloc(reinterpret_cast<void**>(&e.big_buf), want) != cudaSuccess) {
-        cudaGetLastError();
-        e.big_buf = nullptr;
-        return e.fail(UC_ENOMEM, "scratch for oversized buckets");
-      }
-      e.big_cap = want;
+    } else {
+      const int r = e.big_scratch(want, big, "scratch for oversized buckets");
+      if (r) return r;
     }
-    if (!big) big = e.big_buf;
     unsigned long long* d_off = reinterpret_cast<unsigned long long*>(big);
     char* scratch = big + ((size_t(nbig) * 8 + 255) & ~size_t(255));
     UC_CK(cudaMemcpyAsync(d_off, off.data(), nbig * 8, cudaMemcpyHostToDevice, e.stream));
@@ -3761,7 +3822,7 @@ static int run_graph(Env& e, int slot, uint64_t key, F&& body) {
 // prefilled: X already holds a state (written by the tiles and the line
 // walk) and the first round runs over the ids [0, cnt[0]), cnt[0] set on the
 // device before.
-static int rank_lists(Env& e, const uint32_t* prev, const uint32_t* w, uint64_t nmax, bool count_on_device,
+static int rank_lists(Env& e, const uint32_t* prev, const uint32_t* w, uint64_t nmax,
                       unsigned long long* X, uint32_t* act0, uint32_t* act1, uint32_t* cnt, uint32_t& rounds,
                       uint32_t*& act_final, uint32_t*& cnt_final, bool prefilled = false) {
   rounds = 2;
@@ -3772,7 +3833,7 @@ static int rank_lists(Env& e, const uint32_t* prev, const uint32_t* w, uint64_t 
   } else {
     UC_CK(cudaMemsetAsync(cnt, 0, (rounds + 1) * 4, e.stream));
     ++e.launches;
-    k_rank_init<<<grid, 256, 0, e.stream>>>(prev, w, nmax, count_on_device ? e.ctr : nullptr, X, act0, cnt);
+    k_rank_init<<<grid, 256, 0, e.stream>>>(prev, w, nmax, X, act0, cnt);
   }
   uint32_t* lists[2] = {act0, act1};
   for (uint32_t r = 0; r < rounds; ++r) {
@@ -3820,13 +3881,13 @@ static uint32_t hec_rounds(const Env& e, uint64_t nmax) {
 // ranking's first state in X (built from them by k_seg_xinit; nx cross
 // indices) instead of (prev, next, w).
 static void hec_contract(Env& e, HecPool& h, uint32_t R, const uint32_t* prev, const uint32_t* next,
-                         const uint32_t* w, uint64_t nmax, bool count_on_device, unsigned long long* X,
+                         const uint32_t* w, uint64_t nmax, unsigned long long* X,
                          uint8_t* oncycle, const SegRec* seg = nullptr, uint32_t nx = 0, int k = 0) {
   const int grid = grid_for(e, nmax ? nmax : 1, 256);
   cudaMemsetAsync(h.ln, 0, (R + 1) * 4, e.stream);
   ++e.launches;
   if (seg) k_hec_level0_seg<<<grid, 256, 0, e.stream>>>(h, seg, X, nmax, nx, k);
-  else k_hec_level0<<<grid, 256, 0, e.stream>>>(h, prev, next, w, nmax, count_on_device ? e.ctr : nullptr);
+  else k_hec_level0<<<grid, 256, 0, e.stream>>>(h, prev, next, w, nmax);
   for (uint32_t r = 0; r < R; ++r) {
     e.launches += 6;
     k_hec_prep<<<grid, 256, 0, e.stream>>>(h, int(r));
@@ -3860,11 +3921,11 @@ static int contract_hec(Env& e, const uint64_t* d_keys, const uint32_t* succ, co
   if (!dcyc) return e.fail(UC_EBUDGET, "arena overflow");
   UC_CK(cudaMemsetAsync(&e.ctr->err, 0, 4, e.stream));
   UC_CK(cudaMemsetAsync(flag, 0, n, e.stream));
-  hec_contract(e, h, R, pred, succ, nullptr, n, false, X, flag);
+  hec_contract(e, h, R, pred, succ, nullptr, n, X, flag);
   e.launches += 2;
   k_head_rank<<<grid_for(e, n, 256), 256, 0, e.stream>>>(X, n, head, rank);
   UC_CK(cudaMemsetAsync(cnt, 0, 4, e.stream));
-  k_cycle_list<<<grid_for(e, n, 256), 256, 0, e.stream>>>(flag, n, nullptr, act, cnt);
+  k_cycle_list<<<grid_for(e, n, 256), 256, 0, e.stream>>>(flag, n, act, cnt);
   uint32_t hleft = 0;
   UC_CK(cudaMemcpyAsync(&hleft, cnt, 4, cudaMemcpyDeviceToHost, e.stream));
   r = e.read_ctr();
@@ -3921,7 +3982,7 @@ int contract(Env& e, const uint64_t* d_keys, const uint32_t* succ, const uint32_
   if (!dcyc) return e.fail(UC_EBUDGET, "arena overflow");
   uint32_t rounds = 0;
   uint32_t *act = nullptr, *left = nullptr;
-  r = rank_lists(e, pred, nullptr, n, false, X, a0, a1, cnt, rounds, act, left);
+  r = rank_lists(e, pred, nullptr, n, X, a0, a1, cnt, rounds, act, left);
   if (r) return r;
   ++e.launches;
   k_head_rank<<<grid_for(e, n, 256), 256, 0, e.stream>>>(X, n, head, rank);
@@ -4122,10 +4183,10 @@ static int run_stitch(Env& e, const StitchBufs& b, uint64_t X, uint64_t Hp, int 
     // HEC matching rounds, captured as one graph
     r = run_graph(e, 1, (uint64_t(RH) << 32) | uint32_t(gs), [&] {
       cudaMemsetAsync(oncyc, 0, S, e.stream);
-      hec_contract(e, hp, RH, nullptr, nullptr, nullptr, S, false, Xr, oncyc, seg, nx, k);
+      hec_contract(e, hp, RH, nullptr, nullptr, nullptr, S, Xr, oncyc, seg, nx, k);
       cudaMemsetAsync(rcnt, 0, 4, e.stream);
       ++e.launches;
-      k_cycle_list<<<gs, 256, 0, e.stream>>>(oncyc, S, nullptr, act0, rcnt);
+      k_cycle_list<<<gs, 256, 0, e.stream>>>(oncyc, S, act0, rcnt);
     });
     if (r) return r;
     act = act0;
@@ -4148,8 +4209,8 @@ static int run_stitch(Env& e, const StitchBufs& b, uint64_t X, uint64_t Hp, int 
     int rl = UC_OK;
     const bool prefilled = !want_hec;
     r = run_graph(e, 0, (uint64_t(rr) << 33) | (uint64_t(prefilled) << 32) | uint32_t(gs), [&] {
-      rl = prefilled ? rank_lists(e, nullptr, nullptr, S, false, Xr, act0, act1, rcnt, rounds, act, left, true)
-                     : rank_lists(e, hp.prv, hp.wt, S, false, Xr, act0, act1, rcnt, rounds, act, left);
+      rl = prefilled ? rank_lists(e, nullptr, nullptr, S, Xr, act0, act1, rcnt, rounds, act, left, true)
+                     : rank_lists(e, hp.prv, hp.wt, S, Xr, act0, act1, rcnt, rounds, act, left);
       cudaMemsetAsync(oncyc, 0, S, e.stream);
       ++e.launches;
       k_mark_cycle<<<gs, 256, 0, e.stream>>>(act, left, oncyc);
@@ -4233,8 +4294,12 @@ void batch_footprint(const Env& e, uint32_t njobs, const size_t* bytes, int k, i
 // per-bucket arrays; the back arena, sized once the cross k-mers are counted,
 // holds the bucketed copies and the segment pools (a job with X cross k-mers
 // has at most 2X open segments: each holds an S-only start or a P-only end).
-int compact_batch(Env& e, uint32_t njobs, const char* const* texts, const size_t* bytes, int k, int l, char* out,
-                  uint64_t out_cap, uint64_t* out_off, uint64_t* out_len, uc_stats* st) {
+//
+// recs (a batch of one job whose lines are sorted next): the warp tiles' closed
+// lines are left as records in the scatter's spare region; out_len counts the
+// text lines alone.
+static int compact_jobs(Env& e, uint32_t njobs, const char* const* texts, const size_t* bytes, int k, int l, char* out,
+                        uint64_t out_cap, uint64_t* out_off, uint64_t* out_len, uc_stats* st, LineRecs* recs) {
   if (k < 2 || k > 63) return e.fail(UC_EINPUT, "k must be in [2, 63]");
   if (l < 1 || l > 16 || l > k - 1) return e.fail(UC_EINPUT, "l must be in [1, min(16, k-1)]");
   if (njobs == 0) return UC_OK;
@@ -4350,12 +4415,23 @@ int compact_batch(Env& e, uint32_t njobs, const char* const* texts, const size_t
   const bool want_hec = e.tune.contract_method == UC_CONTRACT_HEC;
   const uint32_t RH = hec_rounds(e, Sp);
   const size_t back = back_bytes(e, copies, X, Sp, nw, k, want_hec);
-  r = e.reserve(1, back);
+  // (half of the k-mers start a line at most in canonical input)
+  const int rbits = recs ? line_bin_bits(N / 2, k) : 0;
+  const size_t rcount = recs ? size_t(4) << rbits : 0;
+  r = e.reserve(1, back + rcount + 256);
   if (r) return r;
   auto T64 = [&](uint64_t c) { return static_cast<unsigned long long*>(e.take(1, c * 8)); };
   auto T32 = [&](uint64_t c) { return static_cast<uint32_t*>(e.take(1, c * 4)); };
   char* region1 = static_cast<char*>(e.take(1, scatter_stage_bytes(copies, nw)));
   char* region2 = static_cast<char*>(e.take(1, scatter_stage_bytes(copies, nw)));
+  if (recs) {
+    recs->counts = static_cast<uint32_t*>(e.take(1, rcount));
+    recs->bits = rbits;
+    recs->cap = copies;
+    recs->used = (e.ar[1].used + 255) & ~size_t(255);
+    if (!recs->counts) return e.fail(UC_EBUDGET, "back arena overflow");
+    UC_CK(cudaMemsetAsync(recs->counts, 0, rcount, e.stream));
+  }
   SegRec* seg = static_cast<SegRec*>(e.take(1, Sp * sizeof(SegRec)));
   unsigned long long* Xr = T64(Sp);
   char* segc = static_cast<char*>(e.take(1, segchars));
@@ -4405,6 +4481,16 @@ int compact_batch(Env& e, uint32_t njobs, const char* const* texts, const size_t
   tp.jobs = jd.tab;
   tp.jout = jd.jout;
   tp.jseg = jd.jseg;
+  if (recs) {
+    // the scatter's region that does not hold the copies, and after the
+    // tiles the other one
+    recs->a = reinterpret_cast<char*>(pkeys) == region1 ? region2 : region1;
+    recs->b = reinterpret_cast<char*>(pkeys) == region1 ? region1 : region2;
+    tp.rec_a = reinterpret_cast<ulonglong2*>(recs->a);
+    tp.rec_t = reinterpret_cast<unsigned long long*>(tp.rec_a + copies);
+    tp.rec_counts = recs->counts;
+    tp.rec_bits = rbits;
+  }
   const uint32_t threads = e.tune.tile_threads ? e.tune.tile_threads : 512;
   r = run_tiles_k(e, tp, f, threads, nw);
   if (r) return r;
@@ -4426,6 +4512,11 @@ int compact_batch(Env& e, uint32_t njobs, const char* const* texts, const size_t
   if (r) return r;
   if (e.h_ctr->err) return e.check_err(e.h_ctr);
   uint64_t total = 0;
+  if (recs) {
+    recs->n = uint32_t(e.h_ctr->rec_slots);
+    recs->bytes = total = e.h_ctr->rec_bytes;
+    if (jo[0] + total > J[0].ocap) return e.fail(UC_EINTERNAL, "output bound exceeded");
+  }
   for (uint32_t j = 0; j < njobs; ++j) {
     if (jo[j] > J[j].ocap) return e.fail(UC_EINTERNAL, "output bound exceeded");
     if (out_off) out_off[j] = J[j].obase;
@@ -4440,7 +4531,7 @@ int compact_batch(Env& e, uint32_t njobs, const char* const* texts, const size_t
     st->n_big_tiles = e.h_ctr->nbig;
     st->n_segments = Sp;
     st->n_cycles = e.h_ctr->cycles;
-    st->closed_bytes = 0;
+    st->closed_bytes = recs ? recs->bytes : 0;
     for (uint32_t j = 0; j < njobs; ++j) st->closed_bytes += jc[j];
     st->seg_chars = e.h_ctr->seg_char_cursor;
     st->out_bytes = total;
@@ -4467,6 +4558,11 @@ int compact_batch(Env& e, uint32_t njobs, const char* const* texts, const size_t
   }
   e.reset();
   return UC_OK;
+}
+
+int compact_batch(Env& e, uint32_t njobs, const char* const* texts, const size_t* bytes, int k, int l, char* out,
+                  uint64_t out_cap, uint64_t* out_off, uint64_t* out_len, uc_stats* st) {
+  return compact_jobs(e, njobs, texts, bytes, k, l, out, out_cap, out_off, out_len, st, nullptr);
 }
 
 // The streamed form of the fused path, for a job from host memory whose text
@@ -4702,7 +4798,8 @@ int compact_streamed(Env& e, const char* h_text, size_t bytes, int k, int l, cha
     // per group: the tier lists and their counters, the group's line cursor
     UC_CK(cudaMemsetAsync(&e.ctr->tile_next, 0, 4, e.stream));
     UC_CK(cudaMemsetAsync(&e.ctr->nbig, 0, 4, e.stream));
-    UC_CK(cudaMemsetAsync(&e.ctr->nwarp, 0, 12, e.stream));  // nwarp, nblock, wtile_next
+    UC_CK(cudaMemsetAsync(&e.ctr->nwarp, 0, 8, e.stream));  // nwarp, nblock
+    UC_CK(cudaMemsetAsync(&e.ctr->wtile_next, 0, 4, e.stream));
     UC_CK(cudaMemsetAsync(jd.jout, 0, 8, e.stream));
     r = classify_tiles(e, f, P, nw, groups[g], groups[g + 1]);
     if (r) return r;
@@ -4775,9 +4872,10 @@ int compact_streamed(Env& e, const char* h_text, size_t bytes, int k, int l, cha
 int compact_device(Env& e, const char* d_text, size_t bytes, int k, int l, char* out, uint64_t cap,
                    uint64_t& out_bytes, uc_stats* st) {
   uint64_t off = 0, len = 0;
-  int r = compact_batch(e, 1, &d_text, &bytes, k, l, out, cap, &off, &len, st);
-  out_bytes = len;
-  if (r == UC_OK && e.sorted && len) r = sort_lines(e, out, len, k);
+  LineRecs recs;
+  int r = compact_jobs(e, 1, &d_text, &bytes, k, l, out, cap, &off, &len, st, e.sorted ? &recs : nullptr);
+  out_bytes = len + recs.bytes;
+  if (r == UC_OK && e.sorted) r = sort_lines(e, out, len, k, recs);
   return r;
 }
 

@@ -69,6 +69,8 @@ struct Env {
   // Make an arena hold `bytes`; only while nothing is taken from it.
   int reserve(int arena, size_t bytes);
   void reset() { ar[0].used = ar[1].used = 0; }
+  // The oversized tiles' scratch, grown to hold `bytes` (not in pool mode).
+  int big_scratch(size_t bytes, char*& p, const char* what);
   int read_ctr();
   int check_err(const Counters* h);
 };
@@ -112,9 +114,12 @@ uint64_t output_bound(size_t text_bytes, int k);
 // for jobs whose text and lines exceed the device budget (0 = defaults).
 int compact_streamed(Env& e, const char* h_text, size_t bytes, int k, int l, char* h_out, uint64_t cap,
                      uint64_t& out_bytes, uc_stats* st, uint64_t chunk_lines, uint64_t group_copies);
-// Reorder the lines of out[0, bytes) into byte order in place (scratch from
-// the back arena).
-int sort_lines(Env& e, char* out, uint64_t bytes, int k);
+// The lines of a job in byte order (sorted output): those of out[0, bytes)
+// and of the records in pre, into out (the records' arrays and, above them,
+// the back arena or big_scratch are used).
+int sort_lines(Env& e, char* out, uint64_t bytes, int k, const LineRecs& pre);
+// Leading key bits by which that many lines are counted for sort_lines.
+int line_bin_bits(uint64_t lines, int k);
 // Upper bound of the front and back arena bytes (reserve slack included)
 // that compact_batch needs for these jobs under the current tuning, from the
 // text sizes alone: every line holds at least k+1 bytes and at most every

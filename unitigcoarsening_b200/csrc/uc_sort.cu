@@ -4,6 +4,7 @@
 // most lines are that k-mer plus a few chars.  A line is therefore sorted as
 // a record that holds all of it in 2-bit codes (one or two key words and a
 // tail word), and the sorted text is spelled from the records:
+//   (k_tile_warp   closed lines of warp tiles come as records already)
 //   k_line_recs    text -> records, and a count per bin of leading key bits
 //   k_line_plan    bins -> tiles of about TILE_WINDOW records
 //   k_line_group   records -> their tiles (by groups of tiles first)
@@ -27,9 +28,6 @@ namespace uc {
 
 namespace {
 
-constexpr int TAIL_MAX = 28;                         // chars after the k-mer that a tail word holds
-constexpr uint64_t TAIL_LONG = 1ull << 63;           // tail word: index of a LongLine
-constexpr int TAIL_LEN_SHIFT = 58;                   // else: char count above the codes (first char lowest)
 constexpr unsigned long long HUGE_LINE = 1ull << 16; // bytes from which a line is copied by the whole grid
 
 constexpr uint32_t LR_CHUNK = 16384;  // text bytes whose line starts one block pass takes
@@ -49,7 +47,6 @@ constexpr uint32_t PLAN_ITEMS = 16;  // bins per thread of the plan
 // Cursors lie 32 bytes apart: atomics on words of one L2 line queue up (about
 // 2 ns each).
 constexpr uint32_t CUR_STRIDE = 8;
-constexpr int MAX_BIN_BITS = 23;     // counts stay in L2 (32 MiB)
 
 struct LongLine {
   unsigned long long at;   // offset in the text
@@ -61,34 +58,6 @@ struct SortCtr {
   uint32_t nrec, nlong, nhuge, ntiles;
   uint32_t plan_ticket, tile_ticket, fail, pad;
 };
-
-// One record: keys big-endian (first char in the top bits), so that numeric
-// order is byte order.  RW words: (key, tail) for k <= 31, (key, key, tail)
-// otherwise; the first two words lie together.
-template <int RW>
-struct Rec {
-  uint64_t hi, lo, tail;
-};
-template <int RW>
-struct RecArr {
-  ulonglong2* a;
-  unsigned long long* t;  // tails (RW == 3)
-};
-template <int RW>
-__device__ __forceinline__ Rec<RW> ld_rec(const RecArr<RW>& r, uint64_t i) {
-  const ulonglong2 v = r.a[i];
-  if constexpr (RW == 2) return Rec<RW>{v.x, 0ull, v.y};
-  else return Rec<RW>{v.x, v.y, r.t[i]};
-}
-template <int RW>
-__device__ __forceinline__ void st_rec(const RecArr<RW>& r, uint64_t i, const Rec<RW>& x) {
-  if constexpr (RW == 2) {
-    r.a[i] = make_ulonglong2(x.hi, x.tail);
-  } else {
-    r.a[i] = make_ulonglong2(x.hi, x.lo);
-    r.t[i] = x.tail;
-  }
-}
 
 __device__ __forceinline__ unsigned long long line_bytes_of(uint64_t tail, int k, const LongLine* longs) {
   return (tail & TAIL_LONG) ? longs[uint32_t(tail)].len : uint64_t(k) + 1u + ((tail >> TAIL_LEN_SHIFT) & 31u);
@@ -794,15 +763,13 @@ __global__ void __launch_bounds__(256) k_huge_lines(char* out, const char* keep,
   }
 }
 
-// The launch sequence for one key width.
+// The launch sequence for one key width: the lines of out[0, bytes) and
+// those of pre.
 template <int RW>
-int sort_lines_rw(Env& e, char* out, uint64_t bytes, int k) {
-  const uint64_t lmax = bytes / uint64_t(k + 1) + 1;
-  if (lmax >= 0xFFFFFFF0ull) return e.fail(UC_EINTERNAL, "line count of the output out of range");
-  // about 32 records per bin: a tile then is a window and a fraction of one,
-  // and a bin can be 32 times as dense before its tile outgrows shared memory
-  int bits = 4;
-  while (bits < std::min(MAX_BIN_BITS, 2 * k) && (lmax >> bits) > 32) ++bits;
+int sort_lines_rw(Env& e, char* out, uint64_t bytes, int k, const LineRecs& pre) {
+  const uint64_t lmax = bytes / uint64_t(k + 1) + pre.n;  // lines at most
+  const int bits = pre.bits;
+  if (lmax > pre.cap) return e.fail(UC_EINTERNAL, "more lines than k-mers");
   const uint32_t m = 1u << bits;
   // windows of 1000 records; shorter ones while there are fewer than two
   // tiles per SM.  (Not a power of two: the tiles fill at one pace, and with
@@ -817,41 +784,49 @@ int sort_lines_rw(Env& e, char* out, uint64_t bytes, int k) {
   uint32_t gsh = 0;
   if (ntmax > GRP_BINS)
     for (gsh = 5; (ntmax >> gsh) > GRP_BINS / 2; ) ++gsh;
-  // cleared: the counters, the look-back words, the bin counts
-  const size_t zero = 256 + (nplan + ntmax) * 8 + m * 4ull + 256;
+  // cleared: the counters and the look-back words
+  const size_t zero = 256 + (nplan + ntmax) * 8;
   size_t need = 0;
   auto add = [&](size_t b) { need += (b + 255) & ~size_t(255); };
   add(zero);
-  for (int q = 0; q < 2; ++q) {
-    add(lmax * 16);
-    if (RW == 3) add(lmax * 8);
-  }
   add((ntmax + 1) * 8);
   add((ntmax + GRP_BINS) * CUR_STRIDE * 4);
   add(((ntmax >> gsh) + 1 + GRP_BINS) * CUR_STRIDE * 4);
   add(nlongs * sizeof(LongLine));
   add(nhuges * 4);
   add(bytes + 16);
-  int r = e.reserve(1, need);
-  if (r) return r;
-  char* z = static_cast<char*>(e.take(1, zero));
-  RecArr<RW> ra{}, rb{};
-  for (RecArr<RW>* q : {&ra, &rb}) {
-    q->a = static_cast<ulonglong2*>(e.take(1, lmax * 16));
-    if (RW == 3) q->t = static_cast<unsigned long long*>(e.take(1, lmax * 8));
+  // above the records in the back arena, or, where they leave too little
+  // there, in the oversized tiles' scratch (free by now)
+  char* at = nullptr;
+  if (e.ar[1].cap >= pre.used + need) {
+    at = e.ar[1].base + pre.used;
+  } else {
+    const int r = e.big_scratch(need, at, "scratch for sorted output");
+    if (r) return r;
   }
-  uint2* tile = static_cast<uint2*>(e.take(1, (ntmax + 1) * 8));
-  uint32_t* cur = static_cast<uint32_t*>(e.take(1, (ntmax + GRP_BINS) * CUR_STRIDE * 4));
-  uint32_t* gcur = static_cast<uint32_t*>(e.take(1, ((ntmax >> gsh) + 1 + GRP_BINS) * CUR_STRIDE * 4));
-  LongLine* longs = static_cast<LongLine*>(e.take(1, nlongs * sizeof(LongLine)));
-  uint32_t* huge = static_cast<uint32_t*>(e.take(1, nhuges * 4));
-  char* keep = static_cast<char*>(e.take(1, bytes + 16));
-  if (!keep) return e.fail(UC_EBUDGET, "arena overflow (sorted output)");
+  auto take = [&](size_t b) {
+    char* p = at;
+    at += (b + 255) & ~size_t(255);
+    return p;
+  };
+  char* z = take(zero);
+  RecArr<RW> ra{reinterpret_cast<ulonglong2*>(pre.a), nullptr}, rb{reinterpret_cast<ulonglong2*>(pre.b), nullptr};
+  if (RW == 3) {
+    ra.t = reinterpret_cast<unsigned long long*>(ra.a + pre.cap);
+    rb.t = reinterpret_cast<unsigned long long*>(rb.a + pre.cap);
+  }
+  uint2* tile = reinterpret_cast<uint2*>(take((ntmax + 1) * 8));
+  uint32_t* cur = reinterpret_cast<uint32_t*>(take((ntmax + GRP_BINS) * CUR_STRIDE * 4));
+  uint32_t* gcur = reinterpret_cast<uint32_t*>(take(((ntmax >> gsh) + 1 + GRP_BINS) * CUR_STRIDE * 4));
+  LongLine* longs = reinterpret_cast<LongLine*>(take(nlongs * sizeof(LongLine)));
+  uint32_t* huge = reinterpret_cast<uint32_t*>(take(nhuges * 4));
+  char* keep = take(bytes + 16);
   SortCtr* sc = reinterpret_cast<SortCtr*>(z);
   unsigned long long* st_plan = reinterpret_cast<unsigned long long*>(z + 256);
   unsigned long long* st_tile = st_plan + nplan;
-  uint32_t* counts = reinterpret_cast<uint32_t*>((reinterpret_cast<uintptr_t>(st_tile + ntmax) + 255) & ~uintptr_t(255));
+  uint32_t* counts = pre.counts;
   UC_CK(cudaMemsetAsync(z, 0, zero, e.stream));
+  if (pre.n) UC_CK(cudaMemcpyAsync(&sc->nrec, &e.ctr->rec_slots, 4, cudaMemcpyDeviceToDevice, e.stream));
   auto grid = [&](uint64_t want, int occ) {
     return unsigned(std::max<uint64_t>(1, std::min<uint64_t>(want, uint64_t(e.sm_count) * uint64_t(std::max(1, occ)))));
   };
@@ -860,14 +835,15 @@ int sort_lines_rw(Env& e, char* out, uint64_t bytes, int k) {
   const size_t sm_tile = tile_smem<RW>(k);
   int occ = 0;
   UC_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_line_recs<RW>, 256, sm_recs));
-  e.launches += 4;
-  k_line_recs<RW><<<grid(nchunks, occ), 256, sm_recs, e.stream>>>(out, bytes, k, bits, ra, counts, longs, huge, sc);
+  e.launches += 2;
+  if (bytes) ++e.launches;
+  if (bytes) k_line_recs<RW><<<grid(nchunks, occ), 256, sm_recs, e.stream>>>(out, bytes, k, bits, ra, counts, longs, huge, sc);
   k_line_plan<<<unsigned(nplan), 256, 0, e.stream>>>(counts, m, win, tile, cur, gcur, gsh, st_plan, sc);
   if (nlongs > 1) {
     ++e.launches;
     k_line_keep<<<grid((nlongs + 7) / 8, 4), 256, 0, e.stream>>>(out, keep, longs, huge, sc);
   }
-  r = allow_max_smem(e, k_line_group<RW>);
+  int r = allow_max_smem(e, k_line_group<RW>);
   if (r) return r;
   RecArr<RW> from = ra, to = rb;
   for (uint32_t level = gsh ? 0u : 1u; level < 2; ++level) {
@@ -894,16 +870,25 @@ int sort_lines_rw(Env& e, char* out, uint64_t bytes, int k) {
     UC_CK(cudaGetLastError());
     UC_CK(cudaStreamSynchronize(e.stream));
   }
-  e.reset();
   return UC_OK;
 }
 
 }  // namespace
 
-int sort_lines(Env& e, char* out, uint64_t bytes, int k) {
-  if (bytes == 0) return UC_OK;
+int line_bin_bits(uint64_t lines, int k) {
+  // about 32 records per bin at most: a tile then is a window and a fraction
+  // of one, and a bin can be 32 times as dense before its tile outgrows
+  // shared memory.  Counts of 23 bits stay in L2 (32 MiB).
+  int bits = 4;
+  while (bits < std::min(23, 2 * k) && (lines >> bits) > 32) ++bits;
+  return bits;
+}
+
+int sort_lines(Env& e, char* out, uint64_t bytes, int k, const LineRecs& pre) {
+  if (bytes == 0 && pre.n == 0) return UC_OK;
+  const int r = k <= 31 ? sort_lines_rw<2>(e, out, bytes, k, pre) : sort_lines_rw<3>(e, out, bytes, k, pre);
   e.reset();
-  return k <= 31 ? sort_lines_rw<2>(e, out, bytes, k) : sort_lines_rw<3>(e, out, bytes, k);
+  return r;
 }
 
 }  // namespace uc
