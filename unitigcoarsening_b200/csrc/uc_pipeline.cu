@@ -2613,15 +2613,18 @@ __global__ void k_seg_cycles(Counters* ctr, uint32_t S, const uint32_t* __restri
 // transpose_and_sort, coarseners.h:182-235) and their offsets are composed
 // top-down (instead of copying member lists, compact_graph.h:55-112).
 // Levels live in one node pool; level r occupies [lb[r], lb[r] + ln[r]).
-// Kernels read the level sizes on the device, so every round is enqueued
-// without host round trips.
+// All rounds run in one cooperative kernel (k_hec_all) whose blocks meet at a
+// barrier between the steps and stop at the first empty level: paths of
+// canonical k-mers are short, so a few of the rounds a list could need are
+// enough.  (2M k-mers, k = 63: 0.40 ms for the call; six launches per round for
+// the 50 rounds of the bound took 1.78, most of them on empty levels.)
 constexpr uint32_t HV_UNSET = 0xFFFFFFFFu, HV_LOCK = 0xFFFFFFFEu, HV_FIN = 0xFFFFFFFDu, HV_CYC = 0xFFFFFFFCu;
 constexpr uint32_t HP_SENT = 0xFFFFFFFBu;  // coarse node not yet given a first member
 
 struct HecPool {
   uint32_t *prv, *nxt, *wt, *hn, *vc, *agg, *loc, *first0;
   uint32_t* lb;  // [R+1] level base
-  uint32_t* ln;  // [R+1] level size
+  uint32_t* ln;  // [R+1] level size, then the blocks' meeting place (two words)
   uint32_t cap;
   Counters* ctr;
 };
@@ -2666,169 +2669,256 @@ __global__ void k_hec_level0_seg(HecPool h, const SegRec* __restrict__ seg, cons
   }
 }
 
+// Values other blocks wrote in an earlier step are read past L1.
+__device__ __forceinline__ uint32_t hec_ld(const uint32_t* p) { return __ldcg(p); }
+
 // choice (hn) per node; isolated nodes are finished chains; a node whose
-// predecessor is still the sentinel is a whole cycle collapsed into one
-__global__ void k_hec_prep(HecPool h, int r) {
-  const uint32_t b = h.lb[r], N = h.ln[r];
-  for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < N; j += gridDim.x * blockDim.x) {
-    const uint32_t u = b + j;
-    const uint32_t pv = h.prv[u], nx = h.nxt[u];
-    if (pv == HP_SENT) {
-      h.hn[u] = NONE;
-      h.vc[u] = HV_CYC;
-    } else if (pv == u) {  // a one-node cycle
-      h.hn[u] = NONE;
-      h.vc[u] = HV_CYC;
-    } else {
-      const uint32_t c = (pv != NONE) ? pv : nx;
-      h.hn[u] = c;
-      h.vc[u] = (c == NONE) ? HV_FIN : HV_UNSET;
-    }
-  }
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    h.lb[r + 1] = b + N;
-    h.ln[r + 1] = 0;
-  }
+// predecessor is itself is a one-node cycle
+__device__ __forceinline__ void hec_prep(const HecPool& h, uint32_t u, uint32_t pv, uint32_t nx) {
+  const uint32_t c = (pv != NONE) ? pv : nx;
+  const bool cyc = pv == u;
+  h.hn[u] = cyc ? NONE : c;
+  h.vc[u] = cyc ? HV_CYC : (c == NONE) ? HV_FIN : HV_UNSET;
 }
 
 // One pass of the two-CAS pairing.  A label is the pool index of the
 // aggregate's root.  Pass 1 gives up after 10 tries when u > v (the
 // reference's deadlock break, heuristics.h:142-146); pass 2 retries the rest
 // a bounded number of times and then leaves u a singleton aggregate.
-__global__ void k_hec_match(HecPool h, int r, int pass) {
-  const uint32_t b = h.lb[r], N = h.ln[r];
-  for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < N; j += gridDim.x * blockDim.x) {
-    const uint32_t u = b + j;
-    const uint32_t v = h.hn[u];
-    if (v == NONE) continue;
-    if (pass == 2 && atomicAdd(h.vc + u, 0u) != HV_UNSET) continue;
-    bool done = false;
-    const int limit = (pass == 1) ? 64 : 256;
-    for (int it = 0; it < limit && !done; ++it) {
-      if (atomicCAS(h.vc + u, HV_UNSET, HV_LOCK) == HV_UNSET) {
-        if (atomicCAS(h.vc + v, HV_UNSET, HV_LOCK) == HV_UNSET) {
-          atomicExch(h.vc + v, u);
-          atomicExch(h.vc + u, u);
+__device__ __forceinline__ void hec_match(const HecPool& h, uint32_t u, uint32_t v, int pass) {
+  bool done = false;
+  const int limit = (pass == 1) ? 64 : 256;
+  for (int it = 0; it < limit && !done; ++it) {
+    if (atomicCAS(h.vc + u, HV_UNSET, HV_LOCK) == HV_UNSET) {
+      if (atomicCAS(h.vc + v, HV_UNSET, HV_LOCK) == HV_UNSET) {
+        atomicExch(h.vc + v, u);
+        atomicExch(h.vc + u, u);
+        done = true;
+      } else {
+        const uint32_t lv = atomicAdd(h.vc + v, 0u);
+        if (lv < HV_CYC) {  // v already labelled: join its aggregate
+          atomicExch(h.vc + u, lv);
           done = true;
         } else {
-          const uint32_t lv = atomicAdd(h.vc + v, 0u);
-          if (lv < HV_CYC) {  // v already labelled: join its aggregate
-            atomicExch(h.vc + u, lv);
-            done = true;
-          } else {
-            atomicExch(h.vc + u, HV_UNSET);  // release and retry
-          }
+          atomicExch(h.vc + u, HV_UNSET);  // release and retry
         }
-      } else {
-        done = true;  // u is labelled (or being labelled) by a neighbour
       }
-      if (pass == 1 && it > 10 && u > v) break;
+    } else {
+      done = true;  // u is labelled (or being labelled) by a neighbour
     }
-    if (pass == 2 && !done) atomicCAS(h.vc + u, HV_UNSET, u);  // singleton
+    if (pass == 1 && it > 10 && u > v) break;
   }
-}
-
-// Roots (label == self) take the next level's pool slots; the root's hn
-// holds its new index afterwards.
-__global__ void k_hec_roots(HecPool h, int r) {
-  const uint32_t b = h.lb[r], N = h.ln[r];
-  const uint32_t nb = h.lb[r + 1];
-  const int lane = threadIdx.x & 31;
-  for (uint32_t j0 = blockIdx.x * blockDim.x; j0 < N; j0 += gridDim.x * blockDim.x) {
-    const uint32_t j = j0 + threadIdx.x;
-    const uint32_t u = b + j;
-    const bool root = (j < N) && (h.vc[u] == u);
-    const uint32_t m = __ballot_sync(0xFFFFFFFFu, root);
-    uint32_t base = 0;
-    if (m) {
-      if (lane == __ffs(m) - 1) base = atomicAdd(h.ln + r + 1, uint32_t(__popc(m)));
-      base = __shfl_sync(0xFFFFFFFFu, base, __ffs(m) - 1);
-    }
-    if (root) {
-      const uint32_t a = nb + base + __popc(m & ((1u << lane) - 1u));
-      if (a >= h.cap) {
-        atomicOr(&h.ctr->err, ERR_CAPACITY);
-      } else {
-        h.hn[u] = a;
-        h.prv[a] = HP_SENT;
-        h.nxt[a] = NONE;
-        h.wt[a] = 0;
-        h.first0[a] = NONE;
-      }
-    }
-  }
-}
-
-__global__ void k_hec_assign(HecPool h, int r) {
-  const uint32_t b = h.lb[r], N = h.ln[r];
-  for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < N; j += gridDim.x * blockDim.x) {
-    const uint32_t u = b + j;
-    const uint32_t c = h.vc[u];
-    h.agg[u] = (c < HV_CYC) ? h.hn[c] : NONE;
-  }
+  if (pass == 2 && !done) atomicCAS(h.vc + u, HV_UNSET, u);  // singleton
 }
 
 // The first member of each aggregate (predecessor outside it) walks its
-// members along next: local offsets, total weight, coarse neighbours.
-__global__ void k_hec_order(HecPool h, int r) {
-  const uint32_t b = h.lb[r], N = h.ln[r];
-  for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < N; j += gridDim.x * blockDim.x) {
-    const uint32_t u = b + j;
-    const uint32_t A = h.agg[u];
-    if (A == NONE || A >= h.cap) continue;
-    const uint32_t pv = h.prv[u];
-    if (pv != NONE && h.agg[pv] == A) continue;  // not the first member
-    uint32_t off = 0, m = u, last = u;
-    for (uint32_t guard = 0; guard < N; ++guard) {
-      h.loc[m] = off;
-      off += h.wt[m];
-      last = m;
-      const uint32_t nx = h.nxt[m];
-      if (nx == NONE || h.agg[nx] != A) break;
-      m = nx;
-    }
-    h.wt[A] = off;
-    h.first0[A] = h.first0[u];
-    h.nxt[A] = (h.nxt[last] == NONE) ? NONE : h.agg[h.nxt[last]];
-    h.prv[A] = (pv == NONE) ? NONE : h.agg[pv];
+// members along next: local offsets, total weight, coarse neighbours, and the
+// coarse node's choice.  (ap: the aggregate of u's predecessor)
+__device__ __forceinline__ void hec_order(const HecPool& h, uint32_t u, uint32_t A, uint32_t ap, uint32_t N) {
+  uint32_t off = 0, m = u, nx = NONE;
+  for (uint32_t guard = 0; guard < N; ++guard) {
+    h.loc[m] = off;
+    off += hec_ld(h.wt + m);
+    nx = hec_ld(h.nxt + m);
+    if (nx == NONE || hec_ld(h.agg + nx) != A) break;
+    m = nx;
   }
+  const uint32_t an = (nx == NONE) ? NONE : hec_ld(h.agg + nx);
+  h.wt[A] = off;
+  h.first0[A] = hec_ld(h.first0 + u);
+  h.nxt[A] = an;
+  h.prv[A] = ap;
+  hec_prep(h, A, ap, an);
 }
 
 // Top-down: (head, offset) of every node from its aggregate's, stored in
 // (hn, loc).  A finished node is a whole chain headed by its first member; a
 // cycle node marks its members with head NONE.
-__global__ void k_hec_down(HecPool h, int r) {
-  const uint32_t b = h.lb[r], N = h.ln[r];
-  for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < N; j += gridDim.x * blockDim.x) {
-    const uint32_t u = b + j;
-    const uint32_t c = h.vc[u];
-    uint32_t hd, of;
-    if (c == HV_FIN) {
-      hd = h.first0[u];
-      of = 0;
-    } else if (c == HV_CYC) {
-      hd = NONE;
-      of = 0;
-    } else {
-      const uint32_t A = h.agg[u];
-      hd = (A == NONE || A >= h.cap) ? NONE : h.hn[A];
-      of = (hd == NONE) ? 0 : h.loc[A] + h.loc[u];
-    }
-    h.hn[u] = hd;
-    h.loc[u] = of;
+__device__ __forceinline__ void hec_down(const HecPool& h, uint32_t u) {
+  const uint32_t c = hec_ld(h.vc + u);
+  uint32_t hd = NONE, of = 0;
+  if (c == HV_FIN) {
+    hd = hec_ld(h.first0 + u);
+  } else if (c != HV_CYC) {
+    const uint32_t A = hec_ld(h.agg + u);
+    hd = (A == NONE || A >= h.cap) ? NONE : hec_ld(h.hn + A);
+    of = (hd == NONE) ? 0 : hec_ld(h.loc + A) + hec_ld(h.loc + u);
   }
+  h.hn[u] = hd;
+  h.loc[u] = of;
 }
 
-// Level-0 results into the (pointer | HEAD_BIT, offset) form of the ranking.
-__global__ void k_hec_emit(HecPool h, unsigned long long* __restrict__ X, uint8_t* __restrict__ oncycle) {
-  const uint32_t N = h.ln[0];
-  for (uint32_t s = blockIdx.x * blockDim.x + threadIdx.x; s < N; s += gridDim.x * blockDim.x) {
-    const uint32_t hd = h.hn[s];
+// All blocks of a cooperative grid meet here (gen counts the meetings): the
+// last one to arrive (bar[0]) lets the others go (bar[1]).  A wait that runs
+// out, or meets another block's, sets the error flag and returns false; the
+// kernel then ends.
+__device__ __forceinline__ bool grid_meet(uint32_t* bar, uint32_t& gen, uint32_t* err) {
+  __shared__ int s_ok;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    ++gen;
+    int ok = 1;
+    __threadfence();
+    if (atomicAdd(bar, 1u) + 1u == gen * gridDim.x) {
+      atomicExch(bar + 1, gen);
+    } else {
+      uint32_t p = 0;
+      while (*reinterpret_cast<volatile uint32_t*>(bar + 1) < gen) {
+        __nanosleep(20);
+        if (++p >= (1u << 22) || ((p & 1023u) == 0 && (*reinterpret_cast<volatile uint32_t*>(err) & ERR_INTERNAL))) {
+          atomicOr(err, ERR_INTERNAL | ERR_TIMEOUT);
+          ok = 0;
+          break;
+        }
+      }
+    }
+    __threadfence();
+    s_ok = ok;
+  }
+  __syncthreads();
+  return s_ok != 0;
+}
+
+// One round over level r (base b, N nodes; level 0 and coarse nodes have
+// their choices): threads t0, t0 + span, ... of all blocks or of one, meet()
+// between the steps.  Sets the next level's base, size and choices.
+template <class Meet>
+__device__ __forceinline__ bool hec_round(const HecPool& h, uint32_t r, uint32_t& b, uint32_t& N, uint32_t t0,
+                                          uint32_t span, Meet meet) {
+  __shared__ uint32_t sc[33];
+  uint32_t* const err = &h.ctr->err;
+  for (int pass = 1; pass <= 2; ++pass) {
+    for (uint32_t j0 = t0; j0 < N; j0 += 4 * span) {
+      uint32_t v[4];
+#pragma unroll
+      for (uint32_t q = 0; q < 4; ++q) v[q] = j0 + q * span < N ? hec_ld(h.hn + b + j0 + q * span) : NONE;
+      if (pass == 2) {
+#pragma unroll
+        for (uint32_t q = 0; q < 4; ++q)
+          if (v[q] != NONE && hec_ld(h.vc + b + j0 + q * span) != HV_UNSET) v[q] = NONE;
+      }
+#pragma unroll
+      for (uint32_t q = 0; q < 4; ++q)
+        if (v[q] != NONE) hec_match(h, b + j0 + q * span, v[q], pass);
+    }
+    if (!meet()) return false;
+  }
+  // roots (label == self) take the next level's pool slots; the root's hn
+  // holds its new index.  A coarse node no first member reaches (hec_order)
+  // is a whole cycle collapsed into one.
+  // (whole blocks iterate together: one append per block and pass)
+  for (uint32_t j0 = t0 - threadIdx.x; j0 < N; j0 += 4 * span) {
+    uint32_t root = 0;
+#pragma unroll
+    for (uint32_t q = 0; q < 4; ++q) {
+      const uint32_t j = j0 + threadIdx.x + q * span;
+      if (j < N && hec_ld(h.vc + b + j) == b + j) root |= 1u << q;
+    }
+    uint32_t a = b + N + block_append(h.ln + r + 1, uint32_t(__popc(root)), sc);
+#pragma unroll
+    for (uint32_t q = 0; q < 4; ++q) {
+      if (!((root >> q) & 1u)) continue;
+      if (a >= h.cap) {
+        atomicOr(err, ERR_CAPACITY);
+      } else {
+        h.hn[b + j0 + threadIdx.x + q * span] = a;
+        h.prv[a] = HP_SENT;
+        h.nxt[a] = NONE;
+        h.wt[a] = 0;
+        h.first0[a] = NONE;
+        h.hn[a] = NONE;
+        h.vc[a] = HV_CYC;
+      }
+      ++a;
+    }
+  }
+  if (!meet()) return false;
+  for (uint32_t j0 = t0; j0 < N; j0 += 4 * span) {
+    uint32_t c[4], a[4];
+#pragma unroll
+    for (uint32_t q = 0; q < 4; ++q) c[q] = j0 + q * span < N ? hec_ld(h.vc + b + j0 + q * span) : NONE;
+#pragma unroll
+    for (uint32_t q = 0; q < 4; ++q) a[q] = c[q] < HV_CYC ? hec_ld(h.hn + c[q]) : NONE;
+#pragma unroll
+    for (uint32_t q = 0; q < 4; ++q)
+      if (j0 + q * span < N) h.agg[b + j0 + q * span] = a[q];
+  }
+  if (!meet()) return false;
+  for (uint32_t j0 = t0; j0 < N; j0 += 4 * span) {
+    // which nodes are first members, then their walks
+    uint32_t A[4], pv[4], ap[4];
+#pragma unroll
+    for (uint32_t q = 0; q < 4; ++q) {
+      const uint32_t u = b + j0 + q * span;
+      A[q] = j0 + q * span < N ? hec_ld(h.agg + u) : NONE;
+      pv[q] = j0 + q * span < N ? hec_ld(h.prv + u) : NONE;
+    }
+#pragma unroll
+    for (uint32_t q = 0; q < 4; ++q) ap[q] = (A[q] != NONE && pv[q] != NONE) ? hec_ld(h.agg + pv[q]) : NONE;
+#pragma unroll
+    for (uint32_t q = 0; q < 4; ++q)
+      if (A[q] != NONE && A[q] < h.cap && ap[q] != A[q]) hec_order(h, b + j0 + q * span, A[q], ap[q], N);
+  }
+  if (t0 == 0) h.lb[r + 1] = b + N;
+  if (!meet()) return false;
+  b += N;
+  N = min(hec_ld(h.ln + r + 1), h.cap - min(h.cap, b));
+  return true;
+}
+
+// The rounds (level 0 is set), at most R of them, then the way down and the
+// level-0 results in the (pointer | HEAD_BIT, offset) form of the ranking.
+// Levels of at most HEC_SOLO nodes are worked by one block, up and down, while
+// the others wait at one meeting.  Lists still open after R rounds set
+// ERR_TIMEOUT.
+constexpr uint32_t HEC_THREADS = 1024, HEC_SOLO = 4096;
+__global__ void __launch_bounds__(HEC_THREADS, 2) k_hec_all(HecPool h, uint32_t R, unsigned long long* __restrict__ X,
+                                                         uint8_t* __restrict__ oncycle) {
+  const uint32_t t0 = blockIdx.x * blockDim.x + threadIdx.x, span = gridDim.x * blockDim.x;
+  uint32_t* const bar = h.ln + R + 1;
+  uint32_t* const err = &h.ctr->err;
+  uint32_t gen = 0, r = 0, b = 0, N = hec_ld(h.ln);
+  const uint32_t N0 = N;
+  auto all = [&] { return grid_meet(bar, gen, err); };
+  auto own = [] {
+    __syncthreads();
+    return true;
+  };
+  for (uint32_t u = t0; u < N; u += span) hec_prep(h, u, hec_ld(h.prv + u), hec_ld(h.nxt + u));
+  if (!all()) return;
+  for (; r < R && N > HEC_SOLO; ++r)
+    if (!hec_round(h, r, b, N, t0, span, all)) return;
+  const uint32_t rs = r;
+  if (N) {
+    if (blockIdx.x == 0) {
+      for (; r < R && N; ++r) hec_round(h, r, b, N, threadIdx.x, HEC_THREADS, own);
+      if (N) {
+        if (threadIdx.x == 0) atomicOr(err, ERR_TIMEOUT);
+      } else {
+        while (r-- > rs) {
+          b = r ? hec_ld(h.lb + r) : 0u;
+          N = hec_ld(h.ln + r);
+          for (uint32_t j = threadIdx.x; j < N; j += HEC_THREADS) hec_down(h, b + j);
+          __syncthreads();
+        }
+      }
+    }
+    if (!all()) return;
+    if (hec_ld(err) & ERR_TIMEOUT) return;  // the rounds ran out
+  }
+  for (r = rs; r-- > 0;) {
+    b = r ? hec_ld(h.lb + r) : 0u;
+    N = hec_ld(h.ln + r);
+    for (uint32_t j = t0; j < N; j += span) hec_down(h, b + j);
+    if (!all()) return;
+  }
+  for (uint32_t s = t0; s < N0; s += span) {
+    const uint32_t hd = hec_ld(h.hn + s);
     if (hd == NONE) {
       X[s] = pk(s, 0);
       if (oncycle) oncycle[s] = 1;
     } else {
-      X[s] = pk(hd == s ? (hd | HEAD_BIT) : hd, h.loc[s]);
+      X[s] = pk(hd == s ? (hd | HEAD_BIT) : hd, hec_ld(h.loc + s));
     }
   }
 }
@@ -2838,10 +2928,6 @@ __global__ void k_cycle_list(const uint8_t* __restrict__ oncycle, uint64_t n,
   const uint64_t N = n;
   for (uint64_t s = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; s < N; s += uint64_t(gridDim.x) * blockDim.x)
     if (oncycle[s]) act[atomicAdd(cnt, 1u)] = uint32_t(s);
-}
-
-__global__ void k_hec_check(HecPool h, int R) {
-  if (h.ln[R] != 0) atomicOr(&h.ctr->err, ERR_TIMEOUT);
 }
 
 // ======================================================= phase-API helpers
@@ -3857,7 +3943,7 @@ static int hec_take(Env& e, uint64_t nmax, uint32_t R, HecPool& h) {
   uint32_t** arr[8] = {&h.prv, &h.nxt, &h.wt, &h.hn, &h.vc, &h.agg, &h.loc, &h.first0};
   for (auto a : arr) *a = static_cast<uint32_t*>(e.take(1, cap * 4));
   h.lb = static_cast<uint32_t*>(e.take(1, (R + 1) * 4));
-  h.ln = static_cast<uint32_t*>(e.take(1, (R + 1) * 4));
+  h.ln = static_cast<uint32_t*>(e.take(1, (R + 3) * 4));
   h.cap = uint32_t(std::min<uint64_t>(cap, 0xFFFFFFF0ull));
   h.ctr = e.ctr;
   if (!h.ln) return e.fail(UC_EBUDGET, "arena overflow (HEC pool)");
@@ -3876,31 +3962,27 @@ static uint32_t hec_rounds(const Env& e, uint64_t nmax) {
 }
 
 // HEC contraction of the lists (prev, next, w) into X (pointer | HEAD_BIT,
-// offset) and cycle flags, all rounds enqueued on the stream.
+// offset) and cycle flags, enqueued on the stream (one kernel for all rounds).
 // With seg, level 0 comes from the fused path's segment records and the
 // ranking's first state in X (built from them by k_seg_xinit; nx cross
 // indices) instead of (prev, next, w).
-static void hec_contract(Env& e, HecPool& h, uint32_t R, const uint32_t* prev, const uint32_t* next,
+static int hec_contract(Env& e, HecPool& h, uint32_t R, const uint32_t* prev, const uint32_t* next,
                          const uint32_t* w, uint64_t nmax, unsigned long long* X,
                          uint8_t* oncycle, const SegRec* seg = nullptr, uint32_t nx = 0, int k = 0) {
   const int grid = grid_for(e, nmax ? nmax : 1, 256);
-  cudaMemsetAsync(h.ln, 0, (R + 1) * 4, e.stream);
-  ++e.launches;
+  UC_CK(cudaMemsetAsync(h.ln, 0, (R + 3) * 4, e.stream));
+  e.launches += 2;
   if (seg) k_hec_level0_seg<<<grid, 256, 0, e.stream>>>(h, seg, X, nmax, nx, k);
   else k_hec_level0<<<grid, 256, 0, e.stream>>>(h, prev, next, w, nmax);
-  for (uint32_t r = 0; r < R; ++r) {
-    e.launches += 6;
-    k_hec_prep<<<grid, 256, 0, e.stream>>>(h, int(r));
-    k_hec_match<<<grid, 256, 0, e.stream>>>(h, int(r), 1);
-    k_hec_match<<<grid, 256, 0, e.stream>>>(h, int(r), 2);
-    k_hec_roots<<<grid, 256, 0, e.stream>>>(h, int(r));
-    k_hec_assign<<<grid, 256, 0, e.stream>>>(h, int(r));
-    k_hec_order<<<grid, 256, 0, e.stream>>>(h, int(r));
-  }
-  e.launches += 1 + R + 1;
-  k_hec_check<<<1, 1, 0, e.stream>>>(h, int(R));
-  for (int r = int(R) - 1; r >= 0; --r) k_hec_down<<<grid, 256, 0, e.stream>>>(h, r);
-  k_hec_emit<<<grid, 256, 0, e.stream>>>(h, X, oncycle);
+  // every block resident (they meet)
+  int occ = 0;
+  UC_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_hec_all, int(HEC_THREADS), 0));
+  const uint64_t want = (nmax + HEC_THREADS - 1) / HEC_THREADS;
+  const unsigned g = unsigned(std::max<uint64_t>(1, std::min<uint64_t>(want, uint64_t(e.sm_count) * std::max(1, occ))));
+  void* args[] = {&h, &R, &X, &oncycle};
+  UC_CK(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(k_hec_all), dim3(g), dim3(HEC_THREADS), args, 0,
+                                    e.stream));
+  return UC_OK;
 }
 
 static int contract_hec(Env& e, const uint64_t* d_keys, const uint32_t* succ, const uint32_t* pred, uint64_t n,
@@ -3921,7 +4003,8 @@ static int contract_hec(Env& e, const uint64_t* d_keys, const uint32_t* succ, co
   if (!dcyc) return e.fail(UC_EBUDGET, "arena overflow");
   UC_CK(cudaMemsetAsync(&e.ctr->err, 0, 4, e.stream));
   UC_CK(cudaMemsetAsync(flag, 0, n, e.stream));
-  hec_contract(e, h, R, pred, succ, nullptr, n, X, flag);
+  r = hec_contract(e, h, R, pred, succ, nullptr, n, X, flag);
+  if (r) return r;
   e.launches += 2;
   k_head_rank<<<grid_for(e, n, 256), 256, 0, e.stream>>>(X, n, head, rank);
   UC_CK(cudaMemsetAsync(cnt, 0, 4, e.stream));
@@ -4180,15 +4263,12 @@ static int run_stitch(Env& e, const StitchBufs& b, uint64_t X, uint64_t Hp, int 
   k_seg_xinit<<<gs, 256, 0, e.stream>>>(S, seg, nx, k, Xr);
   bool hec = want_hec;
   if (hec) {
-    // HEC matching rounds, captured as one graph
-    r = run_graph(e, 1, (uint64_t(RH) << 32) | uint32_t(gs), [&] {
-      cudaMemsetAsync(oncyc, 0, S, e.stream);
-      hec_contract(e, hp, RH, nullptr, nullptr, nullptr, S, Xr, oncyc, seg, nx, k);
-      cudaMemsetAsync(rcnt, 0, 4, e.stream);
-      ++e.launches;
-      k_cycle_list<<<gs, 256, 0, e.stream>>>(oncyc, S, act0, rcnt);
-    });
+    UC_CK(cudaMemsetAsync(oncyc, 0, S, e.stream));
+    r = hec_contract(e, hp, RH, nullptr, nullptr, nullptr, S, Xr, oncyc, seg, nx, k);
     if (r) return r;
+    UC_CK(cudaMemsetAsync(rcnt, 0, 4, e.stream));
+    ++e.launches;
+    k_cycle_list<<<gs, 256, 0, e.stream>>>(oncyc, S, act0, rcnt);
     act = act0;
     left = rcnt;
     rounds = RH;

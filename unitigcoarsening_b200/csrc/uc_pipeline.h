@@ -42,8 +42,8 @@ struct Env {
   uint32_t graph_nodes = 0; // of which inside CUDA graphs
   // instantiated graphs of the contraction rounds, reused while the round
   // count (the graph's shape) stays the same
-  cudaGraphExec_t gexec[2] = {nullptr, nullptr};
-  uint64_t gkey[2] = {0, 0};
+  cudaGraphExec_t gexec[1] = {nullptr};
+  uint64_t gkey[1] = {0};
   bool use_graphs = true;
   cudaStream_t gstream = nullptr;  // capture stream when the caller's stream is the legacy one
   // pool mode (serving): the arenas are fixed slices of a device pool that a
