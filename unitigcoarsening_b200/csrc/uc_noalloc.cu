@@ -38,9 +38,9 @@
 namespace {
 
 constexpr uint64_t kMaxKmers = UC_EMIT_NOALLOC_MAX_KMERS;
-// member counts and line lengths (4 B each), line offsets (8 B), scan block
-// sums: 16 MiB + 2.3 KiB at the maximum; the array keeps 64 KiB of slack.
-constexpr size_t kScratchBytes = (size_t(16) << 20) + (size_t(64) << 10);
+// member counts and line positions (4 B each per k-mer), later chars (1 B),
+// tile sums: 9 MiB + 17 KiB at the maximum; the array keeps some slack.
+constexpr size_t kScratchBytes = (size_t(9) << 20) + (size_t(64) << 10);
 
 // One cache entry per CUDA context that has called: the context's unique id
 // (cuCtxGetId), the array's address in it and the device's SM count.

@@ -2981,32 +2981,215 @@ __global__ void k_count_members(const uint32_t* __restrict__ head, uint64_t n, u
     atomicAdd(cnt + head[v], 1u);
 }
 
-__global__ void k_line_len(const uint32_t* __restrict__ head, const uint32_t* __restrict__ cnt,
-                           uint64_t n, int k, uint32_t* __restrict__ len) {
-  for (uint64_t v = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; v < n;
-       v += uint64_t(gridDim.x) * blockDim.x)
-    len[v] = (head[v] == uint32_t(v)) ? uint32_t(k) + cnt[v] : 0u;
+// Unitig lines from (head, rank), ordered by head id (write_intra_bucket_
+// outputs, compact.h:187-208).  A line is its head's k-mer and the last char
+// of each later member.  The members counted per head (k_count_members) give,
+// by one look-back pass, each line's first position among all members
+// (k_emit_scan); each later member stores its char at its position, one byte
+// into an n-byte array that L2 holds (k_emit_chars); then blocks take heads in
+// id order and store their lines as one stream, spelled in shared memory
+// (k_emit_lines).  17M k-mers, k = 31: 540 us in all; every member storing its
+// char straight into the output (290 MB, a random byte each) took 950 of 1600.
+constexpr uint32_t EMIT_TILE = 1024;  // vertices per block of k_emit_scan and k_emit_lines
+
+// heads among [0, n)
+__global__ void __launch_bounds__(256) k_count_heads(const uint32_t* __restrict__ head, uint64_t n,
+                                                     unsigned long long* total) {
+  uint32_t acc = 0;
+  for (uint64_t v = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; v < n; v += uint64_t(gridDim.x) * blockDim.x)
+    acc += head[v] == uint32_t(v);
+  acc = __reduce_add_sync(0xFFFFFFFFu, acc);
+  if ((threadIdx.x & 31u) == 0 && acc) atomicAdd(total, (unsigned long long)acc);
 }
 
-// Spell each vertex's chars at its line offset (write_intra_bucket_outputs,
-// compact.h:187-208): rank 0 writes the whole k-mer, rank r writes its last
-// char at k-1+r, the last member adds '\n'.
+// voff[v]: members of the heads before v.  base[b]: lines (high half) and
+// members (low half) before block b's vertices; base[blocks] the totals.
+__global__ void __launch_bounds__(256) k_emit_scan(const uint32_t* __restrict__ head, const uint32_t* __restrict__ cnt,
+                                                   uint64_t n, uint32_t* __restrict__ voff,
+                                                   unsigned long long* __restrict__ base, unsigned long long* st,
+                                                   uint32_t* ctl) {
+  __shared__ unsigned long long scan[33], s_base;
+  __shared__ uint32_t s_b;
+  if (threadIdx.x == 0) s_b = atomicAdd(ctl, 1u);
+  __syncthreads();
+  const uint32_t b = s_b;
+  const uint64_t v0 = uint64_t(b) * EMIT_TILE + 4u * threadIdx.x;
+  uint32_t c[4];
+  unsigned long long sum = 0;
+#pragma unroll
+  for (uint32_t q = 0; q < 4; ++q) {
+    c[q] = (v0 + q < n && head[v0 + q] == uint32_t(v0 + q)) ? cnt[v0 + q] : 0u;
+    sum += c[q] ? (1ull << 31) + c[q] : 0ull;  // (62 bits travel: both below 2^31)
+  }
+  unsigned long long tot;
+  const unsigned long long pre = block_excl_scan(sum, scan, &tot);
+  if (threadIdx.x < 32) {
+    if (threadIdx.x == 0) lb_publish(st, b, LB_SUM, tot);
+    __syncwarp();
+    const unsigned long long e = lb_exclusive(st, b, tot, ctl + 1);
+    if (threadIdx.x == 0) s_base = e;
+  }
+  __syncthreads();
+  uint32_t p = uint32_t((s_base + pre) & 0x7FFFFFFFull);
+#pragma unroll
+  for (uint32_t q = 0; q < 4; ++q) {
+    if (v0 + q < n) voff[v0 + q] = p;
+    p += c[q];
+  }
+  auto split = [](unsigned long long x) { return ((x >> 31) << 32) | (x & 0x7FFFFFFFull); };
+  if (threadIdx.x == 0) {
+    base[b] = split(s_base);
+    if (b == gridDim.x - 1) base[b + 1] = split(s_base + tot);
+  }
+}
+
+// Each later member's last char at its position, four members per thread and
+// pass in flight.
 template <int NW>
-__global__ void k_spell(const uint64_t* __restrict__ keys, const uint32_t* __restrict__ head,
-                        const uint32_t* __restrict__ rank, const uint32_t* __restrict__ cnt,
-                        const unsigned long long* __restrict__ loff, uint64_t n, int k,
-                        char* __restrict__ out) {
-  for (uint64_t v = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; v < n;
-       v += uint64_t(gridDim.x) * blockDim.x) {
-    const Key<NW> x = ld_key<NW>(keys, v);
-    const uint32_t h = head[v], r = rank[v];
-    char* dst = out + loff[h];
-    if (r == 0) {
-      spell_key<NW>(dst, x, k);
-    } else {
-      dst[k - 1 + r] = acgt(key_char(x, k - 1));
+__global__ void __launch_bounds__(256) k_emit_chars(const uint64_t* __restrict__ keys, const uint32_t* __restrict__ head,
+                                                    const uint32_t* __restrict__ rank,
+                                                    const uint32_t* __restrict__ voff, uint64_t n, int k,
+                                                    char* __restrict__ chars) {
+  constexpr int PER = 4;
+  const uint64_t span = uint64_t(gridDim.x) * blockDim.x;
+  // the word that holds char k - 1
+  const uint32_t w = (NW == 2 && k > 32) ? 1u : 0u, sh = 2u * uint32_t(k - 1 - 32 * int(w));
+  for (uint64_t v0 = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; v0 < n; v0 += span * PER) {
+    uint32_t r[PER], h[PER];
+    uint64_t x[PER];
+#pragma unroll
+    for (int q = 0; q < PER; ++q) {
+      const uint64_t v = v0 + q * span;
+      r[q] = v < n ? rank[v] : 0u;
+      h[q] = v < n ? head[v] : 0u;
+      x[q] = v < n ? keys[v * NW + w] : 0u;
     }
-    if (r + 1 == cnt[h]) dst[k + r] = '\n';
+    uint32_t at[PER];
+#pragma unroll
+    for (int q = 0; q < PER; ++q) at[q] = r[q] ? voff[h[q]] + r[q] : 0u;
+#pragma unroll
+    for (int q = 0; q < PER; ++q)
+      if (r[q] && at[q] < n) chars[at[q]] = acgt(uint32_t(x[q] >> sh) & 3u);
+  }
+}
+
+// The lines of a tile's heads, in id order.  Lines of EMIT_HUGE members or
+// more leave their chars to k_emit_huge.
+constexpr uint32_t EMIT_HUGE = 1u << 16;
+template <int NW>
+__global__ void __launch_bounds__(256) k_emit_lines(const uint64_t* __restrict__ keys, const uint32_t* __restrict__ head,
+                                                    const uint32_t* __restrict__ cnt,
+                                                    const uint32_t* __restrict__ voff, const char* __restrict__ chars,
+                                                    const unsigned long long* __restrict__ base, uint64_t n, int k,
+                                                    char* __restrict__ out, uint32_t* ctl, uint32_t* __restrict__ huge) {
+  constexpr int NC = NW == 1 ? 4 : 6;
+  constexpr uint32_t BUF = (16 + 32 * (32 * NW + TAIL_MAX + 4) + 16) / 4;  // a warp's text: 32 lines
+  __shared__ __align__(16) uint32_t buf_all[8][BUF];
+  __shared__ uint16_t list[EMIT_TILE];
+  __shared__ uint32_t scan[33];
+  const uint32_t lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
+  uint32_t* buf = buf_all[wid];
+  const uint64_t t0 = uint64_t(blockIdx.x) * EMIT_TILE, v0 = t0 + 4u * threadIdx.x;
+  uint32_t mask = 0;
+#pragma unroll
+  for (uint32_t q = 0; q < 4; ++q)
+    if (v0 + q < n && head[v0 + q] == uint32_t(v0 + q)) mask |= 1u << q;
+  uint32_t nl;
+  uint32_t at = block_excl_scan(uint32_t(__popc(mask)), scan, &nl);
+  for (uint32_t m = mask; m; m &= m - 1) list[at++] = uint16_t(4 * threadIdx.x + uint32_t(__ffs(m)) - 1u);
+  __syncthreads();
+  const unsigned long long line0 = base[blockIdx.x] >> 32;
+  const uint32_t per = ((nl + 7) / 8 + 31u) & ~31u;
+  const uint32_t r0 = min(nl, wid * per), r1 = min(nl, r0 + per);
+  if (r0 >= r1) return;
+  WarpText T;
+  T.begin(out + (line0 + r0) * uint64_t(k) + voff[t0 + list[r0]]);
+  for (uint32_t i0 = r0; i0 < r1; i0 += 32) {
+    const bool live = i0 + lane < r1;
+    uint64_t v = 0;
+    uint32_t c = 0, p = 0;
+    Key<NW> x;
+#pragma unroll
+    for (int w = 0; w < NW; ++w) x.w[w] = 0;
+    if (live) {
+      v = t0 + list[i0 + lane];
+      c = cnt[v];
+      p = voff[v];
+      x = ld_key<NW>(keys, v);
+    }
+    const unsigned long long nb = live ? uint64_t(k) + c : 0ull;
+    unsigned long long inc = nb;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned long long u = __shfl_up_sync(0xFFFFFFFFu, inc, o);
+      if (lane >= uint32_t(o)) inc += u;
+    }
+    const unsigned long long total = __shfl_sync(0xFFFFFFFFu, inc, 31);
+    if (!__any_sync(0xFFFFFFFFu, c > uint32_t(TAIL_MAX) + 1u)) {
+      if (live) {
+        uint64_t codes = 0;
+        for (uint32_t r = 1; r < c; ++r) {
+          const uint32_t b = uint32_t(chars[p + r]);
+          codes |= uint64_t(codes_of_bits((b >> 1) & 3u)) << (2 * (r - 1));
+        }
+        uint64_t w[3] = {x.w[0], 0, 0};
+        if constexpr (NW == 1) {
+          w[0] |= codes << (2 * k);
+          w[1] = codes >> (64 - 2 * k);
+        } else {
+          const int u = 2 * k - 64;
+          w[1] = x.w[1] | (codes << u);
+          w[2] = u ? codes >> (64 - u) : 0ull;
+        }
+        uint32_t xx[NC];
+#pragma unroll
+        for (int q = 0; q < NC; ++q) xx[q] = uint32_t(w[q >> 1] >> (32 * (q & 1)));
+        spell_text<NC>(buf, T.fill + uint32_t(inc - nb), xx, uint32_t(k) - 1u + c, 1u);
+      }
+      __syncwarp();
+      T.flush(buf, uint32_t(total));
+    } else {
+      // a longer line among the 32: k-mers by their lanes, later chars by the
+      // warp, line after line
+      T.end(buf);
+      char* const dst = T.dst + (inc - nb);
+      if (live) {
+        spell_key<NW>(dst, x, k);
+        dst[uint64_t(k) - 1 + c] = '\n';
+        if (c >= EMIT_HUGE) huge[atomicAdd(ctl + 2, 1u)] = uint32_t(v);
+      }
+      for (uint32_t q = 0; q < 32; ++q) {
+        const uint32_t m = __shfl_sync(0xFFFFFFFFu, c, int(q)), f = __shfl_sync(0xFFFFFFFFu, p, int(q));
+        char* const d = reinterpret_cast<char*>(
+            __shfl_sync(0xFFFFFFFFu, (unsigned long long)reinterpret_cast<uintptr_t>(dst), int(q)));
+        if (m > 1 && m < EMIT_HUGE) copy_bytes(d + k, chars + f + 1, m - 1, lane, 32u);
+      }
+      __syncwarp();
+      T.begin(T.dst + total);
+    }
+  }
+  T.end(buf);
+}
+
+// The later chars of the lines of EMIT_HUGE members or more, each line by the
+// whole grid.
+__global__ void __launch_bounds__(256) k_emit_huge(const uint32_t* __restrict__ head, const uint32_t* __restrict__ cnt,
+                                                   const uint32_t* __restrict__ voff, const char* __restrict__ chars,
+                                                   const unsigned long long* __restrict__ base, int k,
+                                                   char* __restrict__ out, const uint32_t* __restrict__ huge,
+                                                   uint32_t nhuge) {
+  __shared__ uint32_t scan[33];
+  for (uint32_t i = 0; i < nhuge; ++i) {
+    const uint32_t v = huge[i], c = cnt[v], p = voff[v];
+    // the line's index: its tile's first and the heads before it there
+    const uint64_t t0 = uint64_t(v) / EMIT_TILE * EMIT_TILE;
+    uint32_t before = 0;
+    for (uint64_t u = t0 + threadIdx.x; u < v; u += blockDim.x) before += head[u] == uint32_t(u);
+    uint32_t tot;
+    block_excl_scan(before, scan, &tot);
+    char* const dst = out + ((base[v / EMIT_TILE] >> 32) + tot) * uint64_t(k) + p + k;
+    for (uint64_t x = uint64_t(blockIdx.x) * EMIT_HUGE; x < c - 1u; x += uint64_t(gridDim.x) * EMIT_HUGE)
+      copy_bytes(dst + x, chars + p + 1 + x, min((unsigned long long)EMIT_HUGE, c - 1ull - x), threadIdx.x, blockDim.x);
   }
 }
 
@@ -4087,57 +4270,120 @@ int contract(Env& e, const uint64_t* d_keys, const uint32_t* succ, const uint32_
   return UC_OK;
 }
 
+// emit() and emit_in() over scratch of emit_scratch_bytes(n) bytes.  With out
+// null only the size: every member but a line's first adds one char.
+static int emit_over(cudaStream_t s, int sm_count, const uint64_t* keys, const uint32_t* head, const uint32_t* rank,
+                     uint64_t n, int k, char* out, uint64_t cap, uint64_t& out_bytes, char* scratch, uint32_t& launches,
+                     std::string& err) {
+  auto al = [](uint64_t b) { return (b + 255) & ~uint64_t(255); };
+  const uint64_t tiles = (n + EMIT_TILE - 1) / EMIT_TILE;
+  auto ck = [&](cudaError_t c, const char* what) -> int {
+    if (c == cudaSuccess) return UC_OK;
+    err = std::string(what) + ": " + cudaGetErrorString(c);
+    return int(UC_ECUDA);
+  };
+  auto take = [&](uint64_t b) {
+    char* p = scratch;
+    scratch += al(b);
+    return p;
+  };
+  // cleared: the control words (ticket, wait flag, long lines, heads), the
+  // look-back words, the member counts
+  char* z = take(256 + tiles * 8);
+  uint32_t* ctl = reinterpret_cast<uint32_t*>(z);
+  unsigned long long* heads = reinterpret_cast<unsigned long long*>(z + 16);
+  unsigned long long* st = reinterpret_cast<unsigned long long*>(z + 256);
+  unsigned long long* base = reinterpret_cast<unsigned long long*>(take((tiles + 1) * 8));
+  uint32_t* cnt = reinterpret_cast<uint32_t*>(take(n * 4));
+  uint32_t* voff = reinterpret_cast<uint32_t*>(take(n * 4));
+  uint32_t* huge = reinterpret_cast<uint32_t*>(take((n / EMIT_HUGE + 1) * 4));
+  char* chars = take(n + 16);
+  const uint64_t want = (n + 255) / 256, gcap = uint64_t(sm_count) * 16;
+  const int grid = int(std::max<uint64_t>(1, std::min(want, gcap)));
+  int r = ck(cudaMemsetAsync(z, 0, 256 + tiles * 8, s), "cudaMemsetAsync");
+  if (r) return r;
+  unsigned long long got = 0;
+  if (!out) {
+    ++launches;
+    k_count_heads<<<grid, 256, 0, s>>>(head, n, heads);
+    if ((r = ck(cudaGetLastError(), "launch"))) return r;
+    if ((r = ck(cudaMemcpyAsync(&got, heads, 8, cudaMemcpyDeviceToHost, s), "cudaMemcpyAsync"))) return r;
+    if ((r = ck(cudaStreamSynchronize(s), "cudaStreamSynchronize"))) return r;
+    out_bytes = got * uint64_t(k) + n;
+    return UC_OK;
+  }
+  if ((r = ck(cudaMemsetAsync(cnt, 0, n * 4, s), "cudaMemsetAsync"))) return r;
+  launches += 2;
+  k_count_members<<<grid, 256, 0, s>>>(head, n, cnt);
+  k_emit_scan<<<unsigned(tiles), 256, 0, s>>>(head, cnt, n, voff, base, st, ctl);
+  if ((r = ck(cudaGetLastError(), "launch"))) return r;
+  if ((r = ck(cudaMemcpyAsync(&got, base + tiles, 8, cudaMemcpyDeviceToHost, s), "cudaMemcpyAsync"))) return r;
+  uint32_t c[3] = {0, 0, 0};
+  if ((r = ck(cudaMemcpyAsync(c, ctl, 12, cudaMemcpyDeviceToHost, s), "cudaMemcpyAsync"))) return r;
+  if ((r = ck(cudaStreamSynchronize(s), "cudaStreamSynchronize"))) return r;
+  if (c[1]) {
+    err = "a bounded device wait ran out";
+    return UC_ETIMEOUT;
+  }
+  out_bytes = (got >> 32) * uint64_t(k) + (got & 0xFFFFFFFFull);
+  if (out_bytes > cap) {
+    err = "output buffer too small";
+    return UC_EINPUT;
+  }
+  launches += 2;
+  if (k <= 31) {
+    k_emit_chars<1><<<grid, 256, 0, s>>>(keys, head, rank, voff, n, k, chars);
+    k_emit_lines<1><<<unsigned(tiles), 256, 0, s>>>(keys, head, cnt, voff, chars, base, n, k, out, ctl, huge);
+  } else {
+    k_emit_chars<2><<<grid, 256, 0, s>>>(keys, head, rank, voff, n, k, chars);
+    k_emit_lines<2><<<unsigned(tiles), 256, 0, s>>>(keys, head, cnt, voff, chars, base, n, k, out, ctl, huge);
+  }
+  if ((r = ck(cudaGetLastError(), "launch"))) return r;
+  if ((r = ck(cudaMemcpyAsync(c, ctl, 12, cudaMemcpyDeviceToHost, s), "cudaMemcpyAsync"))) return r;
+  if ((r = ck(cudaStreamSynchronize(s), "cudaStreamSynchronize"))) return r;
+  if (c[2]) {
+    ++launches;
+    k_emit_huge<<<unsigned(sm_count) * 4u, 256, 0, s>>>(head, cnt, voff, chars, base, k, out, huge, c[2]);
+    if ((r = ck(cudaGetLastError(), "launch"))) return r;
+    if ((r = ck(cudaStreamSynchronize(s), "cudaStreamSynchronize"))) return r;
+  }
+  return UC_OK;
+}
+
+uint64_t emit_scratch_bytes(uint64_t n) {
+  auto al = [](uint64_t b) { return (b + 255) & ~uint64_t(255); };
+  const uint64_t tiles = (n + EMIT_TILE - 1) / EMIT_TILE;
+  return al(256 + tiles * 8) + al((tiles + 1) * 8) + 2 * al(n * 4) + al((n / EMIT_HUGE + 1) * 4) + al(n + 16);
+}
+
 int emit(Env& e, const uint64_t* d_keys, const uint32_t* succ, const uint32_t* head, const uint32_t* rank,
          uint64_t n, int k, char* out, uint64_t cap, uint64_t& out_bytes) {
   (void)succ;
   if (k < 2 || k > 63) return e.fail(UC_EINPUT, "k must be in [2, 63]");
   out_bytes = 0;
   if (n == 0) return UC_OK;
+  if (n >= 0x7FFFFFFFull) return e.fail(UC_EINPUT, "too many k-mers for 31-bit ids");
   e.reset();
-  int r = e.reserve(1, n * 16 + scan_tmp_elems(n) * 8 + 4096);
+  int r = e.reserve(1, emit_scratch_bytes(n) + 4096);
   if (r) return r;
-  uint32_t* cnt = static_cast<uint32_t*>(e.take(1, n * 4));
-  uint32_t* len = static_cast<uint32_t*>(e.take(1, n * 4));
-  unsigned long long* loff = static_cast<unsigned long long*>(e.take(1, (n + 1) * 8));
-  unsigned long long* tmp = static_cast<unsigned long long*>(e.take(1, scan_tmp_elems(n) * 8));
-  if (!tmp) return e.fail(UC_EBUDGET, "arena overflow");
-  UC_CK(cudaMemsetAsync(cnt, 0, n * 4, e.stream));
-  const int grid = grid_for(e, n, 256);
-  e.launches += 2 + 6;
-  k_count_members<<<grid, 256, 0, e.stream>>>(head, n, cnt);
-  k_line_len<<<grid, 256, 0, e.stream>>>(head, cnt, n, k, len);
-  scan_excl<uint32_t, unsigned long long>(len, n, loff, tmp, e.stream);
-  unsigned long long total = 0;
-  UC_CK(cudaMemcpyAsync(&total, loff + n, 8, cudaMemcpyDeviceToHost, e.stream));
-  UC_CK(cudaStreamSynchronize(e.stream));
-  out_bytes = total;
-  if (out) {
-    if (total > cap) return e.fail(UC_EINPUT, "output buffer too small");
-    ++e.launches;
-    if (k <= 31) k_spell<1><<<grid, 256, 0, e.stream>>>(d_keys, head, rank, cnt, loff, n, k, out);
-    else k_spell<2><<<grid, 256, 0, e.stream>>>(d_keys, head, rank, cnt, loff, n, k, out);
-    UC_CK(cudaGetLastError());
-    UC_CK(cudaStreamSynchronize(e.stream));
-  }
+  char* scratch = static_cast<char*>(e.take(1, emit_scratch_bytes(n)));
+  if (!scratch) return e.fail(UC_EBUDGET, "arena overflow");
+  std::string err;
+  r = emit_over(e.stream, e.sm_count, d_keys, head, rank, n, k, out, cap, out_bytes, scratch, e.launches, err);
   e.reset();
-  return UC_OK;
-}
-
-uint64_t emit_scratch_bytes(uint64_t n) {
-  auto al = [](uint64_t b) { return (b + 255) & ~uint64_t(255); };
-  return 2 * al(n * 4) + al((n + 1) * 8) + al(scan_tmp_elems(n) * 8);
+  return r ? e.fail(r, err) : UC_OK;
 }
 
 int emit_preload(std::string& err) {
   const void* fns[] = {
       reinterpret_cast<const void*>(k_count_members),
-      reinterpret_cast<const void*>(k_line_len),
-      reinterpret_cast<const void*>(k_scan_reduce<uint32_t, unsigned long long>),
-      reinterpret_cast<const void*>(k_scan_down<uint32_t, unsigned long long>),
-      reinterpret_cast<const void*>(k_scan_reduce<unsigned long long, unsigned long long>),
-      reinterpret_cast<const void*>(k_scan_down<unsigned long long, unsigned long long>),
-      reinterpret_cast<const void*>(k_spell<1>),
-      reinterpret_cast<const void*>(k_spell<2>)};
+      reinterpret_cast<const void*>(k_count_heads),
+      reinterpret_cast<const void*>(k_emit_scan),
+      reinterpret_cast<const void*>(k_emit_chars<1>),
+      reinterpret_cast<const void*>(k_emit_chars<2>),
+      reinterpret_cast<const void*>(k_emit_lines<1>),
+      reinterpret_cast<const void*>(k_emit_lines<2>),
+      reinterpret_cast<const void*>(k_emit_huge)};
   for (const void* f : fns) {
     cudaFuncAttributes a;
     const cudaError_t c = cudaFuncGetAttributes(&a, f);
@@ -4158,40 +4404,9 @@ int emit_in(cudaStream_t s, int sm_count, const uint64_t* d_keys, const uint32_t
     return UC_EINPUT;
   }
   if (n == 0) return UC_OK;
-  auto al = [](uint64_t b) { return (b + 255) & ~uint64_t(255); };
-  char* p = static_cast<char*>(scratch);
-  uint32_t* cnt = reinterpret_cast<uint32_t*>(p);
-  uint32_t* len = reinterpret_cast<uint32_t*>(p + al(n * 4));
-  unsigned long long* loff = reinterpret_cast<unsigned long long*>(p + 2 * al(n * 4));
-  unsigned long long* tmp = reinterpret_cast<unsigned long long*>(p + 2 * al(n * 4) + al((n + 1) * 8));
-  auto ck = [&](cudaError_t c, const char* what) -> int {
-    if (c == cudaSuccess) return UC_OK;
-    err = std::string(what) + ": " + cudaGetErrorString(c);
-    return int(UC_ECUDA);
-  };
-  const uint64_t want = (n + 255) / 256, gcap = uint64_t(sm_count) * 16;
-  const int grid = int(std::max<uint64_t>(1, std::min(want, gcap)));
-  int r = ck(cudaMemsetAsync(cnt, 0, n * 4, s), "cudaMemsetAsync");
-  if (r) return r;
-  k_count_members<<<grid, 256, 0, s>>>(head, n, cnt);
-  k_line_len<<<grid, 256, 0, s>>>(head, cnt, n, k, len);
-  scan_excl<uint32_t, unsigned long long>(len, n, loff, tmp, s);
-  unsigned long long total = 0;
-  if ((r = ck(cudaGetLastError(), "launch"))) return r;
-  if ((r = ck(cudaMemcpyAsync(&total, loff + n, 8, cudaMemcpyDeviceToHost, s), "cudaMemcpyAsync"))) return r;
-  if ((r = ck(cudaStreamSynchronize(s), "cudaStreamSynchronize"))) return r;
-  out_bytes = total;
-  if (out) {
-    if (total > cap) {
-      err = "output buffer too small";
-      return UC_EINPUT;
-    }
-    if (k <= 31) k_spell<1><<<grid, 256, 0, s>>>(d_keys, head, rank, cnt, loff, n, k, out);
-    else k_spell<2><<<grid, 256, 0, s>>>(d_keys, head, rank, cnt, loff, n, k, out);
-    if ((r = ck(cudaGetLastError(), "launch"))) return r;
-    if ((r = ck(cudaStreamSynchronize(s), "cudaStreamSynchronize"))) return r;
-  }
-  return UC_OK;
+  uint32_t launches = 0;
+  return emit_over(s, sm_count, d_keys, head, rank, n, k, out, cap, out_bytes, static_cast<char*>(scratch), launches,
+                   err);
 }
 
 uint64_t output_bound(size_t text_bytes, int k) {

@@ -301,29 +301,6 @@ __global__ void __launch_bounds__(256) k_line_plan(uint32_t* __restrict__ counts
   }
 }
 
-// n bytes from src to dst (any alignment) by `size` threads: 16-byte stores
-// of the destination, each from five source words.  Reads up to 3 bytes on
-// either side of the source bytes' words.
-__device__ __forceinline__ void copy_bytes(char* dst, const char* src, unsigned long long n, uint32_t rank,
-                                           uint32_t size) {
-  const uint32_t head = uint32_t(min((unsigned long long)((16u - uint32_t(reinterpret_cast<uintptr_t>(dst) & 15u)) & 15u), n));
-  if (rank < head) dst[rank] = src[rank];
-  dst += head;
-  src += head;
-  n -= head;
-  const uint32_t sh = 8u * uint32_t(reinterpret_cast<uintptr_t>(src) & 3u);
-  const uint32_t* w = reinterpret_cast<const uint32_t*>(reinterpret_cast<uintptr_t>(src) & ~uintptr_t(3));
-  const unsigned long long np = n >> 4;
-  for (unsigned long long p = rank; p < np; p += size) {
-    const uint32_t a = w[4 * p], b = w[4 * p + 1], c = w[4 * p + 2], d = w[4 * p + 3];
-    const uint32_t e = sh ? w[4 * p + 4] : 0u;
-    reinterpret_cast<uint4*>(dst)[p] = make_uint4(__funnelshift_r(a, b, sh), __funnelshift_r(b, c, sh),
-                                                  __funnelshift_r(c, d, sh), __funnelshift_r(d, e, sh));
-  }
-  const uint32_t rest = uint32_t(n & 15u);
-  for (uint32_t q = rank; q < rest; q += size) dst[16 * np + q] = src[16 * np + q];
-}
-
 // Records -> groups of 2^sh tiles (sh = 0: their tiles), in any order inside a
 // group.  A block takes a chunk of records, counts them per group in shared
 // memory, reserves one run per group present (cursors at cur) and writes the
