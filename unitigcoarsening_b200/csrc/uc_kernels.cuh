@@ -20,14 +20,20 @@ struct Counters {
   alignas(128) uint32_t wtile_next;
   alignas(128) unsigned long long rec_bytes;  // the records' lines
   unsigned long long cycles;
+  unsigned long long copies;         // total of the bucket counts
   uint32_t cross_count;
   uint32_t ntiles;
   uint32_t tile_next;
   uint32_t nbig;
   uint32_t err;
-  uint32_t work_next;                // scatter work counter
+  uint32_t work_mid, work_sub;       // work counters of scatter levels 2 and 3
   uint32_t nwarp, nblock;            // tiles per tier
 };
+
+// After the counters, cleared with them: the look-back words of the tile plan
+// and of the bucket offsets, each behind its ticket (uc_lookback.cuh).
+constexpr size_t PLAN_LB_WORDS = 512, SCAN_LB_WORDS = 8192 + 1;
+constexpr size_t COUNTERS_BYTES = sizeof(Counters) + (PLAN_LB_WORDS + SCAN_LB_WORDS) * 8;
 
 // A line as a record (sorted output): its k-mer big-endian (first char in the
 // top bits of hi, chars 32.. in lo), so that numeric order is byte order, and a

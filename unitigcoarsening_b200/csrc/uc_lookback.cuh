@@ -23,10 +23,11 @@ __device__ __forceinline__ void lb_publish(unsigned long long* st, uint32_t i, u
 }
 
 // Sum of the items before item i (every lane of one warp calls; item i's own
-// sum is published already).  Publishes item i's inclusive prefix.  A wait
-// that runs out, or one that meets another block's failure, sets *fail.
+// sum is published already).  Publishes item i's inclusive prefix.  A wait that
+// runs out sets `bit` in *fail; one that meets a failure (any bit) gives up.
 __device__ __forceinline__ unsigned long long lb_exclusive(unsigned long long* st, uint32_t i,
-                                                           unsigned long long own, uint32_t* fail) {
+                                                           unsigned long long own, uint32_t* fail,
+                                                           uint32_t bit = 1u) {
   const uint32_t lane = threadIdx.x & 31u;
   unsigned long long sum = 0;
   int64_t j = int64_t(i) - 1;  // nearest item of the window of 32
@@ -41,7 +42,7 @@ __device__ __forceinline__ unsigned long long lb_exclusive(unsigned long long* s
         if ((p & 1023u) == 1023u && *reinterpret_cast<volatile uint32_t*>(fail)) break;
       }
       if (!v) {
-        atomicOr(fail, 1u);
+        atomicOr(fail, bit);
         v = LB_PREFIX;
       }
     }

@@ -31,73 +31,52 @@ namespace uc {
 
 // ===================================================================== scan
 
-template <typename Tin, typename Tout>
-__global__ void k_scan_reduce(const Tin* __restrict__ in, uint64_t n, Tout* __restrict__ bsum,
-                              uint32_t per_block) {
-  __shared__ Tout sh[33];
-  const uint64_t b0 = uint64_t(blockIdx.x) * per_block;
-  Tout acc = 0;
-  for (uint64_t i = b0 + threadIdx.x; i < min(n, b0 + per_block); i += blockDim.x) acc += Tout(in[i]);
-  Tout total;
-  block_excl_scan(acc, sh, &total);
-  if (threadIdx.x == 0) bsum[blockIdx.x] = total;
-}
-
-// Exclusive scan of one block's slice, offset by the scanned block sums.
-template <typename Tin, typename Tout>
-__global__ void k_scan_down(const Tin* __restrict__ in, uint64_t n, Tout* __restrict__ out,
-                            const Tout* __restrict__ boff, uint32_t per_block, Tout* total_out) {
-  __shared__ Tout sh[33];
-  const uint64_t b0 = uint64_t(blockIdx.x) * per_block;
-  const uint64_t b1 = min(n, b0 + per_block);
-  const uint32_t per_thread = (per_block + blockDim.x - 1) / blockDim.x;
-  const uint64_t lo = b0 + uint64_t(threadIdx.x) * per_thread;
-  const uint64_t hi = min(b1, lo + per_thread);
-  Tout acc = 0;
-  for (uint64_t i = lo; i < hi; ++i) acc += Tout(in[i]);
-  Tout total;
-  Tout pre = block_excl_scan(acc, sh, &total) + boff[blockIdx.x];
-  for (uint64_t i = lo; i < hi; ++i) {
-    const Tout v = Tout(in[i]);
-    out[i] = pre;
-    pre += v;
+// Exclusive prefix sums of the bucket (or count group) counts, and their
+// total, in one look-back pass: 4096 counts per block.
+constexpr uint32_t SCAN_TILE = 4096;
+__global__ void __launch_bounds__(256) k_bucket_offsets(const uint32_t* __restrict__ in, uint64_t n,
+                                                        unsigned long long* __restrict__ out, unsigned long long* lb,
+                                                        uint32_t* err, unsigned long long* total) {
+  __shared__ unsigned long long scan[33], s_base;
+  __shared__ uint32_t s_b;
+  if (threadIdx.x == 0) s_b = atomicAdd(reinterpret_cast<uint32_t*>(lb), 1u);
+  __syncthreads();
+  const uint32_t b = s_b;
+  const uint64_t i0 = uint64_t(b) * SCAN_TILE + 16u * threadIdx.x;
+  uint32_t c[16];
+  unsigned long long sum = 0;
+#pragma unroll
+  for (int v = 0; v < 4; ++v) {  // (the counts start 256-byte aligned)
+    uint4 x = make_uint4(0u, 0u, 0u, 0u);
+    if (i0 + 4 * v + 4 <= n) {
+      x = reinterpret_cast<const uint4*>(in + i0)[v];
+    } else {
+      if (i0 + 4 * v < n) x.x = in[i0 + 4 * v];
+      if (i0 + 4 * v + 1 < n) x.y = in[i0 + 4 * v + 1];
+      if (i0 + 4 * v + 2 < n) x.z = in[i0 + 4 * v + 2];
+    }
+    c[4 * v] = x.x;
+    c[4 * v + 1] = x.y;
+    c[4 * v + 2] = x.z;
+    c[4 * v + 3] = x.w;
+    sum += uint64_t(x.x) + x.y + x.z + x.w;
   }
-  if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) {
-    out[n] = boff[blockIdx.x] + total;
-    if (total_out) *total_out = boff[blockIdx.x] + total;
+  unsigned long long tot;
+  const unsigned long long pre = block_excl_scan(sum, scan, &tot);
+  if (threadIdx.x < 32) {
+    if (threadIdx.x == 0) lb_publish(lb + 1, b, LB_SUM, tot);
+    __syncwarp();
+    const unsigned long long e = lb_exclusive(lb + 1, b, tot, err, ERR_TIMEOUT);
+    if (threadIdx.x == 0) s_base = e;
   }
-}
-
-// Exclusive scan in[0..n) -> out[0..n], out[n] = total.  tmp needs
-// scan_tmp_elems(n) elements of Tout.
-template <typename Tin, typename Tout>
-static void scan_excl(const Tin* in, uint64_t n, Tout* out, Tout* tmp, cudaStream_t s,
-                      Tout* total_out = nullptr) {
-  const uint32_t per_block = 1024 * 8;
-  const uint64_t nb = std::max<uint64_t>(1, (n + per_block - 1) / per_block);
-  Tout* bsum = tmp;
-  Tout* boff = tmp + nb;
-  Tout* rest = tmp + 2 * nb + 1;
-  k_scan_reduce<Tin, Tout><<<unsigned(nb), 1024, 0, s>>>(in, n, bsum, per_block);
-  if (nb == 1) {
-    cudaMemsetAsync(boff, 0, sizeof(Tout), s);
-  } else {
-    scan_excl<Tout, Tout>(bsum, nb, boff, rest, s);
+  __syncthreads();
+  unsigned long long p = s_base + pre;
+#pragma unroll
+  for (int q = 0; q < 16; ++q) {
+    if (i0 + q < n) out[i0 + q] = p;
+    p += c[q];
   }
-  k_scan_down<Tin, Tout><<<unsigned(nb), 1024, 0, s>>>(in, n, out, boff, per_block, total_out);
-}
-
-
-static uint64_t scan_tmp_elems(uint64_t n) {
-  uint64_t t = 0;
-  const uint64_t per_block = 1024 * 8;
-  for (;;) {
-    const uint64_t nb = std::max<uint64_t>(1, (n + per_block - 1) / per_block);
-    t += 2 * nb + 1;
-    if (nb == 1) break;
-    n = nb;
-  }
-  return t + 8;
+  if (b == gridDim.x - 1 && threadIdx.x == 0) out[n] = *total = s_base + tot;
 }
 
 // ===================================================================== pack
@@ -652,22 +631,55 @@ __global__ void __launch_bounds__(256) k_lmin_count(const uint64_t* __restrict__
 
 // ============================================================ tile planning
 
+// One tile's tier by its size: warp tiles and block tiles up to wcap and cap
+// copies, larger ones with the global scratch they need.
+struct Tiers {
+  uint32_t wcap, cap, lf;
+  int nw;
+  uint32_t *wlist, *blist, *big_list;
+  unsigned long long* big_size;
+};
+__device__ __forceinline__ void list_larger_tile(const Tiers& T, Counters* ctr, uint32_t t, uint64_t c) {
+  // (a tile's line bytes must fit 32-bit offsets: c * 64 < 2^32)
+  if (c > (1ull << 26)) {
+    atomicOr(&ctr->err, ERR_INTERNAL);
+  } else if (c <= T.cap) {
+    T.blist[atomicAdd(&ctr->nblock, 1u)] = t;
+  } else {
+    const uint32_t i = atomicAdd(&ctr->nbig, 1u);
+    T.big_list[i] = t;
+    const uint64_t ts = big_slots(c, T.lf);
+    T.big_size[i] = (c * 8ull * T.nw + ((c + 3ull) & ~3ull) * 16ull + ts * 4ull + 255ull) & ~255ull;
+  }
+}
+
 // Tiles pack consecutive whole buckets, next fit: each thread walks a run of
 // `runlen` buckets (a multiple of 16) and starts a new tile at the run's
 // first bucket, at a job's first bucket, and wherever the next bucket would
 // take the tile past `cap` copies.  A tile of several buckets therefore
 // holds at most `cap` copies; a bucket larger than `cap` sits alone.  Counts
-// and flags move 16 at a time (the arrays start 256-byte aligned).
-__global__ void k_tile_flags(const uint32_t* __restrict__ counts, uint32_t m, uint32_t cap, uint32_t jb,
-                             uint32_t runlen, uint32_t* __restrict__ flag) {
-  const uint32_t nruns = (m + runlen - 1) / runlen;
-  for (uint32_t r = blockIdx.x * blockDim.x + threadIdx.x; r < nruns; r += gridDim.x * blockDim.x) {
-    const uint32_t b0 = r * runlen, b1 = min(m, b0 + runlen);
+// move 16 at a time (the array starts 256-byte aligned).  A first walk counts
+// the run's tiles and warp tiles, a look-back numbers them, a second walk
+// writes them and, with lists, sorts them into tiers: one kernel for what took
+// six (flags, three for a scan, writing, classification).
+__global__ void __launch_bounds__(256) k_tile_plan(const uint32_t* __restrict__ counts,
+                                                   const unsigned long long* __restrict__ off, uint32_t m,
+                                                   uint32_t cap, uint32_t jb, uint32_t runlen,
+                                                   unsigned long long* __restrict__ tile_begin,
+                                                   uint32_t* __restrict__ tile_job, Tiers T, int lists,
+                                                   unsigned long long* lb, Counters* ctr) {
+  __shared__ unsigned long long scan[33], s_base;
+  __shared__ uint32_t s_b;
+  if (threadIdx.x == 0) s_b = atomicAdd(reinterpret_cast<uint32_t*>(lb), 1u);
+  __syncthreads();
+  const uint32_t r = s_b * 256u + threadIdx.x, nruns = (m + runlen - 1) / runlen;
+  const uint32_t b0 = r < nruns ? r * runlen : m, b1 = min(m, b0 + min(runlen, m - b0));
+  // open(bucket): a tile starts there; close(copies): the tile before it ends
+  auto walk = [&](auto open, auto close) {
     uint32_t run = 0;
     for (uint32_t c0 = b0; c0 < b1; c0 += 16) {
-      const bool full = c0 + 16 <= b1;
-      uint32_t c[16], f[16];
-      if (full) {
+      uint32_t c[16];
+      if (c0 + 16 <= b1) {
         const uint4* src = reinterpret_cast<const uint4*>(counts + c0);
 #pragma unroll
         for (int v = 0; v < 4; ++v) {
@@ -684,65 +696,63 @@ __global__ void k_tile_flags(const uint32_t* __restrict__ counts, uint32_t m, ui
 #pragma unroll
       for (int q = 0; q < 16; ++q) {
         const uint32_t b = c0 + uint32_t(q);
-        const bool st = (b == b0) || ((b >> jb) != ((b - 1) >> jb)) || (run + c[q] > cap);
-        f[q] = st;
-        run = st ? c[q] : run + c[q];
-      }
-      if (full) {
-        uint4* dst = reinterpret_cast<uint4*>(flag + c0);
-#pragma unroll
-        for (int v = 0; v < 4; ++v) dst[v] = make_uint4(f[4 * v], f[4 * v + 1], f[4 * v + 2], f[4 * v + 3]);
-      } else {
-#pragma unroll
-        for (int q = 0; q < 16; ++q)
-          if (c0 + q < b1) flag[c0 + q] = f[q];
+        if (b >= b1) break;
+        if (b == b0 || ((b >> jb) != ((b - 1) >> jb)) || run + c[q] > cap) {
+          if (b > b0) close(run);
+          open(b);
+          run = c[q];
+        } else {
+          run += c[q];
+        }
       }
     }
+    if (b1 > b0) close(run);
+  };
+  uint32_t nt = 0, nwt = 0;
+  walk([&](uint32_t) { ++nt; }, [&](uint32_t c) { nwt += (c && c <= T.wcap) ? 1u : 0u; });
+  // (62 bits travel: tiles and warp tiles are both below 2^31)
+  unsigned long long tot;
+  const unsigned long long pre = block_excl_scan((static_cast<unsigned long long>(nwt) << 31) | nt, scan, &tot);
+  if (threadIdx.x < 32) {
+    if (threadIdx.x == 0) lb_publish(lb + 1, s_b, LB_SUM, tot);
+    __syncwarp();
+    const unsigned long long e = lb_exclusive(lb + 1, s_b, tot, &ctr->err, ERR_TIMEOUT);
+    if (threadIdx.x == 0) s_base = e;
+  }
+  __syncthreads();
+  if (b0 >= b1) return;
+  uint32_t t = uint32_t((s_base + pre) & 0x7FFFFFFFull), w = uint32_t((s_base + pre) >> 31);
+  unsigned long long o = off[b0];
+  walk(
+      [&](uint32_t b) {
+        tile_begin[t] = o;
+        tile_job[t] = b >> jb;
+      },
+      [&](uint32_t c) {
+        if (lists && c) {
+          if (c <= T.wcap) T.wlist[w++] = t;
+          else list_larger_tile(T, ctr, t, c);
+        }
+        o += c;
+        ++t;
+      });
+  if (b1 == m) {
+    tile_begin[t] = o;
+    ctr->ntiles = t;
+    if (lists) ctr->nwarp = w;
   }
 }
 
-__global__ void k_tile_write(const uint32_t* __restrict__ flag, const uint32_t* __restrict__ fidx,
-                             const unsigned long long* __restrict__ off, uint32_t m, uint32_t jb,
-                             unsigned long long* __restrict__ tile_begin, uint32_t* __restrict__ tile_job,
-                             Counters* ctr) {
-  for (uint32_t b = blockIdx.x * blockDim.x + threadIdx.x; b < m; b += gridDim.x * blockDim.x) {
-    if (flag[b]) {
-      tile_begin[fidx[b]] = off[b];
-      tile_job[fidx[b]] = b >> jb;
-    }
-    if (b == m - 1) {
-      const uint32_t nt = fidx[b] + flag[b];
-      tile_begin[nt] = off[m];
-      ctr->ntiles = nt;
-    }
-  }
-}
-
-// Sort the tiles into tiers by size: warp tiles, block tiles and oversized
-// tiles (with the global scratch each one needs).
-__global__ void k_classify(const unsigned long long* __restrict__ tile_begin, Counters* ctr, uint32_t wcap,
-                           uint32_t cap, uint32_t* __restrict__ wlist, uint32_t* __restrict__ blist,
-                           uint32_t* __restrict__ big_list, unsigned long long* __restrict__ big_size, int nw,
-                           uint32_t lf, uint32_t t0, uint32_t t1) {
+// The tiles [t0, t1) into tiers (the streamed path's groups; the resident
+// path's tiers come with the plan).
+__global__ void k_classify(const unsigned long long* __restrict__ tile_begin, Counters* ctr, Tiers T, uint32_t t0,
+                           uint32_t t1) {
   const uint32_t nt = min(ctr->ntiles, t1);
   for (uint32_t t = t0 + blockIdx.x * blockDim.x + threadIdx.x; t < nt; t += gridDim.x * blockDim.x) {
     const uint64_t c = tile_begin[t + 1] - tile_begin[t];
-    // (a tile's line bytes must fit 32-bit offsets: c * 64 < 2^32)
-    if (tile_begin[t + 1] < tile_begin[t] || c > (1ull << 26)) {
-      atomicOr(&ctr->err, ERR_INTERNAL);
-      continue;
-    }
     if (c == 0) continue;
-    if (c <= wcap) {
-      wlist[atomicAdd(&ctr->nwarp, 1u)] = t;
-    } else if (c <= cap) {
-      blist[atomicAdd(&ctr->nblock, 1u)] = t;
-    } else {
-      const uint32_t i = atomicAdd(&ctr->nbig, 1u);
-      big_list[i] = t;
-      const uint64_t ts = big_slots(c, lf);
-      big_size[i] = (c * 8ull * nw + ((c + 3ull) & ~3ull) * 16ull + ts * 4ull + 255ull) & ~255ull;
-    }
+    if (c <= T.wcap) T.wlist[atomicAdd(&ctr->nwarp, 1u)] = t;
+    else list_larger_tile(T, ctr, t, c);
   }
 }
 
@@ -973,7 +983,7 @@ __global__ void __launch_bounds__(MID_THREADS, NW == 1 ? 2 : 1) k_scatter_mid(
   const uint32_t j0 = min(nb, threadIdx.x * per), j1 = min(nb, j0 + per);
   for (;;) {
     if (threadIdx.x == 0) {
-      const uint32_t t = atomicAdd(&ctr->work_next, 1u);
+      const uint32_t t = atomicAdd(&ctr->work_mid, 1u);
       uint32_t lo = 0, hi = mc;  // the partition p with istart[p] <= t < istart[p + 1]
       while (hi - lo > 1) {
         const uint32_t mid = (lo + hi) >> 1;
@@ -1095,7 +1105,7 @@ __global__ void __launch_bounds__(512, 2) k_scatter_sub(const uint64_t* __restri
   // CTAs per SM fit the registers)
   constexpr int PER = NW == 1 ? 8 : 4;
   for (;;) {
-    if (threadIdx.x == 0) s_sp = atomicAdd(&ctr->work_next, 1u);
+    if (threadIdx.x == 0) s_sp = atomicAdd(&ctr->work_sub, 1u);
     __syncthreads();
     const uint32_t sp = s_sp;
     if (sp >= nsub) break;
@@ -2002,6 +2012,7 @@ __global__ void __launch_bounds__(256, NW == 1 ? 4 : 3) k_tile_warp(TileParams p
   extern __shared__ __align__(16) char smem[];
   const uint32_t wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const TileMem<NW, uint16_t> m = carve<NW, uint16_t>(smem + size_t(wid) * p.wbytes, p.wcap, p.wts);
+  if (p.ctr->err & ERR_TIMEOUT) return;  // the plan did not finish
   const uint32_t nt = p.ctr->nwarp, nw = gridDim.x * (blockDim.x >> 5);
   unsigned long long rec_bytes = 0;
   uint32_t j = blockIdx.x * (blockDim.x >> 5) + wid;  // the first tile needs no counter
@@ -2023,6 +2034,7 @@ __global__ void __launch_bounds__(512) k_tile(TileParams p) {
   extern __shared__ __align__(16) char smem[];
   __shared__ uint32_t s_t;
   const TileMem<NW, uint16_t> m = carve<NW, uint16_t>(smem, p.cap, p.tslots);
+  if (p.ctr->err & ERR_TIMEOUT) return;  // the plan did not finish
   const uint32_t nt = p.ctr->nblock;
   for (;;) {
     if (threadIdx.x == 0) s_t = atomicAdd(&p.ctr->tile_next, 1u);
@@ -3627,8 +3639,8 @@ static Plan plan_buckets(const Env& e, uint64_t nmax, uint32_t njobs, int k, int
 struct Front {
   uint64_t* keys;
   uint32_t *b1, *b2, *counts, *c16, *gcount;
-  unsigned long long *boff, *cursor, *fcur, *tile_begin, *scan_tmp, *goff;
-  uint32_t *flag, *fidx, *big_list, *wlist, *blist, *tile_job;
+  unsigned long long *boff, *cursor, *fcur, *tile_begin, *goff;
+  uint32_t *big_list, *wlist, *blist, *tile_job;
   unsigned long long* big_size;
 };
 
@@ -3637,7 +3649,7 @@ static size_t front_bytes(uint64_t n, int nw, uint64_t M, bool own_keys) {
   auto add = [&](size_t b) { need += (b + 255) & ~size_t(255); };
   if (own_keys) add(n * 8 * nw);
   add(n * 4); add(n * 4); add(M * 4); add((M + 1) * 8); add(M * 8); add(M * 8); add((M + 2) * 8);
-  add(scan_tmp_elems(M) * 8); add(M * 4); add((M + 1) * 4); add(M * 4); add(M * 8);
+  add(M * 4); add(M * 8);
   add(M * 4); add(M * 4); add(M * 4);
   add((M + 1) / 2 * 4);
   add(count_groups(M) * 4); add((count_groups(M) + 1) * 8);
@@ -3653,9 +3665,6 @@ static int take_front(Env& e, uint64_t n, int nw, uint64_t M, bool own_keys, Fro
   f.cursor = static_cast<unsigned long long*>(e.take(0, M * 8));
   f.fcur = static_cast<unsigned long long*>(e.take(0, M * 8));
   f.tile_begin = static_cast<unsigned long long*>(e.take(0, (M + 2) * 8));
-  f.scan_tmp = static_cast<unsigned long long*>(e.take(0, scan_tmp_elems(M) * 8));
-  f.flag = static_cast<uint32_t*>(e.take(0, M * 4));
-  f.fidx = static_cast<uint32_t*>(e.take(0, (M + 1) * 4));
   f.big_list = static_cast<uint32_t*>(e.take(0, M * 4));
   f.big_size = static_cast<unsigned long long*>(e.take(0, M * 8));
   f.wlist = static_cast<uint32_t*>(e.take(0, M * 4));
@@ -3668,20 +3677,37 @@ static int take_front(Env& e, uint64_t n, int nw, uint64_t M, bool own_keys, Fro
   return UC_OK;
 }
 
-// counts -> offsets (M entries: buckets or count groups); returns the total
-// number of copies (host sync).
-static int bucket_offsets(Env& e, const Front& f, const uint32_t* counts, uint64_t M, unsigned long long* offs,
-                          uint64_t& copies) {
-  e.launches += 6;
-  scan_excl<uint32_t, unsigned long long>(counts, M, offs, f.scan_tmp, e.stream);
-  unsigned long long tot = 0;
-  UC_CK(cudaMemcpyAsync(&tot, offs + M, 8, cudaMemcpyDeviceToHost, e.stream));
-  UC_CK(cudaStreamSynchronize(e.stream));
-  copies = tot;
+// Clears the counters and the look-back words behind them.
+static int clear_counters(Env& e) {
+  UC_CK(cudaMemsetAsync(e.ctr, 0, COUNTERS_BYTES, e.stream));
   return UC_OK;
 }
+static unsigned long long* plan_lb(const Env& e) { return reinterpret_cast<unsigned long long*>(e.ctr + 1); }
+static unsigned long long* scan_lb(const Env& e) { return plan_lb(e) + PLAN_LB_WORDS; }
+
+// counts -> offsets (M entries: buckets or count groups) and their total in
+// the counters.
+static int launch_bucket_offsets(Env& e, const uint32_t* counts, uint64_t M, unsigned long long* offs) {
+  const uint64_t nb = (M + SCAN_TILE - 1) / SCAN_TILE;
+  if (nb + 1 > SCAN_LB_WORDS) return e.fail(UC_EINTERNAL, "bucket count beyond the look-back words");
+  ++e.launches;
+  k_bucket_offsets<<<unsigned(nb), 256, 0, e.stream>>>(counts, M, offs, scan_lb(e), &e.ctr->err, &e.ctr->copies);
+  UC_CK(cudaGetLastError());
+  return UC_OK;
+}
+// The same, and the total (host sync).  Clears the scan's look-back words
+// first: a run may take offsets more than once.
+static int bucket_offsets(Env& e, const uint32_t* counts, uint64_t M, unsigned long long* offs, uint64_t& copies) {
+  UC_CK(cudaMemsetAsync(scan_lb(e), 0, SCAN_LB_WORDS * 8, e.stream));
+  int r = launch_bucket_offsets(e, counts, M, offs);
+  if (r) return r;
+  r = e.read_ctr();
+  if (r) return r;
+  copies = e.h_ctr->copies;
+  return (e.h_ctr->err & ERR_TIMEOUT) ? e.check_err(e.h_ctr) : UC_OK;
+}
 static int bucket_offsets(Env& e, const Front& f, uint64_t M, uint64_t& copies) {
-  return bucket_offsets(e, f, f.counts, M, f.boff, copies);
+  return bucket_offsets(e, f.counts, M, f.boff, copies);
 }
 
 // Level split of the scatter: 2^mcb coarse partitions of 2^fb buckets.
@@ -3692,23 +3718,22 @@ static void scatter_split(uint32_t bbits, uint32_t& mcb, uint32_t& fb) {
 
 static size_t scatter_stage_bytes(uint64_t copies, int nw) { return copies * (8ull * nw + 8ull); }
 
-// tile plan + scatter of every k-mer into its bucket(s).  stage: staging
-// records for level 1 (scatter_stage_bytes).
-// Tiles from the bucket counts: next-fit runs of whole buckets.
-static int plan_tiles(Env& e, const Front& f, const Plan& P) {
+static Tiers tiers_of(const Front& f, const Plan& P, int nw) {
+  return Tiers{P.wcap, P.cap, P.lf, nw, f.wlist, f.blist, f.big_list, f.big_size};
+}
+// Tiles from the bucket counts: next-fit runs of whole buckets.  lists: sorted
+// into their tiers too.
+static int plan_tiles(Env& e, const Front& f, const Plan& P, int nw, bool lists) {
   const uint64_t M = P.M;
-  const int gm = grid_for(e, M, 256);
-  e.launches += 2 + 6;
-  {
-    // about 256 threads per SM; each run ends a tile, so runs stay long
-    // where there are enough buckets
-    const uint64_t want = (M + uint64_t(e.sm_count) * 256 - 1) / (uint64_t(e.sm_count) * 256);
-    const uint32_t runlen = uint32_t(std::min<uint64_t>(512, std::max<uint64_t>(16, (want + 15) & ~uint64_t(15))));
-    k_tile_flags<<<grid_for(e, (M + runlen - 1) / runlen, 256), 256, 0, e.stream>>>(f.counts, uint32_t(M), P.pack,
-                                                                                     P.jb, runlen, f.flag);
-  }
-  scan_excl<uint32_t, uint32_t>(f.flag, M, f.fidx, reinterpret_cast<uint32_t*>(f.scan_tmp), e.stream);
-  k_tile_write<<<gm, 256, 0, e.stream>>>(f.flag, f.fidx, f.boff, uint32_t(M), P.jb, f.tile_begin, f.tile_job, e.ctr);
+  ++e.launches;
+  // about 256 threads per SM; each run ends a tile, so runs stay long where
+  // there are enough buckets
+  const uint64_t want = (M + uint64_t(e.sm_count) * 256 - 1) / (uint64_t(e.sm_count) * 256);
+  const uint32_t runlen = uint32_t(std::min<uint64_t>(512, std::max<uint64_t>(16, (want + 15) & ~uint64_t(15))));
+  const uint64_t nb = ((M + runlen - 1) / runlen + 255) / 256;
+  if (nb + 1 > PLAN_LB_WORDS) return e.fail(UC_EINTERNAL, "bucket count beyond the look-back words");
+  k_tile_plan<<<unsigned(nb), 256, 0, e.stream>>>(f.counts, f.boff, uint32_t(M), P.pack, P.jb, runlen, f.tile_begin,
+                                                   f.tile_job, tiers_of(f, P, nw), lists ? 1 : 0, plan_lb(e), e.ctr);
   UC_CK(cudaGetLastError());
   return UC_OK;
 }
@@ -3780,7 +3805,6 @@ static int scatter_begin(Env& e, const Front& f, const Plan& P, int nw, char* r1
   if (!r0) r0 = allow_max_smem(e, k_scatter_sub<1>);
   if (!r0) r0 = allow_max_smem(e, k_scatter_sub<2>);
   if (r0) return r0;
-  UC_CK(cudaMemsetAsync(&e.ctr->cross_count, 0, 4, e.stream));
   e.launches += 1;
   k_coarse_init<<<grid_for(e, sc.mc, 256), 256, 0, e.stream>>>(sc.goff, sc.fb - sc.cg, sc.mc, f.cursor);
   UC_CK(cudaGetLastError());
@@ -3834,7 +3858,6 @@ static int scatter_finish(Env& e, const Front& f, const Scatter& sc, uint64_t*& 
     e.launches += 3;
     k_mid_items<<<1, 256, 0, e.stream>>>(sc.goff, sc.fb - sc.cg, sc.mc, item_start);
     k_coarse_init<<<grid_for(e, sc.nsub, 256), 256, 0, e.stream>>>(sc.goff, sc.sb - sc.cg, sc.nsub, f.fcur);
-    UC_CK(cudaMemsetAsync(&e.ctr->work_next, 0, 4, e.stream));
     if (nw == 1)
       k_scatter_mid<1><<<e.sm_count * o2, MID_THREADS, sm2, e.stream>>>(sc.k1, sc.l1, sc.b1, sc.goff, sc.cg,
                                                                         item_start, sc.fb, sc.sb, sc.mc, f.fcur,
@@ -3849,7 +3872,6 @@ static int scatter_finish(Env& e, const Front& f, const Scatter& sc, uint64_t*& 
   const uint64_t* ik = sc.mid ? sc.k2 : sc.k1;
   const uint32_t* il = sc.mid ? sc.l2 : sc.l1;
   const uint32_t* ib = sc.mid ? sc.b2 : sc.b1;
-  UC_CK(cudaMemsetAsync(&e.ctr->work_next, 0, 4, e.stream));
   e.launches += 1;
   const size_t sm3 = size_t(sc.cap3) * (8 * nw + 4);
   int o3 = 0;
@@ -3876,8 +3898,7 @@ static int scatter_finish(Env& e, const Front& f, const Scatter& sc, uint64_t*& 
 static int classify_tiles(Env& e, const Front& f, const Plan& P, int nw, uint32_t t0 = 0,
                           uint32_t t1 = 0xFFFFFFFFu) {
   ++e.launches;
-  k_classify<<<grid_for(e, P.M, 256), 256, 0, e.stream>>>(f.tile_begin, e.ctr, P.wcap, P.cap, f.wlist, f.blist,
-                                                           f.big_list, f.big_size, nw, P.lf, t0, t1);
+  k_classify<<<grid_for(e, P.M, 256), 256, 0, e.stream>>>(f.tile_begin, e.ctr, tiers_of(f, P, nw), t0, t1);
   UC_CK(cudaGetLastError());
   return UC_OK;
 }
@@ -3894,9 +3915,7 @@ static int plan_and_scatter(Env& e, const Front& f, const Plan& P, uint64_t n, i
   if (r) return r;
   r = scatter_finish(e, f, sc, pkeys, plink);
   if (r) return r;
-  r = plan_tiles(e, f, P);
-  if (r) return r;
-  return classify_tiles(e, f, P, nw);
+  return plan_tiles(e, f, P, nw, true);
 }
 
 template <int NW, int KC>
@@ -3988,7 +4007,8 @@ int find_edges(Env& e, const uint64_t* d_keys, uint64_t n, int k, int l, uint64_
   r = take_front(e, n, nw, P.M, false, f);
   if (r) return r;
   f.keys = const_cast<uint64_t*>(d_keys);
-  UC_CK(cudaMemsetAsync(e.ctr, 0, sizeof(Counters), e.stream));
+  r = clear_counters(e);
+  if (r) return r;
   UC_CK(cudaMemsetAsync(f.counts, 0, P.M * 4, e.stream));
   ++e.launches;
   if (nw == 1) k_lmin_count<1><<<grid_for(e, n, 256), 256, 0, e.stream>>>(d_keys, n, k, P.l_used, seed, P.jb, f.b1, f.b2, f.counts);
@@ -4650,7 +4670,8 @@ static int compact_jobs(Env& e, uint32_t njobs, const char* const* texts, const 
   const uint64_t G = P.M >> P.cg;
   uint32_t* gcount = P.cg ? f.gcount : f.counts;
   unsigned long long* goff = P.cg ? f.goff : f.boff;
-  UC_CK(cudaMemsetAsync(e.ctr, 0, sizeof(Counters), e.stream));
+  r = clear_counters(e);
+  if (r) return r;
   UC_CK(cudaMemsetAsync(gcount, 0, G * 4, e.stream));
   UC_CK(cudaMemsetAsync(jd.jcross, 0, njobs * 4, e.stream));
   UC_CK(cudaMemcpyAsync(jd.tab, J.data(), njobs * sizeof(JobTab), cudaMemcpyHostToDevice, e.stream));
@@ -4677,7 +4698,7 @@ static int compact_jobs(Env& e, uint32_t njobs, const char* const* texts, const 
   cudaEventRecord(e.ev[1], e.stream);
   if (e.after_pack) e.after_pack();
   uint64_t copies = 0;
-  r = bucket_offsets(e, f, gcount, G, goff, copies);
+  r = bucket_offsets(e, gcount, G, goff, copies);
   if (r) return r;
   std::vector<uint32_t> xc(njobs);
   UC_CK(cudaMemcpyAsync(xc.data(), jd.jcross, njobs * 4, cudaMemcpyDeviceToHost, e.stream));
@@ -4917,7 +4938,8 @@ int compact_streamed(Env& e, const char* h_text, size_t bytes, int k, int l, cha
   r = job_buffers(e, 1);
   if (r) return r;
   JobDev jd = job_dev(e, 1);
-  UC_CK(cudaMemsetAsync(e.ctr, 0, sizeof(Counters), e.stream));
+  r = clear_counters(e);
+  if (r) return r;
   UC_CK(cudaMemsetAsync(f.c16, 0, (P.M + 1) / 2 * 4, e.stream));
   UC_CK(cudaMemsetAsync(jd.jcross, 0, 4, e.stream));
   FuseArgs fz;
@@ -4990,7 +5012,7 @@ int compact_streamed(Env& e, const char* h_text, size_t bytes, int k, int l, cha
   if (segchars > SEG_OFF_MASK) return e.fail(UC_EINPUT, "segment chars beyond the 40-bit offsets");
   // the tiles, grouped: whole tiles up to group_copies copies (a larger tile
   // alone); a group's closed lines fit its copies' lines
-  r = plan_tiles(e, f, P);
+  r = plan_tiles(e, f, P, nw, false);
   if (r) return r;
   r = e.read_ctr();
   if (r) return r;

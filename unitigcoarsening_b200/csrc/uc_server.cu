@@ -463,7 +463,7 @@ uc_status uc_server_create(const uc_server_config* cfg, uc_server** out) {
     e.tune = s->cfg.tuning;
     cudaError_t ce = cudaStreamCreateWithFlags(&e.stream, cudaStreamNonBlocking);
     e.own_stream = true;
-    if (ce == cudaSuccess) ce = cudaMalloc(&e.ctr, sizeof(uc::Counters));
+    if (ce == cudaSuccess) ce = cudaMalloc(&e.ctr, uc::COUNTERS_BYTES);
     if (ce == cudaSuccess) ce = cudaMallocHost(&e.h_ctr, sizeof(uc::Counters));
     for (int q = 0; q < uc::Env::NEV && ce == cudaSuccess; ++q) ce = cudaEventCreate(&e.ev[q]);
     // job table for the largest batch, allocated once
