@@ -197,8 +197,7 @@ class Compactor:
         self.close()
 
     def _bind_stream(self):
-        with torch.cuda.device(self.device):
-            s = torch.cuda.current_stream().cuda_stream
+        s = torch.cuda.current_stream(self.device).cuda_stream
         self._L.uc_ctx_set_stream(self._h, ctypes.c_void_p(s))
 
     def _check(self, st: int):
@@ -305,7 +304,7 @@ class Compactor:
         nb = ctypes.c_uint64()
         st = Stats()
         self._check(self._L.uc_compact_device(self._h, _ptr(text), text.numel(), k, l, _ptr(out), out.numel(),
-                                              ctypes.byref(nb), ctypes.byref(st)))
+                                              ctypes.byref(nb), ctypes.byref(st) if stats else None))
         res = out[: nb.value]
         return (res, st.as_dict()) if stats else res
 
@@ -323,7 +322,7 @@ class Compactor:
         ln = (ctypes.c_uint64 * max(nj, 1))()
         st = Stats()
         self._check(self._L.uc_compact_batch(self._h, nj, ptrs, sizes, k, l, _ptr(out), out.numel(), off, ln,
-                                             ctypes.byref(st)))
+                                             ctypes.byref(st) if stats else None))
         res = [out[off[j]: off[j] + ln[j]] for j in range(nj)]
         return (res, st.as_dict()) if stats else res
 
@@ -343,7 +342,7 @@ class Compactor:
         ob = ctypes.c_size_t()
         st = Stats()
         self._check(self._L.uc_compact_host(self._h, tp, tn, k, l, ctypes.c_void_p(out.data_ptr()), out.numel(),
-                                            ctypes.byref(ob), ctypes.byref(st)))
+                                            ctypes.byref(ob), ctypes.byref(st) if stats else None))
         res = out[: ob.value]
         return (res, st.as_dict()) if stats else res
 
@@ -400,7 +399,7 @@ class Compactor:
         olen = (ctypes.c_size_t * max(nj, 1))()
         st = Stats()
         self._bind_stream()
-        self._check(self._L.uc_compact_host_many(self._h, nj, ptrs, sizes, k, l, optr, ocap, olen, ctypes.byref(st)))
+        self._check(self._L.uc_compact_host_many(self._h, nj, ptrs, sizes, k, l, optr, ocap, olen, ctypes.byref(st) if stats else None))
         res = [outs[j][: olen[j]] for j in range(nj)]
         return (res, st.as_dict()) if stats else res
 

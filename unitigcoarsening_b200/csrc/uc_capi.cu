@@ -198,7 +198,7 @@ uc_status uc_ctx_create(int device, size_t hbm_budget, uc_ctx** out) {
   c->env.budget = hbm_budget ? hbm_budget : size_t(double(fr) * 0.9);
   e = cudaStreamCreateWithFlags(&c->env.stream, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaMalloc(&c->env.ctr, uc::COUNTERS_BYTES);
-  if (e == cudaSuccess) e = cudaMallocHost(&c->env.h_ctr, sizeof(uc::Counters));
+  if (e == cudaSuccess) e = cudaMallocHost(&c->env.h_ctr, sizeof(uc::Counters) + uc::Env::HOST_IO);
   for (int i = 0; i < uc::Env::NEV && e == cudaSuccess; ++i) e = cudaEventCreate(&c->env.ev[i]);
   if (e != cudaSuccess) {
     cudaGetLastError();

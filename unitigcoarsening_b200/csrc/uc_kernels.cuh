@@ -28,6 +28,7 @@ struct Counters {
   uint32_t err;
   uint32_t work_mid, work_sub;       // work counters of scatter levels 2 and 3
   uint32_t nwarp, nblock;            // tiles per tier
+  uint32_t walked, left;             // line walk: segments on lines written, lines left
 };
 
 // After the counters, cleared with them: the look-back words of the tile plan

@@ -2276,14 +2276,19 @@ __device__ __forceinline__ void line_end(LineOut& L) {
 // the head; the first WALK_REG records stay in registers), the warp
 // reserves its lines' bytes, and the walk copies each segment's chars into
 // the line (records past the kept ones read again, now mostly in L2).  A line that goes on past WALK_CAP segments is left to the ranking
-// path: its head goes to longl.  wst[0] counts the segments of the lines
-// written (those with ids below nx), wst[1] the lines left.  cap <=
+// path: its head goes to longl.  walked counts the segments of the lines
+// written (those with ids below nx), left the lines left.  cap <=
 // WALK_CAP (smaller only to test the ranking path).
 __global__ void __launch_bounds__(256) k_walk_emit(uint32_t H, const SegRec* __restrict__ seg, uint32_t nx, int k,
                                                    const JobTab* __restrict__ jobs, unsigned long long* __restrict__ jout,
                                                    const char* __restrict__ segchars, char* __restrict__ out,
                                                    uint32_t cap, uint32_t* __restrict__ longl, uint32_t lcap,
-                                                   uint32_t* wst, Counters* ctr) {
+                                                   int guard, Counters* ctr) {
+  // guard: enqueued before it was known that the tiles are complete
+  __shared__ uint32_t skip;
+  if (threadIdx.x == 0) skip = guard ? ctr->nbig | ctr->err : 0u;
+  __syncthreads();
+  if (skip) return;
   __shared__ uint32_t sc[33];
   const uint64_t stride = uint64_t(gridDim.x) * blockDim.x;
   uint32_t walked = 0;
@@ -2317,7 +2322,7 @@ __global__ void __launch_bounds__(256) k_walk_emit(uint32_t H, const SegRec* __r
     const uint32_t job = done ? uint32_t(r.off_job >> SEG_OFF_BITS) : JOB_NONE;
     const unsigned long long o = warp_reserve(jout, job, done ? len + 1u : 0ull);
     if (live && !done) {
-      const uint32_t i = atomicAdd(wst + 1, 1u);
+      const uint32_t i = atomicAdd(&ctr->left, 1u);
       if (i < lcap) longl[i] = uint32_t(h);
       else atomicOr(&ctr->err, ERR_INTERNAL);  // a left line holds more than cap cross ids
     }
@@ -2356,7 +2361,7 @@ __global__ void __launch_bounds__(256) k_walk_emit(uint32_t H, const SegRec* __r
   }
   uint32_t tot;
   block_excl_scan(walked, sc, &tot);
-  if (threadIdx.x == 0 && tot) atomicAdd(wst, tot);
+  if (threadIdx.x == 0 && tot) atomicAdd(&ctr->walked, tot);
 }
 
 // The ranking's first state from the segment records (when the walk left
@@ -3372,7 +3377,7 @@ static void launch_pack_as(Env& e, const JobTab* jobs, const JobTab& J, uint32_t
   const size_t sm = pack_smem(pcap);
   if (sm > 48 * 1024) allow_max_smem(e, k_pack<NW, FUSE, MULTI, KC>);
   int occ = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_pack<NW, FUSE, MULTI, KC>, 256, sm);
+  occupancy(e, occ, k_pack<NW, FUSE, MULTI, KC>, 256, sm);
   const int grid = int(std::max<uint64_t>(1, std::min<uint64_t>(nblocks, uint64_t(e.sm_count) * std::max(1, occ))));
   ++e.launches;
   k_pack<NW, FUSE, MULTI, KC><<<grid, 256, sm, e.stream>>>(jobs, J, njobs, nblocks, starts, k, keys, &e.ctr->err, fz.l,
@@ -3440,11 +3445,13 @@ static JobDev job_dev(Env& e, uint32_t njobs) {
 // Text -> keys for one job (and, with fz, buckets + counts).  Fixed-width
 // lines are packed directly; any other layout indexes the line starts first
 // (back arena, which must be empty).
+// defer: fixed-width lines are only enqueued; the caller reads the counters
+// and, on ERR_LAYOUT, clears them and calls again with J.fixed = 0.
 static int pack_single(Env& e, const char* d_text, size_t bytes, int k, uint64_t* d_keys, const FuseArgs* fz,
-                       JobTab& J, JobTab* jdev) {
+                       JobTab& J, JobTab* jdev, bool defer = false) {
   const uint8_t* text = reinterpret_cast<const uint8_t*>(d_text);
   const uint64_t n = J.n, body = J.body, end = J.end;
-  UC_CK(cudaMemsetAsync(&e.ctr->err, 0, 4, e.stream));
+  if (!defer) UC_CK(cudaMemsetAsync(&e.ctr->err, 0, 4, e.stream));  // (cleared with the counters)
   if (n == 0) {
     if (end > body) return e.fail(UC_EINPUT, "header count differs from the number of lines");
     return UC_OK;
@@ -3457,6 +3464,7 @@ static int pack_single(Env& e, const char* d_text, size_t bytes, int k, uint64_t
     if (nw == 1) launch_pack<1>(e, jdev, &J, 1, nblocks, nullptr, k, d_keys, fz);
     else launch_pack<2>(e, jdev, &J, 1, nblocks, nullptr, k, d_keys, fz);
     UC_CK(cudaGetLastError());
+    if (defer) return UC_OK;
     st = e.read_ctr();
     if (st) return st;
     if (e.h_ctr->err & ERR_LAYOUT) {
@@ -3501,13 +3509,41 @@ static int pack_single(Env& e, const char* d_text, size_t bytes, int k, uint64_t
   return UC_OK;
 }
 
-// Host view of one job's text: count line, body offset, end, layout.
+// Host view of one job's text: count line, body offset, end, layout.  The
+// first and the last bytes come back in one wait; a longer count line or tail
+// is read by parse_header and text_end.
 static int host_job(Env& e, const char* d_text, size_t bytes, int k, JobTab& J) {
   uint64_t n = 0, body = 0, end = 0;
-  int st = parse_header(e, d_text, bytes, n, body);
-  if (st) return st;
-  st = text_end(e, d_text, bytes, body, end);
-  if (st) return st;
+  constexpr size_t W = 256;
+  const size_t w = std::min<size_t>(bytes, W);
+  char *head = e.h_io(), *tail = e.h_io() + W;
+  if (w) {
+    UC_CK(cudaMemcpyAsync(head, d_text, w, cudaMemcpyDeviceToHost, e.stream));
+    UC_CK(cudaMemcpyAsync(tail, d_text + bytes - w, w, cudaMemcpyDeviceToHost, e.stream));
+    UC_CK(cudaStreamSynchronize(e.stream));
+  }
+  size_t p = 0;
+  while (p < w && (head[p] == ' ' || head[p] == '\t' || head[p] == '\r')) ++p;
+  bool known = p < w && head[p] >= '0' && head[p] <= '9';
+  for (; known && p < w && head[p] >= '0' && head[p] <= '9'; ++p) {
+    n = n * 10 + uint64_t(head[p] - '0');
+    if (n > 0xFFFFFFFEull) known = false;
+  }
+  while (p < w && head[p] != '\n') ++p;
+  known = known && (p < w || w == bytes);
+  if (known) {
+    body = (p < w) ? p + 1 : w;
+  } else {
+    const int st = parse_header(e, d_text, bytes, n, body);
+    if (st) return st;
+  }
+  end = bytes;
+  const size_t at = bytes - w;  // of the tail
+  while (end > body && end > at && (tail[end - at - 1] == '\n' || tail[end - at - 1] == '\r')) --end;
+  if (end > body && end == at) {  // nothing but line breaks there
+    const int st = text_end(e, d_text, bytes, body, end);
+    if (st) return st;
+  }
   J = JobTab{};
   J.text = reinterpret_cast<const uint8_t*>(d_text);
   J.tbytes = bytes;
@@ -3529,7 +3565,6 @@ int pack(Env& e, const char* d_text, size_t bytes, int k, uint64_t* d_keys, uint
   r = job_buffers(e, 1);
   if (r) return r;
   JobDev jd = job_dev(e, 1);
-  UC_CK(cudaMemcpyAsync(jd.tab, &J, sizeof(JobTab), cudaMemcpyHostToDevice, e.stream));
   r = pack_single(e, d_text, bytes, k, d_keys, nullptr, J, jd.tab);
   e.reset();
   return r;
@@ -3819,8 +3854,9 @@ static int scatter_l1(Env& e, const Front& f, const Scatter& sc, const uint64_t*
   const size_t sm1 = size_t(2 * chunk) * (8 * nw + 8) + size_t(sc.mc) * 16 + 16;
   // one wave of resident CTAs (the chunks are strided statically)
   int o1 = 0;
-  if (nw == 1) UC_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o1, k_scatter_coarse<1>, COARSE_THREADS, sm1));
-  else UC_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o1, k_scatter_coarse<2>, COARSE_THREADS, sm1));
+  if (const int ro = nw == 1 ? occupancy(e, o1, k_scatter_coarse<1>, COARSE_THREADS, sm1)
+                             : occupancy(e, o1, k_scatter_coarse<2>, COARSE_THREADS, sm1))
+    return ro;
   if (o1 < 1) return e.fail(UC_EINTERNAL, "scatter kernel does not fit an SM");
   const int g1 = int(std::max<uint64_t>(1, std::min<uint64_t>((n + chunk - 1) / chunk,
                                                               uint64_t(e.sm_count) * uint64_t(o1))));
@@ -3852,8 +3888,9 @@ static int scatter_finish(Env& e, const Front& f, const Scatter& sc, uint64_t*& 
     uint32_t* item_start = reinterpret_cast<uint32_t*>(f.cursor + sc.mc);
     const size_t sm2 = size_t(MID_CHUNK) * (8 * nw + 8) + size_t(nb) * 16 + 4 + size_t(sc.mc + 1) * 4;
     int o2 = 0;
-    if (nw == 1) UC_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o2, k_scatter_mid<1>, MID_THREADS, sm2));
-    else UC_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o2, k_scatter_mid<2>, MID_THREADS, sm2));
+    if (const int ro = nw == 1 ? occupancy(e, o2, k_scatter_mid<1>, MID_THREADS, sm2)
+                               : occupancy(e, o2, k_scatter_mid<2>, MID_THREADS, sm2))
+      return ro;
     if (o2 < 1) return e.fail(UC_EINTERNAL, "scatter kernel does not fit an SM");
     e.launches += 3;
     k_mid_items<<<1, 256, 0, e.stream>>>(sc.goff, sc.fb - sc.cg, sc.mc, item_start);
@@ -3875,8 +3912,9 @@ static int scatter_finish(Env& e, const Front& f, const Scatter& sc, uint64_t*& 
   e.launches += 1;
   const size_t sm3 = size_t(sc.cap3) * (8 * nw + 4);
   int o3 = 0;
-  if (nw == 1) UC_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o3, k_scatter_sub<1>, 512, sm3));
-  else UC_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o3, k_scatter_sub<2>, 512, sm3));
+  if (const int ro = nw == 1 ? occupancy(e, o3, k_scatter_sub<1>, 512, sm3)
+                             : occupancy(e, o3, k_scatter_sub<2>, 512, sm3))
+    return ro;
   if (o3 < 1) return e.fail(UC_EINTERNAL, "scatter kernel does not fit an SM");
   const int g3 = int(std::min<uint64_t>(sc.nsub, uint64_t(e.sm_count) * uint64_t(o3)));
   if (nw == 1)
@@ -3927,69 +3965,77 @@ static int run_tiles(Env& e, TileParams& tp, const Front& f, uint32_t threads) {
   if (tp.wcap) {
     const int r0 = allow_max_smem(e, k_tile_warp<NW, KC>);
     if (r0) return r0;
-    UC_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&wocc, k_tile_warp<NW, KC>, 256, wsm));
+    if (const int ro = occupancy(e, wocc, k_tile_warp<NW, KC>, 256, wsm)) return ro;
     if (wocc < 1) return e.fail(UC_EINTERNAL, "warp tile kernel does not fit an SM");
   }
-  cudaEventRecord(e.ev[8], e.stream);
+  if (e.timed) cudaEventRecord(e.ev[8], e.stream);
   if (tp.wcap) {
     ++e.launches;
     k_tile_warp<NW, KC><<<e.sm_count * wocc, 256, wsm, e.stream>>>(tp);
     UC_CK(cudaGetLastError());
   }
-  cudaEventRecord(e.ev[9], e.stream);
+  if (e.timed) cudaEventRecord(e.ev[9], e.stream);
   const size_t smem = tile_bytes(NW, tp.cap, tp.tslots);
   const int r1 = allow_max_smem(e, k_tile<NW, KC>);
   if (r1) return r1;
   int occ = 0;
-  UC_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_tile<NW, KC>, int(threads), smem));
+  if (const int ro = occupancy(e, occ, k_tile<NW, KC>, int(threads), smem)) return ro;
   if (occ < 1) return e.fail(UC_EINTERNAL, "tile kernel does not fit an SM");
   ++e.launches;
   k_tile<NW, KC><<<e.sm_count * occ, threads, smem, e.stream>>>(tp);
   UC_CK(cudaGetLastError());
-  cudaEventRecord(e.ev[5], e.stream);
-  e.tiles_timed = true;
-  // oversized tiles: one CTA each in global scratch
-  int st = e.read_ctr();
-  if (st) return st;
-  if (e.h_ctr->err) return e.check_err(e.h_ctr);
-  const uint32_t nbig = e.h_ctr->nbig;
-  if (nbig) {
-    std::vector<unsigned long long> sz(nbig), off(nbig);
-    UC_CK(cudaMemcpyAsync(sz.data(), f.big_size, nbig * 8, cudaMemcpyDeviceToHost, e.stream));
-    UC_CK(cudaStreamSynchronize(e.stream));
-    unsigned long long tot = 0;
-    for (uint32_t i = 0; i < nbig; ++i) {
-      off[i] = tot;
-      tot += sz[i];
-    }
-    const size_t want = size_t(tot) + size_t(nbig) * 8 + 4096;
-    char* big = nullptr;
-    if (e.pool) {
-      big = static_cast<char*>(e.take(1, want));
-      if (!big) return e.fail(UC_EBUDGET, "scratch for oversized buckets exceeds the pool slice");
-    } else {
-      const int r = e.big_scratch(want, big, "scratch for oversized buckets");
-      if (r) return r;
-    }
-    unsigned long long* d_off = reinterpret_cast<unsigned long long*>(big);
-    char* scratch = big + ((size_t(nbig) * 8 + 255) & ~size_t(255));
-    UC_CK(cudaMemcpyAsync(d_off, off.data(), nbig * 8, cudaMemcpyHostToDevice, e.stream));
-    tp.big_list = f.big_list;
-    tp.big_scratch = scratch;
-    tp.big_off = d_off;
-    ++e.launches;
-    k_tile_big<NW><<<nbig, 1024, 0, e.stream>>>(tp);
-    UC_CK(cudaGetLastError());
-    UC_CK(cudaStreamSynchronize(e.stream));
+  if (e.timed) cudaEventRecord(e.ev[5], e.stream);
+  e.tiles_timed = e.timed;
+  return UC_OK;
+}
+
+// The oversized tiles, one CTA each in global scratch: nbig of them, known
+// once the tile kernels' counters are read.  Waits for them.
+static int run_big_tiles(Env& e, TileParams& tp, const Front& f, int nw, uint32_t nbig) {
+  std::vector<unsigned long long> sz(nbig), off(nbig);
+  UC_CK(cudaMemcpyAsync(sz.data(), f.big_size, nbig * 8, cudaMemcpyDeviceToHost, e.stream));
+  UC_CK(cudaStreamSynchronize(e.stream));
+  unsigned long long tot = 0;
+  for (uint32_t i = 0; i < nbig; ++i) {
+    off[i] = tot;
+    tot += sz[i];
   }
+  const size_t want = size_t(tot) + size_t(nbig) * 8 + 4096;
+  char* big = nullptr;
+  if (e.pool) {
+    big = static_cast<char*>(e.take(1, want));
+    if (!big) return e.fail(UC_EBUDGET, "scratch for oversized buckets exceeds the pool slice");
+  } else {
+    const int r = e.big_scratch(want, big, "scratch for oversized buckets");
+    if (r) return r;
+  }
+  unsigned long long* d_off = reinterpret_cast<unsigned long long*>(big);
+  char* scratch = big + ((size_t(nbig) * 8 + 255) & ~size_t(255));
+  UC_CK(cudaMemcpyAsync(d_off, off.data(), nbig * 8, cudaMemcpyHostToDevice, e.stream));
+  tp.big_list = f.big_list;
+  tp.big_scratch = scratch;
+  tp.big_off = d_off;
+  ++e.launches;
+  if (nw == 1) k_tile_big<1><<<nbig, 1024, 0, e.stream>>>(tp);
+  else k_tile_big<2><<<nbig, 1024, 0, e.stream>>>(tp);
+  UC_CK(cudaGetLastError());
+  UC_CK(cudaStreamSynchronize(e.stream));
   return UC_OK;
 }
 
 // The tile kernels for tp.k: compile-time k = 31 (64-bit keys) and 63
 // (128-bit keys), the generic form otherwise.
-static int run_tiles_k(Env& e, TileParams& tp, const Front& f, uint32_t threads, int nw) {
+static int launch_tiles(Env& e, TileParams& tp, const Front& f, uint32_t threads, int nw) {
   if (nw == 1) return tp.k == 31 ? run_tiles<1, 31>(e, tp, f, threads) : run_tiles<1, 0>(e, tp, f, threads);
   return tp.k == 63 ? run_tiles<2, 63>(e, tp, f, threads) : run_tiles<2, 0>(e, tp, f, threads);
+}
+// Every tier, the oversized tiles included (waits once for the counters).
+static int run_tiles_k(Env& e, TileParams& tp, const Front& f, uint32_t threads, int nw) {
+  int r = launch_tiles(e, tp, f, threads, nw);
+  if (!r) r = e.read_ctr();
+  if (r) return r;
+  if (e.h_ctr->err) return e.check_err(e.h_ctr);
+  return e.h_ctr->nbig ? run_big_tiles(e, tp, f, nw, e.h_ctr->nbig) : UC_OK;
 }
 
 int find_edges(Env& e, const uint64_t* d_keys, uint64_t n, int k, int l, uint64_t seed, uint32_t* succ,
@@ -4013,9 +4059,11 @@ int find_edges(Env& e, const uint64_t* d_keys, uint64_t n, int k, int l, uint64_
   ++e.launches;
   if (nw == 1) k_lmin_count<1><<<grid_for(e, n, 256), 256, 0, e.stream>>>(d_keys, n, k, P.l_used, seed, P.jb, f.b1, f.b2, f.counts);
   else k_lmin_count<2><<<grid_for(e, n, 256), 256, 0, e.stream>>>(d_keys, n, k, P.l_used, seed, P.jb, f.b1, f.b2, f.counts);
-  uint64_t copies = 0;
-  r = bucket_offsets(e, f, P.M, copies);
+  r = launch_bucket_offsets(e, f.counts, P.M, f.boff);
+  if (!r) r = e.read_ctr();
   if (r) return r;
+  if (e.h_ctr->err) return e.check_err(e.h_ctr);
+  const uint64_t copies = e.h_ctr->copies;
   r = e.reserve(1, 2 * scatter_stage_bytes(copies, nw) + 4096);
   if (r) return r;
   char* region1 = static_cast<char*>(e.take(1, scatter_stage_bytes(copies, nw)));
@@ -4042,9 +4090,11 @@ int find_edges(Env& e, const uint64_t* d_keys, uint64_t n, int k, int l, uint64_
   tp.mode = 0;
   tp.succ = succ;
   tp.pred = pred;
+  e.timed = false;
   r = run_tiles_k(e, tp, f, 512, nw);
   if (r) return r;
-  r = e.read_ctr();
+  // (oversized tiles may have set the error flag after the counters were read)
+  if (e.h_ctr->nbig) r = e.read_ctr();
   e.reset();
   if (r) return r;
   return e.check_err(e.h_ctr);
@@ -4179,7 +4229,7 @@ static int hec_contract(Env& e, HecPool& h, uint32_t R, const uint32_t* prev, co
   else k_hec_level0<<<grid, 256, 0, e.stream>>>(h, prev, next, w, nmax);
   // every block resident (they meet)
   int occ = 0;
-  UC_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_hec_all, int(HEC_THREADS), 0));
+  if (const int ro = occupancy(e, occ, k_hec_all, int(HEC_THREADS), 0)) return ro;
   const uint64_t want = (nmax + HEC_THREADS - 1) / HEC_THREADS;
   const unsigned g = unsigned(std::max<uint64_t>(1, std::min<uint64_t>(want, uint64_t(e.sm_count) * std::max(1, occ))));
   void* args[] = {&h, &R, &X, &oncycle};
@@ -4462,8 +4512,18 @@ static uint64_t long_cap(const Env& e, uint64_t X) { return X / walk_cap(e) + 64
 // lines it leaves and for cycles, ranking (pointer jumping, or HEC with
 // pointer jumping when its rounds run out), line lengths at the heads, one
 // reservation per line, the segment copies, and the rare segment cycles.
+// The walk alone: enqueued (counters walked and left zero before).
+static int launch_walk(Env& e, const StitchBufs& b, uint64_t X, uint64_t Hp, int k, const JobDev& jd, char* out,
+                       bool guard) {
+  ++e.launches;
+  k_walk_emit<<<grid_for(e, Hp, 256), 256, 0, e.stream>>>(uint32_t(Hp), b.seg, uint32_t(X), k, jd.tab, jd.jout, b.segc,
+                                                          out, walk_cap(e), b.longl, b.lcap, guard ? 1 : 0, e.ctr);
+  UC_CK(cudaGetLastError());
+  return UC_OK;
+}
+// walked: the walk is done and its counters are in h_ctr.
 static int run_stitch(Env& e, const StitchBufs& b, uint64_t X, uint64_t Hp, int k, int nw, bool want_hec,
-                      uint32_t RH, const JobDev& jd, char* out, uint32_t& rounds) {
+                      uint32_t RH, const JobDev& jd, char* out, uint32_t& rounds, bool walked = false) {
   rounds = 0;
   const uint32_t S = uint32_t(X + Hp), nx = uint32_t(X), H = uint32_t(Hp);
   SegRec* seg = b.seg;
@@ -4473,7 +4533,6 @@ static int run_stitch(Env& e, const StitchBufs& b, uint64_t X, uint64_t Hp, int 
   uint8_t* oncyc = b.oncyc;
   unsigned long long* lbase = b.lbase;
   HecPool hp = b.hp;
-  uint32_t* wst = rcnt + 48;  // the walk's counters (the rounds use at most 35 list counts)
   int r = UC_OK;
   const int gs = grid_for(e, S, 256);
   uint32_t *act = nullptr, *left = nullptr;
@@ -4481,15 +4540,15 @@ static int run_stitch(Env& e, const StitchBufs& b, uint64_t X, uint64_t Hp, int 
   if (!want_hec) {
     // the line walk writes every line its head reaches within WALK_CAP
     // segments; the rest is ranked from the first state, built below
-    UC_CK(cudaMemsetAsync(wst, 0, 8, e.stream));
-    ++e.launches;
-    k_walk_emit<<<grid_for(e, H, 256), 256, 0, e.stream>>>(H, seg, nx, k, jd.tab, jd.jout, segc, out, walk_cap(e),
-                                                           b.longl, b.lcap, wst, e.ctr);
-    uint32_t hw[2] = {0, 0};
-    UC_CK(cudaMemcpyAsync(hw, wst, 8, cudaMemcpyDeviceToHost, e.stream));
-    UC_CK(cudaStreamSynchronize(e.stream));
-    if (hw[0] == nx && hw[1] == 0) return UC_OK;
-    nlong = std::min(hw[1], b.lcap);
+    if (!walked) {
+      UC_CK(cudaMemsetAsync(&e.ctr->walked, 0, 8, e.stream));  // walked, left
+      r = launch_walk(e, b, X, Hp, k, jd, out, false);
+      if (!r) r = e.read_ctr();
+      if (r) return r;
+      if (e.h_ctr->err) return e.check_err(e.h_ctr);
+    }
+    if (e.h_ctr->walked == nx && e.h_ctr->left == 0) return UC_OK;
+    nlong = std::min(e.h_ctr->left, b.lcap);
     ++e.launches;
     k_set_u32<<<1, 1, 0, e.stream>>>(rcnt, nx);
   }
@@ -4622,6 +4681,11 @@ static int compact_jobs(Env& e, uint32_t njobs, const char* const* texts, const 
   e.reset();
   e.launches = 0;
   e.graph_nodes = 0;
+  e.timed = st != nullptr;
+  e.tiles_timed = false;
+  auto mark = [&](int i) {
+    if (e.timed) cudaEventRecord(e.ev[i], e.stream);
+  };
   int r = job_buffers(e, njobs);
   if (r) return r;
   JobDev jd = job_dev(e, njobs);
@@ -4673,9 +4737,21 @@ static int compact_jobs(Env& e, uint32_t njobs, const char* const* texts, const 
   r = clear_counters(e);
   if (r) return r;
   UC_CK(cudaMemsetAsync(gcount, 0, G * 4, e.stream));
-  UC_CK(cudaMemsetAsync(jd.jcross, 0, njobs * 4, e.stream));
-  UC_CK(cudaMemcpyAsync(jd.tab, J.data(), njobs * sizeof(JobTab), cudaMemcpyHostToDevice, e.stream));
-  cudaEventRecord(e.ev[0], e.stream);
+  // the per-job counters (jout, jseg, jclosed, jcross) in one piece
+  const size_t jbytes = size_t(reinterpret_cast<char*>(jd.jcross + njobs) - reinterpret_cast<char*>(jd.jout));
+  UC_CK(cudaMemsetAsync(jd.jout, 0, jbytes, e.stream));
+  // their copy on the host: pinned where it fits
+  std::vector<char> jhost(jbytes <= Env::HOST_IO - 1024 ? 0 : jbytes);
+  char* const jh = jhost.empty() ? e.h_io() + 1024 : jhost.data();
+  auto on_host = [&](const void* p) { return jh + (static_cast<const char*>(p) - reinterpret_cast<char*>(jd.jout)); };
+  // counters and per-job counters to the host (waits)
+  auto read_back = [&]() -> int {
+    UC_CK(cudaMemcpyAsync(jh, jd.jout, jbytes, cudaMemcpyDeviceToHost, e.stream));
+    return e.read_ctr();
+  };
+  if (njobs > 1)
+    UC_CK(cudaMemcpyAsync(jd.tab, J.data(), njobs * sizeof(JobTab), cudaMemcpyHostToDevice, e.stream));
+  mark(0);
   FuseArgs fz;
   fz.l = P.l_used;
   fz.seed = e.seed;
@@ -4688,22 +4764,33 @@ static int compact_jobs(Env& e, uint32_t njobs, const char* const* texts, const 
   fz.jcross = jd.jcross;
   fz.M = P.M;
   if (njobs == 1) {
-    r = pack_single(e, texts[0], bytes[0], k, f.keys, &fz, J[0], jd.tab);
+    r = pack_single(e, texts[0], bytes[0], k, f.keys, &fz, J[0], jd.tab, J[0].fixed != 0);
     if (r) return r;
   } else if (N > 0) {
     if (nw == 1) launch_pack<1>(e, jd.tab, nullptr, njobs, lb, nullptr, k, f.keys, &fz);
     else launch_pack<2>(e, jd.tab, nullptr, njobs, lb, nullptr, k, f.keys, &fz);
     UC_CK(cudaGetLastError());
   }
-  cudaEventRecord(e.ev[1], e.stream);
-  if (e.after_pack) e.after_pack();
-  uint64_t copies = 0;
-  r = bucket_offsets(e, gcount, G, goff, copies);
+  if (e.timed || e.after_pack) cudaEventRecord(e.ev[1], e.stream);
+  r = launch_bucket_offsets(e, gcount, G, goff);
+  if (!r) r = read_back();
   if (r) return r;
-  std::vector<uint32_t> xc(njobs);
-  UC_CK(cudaMemcpyAsync(xc.data(), jd.jcross, njobs * 4, cudaMemcpyDeviceToHost, e.stream));
-  r = e.read_ctr();
-  if (r) return r;
+  if (njobs == 1 && J[0].fixed && (e.h_ctr->err & ERR_LAYOUT)) {
+    // not k chars and a break per line after all: again, from the line starts
+    J[0].fixed = 0;
+    r = clear_counters(e);
+    if (r) return r;
+    UC_CK(cudaMemsetAsync(gcount, 0, G * 4, e.stream));
+    UC_CK(cudaMemsetAsync(jd.jout, 0, jbytes, e.stream));
+    r = pack_single(e, texts[0], bytes[0], k, f.keys, &fz, J[0], jd.tab);
+    if (r) return r;
+    if (e.timed || e.after_pack) cudaEventRecord(e.ev[1], e.stream);
+    r = launch_bucket_offsets(e, gcount, G, goff);
+    if (!r) r = read_back();
+    if (r) return r;
+  }
+  const uint64_t copies = e.h_ctr->copies;
+  const uint32_t* xc = reinterpret_cast<const uint32_t*>(on_host(jd.jcross));
   uint64_t xsum = 0;
   for (uint32_t j = 0; j < njobs; ++j) xsum += xc[j];
   if (copies != N + xsum && !e.h_ctr->err) return e.fail(UC_EINTERNAL, "bucket counts disagree with the copies");
@@ -4711,6 +4798,7 @@ static int compact_jobs(Env& e, uint32_t njobs, const char* const* texts, const 
     if (e.h_ctr->err & ERR_LAYOUT) return e.fail(UC_EINPUT, "a k-mer line is shorter than k");
     return e.check_err(e.h_ctr);
   }
+  if (e.after_pack) e.after_pack();
   const uint64_t X = copies - N;
   // segment ids: [0, X) the segments that start at a cross k-mer's S-only
   // copy; then each job's head pool (a line's first open segment ends at a
@@ -4724,7 +4812,15 @@ static int compact_jobs(Env& e, uint32_t njobs, const char* const* texts, const 
   const uint64_t Sp = X + Hp;
   if (Sp >= 0x7FFFFFF0ull) return e.fail(UC_EINPUT, "too many cross-tile segments");
   if (njobs >= (1u << (64 - SEG_OFF_BITS))) return e.fail(UC_EINPUT, "too many jobs in one batch");
-  UC_CK(cudaMemcpyAsync(jd.tab, J.data(), njobs * sizeof(JobTab), cudaMemcpyHostToDevice, e.stream));
+  if (njobs == 1) {
+    // (pinned: the copy does not wait)
+    static_assert(sizeof(JobTab) <= 512, "the job fits the pinned area");
+    JobTab* hj = reinterpret_cast<JobTab*>(e.h_io() + 512);
+    *hj = J[0];
+    UC_CK(cudaMemcpyAsync(jd.tab, hj, sizeof(JobTab), cudaMemcpyHostToDevice, e.stream));
+  } else {
+    UC_CK(cudaMemcpyAsync(jd.tab, J.data(), njobs * sizeof(JobTab), cudaMemcpyHostToDevice, e.stream));
+  }
   const uint64_t segchars = Sp * uint64_t(k) + copies + 64;
   if (segchars > SEG_OFF_MASK) return e.fail(UC_EINPUT, "segment chars beyond the 40-bit offsets");
   const uint32_t R = 64;
@@ -4766,13 +4862,11 @@ static int compact_jobs(Env& e, uint32_t njobs, const char* const* texts, const 
   }
   // unused head-pool ids keep length 0 (every id below X gets a record)
   UC_CK(cudaMemsetAsync(seg + X, 0, Hp * sizeof(SegRec), e.stream));
-  UC_CK(cudaMemsetAsync(jd.jout, 0, njobs * 8, e.stream));
-  UC_CK(cudaMemsetAsync(jd.jseg, 0, njobs * 4, e.stream));
   uint64_t* pkeys = nullptr;
   uint32_t* plink = nullptr;
   r = plan_and_scatter(e, f, P, N, nw, 0, region1, region2, copies, pkeys, plink, P.cg > 0);
   if (r) return r;
-  cudaEventRecord(e.ev[2], e.stream);
+  mark(2);
 
   TileParams tp{};
   tp.pkeys = pkeys;
@@ -4808,25 +4902,40 @@ static int compact_jobs(Env& e, uint32_t njobs, const char* const* texts, const 
     tp.rec_bits = rbits;
   }
   const uint32_t threads = e.tune.tile_threads ? e.tune.tile_threads : 512;
-  r = run_tiles_k(e, tp, f, threads, nw);
-  if (r) return r;
-  cudaEventRecord(e.ev[3], e.stream);
-  r = e.read_ctr();
-  if (r) return r;
-  if (e.h_ctr->err) return e.check_err(e.h_ctr);
-  UC_CK(cudaMemcpyAsync(jd.jclosed, jd.jout, njobs * 8, cudaMemcpyDeviceToDevice, e.stream));
+  // The tiles, and behind them, before the host knows that none is oversized,
+  // the line walk (which does nothing when one is): one wait for both.
   uint32_t rounds = 0;
   StitchBufs sbuf{seg, Xr, segc, act0, act1, oncyc, hlen, lbase, longl, uint32_t(long_cap(e, X)), rcnt, hp};
-  r = run_stitch(e, sbuf, X, Hp, k, nw, want_hec, RH, jd, out, rounds);
-  if (r) return r;
-  UC_CK(cudaGetLastError());
-  cudaEventRecord(e.ev[4], e.stream);
-  std::vector<unsigned long long> jo(njobs), jc(st ? njobs : 0);
-  UC_CK(cudaMemcpyAsync(jo.data(), jd.jout, njobs * 8, cudaMemcpyDeviceToHost, e.stream));
-  if (st) UC_CK(cudaMemcpyAsync(jc.data(), jd.jclosed, njobs * 8, cudaMemcpyDeviceToHost, e.stream));
-  r = e.read_ctr();
+  auto closed_now = [&]() -> int {
+    if (st) UC_CK(cudaMemcpyAsync(jd.jclosed, jd.jout, njobs * 8, cudaMemcpyDeviceToDevice, e.stream));
+    mark(3);
+    return UC_OK;
+  };
+  bool stitched = false;
+  r = launch_tiles(e, tp, f, threads, nw);
+  if (!r) r = closed_now();
+  if (!r && !want_hec) r = launch_walk(e, sbuf, X, Hp, k, jd, out, true);
+  mark(4);
+  if (!r) r = read_back();
   if (r) return r;
   if (e.h_ctr->err) return e.check_err(e.h_ctr);
+  const uint32_t nbig = e.h_ctr->nbig;
+  if (nbig) {
+    r = run_big_tiles(e, tp, f, nw, nbig);
+    if (!r) r = closed_now();
+    if (r) return r;
+  } else {
+    stitched = !want_hec && e.h_ctr->walked == X && e.h_ctr->left == 0;
+  }
+  if (!stitched) {
+    r = run_stitch(e, sbuf, X, Hp, k, nw, want_hec, RH, jd, out, rounds, !nbig && !want_hec);
+    mark(4);
+    if (!r) r = read_back();
+    if (r) return r;
+    if (e.h_ctr->err) return e.check_err(e.h_ctr);
+  }
+  const unsigned long long* jo = reinterpret_cast<const unsigned long long*>(on_host(jd.jout));
+  const unsigned long long* jc = reinterpret_cast<const unsigned long long*>(on_host(jd.jclosed));
   uint64_t total = 0;
   if (recs) {
     recs->n = uint32_t(e.h_ctr->rec_slots);
@@ -4922,6 +5031,7 @@ int compact_streamed(Env& e, const char* h_text, size_t bytes, int k, int l, cha
   e.reset();
   e.launches = 0;
   e.graph_nodes = 0;
+  e.timed = true;
   if (n == 0) return UC_OK;
   if (!chunk_lines) chunk_lines = 64ull << 20;
   if (!group_copies) group_copies = 256ull << 20;

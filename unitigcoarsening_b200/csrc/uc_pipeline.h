@@ -3,6 +3,7 @@
 #include <cstdint>
 #include <functional>
 #include <string>
+#include <vector>
 
 #include <cuda_runtime.h>
 
@@ -32,9 +33,21 @@ struct Env {
   char* jbuf = nullptr;     // job table and per-job counters (grow only)
   size_t jcap = 0;
   Counters* ctr = nullptr;    // device
-  Counters* h_ctr = nullptr;  // pinned host mirror
+  Counters* h_ctr = nullptr;  // pinned host mirror, and HOST_IO bytes more behind it
+  static constexpr size_t HOST_IO = 2048;
+  char* h_io() const { return reinterpret_cast<char*>(h_ctr + 1); }
   static constexpr int NEV = 10;
   cudaEvent_t ev[NEV] = {};
+  bool timed = true;         // the call wants phase times (events are recorded)
+  // kernels whose shared-memory limit is raised, and occupancies asked for
+  std::vector<const void*> smem_raised;
+  struct Occ {
+    const void* fn;
+    int threads;
+    size_t smem;
+    int blocks;
+  };
+  std::vector<Occ> occ;
   bool tiles_timed = false;  // ev[8]/ev[9]/ev[5] bracket the warp and block tile kernels
   uc_tuning tune{};
   uint64_t seed = 0x00C0FFEE5EEDull;
@@ -53,8 +66,8 @@ struct Env {
   // whole-job calls (compact_device and the paths built on it) leave the
   // lines in byte order
   bool sorted = false;
-  // called by the fused path once the pack kernels are enqueued and ev[1]
-  // recorded after them: from then on the job's text is no longer read, so
+  // called by the fused path once the job is packed (its layout is confirmed)
+  // and ev[1] recorded after the pack kernels: from then on the job's text is no longer read, so
   // a host pipeline can upload the next job's text into the same buffer
   std::function<void()> after_pack;
   // failure injection (uc_ctx_set_faults); zeros = off
@@ -81,16 +94,33 @@ struct Env {
     if (_e != cudaSuccess) return e.fail(UC_ECUDA, std::string(#call) + ": " + cudaGetErrorString(_e)); \
   } while (0)
 
-// Let a kernel take all the dynamic shared memory an SM offers a block.  The
-// attribute is process-wide, so it is always set to the same maximum: a
-// per-call size would let one host thread lower it under another thread's
-// launch (concurrent contexts and server lanes).
+// Let a kernel take all the dynamic shared memory an SM offers a block (asked
+// for once per context).  The attribute is process-wide, so it is always set
+// to the same maximum: a per-call size would let one host thread lower it
+// under another thread's launch (concurrent contexts and server lanes).
 template <class K>
 int allow_max_smem(Env& e, K kernel) {
+  const void* fn = reinterpret_cast<const void*>(kernel);
+  for (const void* f : e.smem_raised)
+    if (f == fn) return UC_OK;
   cudaFuncAttributes a{};
   UC_CK(cudaFuncGetAttributes(&a, kernel));
   UC_CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              e.smem_optin - int(a.sharedSizeBytes)));
+  e.smem_raised.push_back(fn);
+  return UC_OK;
+}
+// Resident blocks per SM of a launch (asked for once per context and shape).
+template <class K>
+int occupancy(Env& e, int& blocks, K kernel, int threads, size_t smem) {
+  const void* fn = reinterpret_cast<const void*>(kernel);
+  for (const Env::Occ& o : e.occ)
+    if (o.fn == fn && o.threads == threads && o.smem == smem) {
+      blocks = o.blocks;
+      return UC_OK;
+    }
+  UC_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, kernel, threads, smem));
+  if (e.occ.size() < 256) e.occ.push_back(Env::Occ{fn, threads, smem, blocks});
   return UC_OK;
 }
 

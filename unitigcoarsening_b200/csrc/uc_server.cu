@@ -464,7 +464,7 @@ uc_status uc_server_create(const uc_server_config* cfg, uc_server** out) {
     cudaError_t ce = cudaStreamCreateWithFlags(&e.stream, cudaStreamNonBlocking);
     e.own_stream = true;
     if (ce == cudaSuccess) ce = cudaMalloc(&e.ctr, uc::COUNTERS_BYTES);
-    if (ce == cudaSuccess) ce = cudaMallocHost(&e.h_ctr, sizeof(uc::Counters));
+    if (ce == cudaSuccess) ce = cudaMallocHost(&e.h_ctr, sizeof(uc::Counters) + uc::Env::HOST_IO);
     for (int q = 0; q < uc::Env::NEV && ce == cudaSuccess; ++q) ce = cudaEventCreate(&e.ev[q]);
     // job table for the largest batch, allocated once
     const size_t jb = size_t(s->cfg.max_batch) * (sizeof(uc::JobTab) + 4 * 8) + 1024;

@@ -811,7 +811,7 @@ int sort_lines_rw(Env& e, char* out, uint64_t bytes, int k, const LineRecs& pre)
   const size_t sm_recs = (LR_CHUNK / (uint32_t(k) + 1u) + 2u) * 2u;
   const size_t sm_tile = tile_smem<RW>(k);
   int occ = 0;
-  UC_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_line_recs<RW>, 256, sm_recs));
+  if (const int ro = occupancy(e, occ, k_line_recs<RW>, 256, sm_recs)) return ro;
   e.launches += 2;
   if (bytes) ++e.launches;
   if (bytes) k_line_recs<RW><<<grid(nchunks, occ), 256, sm_recs, e.stream>>>(out, bytes, k, bits, ra, counts, longs, huge, sc);
@@ -831,12 +831,13 @@ int sort_lines_rw(Env& e, char* out, uint64_t bytes, int k, const LineRecs& pre)
   }
   r = allow_max_smem(e, k_line_tiles<RW>);
   if (r) return r;
-  UC_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_line_tiles<RW>, int(TILE_THREADS), sm_tile));
+  if (const int ro = occupancy(e, occ, k_line_tiles<RW>, int(TILE_THREADS), sm_tile)) return ro;
   if (occ < 1) return e.fail(UC_EINTERNAL, "line tile kernel does not fit an SM");
   k_line_tiles<RW><<<grid(ntmax, occ), TILE_THREADS, sm_tile, e.stream>>>(from, to, tile, bits, out, k, longs, keep,
                                                                          st_tile, sc);
   UC_CK(cudaGetLastError());
-  SortCtr h;
+  static_assert(sizeof(SortCtr) <= Env::HOST_IO, "the counters fit the pinned area");
+  SortCtr& h = *reinterpret_cast<SortCtr*>(e.h_io());
   UC_CK(cudaMemcpyAsync(&h, sc, sizeof h, cudaMemcpyDeviceToHost, e.stream));
   UC_CK(cudaStreamSynchronize(e.stream));
   if (h.fail & 1u) return e.fail(UC_ETIMEOUT, "a bounded device wait ran out (sorted output)");
