@@ -1844,8 +1844,9 @@ __device__ void process_tile(const TileParams& p, const TileMem<NW, IT>& m, uint
     for (uint32_t i = G::rank(); i < c; i += G::size()) {
       const uint64_t r = roles(skey(m, i));
       const uint32_t id = p.plink[beg + i];
-      if (r & ROLE_S) p.succ[id] = (m.A[i] == NONE_I) ? NONE : p.plink[beg + m.A[i]];
-      if (r & ROLE_P) p.pred[id] = (m.P[i] == NONE_I) ? NONE : p.plink[beg + m.P[i]];
+      // (both arrays hold NONE: only links are stored)
+      if ((r & ROLE_S) && m.A[i] != NONE_I) p.succ[id] = p.plink[beg + m.A[i]];
+      if ((r & ROLE_P) && m.P[i] != NONE_I) p.pred[id] = p.plink[beg + m.P[i]];
     }
     return;
   }
@@ -4090,6 +4091,13 @@ int find_edges(Env& e, const uint64_t* d_keys, uint64_t n, int k, int l, uint64_
   tp.mode = 0;
   tp.succ = succ;
   tp.pred = pred;
+  // The tiles' stores go to random ids, four bytes to a sector of 32, so the
+  // values that need none (about half of them: a neighbour of a canonical
+  // k-mer is as likely as not to be stored the other way round) are written as
+  // a stream beforehand.  16.3M k-mers: tile kernel 815 -> 507 us, for 24 of
+  // streaming.
+  UC_CK(cudaMemsetAsync(succ, 0xFF, n * 4, e.stream));
+  UC_CK(cudaMemsetAsync(pred, 0xFF, n * 4, e.stream));
   e.timed = false;
   r = run_tiles_k(e, tp, f, 512, nw);
   if (r) return r;
