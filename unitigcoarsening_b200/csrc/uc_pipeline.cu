@@ -2950,6 +2950,125 @@ __global__ void k_cycle_list(const uint8_t* __restrict__ oncycle, uint64_t n,
 
 // ======================================================= phase-API helpers
 
+// Contraction by ranking from the predecessors: every vertex first walks up to
+// RANK_STEPS of them, and one that meets a head on the way is done.  K-mers of a
+// canonical set keep each neighbour with probability about a half, so lines
+// are short and few vertices are left (1 in 2^RANK_STEPS), whose pointer and
+// distance go to X and whose ids go to the list that k_rank_rest works off.
+// The walk is a chain of dependent 4-byte gathers from the predecessors,
+// which L2 holds (65 MB at 16M k-mers), so a thread walks four vertices at a
+// time; pointer jumping from the first state wrote and gathered (pointer,
+// distance) pairs, twice the bytes and past L2.  16.3M k-mers: 134 us, and 29 for
+// the rest, where the first state, the rounds and the split of the pairs took
+// 92, 323 and 50.
+// head[v] == NONE: not ranked yet.
+constexpr uint32_t RANK_STEPS = 8;
+__global__ void __launch_bounds__(256) k_rank_walk(const uint32_t* __restrict__ pred, uint64_t n,
+                                                   uint32_t* __restrict__ head, uint32_t* __restrict__ rank,
+                                                   unsigned long long* __restrict__ X, uint32_t* __restrict__ act,
+                                                   uint32_t* act_count) {
+  __shared__ uint32_t sc[33];
+  // whole blocks iterate together (block_append needs every thread)
+  for (uint64_t s0 = uint64_t(blockIdx.x) * 1024u; s0 < n; s0 += uint64_t(gridDim.x) * 1024u) {
+    uint32_t p[4], h[4], d[4];
+#pragma unroll
+    for (uint32_t q = 0; q < 4; ++q) {
+      const uint64_t v = s0 + q * 256u + threadIdx.x;
+      h[q] = uint32_t(v);
+      d[q] = 0;
+      p[q] = v < n ? pred[v] : NONE;
+    }
+#pragma unroll 1
+    for (uint32_t i = 0; i < RANK_STEPS; ++i) {
+      if ((p[0] & p[1] & p[2] & p[3]) == NONE) break;
+#pragma unroll
+      for (uint32_t q = 0; q < 4; ++q) {
+        if (p[q] != NONE) {
+          h[q] = p[q];
+          ++d[q];
+          p[q] = pred[h[q]];
+        }
+      }
+    }
+    uint32_t open = 0;
+#pragma unroll
+    for (uint32_t q = 0; q < 4; ++q) {
+      const uint64_t v = s0 + q * 256u + threadIdx.x;
+      if (v >= n) continue;
+      if (p[q] == NONE) {
+        head[v] = h[q];
+        rank[v] = d[q];
+      } else {
+        head[v] = NONE;
+        X[v] = pk(h[q], d[q]);
+        ++open;
+      }
+    }
+    // (most blocks have some open vertex, all of them few)
+    uint32_t slot = block_append(act_count, open, sc);
+    if (open) {
+#pragma unroll
+      for (uint32_t q = 0; q < 4; ++q)
+        if (p[q] != NONE) act[slot++] = uint32_t(s0 + q * 256u + threadIdx.x);
+    }
+  }
+}
+
+// The vertices left by k_rank_walk: rounds of pointer jumping over ever
+// shorter lists, in one cooperative kernel whose blocks meet after each round
+// and that ends at the first empty list (a launch per round ran all
+// 2 + log2(n) of them, 2.4 us each when empty).  A vertex whose pointer is
+// ranked takes its head; one whose pointer is not jumps to where that one
+// points.  rank is stored before head, so whoever sees the head sees the rank.
+// Lists open after the last round hold cycles (and what leads into one): count
+// in cnt[rounds].
+__global__ void __launch_bounds__(1024, 2) k_rank_rest(unsigned long long* X, uint32_t* head, uint32_t* rank,
+                                                       uint32_t* list0, uint32_t* list1, uint32_t* cnt,
+                                                       uint32_t rounds, uint32_t* bar, uint32_t* err) {
+  __shared__ uint32_t sc[33];
+  uint32_t gen = 0;
+  volatile unsigned long long* const vX = X;
+  volatile uint32_t *const vh = head, *const vr = rank;
+  for (uint32_t r = 0; r < rounds; ++r) {
+    const uint32_t na = *reinterpret_cast<volatile uint32_t*>(cnt + r);
+    if (na == 0) return;
+    volatile uint32_t* const in = (r & 1) ? list1 : list0;
+    uint32_t* const out = (r & 1) ? list0 : list1;
+    // whole blocks iterate together (block_append needs every thread)
+    for (uint64_t j0 = uint64_t(blockIdx.x) * blockDim.x; j0 < na; j0 += uint64_t(gridDim.x) * blockDim.x) {
+      const uint64_t j = j0 + threadIdx.x;
+      bool keep = false;
+      uint32_t s = 0;
+      if (j < na) {
+        s = in[j];
+        const unsigned long long v = vX[s];
+        const uint32_t p = pk_p(v), hp = vh[p];
+        if (hp != NONE) {
+          __threadfence();
+          vr[s] = vr[p] + pk_o(v);
+          __threadfence();
+          vh[s] = hp;
+        } else {
+          const unsigned long long u = vX[p];
+          vX[s] = pk(pk_p(u), pk_o(v) + pk_o(u));
+          keep = true;
+        }
+      }
+      const uint32_t slot = block_append(cnt + r + 1, keep ? 1u : 0u, sc);
+      if (keep) out[slot] = s;
+    }
+    if (!grid_meet(bar, gen, err)) return;
+  }
+  const uint32_t na = *reinterpret_cast<volatile uint32_t*>(cnt + rounds);
+  volatile uint32_t* const in = (rounds & 1) ? list1 : list0;
+  for (uint64_t j = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; j < na; j += uint64_t(gridDim.x) * blockDim.x) {
+    const uint32_t s = in[j];
+    const unsigned long long v = vX[s];
+    rank[s] = pk_o(v);
+    head[s] = pk_p(v);
+  }
+}
+
 __global__ void k_head_rank(const unsigned long long* __restrict__ X, uint64_t n,
                             uint32_t* __restrict__ head, uint32_t* __restrict__ rank) {
   for (uint64_t v = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; v < n;
@@ -4166,14 +4285,19 @@ static int run_graph(Env& e, int slot, uint64_t key, F&& body) {
   return UC_OK;
 }
 
+static uint32_t rank_rounds(uint64_t nmax) {
+  uint32_t r = 2;
+  for (uint64_t t = 1; t < nmax; t <<= 1) ++r;
+  return r;
+}
+
 // prefilled: X already holds a state (written by the tiles and the line
 // walk) and the first round runs over the ids [0, cnt[0]), cnt[0] set on the
 // device before.
 static int rank_lists(Env& e, const uint32_t* prev, const uint32_t* w, uint64_t nmax,
                       unsigned long long* X, uint32_t* act0, uint32_t* act1, uint32_t* cnt, uint32_t& rounds,
                       uint32_t*& act_final, uint32_t*& cnt_final, bool prefilled = false) {
-  rounds = 2;
-  for (uint64_t t = 1; t < nmax; t <<= 1) ++rounds;
+  rounds = rank_rounds(nmax);
   const int grid = grid_for(e, nmax ? nmax : 1, 256);
   if (prefilled) {
     UC_CK(cudaMemsetAsync(cnt + 1, 0, rounds * 4, e.stream));
@@ -4324,15 +4448,38 @@ int contract(Env& e, const uint64_t* d_keys, const uint32_t* succ, const uint32_
   uint32_t* cnt = static_cast<uint32_t*>(e.take(1, 64 * 4));
   unsigned long long* dcyc = static_cast<unsigned long long*>(e.take(1, 8));
   if (!dcyc) return e.fail(UC_EBUDGET, "arena overflow");
-  uint32_t rounds = 0;
-  uint32_t *act = nullptr, *left = nullptr;
-  r = rank_lists(e, pred, nullptr, n, X, a0, a1, cnt, rounds, act, left);
+  uint32_t rounds = rank_rounds(n);
+  UC_CK(cudaMemsetAsync(cnt, 0, 64 * 4, e.stream));  // list counts (34 at most); the meetings at 48
+  UC_CK(cudaMemsetAsync(&e.ctr->err, 0, 4, e.stream));
+  e.launches += 2;
+  // results over the predecessors: walk a copy (the list that fills later)
+  auto over = [&](const uint32_t* o) { return o < pred + n && pred < o + n; };
+  const uint32_t* from = pred;
+  if (over(head) || over(rank)) {
+    UC_CK(cudaMemcpyAsync(a1, pred, n * 4, cudaMemcpyDeviceToDevice, e.stream));
+    from = a1;
+  }
+  k_rank_walk<<<grid_for(e, (n + 3) / 4, 256), 256, 0, e.stream>>>(from, n, head, rank, X, a0, cnt);
+  UC_CK(cudaGetLastError());
+  int occ = 0;
+  if (const int ro = occupancy(e, occ, k_rank_rest, 1024, 0)) return ro;
+  const uint64_t want = (n + 1023) / 1024;
+  const unsigned g = unsigned(std::max<uint64_t>(1, std::min<uint64_t>(want, uint64_t(e.sm_count) * std::max(1, occ))));
+  uint32_t *bar = cnt + 48, *errp = &e.ctr->err;
+  void* args[] = {&X, &head, &rank, &a0, &a1, &cnt, &rounds, &bar, &errp};
+  UC_CK(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(k_rank_rest), dim3(g), dim3(1024), args, 0, e.stream));
+  uint32_t* const hl = reinterpret_cast<uint32_t*>(e.h_io());
+  UC_CK(cudaMemcpyAsync(hl, cnt + rounds, 4, cudaMemcpyDeviceToHost, e.stream));
+  r = e.read_ctr();
   if (r) return r;
-  ++e.launches;
-  k_head_rank<<<grid_for(e, n, 256), 256, 0, e.stream>>>(X, n, head, rank);
-  uint32_t hleft = 0;
-  UC_CK(cudaMemcpyAsync(&hleft, left, 4, cudaMemcpyDeviceToHost, e.stream));
-  UC_CK(cudaStreamSynchronize(e.stream));
+  if (e.h_ctr->err) {
+    r = e.check_err(e.h_ctr);
+    UC_CK(cudaMemsetAsync(&e.ctr->err, 0, 4, e.stream));
+    e.reset();
+    return r;
+  }
+  const uint32_t hleft = *hl;
+  const uint32_t* act = (rounds & 1) ? a1 : a0;
   if (hleft) {
     UC_CK(cudaMemsetAsync(seen, 0, n, e.stream));
     UC_CK(cudaMemsetAsync(dcyc, 0, 8, e.stream));
