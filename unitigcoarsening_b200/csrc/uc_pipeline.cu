@@ -785,57 +785,124 @@ __host__ __device__ constexpr int sc_chunk() {
 }
 static_assert(2 * sc_chunk<1>() < 65536 && 2 * sc_chunk<2>() < 65536, "chunk copy counts share a 32-bit scan");
 
+// Staged records (key, link, bucket), packed: one 16-byte record with a one-word
+// key; with a two-word key, link and bucket as one word behind the keys.
+// Levels 1 and 2 are bound by the runs that they write more than by their
+// bytes (13 to 16 records each, starting and ending inside a sector in every
+// array), and packed there are a third or half as many.  260M k-mers, k = 31,
+// 289M copies: levels 1, 2, 3 took 2.82, 2.17, 2.12 ms with arrays of their own
+// for key, link and bucket, and 2.40, 1.96, 2.00 now; k = 63, 66M copies:
+// 0.90, 0.85, 0.58 and 0.84, 0.72, 0.55.  (Level 2's staging in shared memory
+// keeps three arrays for one-word keys: 16-byte records there cost it 0.3 ms.)
+template <int NW, bool PACKED>
+struct Stage {
+  uint64_t* k = nullptr;
+  uint32_t *l = nullptr, *b = nullptr;  // (packed: l is the second array of a two-word key's)
+  // over n records at base, 256-byte aligned (scatter_stage_bytes)
+  __host__ __device__ static Stage over(void* base, uint64_t n) {
+    Stage s;
+    s.k = static_cast<uint64_t*>(base);
+    s.l = reinterpret_cast<uint32_t*>(s.k + NW * n);
+    s.b = s.l + n;
+    return s;
+  }
+  __device__ __forceinline__ void get(uint64_t i, Key<NW>& key, uint32_t& link, uint32_t& bkt) const {
+    if constexpr (PACKED) {
+      unsigned long long w;
+      if constexpr (NW == 1) {  // (two loads: one of 16 bytes was 0.15 ms slower in level 2)
+        key.w[0] = k[2 * i];
+        w = k[2 * i + 1];
+      } else {
+        key = ld_key<NW>(k, i);
+        w = reinterpret_cast<const unsigned long long*>(l)[i];
+      }
+      link = uint32_t(w);
+      bkt = uint32_t(w >> 32);
+    } else {
+      bkt = b[i];
+      key = ld_key<NW>(k, i);
+      link = l[i];
+    }
+  }
+  __device__ __forceinline__ void put(uint64_t i, const Key<NW>& key, uint32_t link, uint32_t bkt) const {
+    if constexpr (PACKED) {
+      const unsigned long long w = (static_cast<unsigned long long>(bkt) << 32) | link;
+      if constexpr (NW == 1) {
+        reinterpret_cast<ulonglong2*>(k)[i] = make_ulonglong2(key.w[0], w);
+      } else {
+        st_key<NW>(k, i, key);
+        reinterpret_cast<unsigned long long*>(l)[i] = w;
+      }
+    } else {
+      st_key<NW>(k, i, key);
+      l[i] = link;
+      b[i] = bkt;
+    }
+  }
+  __device__ __forceinline__ uint32_t bucket(uint64_t i) const {
+    static_assert(PACKED, "read from global memory only");
+    if constexpr (NW == 1) return uint32_t(k[2 * i + 1] >> 32);
+    else return uint32_t(reinterpret_cast<const unsigned long long*>(l)[i] >> 32);
+  }
+};
+
 __global__ void k_coarse_init(const unsigned long long* __restrict__ boff, uint32_t fb, uint32_t mc,
                               unsigned long long* __restrict__ ccur) {
   for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < mc; j += gridDim.x * blockDim.x)
     ccur[j] = boff[uint64_t(j) << fb];
 }
 
-constexpr int COARSE_THREADS = 256;
+constexpr int COARSE_THREADS = 512;
 
 template <int NW>
-__global__ void __launch_bounds__(COARSE_THREADS) k_scatter_coarse(const uint64_t* __restrict__ keys,
+__global__ void __launch_bounds__(COARSE_THREADS, 2) k_scatter_coarse(const uint64_t* __restrict__ keys,
                                                         const uint32_t* __restrict__ b1,
                                                         const uint32_t* __restrict__ b2, uint64_t n,
                                                         uint32_t fb, uint32_t mc,
                                                         unsigned long long* __restrict__ ccur,
-                                                        uint64_t* __restrict__ rkey, uint32_t* __restrict__ rlink,
-                                                        uint32_t* __restrict__ rbkt, int ids_mode, Counters* ctr) {
+                                                        Stage<NW, true> to, int ids_mode, Counters* ctr) {
   extern __shared__ __align__(16) unsigned char sm_raw[];
-  uint64_t* skey = reinterpret_cast<uint64_t*>(sm_raw);                         // [2*CHUNK*NW]
   constexpr int SC_CHUNK = sc_chunk<NW>();
-  uint32_t* slink = reinterpret_cast<uint32_t*>(skey + 2 * SC_CHUNK * NW);      // [2*CHUNK]
-  uint32_t* sbkt = slink + 2 * SC_CHUNK;                                        // [2*CHUNK]
-  unsigned long long* gbase = reinterpret_cast<unsigned long long*>(sbkt + 2 * SC_CHUNK);  // [mc]
+  const auto own = Stage<NW, true>::over(sm_raw, 2 * SC_CHUNK);
+  unsigned long long* gbase = reinterpret_cast<unsigned long long*>(sm_raw + 2 * SC_CHUNK * (8 * NW + 8));  // [mc]
   uint32_t* hist = reinterpret_cast<uint32_t*>(gbase + mc);                     // [mc]
   uint32_t* lofs = hist + mc;                                                   // [mc + 1]
   __shared__ uint32_t sc[33];
-  for (uint64_t c0 = uint64_t(blockIdx.x) * SC_CHUNK; c0 < n; c0 += uint64_t(gridDim.x) * SC_CHUNK) {
-    const uint32_t cn = uint32_t((n - c0) < uint64_t(SC_CHUNK) ? (n - c0) : uint64_t(SC_CHUNK));
-    // every load of the chunk is issued at once; the values stay in registers
-    constexpr int PT = SC_CHUNK / COARSE_THREADS;
-    Key<NW> kk[PT];
-    uint32_t aa[PT], bb[PT];
+  // A chunk's loads are all issued at once, for the first chunk here and for
+  // every later one before its predecessor is written out, so that they are
+  // in flight meanwhile; the values stay in registers.  A copy's rank within its
+  // partition is what the count returns: no second atomic to place it.
+  constexpr int PT = SC_CHUNK / COARSE_THREADS;
+  Key<NW> kk[PT];
+  uint32_t aa[PT], bb[PT];
+  auto load = [&](uint64_t at) {
 #pragma unroll
     for (int q = 0; q < PT; ++q) {
-      const uint32_t t = uint32_t(q) * COARSE_THREADS + threadIdx.x;
-      if (t < cn) {
-        kk[q] = ld_key<NW>(keys, c0 + t);
-        aa[q] = b1[c0 + t];
-        bb[q] = b2[c0 + t];
-      }
+      const uint64_t i = at + uint32_t(q) * COARSE_THREADS + threadIdx.x;
+      const uint64_t j = i < n ? i : 0;  // (a load behind a branch is waited for at once)
+      kk[q] = ld_key<NW>(keys, j);
+      aa[q] = b1[j];
+      bb[q] = b2[j];
     }
+  };
+  const uint64_t stride = uint64_t(gridDim.x) * SC_CHUNK;
+  uint64_t c0 = uint64_t(blockIdx.x) * SC_CHUNK;
+  load(c0);
+  for (; c0 < n; c0 += stride) {
+    const uint32_t cn = uint32_t((n - c0) < uint64_t(SC_CHUNK) ? (n - c0) : uint64_t(SC_CHUNK));
     for (uint32_t j = threadIdx.x; j < mc; j += blockDim.x) hist[j] = 0;
     __syncthreads();
     // count copies per coarse partition; bit q of cmask marks a cross k-mer
     uint32_t cmask = 0;
+    uint32_t rr[PT];  // ranks: of the first copy in the low half, of the second in the high half
 #pragma unroll
     for (int q = 0; q < PT; ++q) {
       const uint32_t t = uint32_t(q) * COARSE_THREADS + threadIdx.x;
+      rr[q] = 0;
       if (t < cn) {
-        atomicAdd(hist + (aa[q] >> fb), 1u);
+        rr[q] = atomicAdd(hist + (aa[q] >> fb), 1u);
         if (aa[q] != bb[q]) {
-          atomicAdd(hist + (bb[q] >> fb), 1u);
+          rr[q] |= atomicAdd(hist + (bb[q] >> fb), 1u) << 16;
           cmask |= 1u << q;
         }
       }
@@ -860,9 +927,9 @@ __global__ void __launch_bounds__(COARSE_THREADS) k_scatter_coarse(const uint64_
       for (uint32_t j = j0; j < j1; ++j) {
         const uint32_t h = hist[j];
         lofs[j] = pre;
-        gbase[j] = h ? atomicAdd(ccur + j, (unsigned long long)h) : 0ull;
+        // (less the run's place in the staging area: staged position + gbase)
+        gbase[j] = (h ? atomicAdd(ccur + j, (unsigned long long)h) : 0ull) - pre;
         pre += h;
-        hist[j] = 0;
       }
       if (threadIdx.x == 0) {
         lofs[mc] = tot & 0xFFFFu;
@@ -892,17 +959,13 @@ __global__ void __launch_bounds__(COARSE_THREADS) k_scatter_coarse(const uint64_
         const uint32_t link = ids_mode ? uint32_t(c0 + t) : x;
         Key<NW> kp = key;
         kp.w[NW - 1] |= ROLE_P | (cross ? 0ull : ROLE_S);
-        const uint32_t sp = lofs[a >> fb] + atomicAdd(hist + (a >> fb), 1u);
-        st_key<NW>(skey, sp, kp);
-        slink[sp] = link;
-        sbkt[sp] = a;
+        const uint32_t sp = lofs[a >> fb] + (rr[q] & 0xFFFFu);
+        own.put(sp, kp, link, a);
         if (cross) {
           Key<NW> ks = key;
           ks.w[NW - 1] |= ROLE_S;
-          const uint32_t sq = lofs[b >> fb] + atomicAdd(hist + (b >> fb), 1u);
-          st_key<NW>(skey, sq, ks);
-          slink[sq] = link;
-          sbkt[sq] = b;
+          const uint32_t sq = lofs[b >> fb] + (rr[q] >> 16);
+          own.put(sq, ks, link, b);
         }
       }
     }
@@ -910,13 +973,12 @@ __global__ void __launch_bounds__(COARSE_THREADS) k_scatter_coarse(const uint64_
     // write the runs out: consecutive slots of a partition are consecutive
     // global positions
     const uint32_t total = lofs[mc];
+    load(c0 + stride);
     for (uint32_t sl = threadIdx.x; sl < total; sl += blockDim.x) {
-      const uint32_t bk = sbkt[sl];
-      const uint32_t part = bk >> fb;
-      const uint64_t pos = gbase[part] + (sl - lofs[part]);
-      st_key<NW>(rkey, pos, ld_key<NW>(skey, sl));
-      rlink[pos] = slink[sl];
-      rbkt[pos] = bk;
+      Key<NW> key;
+      uint32_t link, bk;
+      own.get(sl, key, link, bk);
+      to.put(gbase[bk >> fb] + sl, key, link, bk);
     }
     __syncthreads();
   }
@@ -937,7 +999,8 @@ __global__ void __launch_bounds__(COARSE_THREADS) k_scatter_coarse(const uint64_
 // 1024 partly written runs per block, more than L2 holds at 1 Gbp.)
 constexpr int MID_CHUNK = 4096;    // staged records per level-2 chunk
 constexpr int MID_MAX_BINS = 1024; // sub-partitions per coarse partition
-constexpr int SUB_MAX_BITS = 8;    // buckets per sub-partition: at most 2^8
+static_assert(MID_CHUNK <= 4096 && MID_MAX_BINS <= 4096, "a record's rank and bucket share a word");
+constexpr int SUB_MAX_BITS = 9;    // buckets per sub-partition: at most 2^9
 constexpr int MID_THREADS = 512;
 
 // Chunk list of level 2: item_start[p] = first chunk of coarse partition p
@@ -959,21 +1022,20 @@ __global__ void k_mid_items(const unsigned long long* __restrict__ boff, uint32_
 
 template <int NW>
 __global__ void __launch_bounds__(MID_THREADS, NW == 1 ? 2 : 1) k_scatter_mid(
-    const uint64_t* __restrict__ rkey, const uint32_t* __restrict__ rlink, const uint32_t* __restrict__ rbkt,
-    const unsigned long long* __restrict__ goff, uint32_t cg, const uint32_t* __restrict__ item_start, uint32_t fb,
-    uint32_t sb, uint32_t mc, unsigned long long* __restrict__ scur, uint64_t* __restrict__ okey,
-    uint32_t* __restrict__ olink, uint32_t* __restrict__ obkt, Counters* ctr) {
+    Stage<NW, true> from, const unsigned long long* __restrict__ goff, uint32_t cg, const uint32_t* __restrict__ item_start, uint32_t fb,
+    uint32_t sb, uint32_t mc, unsigned long long* __restrict__ scur, Stage<NW, true> to, Counters* ctr) {
   extern __shared__ __align__(16) unsigned char sm_raw[];
-  uint64_t* skey = reinterpret_cast<uint64_t*>(sm_raw);                              // [MID_CHUNK*NW]
-  uint32_t* slink = reinterpret_cast<uint32_t*>(skey + MID_CHUNK * NW);              // [MID_CHUNK]
-  uint32_t* sbkt = slink + MID_CHUNK;                                                // [MID_CHUNK]
-  unsigned long long* gbase = reinterpret_cast<unsigned long long*>(sbkt + MID_CHUNK);  // [nb]
+  const auto own = Stage<NW, NW == 2>::over(sm_raw, MID_CHUNK);
+  unsigned long long* gbase = reinterpret_cast<unsigned long long*>(sm_raw + MID_CHUNK * (8 * NW + 8));  // [nb]
   const uint32_t nb = 1u << (fb - sb);
   uint32_t* hist = reinterpret_cast<uint32_t*>(gbase + nb);                          // [nb]
   uint32_t* lofs = hist + nb;                                                        // [nb + 1]
   uint32_t* istart = lofs + nb + 1;                                                  // [mc + 1]
   __shared__ uint32_t sc[33];
-  __shared__ uint32_t s_t, s_p;
+  // the next chunk, looked up by thread 0 while the block works on this one:
+  // its first record, records and partition (no records: none left)
+  __shared__ unsigned long long s_c0;
+  __shared__ uint32_t s_cn, s_p;
   for (uint32_t j = threadIdx.x; j <= mc; j += blockDim.x) istart[j] = item_start[j];
   __syncthreads();
   const uint32_t nitems = istart[mc];
@@ -981,54 +1043,79 @@ __global__ void __launch_bounds__(MID_THREADS, NW == 1 ? 2 : 1) k_scatter_mid(
   // the bins this thread scans and reserves
   const uint32_t per = (nb + blockDim.x - 1) / blockDim.x;
   const uint32_t j0 = min(nb, threadIdx.x * per), j1 = min(nb, j0 + per);
-  for (;;) {
-    if (threadIdx.x == 0) {
-      const uint32_t t = atomicAdd(&ctr->work_mid, 1u);
-      uint32_t lo = 0, hi = mc;  // the partition p with istart[p] <= t < istart[p + 1]
-      while (hi - lo > 1) {
-        const uint32_t mid = (lo + hi) >> 1;
-        if (istart[mid] <= t) lo = mid;
-        else hi = mid;
-      }
-      s_t = t;
-      s_p = lo;
+  // (goff: offsets of count groups of 2^cg buckets; partition p starts at
+  // group p << (fb - cg))
+  auto item = [&](uint32_t t, unsigned long long& at, unsigned long long& end, uint32_t& part) {
+    at = end = 0;
+    part = 0;
+    if (t >= nitems) return;
+    uint32_t lo = 0, hi = mc;  // the partition p with istart[p] <= t < istart[p + 1]
+    while (hi - lo > 1) {
+      const uint32_t mid = (lo + hi) >> 1;
+      if (istart[mid] <= t) lo = mid;
+      else hi = mid;
     }
-    __syncthreads();
-    const uint32_t t = s_t, p = s_p;
-    __syncthreads();
-    if (t >= nitems) break;
-    // (goff: offsets of count groups of 2^cg buckets; partition p starts at
-    // group p << (fb - cg))
-    const unsigned long long pend = goff[uint64_t(p + 1) << (fb - cg)];
-    const unsigned long long c0 = goff[uint64_t(p) << (fb - cg)] + uint64_t(t - istart[p]) * MID_CHUNK;
-    const uint32_t cn = uint32_t(min(pend - c0, (unsigned long long)MID_CHUNK));
-    const uint32_t sub0 = p << (fb - sb);  // first sub-partition of partition p
-    // the chunk's records, all loads issued at once (in registers), and the
-    // counts per sub-partition
-    uint32_t bb[PT], ll[PT];
-    Key<NW> kk[PT];
+    part = lo;
+    at = goff[uint64_t(lo) << (fb - cg)] + uint64_t(t - istart[lo]) * MID_CHUNK;
+    end = goff[uint64_t(lo + 1) << (fb - cg)];
+  };
+  auto put = [&](unsigned long long at, unsigned long long end, uint32_t part) {
+    s_c0 = at;
+    s_cn = uint32_t(min(end - at, (unsigned long long)MID_CHUNK));
+    s_p = part;
+  };
+  // a chunk's records, all loads issued at once, the first chunk's here and
+  // every later one's before its predecessor is written out
+  uint32_t bb[PT], ll[PT];
+  Key<NW> kk[PT];
+  unsigned long long c0;
+  uint32_t cn, p;
+  auto load = [&] {
+    c0 = s_c0;
+    cn = s_cn;
+    p = s_p;
 #pragma unroll
     for (int q = 0; q < PT; ++q) {
       const uint32_t i = uint32_t(q) * MID_THREADS + threadIdx.x;
-      if (i < cn) {
-        bb[q] = rbkt[c0 + i];
-        kk[q] = ld_key<NW>(rkey, c0 + i);
-        ll[q] = rlink[c0 + i];
-      } else {
-        bb[q] = 0u;
-      }
+      if (i < cn) from.get(c0 + i, kk[q], ll[q], bb[q]);
     }
+  };
+  uint32_t ticket = 0;  // thread 0: the chunk after the one in s_c0
+  if (threadIdx.x == 0) {
+    unsigned long long at, end;
+    uint32_t part;
+    const uint32_t t = atomicAdd(&ctr->work_mid, 1u);
+    ticket = atomicAdd(&ctr->work_mid, 1u);
+    item(t, at, end, part);
+    put(at, end, part);
+  }
+  __syncthreads();
+  load();
+  while (cn) {
+    const uint32_t sub0 = p << (fb - sb);  // first sub-partition of partition p
     for (uint32_t j = threadIdx.x; j < nb; j += blockDim.x) hist[j] = 0;
     __syncthreads();
-    // a record outside partition p would be a broken staging order: flag it
-    // and leave it out rather than index past the counts
+    unsigned long long nat = 0, nend = 0;
+    uint32_t npart = 0;
+    if (threadIdx.x == 0) {
+      item(ticket, nat, nend, npart);
+      ticket = atomicAdd(&ctr->work_mid, 1u);
+    }
+    // The counts per sub-partition; a record keeps its rank there (12 bits)
+    // above its bucket within the partition (fb <= 19 bits).  A record outside
+    // partition p would be a broken staging order: flag it and leave it out
+    // rather than index past the counts.
 #pragma unroll
     for (int q = 0; q < PT; ++q) {
       const uint32_t i = uint32_t(q) * MID_THREADS + threadIdx.x;
       if (i < cn) {
-        const uint32_t bin = (bb[q] >> sb) - sub0;
-        if (bin < nb) atomicAdd(hist + bin, 1u);
-        else atomicOr(&ctr->err, ERR_INTERNAL);
+        const uint32_t lb = bb[q] - (p << fb), bin = lb >> sb;
+        if (bin < nb) {
+          bb[q] = lb | (atomicAdd(hist + bin, 1u) << 20);
+        } else {
+          bb[q] = NONE;
+          atomicOr(&ctr->err, ERR_INTERNAL);
+        }
       }
     }
     __syncthreads();
@@ -1041,34 +1128,33 @@ __global__ void __launch_bounds__(MID_THREADS, NW == 1 ? 2 : 1) k_scatter_mid(
       for (uint32_t j = j0; j < j1; ++j) {
         const uint32_t h = hist[j];
         lofs[j] = pre;
-        gbase[j] = h ? atomicAdd(scur + sub0 + j, (unsigned long long)h) : 0ull;
+        gbase[j] = (h ? atomicAdd(scur + sub0 + j, (unsigned long long)h) : 0ull) - pre;
         pre += h;
-        hist[j] = 0;
       }
-      if (threadIdx.x == 0) lofs[nb] = tot;
+      if (threadIdx.x == 0) {
+        lofs[nb] = tot;
+        put(nat, nend, npart);
+      }
     }
     __syncthreads();
     // place every record in its sub-partition's run of the staging area
 #pragma unroll
     for (int q = 0; q < PT; ++q) {
       const uint32_t i = uint32_t(q) * MID_THREADS + threadIdx.x;
-      const uint32_t bin = (bb[q] >> sb) - sub0;
-      if (i < cn && bin < nb) {
-        const uint32_t sl = lofs[bin] + atomicAdd(hist + bin, 1u);
-        st_key<NW>(skey, sl, kk[q]);
-        slink[sl] = ll[q];
-        sbkt[sl] = bb[q];
+      if (i < cn && bb[q] != NONE) {
+        const uint32_t lb = bb[q] & 0xFFFFFu;
+        const uint32_t sl = lofs[lb >> sb] + (bb[q] >> 20);
+        own.put(sl, kk[q], ll[q], lb);
       }
     }
     __syncthreads();
-    const uint32_t placed = lofs[nb];
+    const uint32_t placed = lofs[nb], b0 = p << fb;
+    load();
     for (uint32_t sl = threadIdx.x; sl < placed; sl += blockDim.x) {
-      const uint32_t bk = sbkt[sl];
-      const uint32_t bin = (bk >> sb) - sub0;
-      const uint64_t pos = gbase[bin] + (sl - lofs[bin]);
-      st_key<NW>(okey, pos, ld_key<NW>(skey, sl));
-      olink[pos] = slink[sl];
-      obkt[pos] = bk;
+      Key<NW> key;
+      uint32_t link, lb;
+      own.get(sl, key, link, lb);
+      to.put(gbase[lb >> sb] + sl, key, link, b0 + lb);
     }
     __syncthreads();
   }
@@ -1085,9 +1171,7 @@ __global__ void __launch_bounds__(MID_THREADS, NW == 1 ? 2 : 1) k_scatter_mid(
 // contiguous range; a larger one (a large repeat bucket) is placed straight
 // into global memory.  Blocks take sub-partitions from a counter.
 template <int NW>
-__global__ void __launch_bounds__(512, 2) k_scatter_sub(const uint64_t* __restrict__ ikey,
-                                                     const uint32_t* __restrict__ ilink,
-                                                     const uint32_t* __restrict__ ibkt,
+__global__ void __launch_bounds__(512, 2) k_scatter_sub(Stage<NW, true> from,
                                                      const unsigned long long* __restrict__ goff, uint32_t gsh,
                                                      uint32_t sb, uint32_t nsub, uint32_t cap,
                                                      uint64_t* __restrict__ pkeys, uint32_t* __restrict__ plink,
@@ -1098,45 +1182,86 @@ __global__ void __launch_bounds__(512, 2) k_scatter_sub(const uint64_t* __restri
   uint32_t* slink = reinterpret_cast<uint32_t*>(skey + size_t(cap) * NW);  // [cap]
   __shared__ unsigned long long s_off[1 << SUB_MAX_BITS];
   __shared__ uint32_t s_cur[1 << SUB_MAX_BITS];
+  // buckets' records among the first batch (when there are more records)
+  __shared__ uint32_t s_first[1 << SUB_MAX_BITS];
+  // the next sub-partition and its records, looked up by thread 0 while the
+  // block works on this one
   __shared__ uint32_t s_sp;
+  __shared__ unsigned long long s_lo, s_hi;
   __shared__ uint32_t sc[33];
   const uint32_t nbk = 1u << sb;  // <= 2^SUB_MAX_BITS <= blockDim.x
   // records per thread and pass: their loads are in flight together (two
   // CTAs per SM fit the registers)
-  constexpr int PER = NW == 1 ? 8 : 4;
-  for (;;) {
-    if (threadIdx.x == 0) s_sp = atomicAdd(&ctr->work_sub, 1u);
-    __syncthreads();
-    const uint32_t sp = s_sp;
-    if (sp >= nsub) break;
+  constexpr int PER = NW == 1 ? 8 : 5;
+  const uint32_t batch = blockDim.x * PER;
+  // known: goff holds every bucket's offset (no count groups)
+  const bool known = cout == nullptr;
+  // The first batch of a sub-partition: loaded before the one before it is
+  // written out, in registers from there to its placement.  Counting it gives
+  // each record its rank in its bucket (kept above the bucket), so
+  // that only records past it take a second atomic to be placed.
+  uint32_t bk[PER];
+  Key<NW> kk[PER];
+  uint32_t ln[PER];
+  uint32_t sp;
+  unsigned long long lo, hi;
+  auto load = [&](unsigned long long i0) {
+#pragma unroll
+    for (int q = 0; q < PER; ++q) {
+      const unsigned long long i = i0 + uint64_t(q) * blockDim.x + threadIdx.x;
+      if (i < hi) from.get(i, kk[q], ln[q], bk[q]);
+    }
+  };
+  auto next = [&] {
+    sp = s_sp;
+    lo = s_lo;
+    hi = s_hi;
+    load(lo);
+  };
+  uint32_t ticket = 0;  // thread 0: the sub-partition after s_sp
+  auto look = [&](uint32_t t, unsigned long long& a, unsigned long long& b) {
+    a = b = 0;
+    if (t < nsub) {
+      a = goff[uint64_t(t) << gsh];
+      b = goff[uint64_t(t + 1) << gsh];
+    }
+  };
+  if (threadIdx.x == 0) {
+    unsigned long long a, b;
+    const uint32_t t = atomicAdd(&ctr->work_sub, 1u);
+    ticket = atomicAdd(&ctr->work_sub, 1u);
+    look(t, a, b);
+    s_sp = t;
+    s_lo = a;
+    s_hi = b;
+  }
+  __syncthreads();
+  next();
+  while (sp < nsub) {
     const uint64_t b0 = uint64_t(sp) << sb;
-    const unsigned long long lo = goff[uint64_t(sp) << gsh], hi = goff[uint64_t(sp + 1) << gsh];
-    // known: goff holds every bucket's offset (no count groups)
-    const bool known = cout == nullptr;
     for (uint32_t j = threadIdx.x; j < nbk; j += blockDim.x) {
       if (known) s_off[j] = goff[b0 + j];
       s_cur[j] = 0;
     }
     __syncthreads();
-    const bool staged = hi - lo <= cap;
-    // the first PER x blockDim records stay in registers from the count to
-    // their placement; the rest are counted from their bucket ids and
-    // loaded again to be placed
-    uint32_t bk[PER];
-    Key<NW> kk[PER];
-    uint32_t ln[PER];
-    auto load = [&](unsigned long long i0) {
-#pragma unroll
-      for (int q = 0; q < PER; ++q) {
-        const unsigned long long i = i0 + uint64_t(q) * blockDim.x + threadIdx.x;
-        bk[q] = 0xFFFFFFFFu;
-        if (i < hi) {
-          bk[q] = ibkt[i];
-          kk[q] = ld_key<NW>(ikey, i);
-          ln[q] = ilink[i];
-        }
+    unsigned long long nlo = 0, nhi = 0;
+    uint32_t nsp = 0;
+    if (threadIdx.x == 0) {
+      nsp = ticket;
+      look(nsp, nlo, nhi);
+      ticket = atomicAdd(&ctr->work_sub, 1u);
+    }
+    const bool staged = hi - lo <= cap, more = hi - lo > batch;
+    auto put = [&](int q, uint64_t pos) {
+      if (staged) {
+        st_key<NW>(skey, pos - lo, kk[q]);
+        slink[pos - lo] = ln[q];
+      } else {
+        st_key<NW>(pkeys, pos, kk[q]);
+        plink[pos] = ln[q];
       }
     };
+    // places the records in registers by the buckets' cursors
     auto place = [&](unsigned long long i0) {
 #pragma unroll
       for (int q = 0; q < PER; ++q) {
@@ -1147,68 +1272,79 @@ __global__ void __launch_bounds__(512, 2) k_scatter_sub(const uint64_t* __restri
             atomicOr(&ctr->err, ERR_INTERNAL);
             continue;
           }
-          const uint64_t pos = s_off[lb] + atomicAdd(s_cur + lb, 1u);
-          if (staged) {
-            st_key<NW>(skey, pos - lo, kk[q]);
-            slink[pos - lo] = ln[q];
-          } else {
-            st_key<NW>(pkeys, pos, kk[q]);
-            plink[pos] = ln[q];
-          }
+          put(q, s_off[lb] + atomicAdd(s_cur + lb, 1u));
         }
       }
     };
-    const uint64_t batch = uint64_t(blockDim.x) * PER;
-    load(lo);
-    if (!known) {
-      // the sub-partition's counts per bucket (records of another
-      // sub-partition are flagged when placed)
+    if (known) {
+      place(lo);
+    } else {
+      // the sub-partition's counts per bucket
 #pragma unroll
       for (int q = 0; q < PER; ++q) {
+        const unsigned long long i = lo + uint64_t(q) * blockDim.x + threadIdx.x;
         const uint32_t lb = bk[q] - uint32_t(b0);
-        if (lb < nbk) atomicAdd(s_cur + lb, 1u);
-      }
-      for (unsigned long long i0 = lo + batch; i0 < hi; i0 += batch) {
-        uint32_t bq[PER];
-#pragma unroll
-        for (int q = 0; q < PER; ++q) {
-          const unsigned long long i = i0 + uint64_t(q) * blockDim.x + threadIdx.x;
-          bq[q] = (i < hi) ? ibkt[i] : 0xFFFFFFFFu;
-        }
-#pragma unroll
-        for (int q = 0; q < PER; ++q) {
-          const uint32_t lb = bq[q] - uint32_t(b0);
-          if (lb < nbk) atomicAdd(s_cur + lb, 1u);
+        bk[q] = 0xFFFFFFFFu;
+        if (i < hi) {
+          if (lb < nbk) bk[q] = lb | (atomicAdd(s_cur + lb, 1u) << SUB_MAX_BITS);
+          else atomicOr(&ctr->err, ERR_INTERNAL);
         }
       }
       __syncthreads();
+      if (more) {
+        for (uint32_t j = threadIdx.x; j < nbk; j += blockDim.x) s_first[j] = s_cur[j];
+        __syncthreads();
+        for (unsigned long long i0 = lo + batch; i0 < hi; i0 += batch) {
+          uint32_t bq[PER];
+#pragma unroll
+          for (int q = 0; q < PER; ++q) {
+            const unsigned long long i = i0 + uint64_t(q) * blockDim.x + threadIdx.x;
+            bq[q] = (i < hi) ? from.bucket(i) : 0xFFFFFFFFu;
+          }
+#pragma unroll
+          for (int q = 0; q < PER; ++q) {
+            const uint32_t lb = bq[q] - uint32_t(b0);
+            if (lb < nbk) atomicAdd(s_cur + lb, 1u);
+          }
+        }
+        __syncthreads();
+      }
       {
         const uint32_t cnt = threadIdx.x < nbk ? s_cur[threadIdx.x] : 0u;
         uint32_t tot;
         const uint32_t ex = block_excl_scan(cnt, sc, &tot);
         if (threadIdx.x < nbk) {
           s_off[threadIdx.x] = lo + ex;
-          s_cur[threadIdx.x] = 0;
+          if (more) s_cur[threadIdx.x] = s_first[threadIdx.x];
           cout[b0 + threadIdx.x] = cnt;
           if (bout) bout[b0 + threadIdx.x] = lo + ex;
         }
       }
       __syncthreads();
+#pragma unroll
+      for (int q = 0; q < PER; ++q)
+        if (bk[q] != 0xFFFFFFFFu) put(q, s_off[bk[q] & ((1u << SUB_MAX_BITS) - 1u)] + (bk[q] >> SUB_MAX_BITS));
     }
-    place(lo);
-    for (unsigned long long i0 = lo + batch; i0 < hi; i0 += batch) {
-      load(i0);
-      place(i0);
-    }
-    __syncthreads();
-    if (staged) {
-      const uint32_t cnt = uint32_t(hi - lo);
-      for (uint32_t t = threadIdx.x; t < cnt; t += blockDim.x) {
-        st_key<NW>(pkeys, lo + t, ld_key<NW>(skey, t));
-        plink[lo + t] = slink[t];
+    if (more) {
+      for (unsigned long long i0 = lo + batch; i0 < hi; i0 += batch) {
+        load(i0);
+        place(i0);
       }
     }
-    __syncthreads();  // the staging area, s_off / s_cur / s_sp are reused
+    if (threadIdx.x == 0) {
+      s_sp = nsp;
+      s_lo = nlo;
+      s_hi = nhi;
+    }
+    __syncthreads();
+    const unsigned long long at = lo;
+    const uint32_t cnt = staged ? uint32_t(hi - lo) : 0u;
+    next();
+    for (uint32_t t = threadIdx.x; t < cnt; t += blockDim.x) {
+      st_key<NW>(pkeys, at + t, ld_key<NW>(skey, t));
+      plink[at + t] = slink[t];
+    }
+    __syncthreads();  // the staging area, s_off / s_cur are reused
   }
 }
 
@@ -3898,7 +4034,7 @@ static int plan_tiles(Env& e, const Front& f, const Plan& P, int nw, bool lists)
 // writes r2 and level 3 (k_scatter_sub) writes back into r1, or, where a
 // coarse partition is already small, level 3 writes r2 straight away.  Both
 // regions hold scatter_stage_bytes(copies, nw); the final copies (pkeys,
-// plink) are the key and link arrays of the region level 3 wrote.  Level 1
+// plink) are arrays at the start of the region level 3 wrote.  Level 1
 // may run over the k-mers in several launches (the streamed path's chunks):
 // its cursors and the cross-index counter carry over.
 struct Scatter {
@@ -3912,8 +4048,7 @@ struct Scatter {
   bool mid = false;
   int nw = 1;
   uint64_t copies = 0;
-  uint64_t *k1 = nullptr, *k2 = nullptr;
-  uint32_t *l1 = nullptr, *l2 = nullptr, *b1 = nullptr, *b2 = nullptr;
+  char *r1 = nullptr, *r2 = nullptr;
 };
 
 // cg > 0: the copies are counted per group of 2^cg buckets (offsets in
@@ -3928,13 +4063,8 @@ static int scatter_begin(Env& e, const Front& f, const Plan& P, int nw, char* r1
   sc.goff = group_offsets ? f.goff : f.boff;
   sc.cout = group_offsets ? f.counts : nullptr;
   sc.bout = group_offsets ? f.boff : nullptr;
-  auto region = [&](char* base, uint64_t*& key, uint32_t*& link, uint32_t*& bkt) {
-    key = reinterpret_cast<uint64_t*>(base);
-    link = reinterpret_cast<uint32_t*>(base + copies * 8ull * nw);
-    bkt = link + copies;
-  };
-  region(r1, sc.k1, sc.l1, sc.b1);
-  region(r2, sc.k2, sc.l2, sc.b2);
+  sc.r1 = r1;
+  sc.r2 = r2;
   scatter_split(P.bits, sc.mcb, sc.fb);
   sc.mc = 1u << sc.mcb;
   // level-3 staging holds cap3 records (two CTAs per SM); sub-partitions of
@@ -3957,8 +4087,6 @@ static int scatter_begin(Env& e, const Front& f, const Plan& P, int nw, char* r1
   if (!r0) r0 = allow_max_smem(e, k_scatter_coarse<2>);
   if (!r0) r0 = allow_max_smem(e, k_scatter_mid<1>);
   if (!r0) r0 = allow_max_smem(e, k_scatter_mid<2>);
-  if (!r0) r0 = allow_max_smem(e, k_scatter_sub<1>);
-  if (!r0) r0 = allow_max_smem(e, k_scatter_sub<2>);
   if (r0) return r0;
   e.launches += 1;
   k_coarse_init<<<grid_for(e, sc.mc, 256), 256, 0, e.stream>>>(sc.goff, sc.fb - sc.cg, sc.mc, f.cursor);
@@ -3982,19 +4110,37 @@ static int scatter_l1(Env& e, const Front& f, const Scatter& sc, const uint64_t*
                                                               uint64_t(e.sm_count) * uint64_t(o1))));
   e.launches += 1;
   if (nw == 1)
-    k_scatter_coarse<1><<<g1, COARSE_THREADS, sm1, e.stream>>>(keys, b1, b2, n, sc.fb, sc.mc, f.cursor, sc.k1, sc.l1,
-                                                               sc.b1, ids_mode, e.ctr);
+    k_scatter_coarse<1><<<g1, COARSE_THREADS, sm1, e.stream>>>(keys, b1, b2, n, sc.fb, sc.mc, f.cursor,
+                                                               Stage<1, true>::over(sc.r1, sc.copies), ids_mode, e.ctr);
   else
-    k_scatter_coarse<2><<<g1, COARSE_THREADS, sm1, e.stream>>>(keys, b1, b2, n, sc.fb, sc.mc, f.cursor, sc.k1, sc.l1,
-                                                               sc.b1, ids_mode, e.ctr);
+    k_scatter_coarse<2><<<g1, COARSE_THREADS, sm1, e.stream>>>(keys, b1, b2, n, sc.fb, sc.mc, f.cursor,
+                                                               Stage<2, true>::over(sc.r1, sc.copies), ids_mode, e.ctr);
   UC_CK(cudaGetLastError());
+  return UC_OK;
+}
+
+template <int NW>
+static int launch_sub(Env& e, const Scatter& sc, char* from, uint64_t* pkeys, uint32_t* plink) {
+  const size_t smem = size_t(sc.cap3) * (8 * NW + 4);
+  int r = allow_max_smem(e, k_scatter_sub<NW>);
+  if (r) return r;
+  int occ = 0;
+  r = occupancy(e, occ, k_scatter_sub<NW>, 512, smem);
+  if (r) return r;
+  if (occ < 1) return e.fail(UC_EINTERNAL, "scatter kernel does not fit an SM");
+  const int g = int(std::min<uint64_t>(sc.nsub, uint64_t(e.sm_count) * uint64_t(occ)));
+  k_scatter_sub<NW><<<g, 512, smem, e.stream>>>(Stage<NW, true>::over(from, sc.copies), sc.goff, sc.sb - sc.cg, sc.sb,
+                                                sc.nsub, sc.cap3, pkeys, plink, sc.cout, sc.bout, e.ctr);
   return UC_OK;
 }
 
 static int scatter_finish(Env& e, const Front& f, const Scatter& sc, uint64_t*& pkeys, uint32_t*& plink) {
   const int nw = sc.nw;
-  pkeys = sc.k2;
-  plink = sc.l2;
+  // the staged records level 3 reads, and the final copies in the other region
+  char* const from = sc.mid ? sc.r2 : sc.r1;
+  char* const to = sc.mid ? sc.r1 : sc.r2;
+  pkeys = reinterpret_cast<uint64_t*>(to);
+  plink = reinterpret_cast<uint32_t*>(to + sc.copies * 8ull * nw);
   if (sc.copies == 0) {
     if (sc.bout) {  // no copies: every bucket empty
       const uint64_t M = uint64_t(sc.nsub) << sc.sb;
@@ -4016,33 +4162,17 @@ static int scatter_finish(Env& e, const Front& f, const Scatter& sc, uint64_t*& 
     k_mid_items<<<1, 256, 0, e.stream>>>(sc.goff, sc.fb - sc.cg, sc.mc, item_start);
     k_coarse_init<<<grid_for(e, sc.nsub, 256), 256, 0, e.stream>>>(sc.goff, sc.sb - sc.cg, sc.nsub, f.fcur);
     if (nw == 1)
-      k_scatter_mid<1><<<e.sm_count * o2, MID_THREADS, sm2, e.stream>>>(sc.k1, sc.l1, sc.b1, sc.goff, sc.cg,
-                                                                        item_start, sc.fb, sc.sb, sc.mc, f.fcur,
-                                                                        sc.k2, sc.l2, sc.b2, e.ctr);
+      k_scatter_mid<1><<<e.sm_count * o2, MID_THREADS, sm2, e.stream>>>(
+          Stage<1, true>::over(sc.r1, sc.copies), sc.goff, sc.cg, item_start, sc.fb, sc.sb, sc.mc, f.fcur,
+          Stage<1, true>::over(sc.r2, sc.copies), e.ctr);
     else
-      k_scatter_mid<2><<<e.sm_count * o2, MID_THREADS, sm2, e.stream>>>(sc.k1, sc.l1, sc.b1, sc.goff, sc.cg,
-                                                                        item_start, sc.fb, sc.sb, sc.mc, f.fcur,
-                                                                        sc.k2, sc.l2, sc.b2, e.ctr);
-    pkeys = sc.k1;
-    plink = sc.l1;
+      k_scatter_mid<2><<<e.sm_count * o2, MID_THREADS, sm2, e.stream>>>(
+          Stage<2, true>::over(sc.r1, sc.copies), sc.goff, sc.cg, item_start, sc.fb, sc.sb, sc.mc, f.fcur,
+          Stage<2, true>::over(sc.r2, sc.copies), e.ctr);
   }
-  const uint64_t* ik = sc.mid ? sc.k2 : sc.k1;
-  const uint32_t* il = sc.mid ? sc.l2 : sc.l1;
-  const uint32_t* ib = sc.mid ? sc.b2 : sc.b1;
   e.launches += 1;
-  const size_t sm3 = size_t(sc.cap3) * (8 * nw + 4);
-  int o3 = 0;
-  if (const int ro = nw == 1 ? occupancy(e, o3, k_scatter_sub<1>, 512, sm3)
-                             : occupancy(e, o3, k_scatter_sub<2>, 512, sm3))
-    return ro;
-  if (o3 < 1) return e.fail(UC_EINTERNAL, "scatter kernel does not fit an SM");
-  const int g3 = int(std::min<uint64_t>(sc.nsub, uint64_t(e.sm_count) * uint64_t(o3)));
-  if (nw == 1)
-    k_scatter_sub<1><<<g3, 512, sm3, e.stream>>>(ik, il, ib, sc.goff, sc.sb - sc.cg, sc.sb, sc.nsub, sc.cap3, pkeys,
-                                                 plink, sc.cout, sc.bout, e.ctr);
-  else
-    k_scatter_sub<2><<<g3, 512, sm3, e.stream>>>(ik, il, ib, sc.goff, sc.sb - sc.cg, sc.sb, sc.nsub, sc.cap3, pkeys,
-                                                 plink, sc.cout, sc.bout, e.ctr);
+  const int r = nw == 1 ? launch_sub<1>(e, sc, from, pkeys, plink) : launch_sub<2>(e, sc, from, pkeys, plink);
+  if (r) return r;
   UC_CK(cudaGetLastError());
   if (sc.bout) {
     // the total after the last bucket, for the tile plan
