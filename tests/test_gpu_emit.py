@@ -55,3 +55,25 @@ def test_tile_edges(comp, oracle, n):
     check(comp, oracle, walk_kmers(random_seq(n + k - 1, n), k)[::-1], k, api.CONTRACT_POINTER_JUMP)
     iso = [random_seq(k, 10_000 + i) for i in range(n)]
     check(comp, oracle, iso, k, api.CONTRACT_HEC)
+
+
+@pytest.mark.parametrize("n", [3, 1023, 1027, 5000])
+@pytest.mark.parametrize("shift", [0, 1, 2, 3])
+def test_head_array_at_any_word(comp, oracle, n, shift):
+    """head and rank may start at any word of a larger array."""
+    k = 31
+    kmers = walk_kmers(random_seq(n // 2 + k - 1, n), k)[::-1] + [random_seq(k, 500 + i) for i in range(n - n // 2)]
+    text = text_of(shuffled(kmers, 4))
+    keys = comp.load_kmers(torch.frombuffer(bytearray(text), dtype=torch.uint8).cuda(), k)
+    succ, pred = comp.assemble_pruned_graph(keys, k, 8)
+    head, rank, _ = comp.coarsen_de_bruijn_full_cycle(keys, succ, pred, k)
+    want = comp.write_unitigs(keys, succ, head, rank, k).cpu().numpy().tobytes()
+    words = oracle.parse(text, k)
+    osucc, opred = oracle.edges(words, k)
+    assert want == oracle.emit(words, k, osucc, *oracle.contract(words, k, osucc, opred)[:2])
+    moved = []
+    for t in (head, rank):
+        buf = torch.empty(n + shift, dtype=t.dtype, device=t.device)
+        buf[shift:] = t
+        moved.append(buf[shift:])
+    assert comp.write_unitigs(keys, succ, *moved, k).cpu().numpy().tobytes() == want
