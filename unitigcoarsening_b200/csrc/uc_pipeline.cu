@@ -1690,26 +1690,31 @@ __device__ __forceinline__ void emit_warp_tile(const TileParams& p, const TileMe
     const uint32_t slot = uint32_t(v);
     __syncwarp();
     const RecArr<NW + 1> out{p.rec_a, p.rec_t};
-    for (uint32_t j = lane; j < nclosed; j += 32) {
-      uint32_t s = m.A[j], len = 1;
-      uint64_t tail = 0;
-      for (uint32_t q = m.P[s]; q != NONE_I && len < c; q = m.P[s]) {
-        tail = (tail << 2) | key_char(skey(m, s), k - 1);
-        s = q;
-        ++len;
+    for (uint32_t base = 0; base < nclosed; base += 32) {
+      const uint32_t j = base + lane;
+      uint32_t bin = NONE;
+      if (j < nclosed) {
+        uint32_t s = m.A[j], len = 1;
+        uint64_t tail = 0;
+        for (uint32_t q = m.P[s]; q != NONE_I && len < c; q = m.P[s]) {
+          tail = (tail << 2) | key_char(skey(m, s), k - 1);
+          s = q;
+          ++len;
+        }
+        const Key<NW> x = strip(skey(m, s));
+        Rec<NW + 1> r;
+        if constexpr (NW == 1) {
+          r.hi = rev2(x.w[0]);
+          r.lo = 0;
+        } else {
+          r.hi = rev2(x.w[0]);
+          r.lo = rev2(x.w[1]);
+        }
+        r.tail = (uint64_t(len - 1u) << TAIL_LEN_SHIFT) | tail;
+        st_rec<NW + 1>(out, uint64_t(slot) + j, r);
+        bin = uint32_t(r.hi >> (64 - p.rec_bits));
       }
-      const Key<NW> x = strip(skey(m, s));
-      Rec<NW + 1> r;
-      if constexpr (NW == 1) {
-        r.hi = rev2(x.w[0]);
-        r.lo = 0;
-      } else {
-        r.hi = rev2(x.w[0]);
-        r.lo = rev2(x.w[1]);
-      }
-      r.tail = (uint64_t(len - 1u) << TAIL_LEN_SHIFT) | tail;
-      atomicAdd(p.rec_counts + (r.hi >> (64 - p.rec_bits)), 1u);
-      st_rec<NW + 1>(out, uint64_t(slot) + j, r);
+      count_bin(p.rec_counts, bin);
     }
   } else {
     if (!WarpGroup::reserve(p, job, U3{cbytes, obytes, heads}, at)) return;

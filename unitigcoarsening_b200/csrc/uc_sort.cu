@@ -10,7 +10,9 @@
 //   k_line_group   records -> their tiles (by groups of tiles first)
 //   k_line_tiles   one block per tile: order in shared memory, the tile's
 //                  place in the output by look-back, lines spelled and stored
-// Nothing returns to the host in between.  The text is read once and written
+// Nothing returns to the host in between, unless a bin holds many tiles' worth
+// of lines (low-complexity k-mers: thousands of lines with the same first chars).
+// Such bins are sorted by the whole grid first (k_over_count, k_over_pass).  The text is read once and written
 // once.  Lines with more than TAIL_MAX chars after the k-mer keep their chars
 // in a copy of the text and are copied.
 //
@@ -19,6 +21,7 @@
 // of the lines (seven passes over pairs or lines) took 28 ms.
 #include <algorithm>
 #include <cstring>
+#include <utility>
 
 #include "uc_kernels.cuh"
 #include "uc_lookback.cuh"
@@ -43,6 +46,10 @@ template <int RW>
 __host__ __device__ constexpr uint32_t tile_cap() {
   return RW == 2 ? 2048u : 1536u;
 }
+// records per tile, give or take a bin (not a power of two: the tiles fill at one
+// pace, and with windows of 1024 their write frontiers lay 16 KB apart, in few
+// of L2's slices and sets)
+constexpr uint32_t WIN = 1000;
 constexpr uint32_t PLAN_ITEMS = 16;  // bins per thread of the plan
 // Cursors lie 32 bytes apart: atomics on words of one L2 line queue up (about
 // 2 ns each).
@@ -56,8 +63,24 @@ struct LongLine {
 
 struct SortCtr {
   uint32_t nrec, nlong, nhuge, ntiles;
-  uint32_t plan_ticket, tile_ticket, fail, pad;
+  uint32_t plan_ticket, tile_ticket, fail;
+  uint32_t nover;  // oversized bins
 };
+
+// An oversized bin's records are sorted beforehand and cut into tiles of their
+// own, marked in the tile's first bin.
+constexpr uint32_t TILE_RUN = 0x80000000u;
+// A bin is oversized from OVER_WINS windows on.  It then spans OVER_WINS tile
+// numbers at least, of which all but the last are its own: at most 1.5 windows
+// per tile, which fit.  Below that a tile of more than its capacity (6 windows at
+// most) is sorted by its block.  At most OVER_MAX bins are oversized (the limit
+// grows with the number of lines).
+constexpr uint32_t OVER_WINS = 5, OVER_MAX = 4096;
+struct OverBin {
+  uint32_t beg, n;   // records
+  uint32_t tile, nt; // tiles of its own
+};
+static_assert(WIN + WIN / 2 + 1 <= tile_cap<2>() && WIN + WIN / 2 + 1 <= tile_cap<3>(), "its tiles fit");
 
 __device__ __forceinline__ unsigned long long line_bytes_of(uint64_t tail, int k, const LongLine* longs) {
   return (tail & TAIL_LONG) ? longs[uint32_t(tail)].len : uint64_t(k) + 1u + ((tail >> TAIL_LEN_SHIFT) & 31u);
@@ -150,7 +173,8 @@ __global__ void __launch_bounds__(256, 5) k_line_recs(const char* __restrict__ o
     }
     if (tid == 0) s_base = nl ? atomicAdd(&sc->nrec, nl) : 0u;
     __syncthreads();
-    auto emit = [&](uint32_t j, uint32_t s, unsigned long long len) {  // len: chars of the line
+    // len: chars of the line; returns its bin
+    auto emit = [&](uint32_t j, uint32_t s, unsigned long long len) -> uint32_t {
       const bool is_long = len > uint64_t(k + TAIL_MAX);
       const uint32_t t = is_long ? 0u : uint32_t(len) - uint32_t(k);
       // the line's code stream from its first char (words past the halo are
@@ -184,13 +208,15 @@ __global__ void __launch_bounds__(256, 5) k_line_recs(const char* __restrict__ o
       } else {
         r.tail = (uint64_t(t) << TAIL_LEN_SHIFT) | (tl & ((1ull << (2 * t)) - 1ull));
       }
-      atomicAdd(counts + (r.hi >> (64 - bits)), 1u);
       st_rec<RW>(rec, s_base + j, r);
+      return uint32_t(r.hi >> (64 - bits));
     };
-    for (uint32_t j = tid; j < nl; j += 256) {
-      const uint32_t s = starts[j];
-      uint32_t len;
-      if (j + 1 < nl) {
+    for (uint32_t j0 = 0; j0 < nl; j0 += 256) {  // (whole warps together)
+      const uint32_t j = j0 + tid, s = j < nl ? starts[j] : 0u;
+      uint32_t len = 0, bin = NONE;
+      if (j >= nl) {
+        // no line
+      } else if (j + 1 < nl) {
         len = uint32_t(starts[j + 1]) - s - 1u;
       } else {
         // the chunk's last line: its break in the bits, or past the halo
@@ -200,8 +226,9 @@ __global__ void __launch_bounds__(256, 5) k_line_recs(const char* __restrict__ o
         len = m ? 32u * w + uint32_t(__ffs(m) - 1) - LR_PRE - s : 0u;
         if (!m) s_open = j + 1u;
       }
-      if (len >= uint32_t(k)) emit(j, s, len);
-      else if (len || j + 1 < nl) atomicOr(&sc->fail, 2u);
+      if (len >= uint32_t(k)) bin = emit(j, s, len);
+      else if (j < nl && (len || j + 1 < nl)) atomicOr(&sc->fail, 2u);
+      count_bin(counts, bin);
     }
     __syncthreads();
     if (s_open) {
@@ -231,7 +258,7 @@ __global__ void __launch_bounds__(256, 5) k_line_recs(const char* __restrict__ o
         __syncthreads();
         if (stop) break;
       }
-      if (tid == 0) emit(j, s, s_end - (c0 + s));
+      if (tid == 0) atomicAdd(counts + emit(j, s, s_end - (c0 + s)), 1u);
     }
     __syncthreads();  // code, nlw, starts are reused
   }
@@ -242,7 +269,12 @@ __global__ void __launch_bounds__(256, 5) k_line_recs(const char* __restrict__ o
 // its last bin.  One pass: prefix sums by look-back, each bin's tile in place
 // of its count, each tile's first record and first bin, and the cursors of
 // the tiles and of the groups of 2^gsh tiles.
+//
+// A bin of more than `big` records is listed, and gets the tile numbers that
+// lie inside it alone: its records go to the first of them as one run, which
+// k_over_items cuts into tiles of equal size.
 __global__ void __launch_bounds__(256) k_line_plan(uint32_t* __restrict__ counts, uint32_t m, uint32_t win,
+                                                   uint32_t big, OverBin* __restrict__ over,
                                                    uint2* __restrict__ tile, uint32_t* __restrict__ cur,
                                                    uint32_t* __restrict__ gcur, uint32_t gsh, unsigned long long* st,
                                                    SortCtr* sc) {
@@ -280,21 +312,50 @@ __global__ void __launch_bounds__(256) k_line_plan(uint32_t* __restrict__ counts
     cur[0] = gcur[0] = 0;
   }
   uint32_t tp = p / win;
+  uint32_t most = 0;
 #pragma unroll
-  for (uint32_t q = 0; q < PLAN_ITEMS; ++q) {
-    const uint32_t nx = p + c[q], tn = nx / win;
-    c[q] = tp;
-    for (uint32_t t = tp + 1; t <= tn; ++t) {
-      tile[t] = make_uint2(nx, i0 + q + 1);
-      cur[t * CUR_STRIDE] = nx;
-      if (!(t & ((1u << gsh) - 1u))) gcur[(t >> gsh) * CUR_STRIDE] = nx;
+  for (uint32_t q = 0; q < PLAN_ITEMS; ++q) most = max(most, c[q]);
+  if (most <= big) {
+#pragma unroll
+    for (uint32_t q = 0; q < PLAN_ITEMS; ++q) {
+      const uint32_t nx = p + c[q], tn = nx / win;
+      c[q] = tp;
+      for (uint32_t t = tp + 1; t <= tn; ++t) {
+        tile[t] = make_uint2(nx, i0 + q + 1);
+        cur[t * CUR_STRIDE] = nx;
+        if (!(t & ((1u << gsh) - 1u))) gcur[(t >> gsh) * CUR_STRIDE] = nx;
+      }
+      p = nx;
+      tp = tn;
     }
-    p = nx;
-    tp = tn;
-  }
 #pragma unroll
-  for (uint32_t q = 0; q < PLAN_ITEMS / 4; ++q)
-    src[q] = make_uint4(c[4 * q], c[4 * q + 1], c[4 * q + 2], c[4 * q + 3]);
+    for (uint32_t q = 0; q < PLAN_ITEMS / 4; ++q)
+      src[q] = make_uint4(c[4 * q], c[4 * q + 1], c[4 * q + 2], c[4 * q + 3]);
+  } else {
+    const uint32_t gm = (1u << gsh) - 1u;
+#pragma unroll 1
+    for (uint32_t q = 0; q < PLAN_ITEMS; ++q) {
+      const uint32_t n = counts[i0 + q], nx = p + n, tn = nx / win;
+      counts[i0 + q] = tp + (n > big ? 1u : 0u);
+      if (n > big) {
+        const uint32_t t0 = tp + 1u;
+        over[atomicAdd(&sc->nover, 1u)] = OverBin{p, n, t0, tn - t0};
+        tile[t0] = make_uint2(p, (i0 + q) | TILE_RUN);
+        cur[t0 * CUR_STRIDE] = p;
+        if (!(t0 & gm)) gcur[(t0 >> gsh) * CUR_STRIDE] = p;
+        if (gsh)
+          for (uint32_t t = (t0 | gm) + 1u; t < tn; t += gm + 1u) gcur[(t >> gsh) * CUR_STRIDE] = nx;
+        tp = tn - 1u;
+      }
+      for (uint32_t t = tp + 1; t <= tn; ++t) {
+        tile[t] = make_uint2(nx, i0 + q + 1);
+        cur[t * CUR_STRIDE] = nx;
+        if (!(t & gm)) gcur[(t >> gsh) * CUR_STRIDE] = nx;
+      }
+      p = nx;
+      tp = tn;
+    }
+  }
   if (i0 + PLAN_ITEMS >= m) {
     tile[tp + 1] = make_uint2(p, m);
     sc->ntiles = tp + 1;
@@ -503,10 +564,203 @@ __device__ __forceinline__ void store_lines(char* out, uint64_t at, uint32_t r0,
   T.end(buf);
 }
 
+// ---- oversized bins: their records, one run per bin, in order by radix passes
+// over the whole grid, 8 bits of the key each, least significant first, between the
+// two record arrays (k_line_group has left the runs in the first).  A pass is
+// one kernel: blocks take chunks in order from a ticket, rank their records per
+// digit, and find the digits' places from the run's counts of them and a look-back over
+// the chunks before theirs.  The time does not depend on how the keys are spread.
+// 2M to 3M lines, k = 31, of which n share 12 chars, whole call: 0.56, 0.83, 1.18, 2.29 ms
+// for n = 10k, 100k, 300k, 1M; with one block for each such bin 0.76, 3.4, 9.3, 30
+// (the call without ordering: 0.35, 0.55, 0.84, 1.78).  A pass is 18 us at 300k
+// records (the round trips of one chunk: few blocks have work).
+constexpr uint32_t OV_THREADS = 256, OV_PER = 8, OV_CHUNK = OV_THREADS * OV_PER;
+constexpr uint32_t OV_PASSES = 16;
+constexpr int OV_PASS_SHIFT = 40;  // look-back words: the tag, the pass, the value (40 bits)
+
+struct OverBins {
+  const OverBin* bin;      // [n]
+  uint32_t* item_start;    // [n + 1] first chunk of each
+  // cleared before the first pass:
+  uint32_t* ticket;        // [OV_PASSES]
+  uint32_t* hist;          // [passes][n][256] digit counts
+  unsigned long long* st;  // [chunks][256] look-back words
+  uint32_t n;
+};
+// The key's bytes that order a run, least significant first: byte position in
+// Rec::hi, or 64 and up in Rec::lo.
+struct Digits {
+  uint32_t n;
+  uint32_t sh[OV_PASSES];
+};
+template <int RW>
+__device__ __forceinline__ uint32_t digit_of(const Rec<RW>& r, uint32_t sh) {
+  if constexpr (RW == 3) return uint32_t((sh & 64u ? r.lo : r.hi) >> (sh & 63u)) & 255u;
+  else return uint32_t(r.hi >> sh) & 255u;
+}
+
+// First chunk of each run, and the runs' tiles.
+__global__ void __launch_bounds__(1024) k_over_items(OverBins o, uint2* __restrict__ tile) {
+  __shared__ uint32_t scan[33];
+  constexpr uint32_t PER = OVER_MAX / 1024;
+  if (blockIdx.x == 0) {
+    uint32_t c[PER], sum = 0;
+#pragma unroll
+    for (uint32_t q = 0; q < PER; ++q) {
+      const uint32_t i = threadIdx.x * PER + q;
+      c[q] = i < o.n ? (o.bin[i].n + OV_CHUNK - 1) / OV_CHUNK : 0u;
+      sum += c[q];
+    }
+    uint32_t tot, at = block_excl_scan(sum, scan, &tot);
+#pragma unroll
+    for (uint32_t q = 0; q < PER; ++q) {
+      const uint32_t i = threadIdx.x * PER + q;
+      if (i < o.n) o.item_start[i] = at;
+      at += c[q];
+    }
+    if (threadIdx.x == 0) o.item_start[o.n] = tot;
+  }
+  for (uint32_t i = blockIdx.x; i < o.n; i += gridDim.x) {
+    const OverBin B = o.bin[i];
+    const uint32_t each = B.n / B.nt, more = B.n % B.nt;
+    for (uint32_t j = threadIdx.x + 1u; j < B.nt; j += blockDim.x)  // (the first is written)
+      tile[B.tile + j] = make_uint2(B.beg + j * each + min(j, more), TILE_RUN);
+  }
+}
+
+// The run of chunk t (one warp calls): the last one that starts at or before it.
+__device__ __forceinline__ uint32_t over_bin_of(const OverBins& o, uint32_t t) {
+  uint32_t lo = 0, n = o.n;  // among [lo, lo + n)
+  while (n > 1) {
+    const uint32_t step = (n + 31u) / 32u, i = step * (threadIdx.x & 31u);
+    const uint32_t m = __ballot_sync(0xFFFFFFFFu, i < n && o.item_start[lo + i] <= t);
+    const uint32_t j = step * (31u - uint32_t(__clz(m)));  // (lane 0 always agrees)
+    lo += j;
+    n = min(step, n - j);
+  }
+  return lo;
+}
+
+// All passes' digit counts of each run.
+template <int RW>
+__global__ void __launch_bounds__(OV_THREADS) k_over_count(RecArr<RW> in, OverBins o, Digits dg) {
+  __shared__ uint32_t cnt[OV_PASSES / (4 - RW)][256], s_bin;  // (8 passes with one key word)
+  const uint32_t tid = threadIdx.x, nitems = o.item_start[o.n];
+  for (uint32_t t = blockIdx.x; t < nitems; t += gridDim.x) {
+    if (tid < 32) {
+      const uint32_t b = over_bin_of(o, t);
+      if (tid == 0) s_bin = b;
+    }
+    for (uint32_t p = 0; p < dg.n; ++p) cnt[p][tid] = 0;
+    __syncthreads();
+    const uint32_t b = s_bin, c0 = (t - o.item_start[b]) * OV_CHUNK;
+    const OverBin B = o.bin[b];
+    const uint32_t cn = min(OV_CHUNK, B.n - c0);
+    for (uint32_t i = tid; i < cn; i += OV_THREADS) {
+      const Rec<RW> r = ld_rec<RW>(in, uint64_t(B.beg) + c0 + i);
+      for (uint32_t p = 0; p < dg.n; ++p) atomicAdd(&cnt[p][digit_of<RW>(r, dg.sh[p])], 1u);
+    }
+    __syncthreads();
+    for (uint32_t p = 0; p < dg.n; ++p)
+      if (cnt[p][tid]) atomicAdd(o.hist + (uint64_t(p) * o.n + b) * 256u + tid, cnt[p][tid]);
+    __syncthreads();
+  }
+}
+
+template <int RW>
+__global__ void __launch_bounds__(OV_THREADS) k_over_pass(RecArr<RW> in, RecArr<RW> to, OverBins o, uint32_t pass,
+                                                          uint32_t sh, SortCtr* sc) {
+  constexpr uint32_t W = OV_THREADS / 32;
+  __shared__ uint32_t wcnt[W][256], place[256], scan[33], s_t, s_bin;
+  const uint32_t tid = threadIdx.x, lane = tid & 31u, wid = tid >> 5;
+  const uint32_t nitems = o.item_start[o.n];
+  const unsigned long long mark = static_cast<unsigned long long>(pass) << OV_PASS_SHIFT;
+  for (;;) {
+    if (tid < 32) {
+      uint32_t t = 0;
+      if (tid == 0) t = atomicAdd(o.ticket + pass, 1u);
+      t = __shfl_sync(0xFFFFFFFFu, t, 0);
+      const uint32_t b = over_bin_of(o, min(t, nitems - 1u));
+      if (tid == 0) {
+        s_t = t;
+        s_bin = b;
+      }
+    }
+#pragma unroll
+    for (uint32_t w = 0; w < W; ++w) wcnt[w][tid] = 0;
+    __syncthreads();
+    const uint32_t t = s_t, b = s_bin;
+    if (t >= nitems) break;
+    const OverBin B = o.bin[b];
+    const uint32_t chunk = t - o.item_start[b], c0 = chunk * OV_CHUNK, cn = min(OV_CHUNK, B.n - c0);
+    // the warp's records, 32 at a time in order, each ranked among the warp's of
+    // its digit
+    Rec<RW> r[OV_PER];
+    uint32_t rk[OV_PER];
+    const uint32_t i0 = wid * (OV_CHUNK / W) + lane;
+#pragma unroll
+    for (uint32_t q = 0; q < OV_PER; ++q)
+      if (i0 + 32 * q < cn) r[q] = ld_rec<RW>(in, uint64_t(B.beg) + c0 + i0 + 32 * q);
+    const uint32_t count = o.hist[(uint64_t(pass) * o.n + b) * 256u + tid];
+#pragma unroll
+    for (uint32_t q = 0; q < OV_PER; ++q) {
+      const bool live = i0 + 32 * q < cn;
+      const uint32_t d = live ? digit_of<RW>(r[q], sh) : 256u;
+      const uint32_t same = __match_any_sync(0xFFFFFFFFu, d), below = same & ((1u << lane) - 1u);
+      const uint32_t before = live ? wcnt[wid][d] : 0u;
+      __syncwarp();
+      if (live && below == 0) wcnt[wid][d] = before + uint32_t(__popc(same));
+      __syncwarp();
+      rk[q] = (before + uint32_t(__popc(below))) | (d << 16);
+    }
+    __syncthreads();
+    // thread d: digit d's records of the warps before each, and of the chunk
+    uint32_t mine = 0;
+#pragma unroll
+    for (uint32_t w = 0; w < W; ++w) {
+      const uint32_t c = wcnt[w][tid];
+      wcnt[w][tid] = mine;
+      mine += c;
+    }
+    unsigned long long* const word = o.st + uint64_t(t) * 256u + tid;
+    atomicExch(word, (chunk ? LB_SUM : LB_PREFIX) | mark | mine);
+    uint32_t tot, first = block_excl_scan(count, scan, &tot);
+    if (chunk) {  // the chunks of the run before this one
+      uint32_t before = 0;
+      for (uint32_t j = 1; j <= chunk; ++j) {
+        unsigned long long v = 0;
+        bool there = false;
+        for (uint32_t p = 0; p < LB_POLLS && !there; ++p) {
+          v = *reinterpret_cast<volatile unsigned long long*>(word - uint64_t(j) * 256u);
+          there = v > LB_VALUE && ((v & LB_VALUE) >> OV_PASS_SHIFT) == pass;
+          if ((p & 1023u) == 1023u && *reinterpret_cast<volatile uint32_t*>(&sc->fail)) break;
+        }
+        if (!there) {
+          atomicOr(&sc->fail, 1u);
+          break;
+        }
+        before += uint32_t(v);
+        if (v & LB_PREFIX) break;
+      }
+      atomicExch(word, LB_PREFIX | mark | (before + mine));
+      first += before;
+    }
+    place[tid] = first;
+    __syncthreads();
+#pragma unroll
+    for (uint32_t q = 0; q < OV_PER; ++q) {
+      if (i0 + 32 * q >= cn) continue;
+      const uint32_t d = rk[q] >> 16, pos = place[d] + wcnt[wid][d] + (rk[q] & 0xFFFFu);
+      if (pos < B.n) st_rec<RW>(to, uint64_t(B.beg) + pos, r[q]);  // (a failed wait: nothing out of bounds)
+    }
+    __syncthreads();  // the shared arrays are reused
+  }
+}
+
 // Stable order of n records of one tile too large for shared memory, by one
 // block: 8 bits of the key per pass, least significant first, between two
 // buffers.  Returns 1 where the result lies in y.  (A bin of more than a
-// tile's records: thousands of lines that share their first chars.)
+// tile's records, up to OVER_WINS windows of them.)
 template <int RW>
 __device__ int order_in_memory(RecArr<RW> x, RecArr<RW> y, uint64_t beg, uint32_t n, int k, uint32_t* hist,
                                uint32_t* wcnt) {
@@ -586,7 +840,7 @@ template <int RW>
 __global__ void __launch_bounds__(TILE_THREADS, RW == 2 ? 4 : 3) k_line_tiles(RecArr<RW> rec, RecArr<RW> spare,
                                                              const uint2* __restrict__ tile, int bits, char* out, int k,
                                                              LongLine* longs, const char* keep,
-                                                             unsigned long long* st, SortCtr* sc) {
+                                                             unsigned long long* st, SortCtr* sc, int runs) {
   extern __shared__ __align__(16) unsigned char sm[];
   constexpr uint32_t TILE_CAP = tile_cap<RW>();
   uint64_t* khi = reinterpret_cast<uint64_t*>(sm);
@@ -601,6 +855,8 @@ __global__ void __launch_bounds__(TILE_THREADS, RW == 2 ? 4 : 3) k_line_tiles(Re
   const uint32_t tid = threadIdx.x, lane = tid & 31u, wid = tid >> 5;
   constexpr uint32_t W = TILE_THREADS / 32, PER = TILE_CAP / TILE_THREADS;
   if (sc->fail) return;  // (of the kernels before; uniform)
+  // oversized bins have to be sorted first (runs: they are, 1 in rec, 2 in spare)
+  if (!runs && sc->nover) return;
   const uint32_t ntiles = sc->ntiles;
   for (;;) {
     if (tid == 0) s_t = atomicAdd(&sc->tile_ticket, 1u);
@@ -609,15 +865,27 @@ __global__ void __launch_bounds__(TILE_THREADS, RW == 2 ? 4 : 3) k_line_tiles(Re
     if (t >= ntiles) break;
     const uint2 T0 = tile[t], T1 = tile[t + 1];
     const uint32_t beg = T0.x, n = T1.x - beg;
-    const bool fits = n <= TILE_CAP;
+    const bool run = (T0.y & TILE_RUN) != 0;  // in order already (and fits)
+    const bool fits = run || n <= TILE_CAP;
     // the tile's key range, spread over the sub-bins
     const uint64_t kmin = T0.y ? uint64_t(T0.y) << (64 - bits) : 0ull;
-    const int sh = max(0, 53 - bits + (T1.y - T0.y > 1u ? 32 - __clz(T1.y - T0.y - 1u) : 0));
+    const uint32_t nbins = (T1.y & ~TILE_RUN) - (T0.y & ~TILE_RUN);
+    const int sh = max(0, 53 - bits + (nbins > 1u ? 32 - __clz(nbins - 1u) : 0));
     unsigned long long bytes = 0;
     uint32_t rk[PER];
     for (uint32_t j = tid; j < TILE_SUB; j += TILE_THREADS) sub[j] = 0;
     __syncthreads();
-    if (fits) {
+    if (run) {
+      const RecArr<RW> src = runs == 2 ? spare : rec;
+      for (uint32_t i = tid; i < n; i += TILE_THREADS) {
+        const Rec<RW> r = ld_rec<RW>(src, uint64_t(beg) + i);
+        khi[i] = r.hi;
+        if constexpr (RW == 3) klo[i] = r.lo;
+        tl[i] = r.tail;
+        bytes += line_bytes_of(r.tail, k, longs);
+        fin[i] = uint16_t(i);
+      }
+    } else if (fits) {
 #pragma unroll
       for (uint32_t q = 0; q < PER; ++q) {
         if (q * TILE_THREADS >= n) break;
@@ -646,7 +914,8 @@ __global__ void __launch_bounds__(TILE_THREADS, RW == 2 ? 4 : 3) k_line_tiles(Re
     for (uint32_t w = 0; w < W; ++w) bytes += s_sum[w];
     if (tid == 0) lb_publish(st, t, LB_SUM, bytes);
     int in_spare = 0;
-    if (fits) {
+    if (run) {
+    } else if (fits) {
       {
         constexpr uint32_t C = TILE_SUB / TILE_THREADS;
         uint32_t c[C], sum = 0;
@@ -740,6 +1009,38 @@ __global__ void __launch_bounds__(256) k_huge_lines(char* out, const char* keep,
   }
 }
 
+// The oversized bins' records in order: in a (runs = 1) or b (2) after it.
+template <int RW>
+int sort_over(Env& e, RecArr<RW> a, RecArr<RW> b, OverBins ov, const SortCtr& h, int k, int bits, uint2* tile,
+              SortCtr* sc, int& runs) {
+  ov.n = h.nover;
+  const uint64_t nchunk = h.nrec / OV_CHUNK + h.nover;  // at most
+  // the bytes that hold chars, but for those within the bins' own bits
+  Digits dg{};
+  for (int sh = 0; RW == 3 && sh < 64; sh += 8)
+    if (sh + 8 > 128 - 2 * k) dg.sh[dg.n++] = uint32_t(64 + sh);
+  for (int sh = 0; sh < 64 - bits; sh += 8)
+    if (sh + 8 > 64 - 2 * k) dg.sh[dg.n++] = uint32_t(sh);
+  runs = 1;
+  int occ = 0;
+  if (const int ro = occupancy(e, occ, k_over_pass<RW>, int(OV_THREADS), 0)) return ro;
+  const unsigned g = unsigned(std::min<uint64_t>(nchunk, uint64_t(e.sm_count) * uint64_t(std::max(1, occ))));
+  e.launches += 2 + dg.n;
+  k_over_items<<<std::min(ov.n, unsigned(e.sm_count)), 1024, 0, e.stream>>>(ov, tile);
+  // tickets, counts and look-back words lie in one piece
+  ov.st = reinterpret_cast<unsigned long long*>(ov.hist + uint64_t(dg.n) * ov.n * 256);
+  UC_CK(cudaMemsetAsync(ov.ticket, 0, size_t(reinterpret_cast<char*>(ov.st + nchunk * 256) -
+                                             reinterpret_cast<char*>(ov.ticket)), e.stream));
+  k_over_count<RW><<<g, OV_THREADS, 0, e.stream>>>(a, ov, dg);
+  for (uint32_t i = 0; i < dg.n; ++i) {
+    k_over_pass<RW><<<g, OV_THREADS, 0, e.stream>>>(a, b, ov, i, dg.sh[i], sc);
+    std::swap(a, b);
+    runs = 3 - runs;
+  }
+  UC_CK(cudaGetLastError());
+  return UC_OK;
+}
+
 // The launch sequence for one key width: the lines of out[0, bytes) and
 // those of pre.
 template <int RW>
@@ -748,14 +1049,14 @@ int sort_lines_rw(Env& e, char* out, uint64_t bytes, int k, const LineRecs& pre)
   const int bits = pre.bits;
   if (lmax > pre.cap) return e.fail(UC_EINTERNAL, "more lines than k-mers");
   const uint32_t m = 1u << bits;
-  // windows of 1000 records; shorter ones while there are fewer than two
-  // tiles per SM.  (Not a power of two: the tiles fill at one pace, and with
-  // windows of 1024 their write frontiers lay 16 KB apart, in few of L2's
-  // slices and sets.)
-  uint32_t win = 1000;
+  // shorter windows while there are fewer than two tiles per SM
+  uint32_t win = WIN;
   while (win > 250 && lmax / win < 2ull * e.sm_count) win /= 2;
   const uint64_t ntmax = lmax / win + 2;
   const uint64_t nplan = (uint64_t(m) + 256 * PLAN_ITEMS - 1) / (256 * PLAN_ITEMS);
+  // (fewer than OVER_MAX bins hold more than lmax / OVER_MAX lines each)
+  const uint32_t big = uint32_t(std::max<uint64_t>(OVER_WINS * win, lmax / OVER_MAX));
+  const uint64_t nover = lmax / big + 1, nchunk = lmax / OV_CHUNK + nover + 1;  // at most
   const uint64_t nlongs = bytes / uint64_t(k + TAIL_MAX + 2) + 1, nhuges = bytes / HUGE_LINE + 1;
   // more tiles than k_line_group counts at once: groups of 2^gsh first
   uint32_t gsh = 0;
@@ -772,6 +1073,10 @@ int sort_lines_rw(Env& e, char* out, uint64_t bytes, int k, const LineRecs& pre)
   add(nlongs * sizeof(LongLine));
   add(nhuges * 4);
   add(bytes + 16);
+  const size_t ovb = OV_PASSES * 4 + (nover * OV_PASSES / (4 - RW) * 4 + nchunk * 8) * 256;
+  add(nover * sizeof(OverBin));
+  add((nover + 1) * 4);
+  add(ovb);
   // above the records in the back arena, or, where they leave too little
   // there, in the oversized tiles' scratch (free by now)
   char* at = nullptr;
@@ -798,6 +1103,12 @@ int sort_lines_rw(Env& e, char* out, uint64_t bytes, int k, const LineRecs& pre)
   LongLine* longs = reinterpret_cast<LongLine*>(take(nlongs * sizeof(LongLine)));
   uint32_t* huge = reinterpret_cast<uint32_t*>(take(nhuges * 4));
   char* keep = take(bytes + 16);
+  OverBins ov{};
+  OverBin* over = reinterpret_cast<OverBin*>(take(nover * sizeof(OverBin)));
+  ov.bin = over;
+  ov.item_start = reinterpret_cast<uint32_t*>(take((nover + 1) * 4));
+  ov.ticket = reinterpret_cast<uint32_t*>(take(ovb));
+  ov.hist = ov.ticket + OV_PASSES;
   SortCtr* sc = reinterpret_cast<SortCtr*>(z);
   unsigned long long* st_plan = reinterpret_cast<unsigned long long*>(z + 256);
   unsigned long long* st_tile = st_plan + nplan;
@@ -812,10 +1123,10 @@ int sort_lines_rw(Env& e, char* out, uint64_t bytes, int k, const LineRecs& pre)
   const size_t sm_tile = tile_smem<RW>(k);
   int occ = 0;
   if (const int ro = occupancy(e, occ, k_line_recs<RW>, 256, sm_recs)) return ro;
-  e.launches += 2;
+  ++e.launches;
   if (bytes) ++e.launches;
   if (bytes) k_line_recs<RW><<<grid(nchunks, occ), 256, sm_recs, e.stream>>>(out, bytes, k, bits, ra, counts, longs, huge, sc);
-  k_line_plan<<<unsigned(nplan), 256, 0, e.stream>>>(counts, m, win, tile, cur, gcur, gsh, st_plan, sc);
+  k_line_plan<<<unsigned(nplan), 256, 0, e.stream>>>(counts, m, win, big, over, tile, cur, gcur, gsh, st_plan, sc);
   if (nlongs > 1) {
     ++e.launches;
     k_line_keep<<<grid((nlongs + 7) / 8, 4), 256, 0, e.stream>>>(out, keep, longs, huge, sc);
@@ -833,13 +1144,25 @@ int sort_lines_rw(Env& e, char* out, uint64_t bytes, int k, const LineRecs& pre)
   if (r) return r;
   if (const int ro = occupancy(e, occ, k_line_tiles<RW>, int(TILE_THREADS), sm_tile)) return ro;
   if (occ < 1) return e.fail(UC_EINTERNAL, "line tile kernel does not fit an SM");
-  k_line_tiles<RW><<<grid(ntmax, occ), TILE_THREADS, sm_tile, e.stream>>>(from, to, tile, bits, out, k, longs, keep,
-                                                                         st_tile, sc);
-  UC_CK(cudaGetLastError());
   static_assert(sizeof(SortCtr) <= Env::HOST_IO, "the counters fit the pinned area");
   SortCtr& h = *reinterpret_cast<SortCtr*>(e.h_io());
-  UC_CK(cudaMemcpyAsync(&h, sc, sizeof h, cudaMemcpyDeviceToHost, e.stream));
-  UC_CK(cudaStreamSynchronize(e.stream));
+  auto tiles = [&](int runs) -> int {
+    ++e.launches;
+    k_line_tiles<RW><<<grid(ntmax, occ), TILE_THREADS, sm_tile, e.stream>>>(from, to, tile, bits, out, k, longs, keep,
+                                                                           st_tile, sc, runs);
+    UC_CK(cudaGetLastError());
+    UC_CK(cudaMemcpyAsync(&h, sc, sizeof h, cudaMemcpyDeviceToHost, e.stream));
+    UC_CK(cudaStreamSynchronize(e.stream));
+    return UC_OK;
+  };
+  r = tiles(0);
+  if (r) return r;
+  if (h.nover && !h.fail) {
+    int runs = 1;
+    r = sort_over<RW>(e, from, to, ov, h, k, bits, tile, sc, runs);
+    if (!r) r = tiles(runs);
+    if (r) return r;
+  }
   if (h.fail & 1u) return e.fail(UC_ETIMEOUT, "a bounded device wait ran out (sorted output)");
   if (h.fail) return e.fail(UC_EINTERNAL, "a line of the output is shorter than k");
   if (h.nhuge) {
