@@ -83,17 +83,17 @@ __device__ __forceinline__ void count_bin(uint32_t* counts, uint32_t bin) {
   if (n) atomicAdd(counts + bin, n);
 }
 
-// Lines the tiles left as records: the records (rec_bytes bytes of lines), a
-// second array as large, and a count per bin of the key's leading bits.  The
-// arrays lie in the back arena below `used`.
+// Lines the tiles left as records: the records (rec_bytes bytes of lines) and a
+// count per bin of the key's leading bits.  The records lie in the back arena, the
+// counts at the start of the front arena (in the keys, which the scatter has
+// read); nothing else of either arena is in use by then.
 struct LineRecs {
-  char *a = nullptr, *b = nullptr;
-  uint64_t cap = 0;  // records either array holds
+  char* a = nullptr;
+  uint64_t cap = 0;  // records that fit at a
   uint32_t* counts = nullptr;
   int bits = 0;
   uint32_t n = 0;
   uint64_t bytes = 0;
-  size_t used = 0;
 };
 
 // One open segment of the fused path (written by the tile that finds it): the

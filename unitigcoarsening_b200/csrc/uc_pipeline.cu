@@ -3557,7 +3557,7 @@ int Env::reserve(int w, size_t bytes) {
   return UC_OK;
 }
 
-int Env::big_scratch(size_t bytes, char*& p, const char* what) {
+int Env::big_scratch(size_t bytes, char*& p, const char* what, size_t beside) {
   if (bytes > big_cap) {
     if (big_buf) {
       cudaStreamSynchronize(stream);
@@ -3565,7 +3565,7 @@ int Env::big_scratch(size_t bytes, char*& p, const char* what) {
     }
     big_buf = nullptr;
     big_cap = 0;
-    if (bytes > budget) return fail(UC_EBUDGET, what);
+    if (bytes + beside > budget) return fail(UC_EBUDGET, what);
     if (dev_malloc(reinterpret_cast<void**>(&big_buf), bytes) != cudaSuccess) {
       cudaGetLastError();
       big_buf = nullptr;
@@ -5149,21 +5149,12 @@ static int compact_jobs(Env& e, uint32_t njobs, const char* const* texts, const 
   const size_t back = back_bytes(e, copies, X, Sp, nw, k, want_hec);
   // (half of the k-mers start a line at most in canonical input)
   const int rbits = recs ? line_bin_bits(N / 2, k) : 0;
-  const size_t rcount = recs ? size_t(4) << rbits : 0;
-  r = e.reserve(1, back + rcount + 256);
+  r = e.reserve(1, back);
   if (r) return r;
   auto T64 = [&](uint64_t c) { return static_cast<unsigned long long*>(e.take(1, c * 8)); };
   auto T32 = [&](uint64_t c) { return static_cast<uint32_t*>(e.take(1, c * 4)); };
   char* region1 = static_cast<char*>(e.take(1, scatter_stage_bytes(copies, nw)));
   char* region2 = static_cast<char*>(e.take(1, scatter_stage_bytes(copies, nw)));
-  if (recs) {
-    recs->counts = static_cast<uint32_t*>(e.take(1, rcount));
-    recs->bits = rbits;
-    recs->cap = copies;
-    recs->used = (e.ar[1].used + 255) & ~size_t(255);
-    if (!recs->counts) return e.fail(UC_EBUDGET, "back arena overflow");
-    UC_CK(cudaMemsetAsync(recs->counts, 0, rcount, e.stream));
-  }
   SegRec* seg = static_cast<SegRec*>(e.take(1, Sp * sizeof(SegRec)));
   unsigned long long* Xr = T64(Sp);
   char* segc = static_cast<char*>(e.take(1, segchars));
@@ -5212,10 +5203,13 @@ static int compact_jobs(Env& e, uint32_t njobs, const char* const* texts, const 
   tp.jout = jd.jout;
   tp.jseg = jd.jseg;
   if (recs) {
-    // the scatter's region that does not hold the copies, and after the
-    // tiles the other one
+    // the scatter's region that does not hold the copies
     recs->a = reinterpret_cast<char*>(pkeys) == region1 ? region2 : region1;
-    recs->b = reinterpret_cast<char*>(pkeys) == region1 ? region1 : region2;
+    recs->cap = copies;
+    // (no more of them than a sixteenth of the lines, or 16)
+    recs->counts = reinterpret_cast<uint32_t*>(f.keys);
+    recs->bits = rbits;
+    UC_CK(cudaMemsetAsync(recs->counts, 0, size_t(4) << rbits, e.stream));
     tp.rec_a = reinterpret_cast<ulonglong2*>(recs->a);
     tp.rec_t = reinterpret_cast<unsigned long long*>(tp.rec_a + copies);
     tp.rec_counts = recs->counts;

@@ -1064,50 +1064,66 @@ int sort_lines_rw(Env& e, char* out, uint64_t bytes, int k, const LineRecs& pre)
     for (gsh = 5; (ntmax >> gsh) > GRP_BINS / 2; ) ++gsh;
   // cleared: the counters and the look-back words
   const size_t zero = 256 + (nplan + ntmax) * 8;
-  size_t need = 0;
-  auto add = [&](size_t b) { need += (b + 255) & ~size_t(255); };
-  add(zero);
-  add((ntmax + 1) * 8);
-  add((ntmax + GRP_BINS) * CUR_STRIDE * 4);
-  add(((ntmax >> gsh) + 1 + GRP_BINS) * CUR_STRIDE * 4);
-  add(nlongs * sizeof(LongLine));
-  add(nhuges * 4);
-  add(bytes + 16);
   const size_t ovb = OV_PASSES * 4 + (nover * OV_PASSES / (4 - RW) * 4 + nchunk * 8) * 256;
-  add(nover * sizeof(OverBin));
-  add((nover + 1) * 4);
-  add(ovb);
-  // above the records in the back arena, or, where they leave too little
-  // there, in the oversized tiles' scratch (free by now)
-  char* at = nullptr;
-  if (e.ar[1].cap >= pre.used + need) {
-    at = e.ar[1].base + pre.used;
-  } else {
-    const int r = e.big_scratch(need, at, "scratch for sorted output");
+  // The job's arrays are used up but for the records and their counts, so the
+  // scratch takes what lies around those in both arenas, and device memory of its own
+  // (the oversized tiles' scratch, free by now) only where that is too little.
+  // Sorted output thus fits where the job itself does, but for jobs with more
+  // text lines than half their k-mers and few cross k-mers.
+  struct Room {
+    uintptr_t at, end;
+  };
+  auto addr = [](const void* p) { return reinterpret_cast<uintptr_t>(p); };
+  const uintptr_t mid = addr(pre.a) + pre.cap * 16;  // the tails (two key words)
+  const uintptr_t last = RW == 3 ? mid + lmax * 8 : addr(pre.a) + lmax * 16;
+  const Room all[4] = {{addr(e.ar[1].base), addr(pre.a)},
+                       {addr(pre.a) + lmax * 16, RW == 3 ? mid : 0},
+                       {last, addr(e.ar[1].base) + e.ar[1].cap},
+                       {addr(pre.counts) + (size_t(4) << bits), addr(e.ar[0].base) + e.ar[0].cap}};
+  char *own = nullptr, *recs, *tails, *keep, *z, *p_longs, *p_cur, *p_gcur, *p_tile, *p_huge, *p_over, *p_item, *p_ov;
+  for (;;) {
+    Room room[4];
+    std::copy(all, all + 4, room);
+    size_t more = 0;
+    auto take = [&](size_t b) {
+      for (Room& r : room) {
+        const uintptr_t at = (r.at + 255) & ~uintptr_t(255);
+        if (at + b > r.end) continue;
+        r.at = at + b;
+        return reinterpret_cast<char*>(at);
+      }
+      char* const p = own + more;
+      more += (b + 255) & ~size_t(255);
+      return p;
+    };
+    keep = take(bytes + 16);
+    recs = take(lmax * 16);
+    tails = RW == 3 ? take(lmax * 8) : nullptr;
+    z = take(zero);
+    p_longs = take(nlongs * sizeof(LongLine));
+    p_cur = take((ntmax + GRP_BINS) * CUR_STRIDE * 4);
+    p_gcur = take(((ntmax >> gsh) + 1 + GRP_BINS) * CUR_STRIDE * 4);
+    p_tile = take((ntmax + 1) * 8);
+    p_huge = take(nhuges * 4);
+    p_over = take(nover * sizeof(OverBin));
+    p_item = take((nover + 1) * 4);
+    p_ov = take(ovb);
+    if (!more || own) break;
+    const int r = e.big_scratch(more, own, "scratch for sorted output", e.ar[0].cap + e.ar[1].cap);
     if (r) return r;
   }
-  auto take = [&](size_t b) {
-    char* p = at;
-    at += (b + 255) & ~size_t(255);
-    return p;
-  };
-  char* z = take(zero);
-  RecArr<RW> ra{reinterpret_cast<ulonglong2*>(pre.a), nullptr}, rb{reinterpret_cast<ulonglong2*>(pre.b), nullptr};
-  if (RW == 3) {
-    ra.t = reinterpret_cast<unsigned long long*>(ra.a + pre.cap);
-    rb.t = reinterpret_cast<unsigned long long*>(rb.a + pre.cap);
-  }
-  uint2* tile = reinterpret_cast<uint2*>(take((ntmax + 1) * 8));
-  uint32_t* cur = reinterpret_cast<uint32_t*>(take((ntmax + GRP_BINS) * CUR_STRIDE * 4));
-  uint32_t* gcur = reinterpret_cast<uint32_t*>(take(((ntmax >> gsh) + 1 + GRP_BINS) * CUR_STRIDE * 4));
-  LongLine* longs = reinterpret_cast<LongLine*>(take(nlongs * sizeof(LongLine)));
-  uint32_t* huge = reinterpret_cast<uint32_t*>(take(nhuges * 4));
-  char* keep = take(bytes + 16);
+  const RecArr<RW> ra{reinterpret_cast<ulonglong2*>(pre.a), reinterpret_cast<unsigned long long*>(mid)};
+  const RecArr<RW> rb{reinterpret_cast<ulonglong2*>(recs), reinterpret_cast<unsigned long long*>(tails)};
+  uint2* tile = reinterpret_cast<uint2*>(p_tile);
+  uint32_t* cur = reinterpret_cast<uint32_t*>(p_cur);
+  uint32_t* gcur = reinterpret_cast<uint32_t*>(p_gcur);
+  LongLine* longs = reinterpret_cast<LongLine*>(p_longs);
+  uint32_t* huge = reinterpret_cast<uint32_t*>(p_huge);
+  OverBin* over = reinterpret_cast<OverBin*>(p_over);
   OverBins ov{};
-  OverBin* over = reinterpret_cast<OverBin*>(take(nover * sizeof(OverBin)));
   ov.bin = over;
-  ov.item_start = reinterpret_cast<uint32_t*>(take((nover + 1) * 4));
-  ov.ticket = reinterpret_cast<uint32_t*>(take(ovb));
+  ov.item_start = reinterpret_cast<uint32_t*>(p_item);
+  ov.ticket = reinterpret_cast<uint32_t*>(p_ov);
   ov.hist = ov.ticket + OV_PASSES;
   SortCtr* sc = reinterpret_cast<SortCtr*>(z);
   unsigned long long* st_plan = reinterpret_cast<unsigned long long*>(z + 256);
