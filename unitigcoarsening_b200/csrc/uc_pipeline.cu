@@ -3103,6 +3103,7 @@ __global__ void k_cycle_list(const uint8_t* __restrict__ oncycle, uint64_t n,
 // distance) pairs, twice the bytes and past L2.  16.3M k-mers: 134 us, and 29 for
 // the rest, where the first state, the rounds and the split of the pairs took
 // 92, 323 and 50.
+// A warp whose vertices are nearly all left halfway stops there (long lines).
 // head[v] == NONE: not ranked yet.
 constexpr uint32_t RANK_STEPS = 8;
 __global__ void __launch_bounds__(256) k_rank_walk(const uint32_t* __restrict__ pred, uint64_t n,
@@ -3120,18 +3121,26 @@ __global__ void __launch_bounds__(256) k_rank_walk(const uint32_t* __restrict__ 
       d[q] = 0;
       p[q] = v < n ? pred[v] : NONE;
     }
+    auto walk = [&](uint32_t steps) {
 #pragma unroll 1
-    for (uint32_t i = 0; i < RANK_STEPS; ++i) {
-      if ((p[0] & p[1] & p[2] & p[3]) == NONE) break;
+      for (uint32_t i = 0; i < steps; ++i) {
+        if ((p[0] & p[1] & p[2] & p[3]) == NONE) break;
 #pragma unroll
-      for (uint32_t q = 0; q < 4; ++q) {
-        if (p[q] != NONE) {
-          h[q] = p[q];
-          ++d[q];
-          p[q] = pred[h[q]];
+        for (uint32_t q = 0; q < 4; ++q) {
+          if (p[q] != NONE) {
+            h[q] = p[q];
+            ++d[q];
+            p[q] = pred[h[q]];
+          }
         }
       }
-    }
+    };
+    walk(RANK_STEPS / 2);
+    // (long lines: the rounds get there sooner)
+    uint32_t left = 0;
+#pragma unroll
+    for (uint32_t q = 0; q < 4; ++q) left += uint32_t(__popc(__ballot_sync(0xFFFFFFFFu, p[q] != NONE)));
+    if (left <= 112) walk(RANK_STEPS - RANK_STEPS / 2);
     uint32_t open = 0;
 #pragma unroll
     for (uint32_t q = 0; q < 4; ++q) {
@@ -3163,17 +3172,17 @@ __global__ void __launch_bounds__(256) k_rank_walk(const uint32_t* __restrict__ 
 // ranked takes its head; one whose pointer is not jumps to where that one
 // points.  rank is stored before head, so whoever sees the head sees the rank.
 // Lists open after the last round hold cycles (and what leads into one): count
-// in cnt[rounds].
+// in cnt[rounds].  More than `most` vertices left by the walk: nothing is done.
 __global__ void __launch_bounds__(1024, 2) k_rank_rest(unsigned long long* X, uint32_t* head, uint32_t* rank,
                                                        uint32_t* list0, uint32_t* list1, uint32_t* cnt,
-                                                       uint32_t rounds, uint32_t* bar, uint32_t* err) {
+                                                       uint32_t rounds, uint32_t most, uint32_t* bar, uint32_t* err) {
   __shared__ uint32_t sc[33];
   uint32_t gen = 0;
   volatile unsigned long long* const vX = X;
   volatile uint32_t *const vh = head, *const vr = rank;
   for (uint32_t r = 0; r < rounds; ++r) {
     const uint32_t na = *reinterpret_cast<volatile uint32_t*>(cnt + r);
-    if (na == 0) return;
+    if (na == 0 || na > most) return;
     volatile uint32_t* const in = (r & 1) ? list1 : list0;
     uint32_t* const out = (r & 1) ? list0 : list1;
     // whole blocks iterate together (block_append needs every thread)
@@ -3209,6 +3218,24 @@ __global__ void __launch_bounds__(1024, 2) k_rank_rest(unsigned long long* X, ui
     rank[s] = pk_o(v);
     head[s] = pk_p(v);
   }
+}
+
+// Long lines (the k-mers of one strand): most vertices are left after the walk, and a
+// round of k_rank_rest gathers head and entry of each pointer.  With more than
+// three quarters of them left (lines of 32 and more) every vertex gets its entry, in
+// k_rank_round's form, and the rounds run as launches of that, two gathers of
+// entries each that make up for two to three rounds of doubling, over all ids first.
+// The host sees the count at the wait it has anyway; below RANK_DENSE vertices
+// that wait and the launches are longer than what they save (100k: 200 us against 155).
+// 8M k-mers, shuffled, lines of 20, 50, 1000 and 1M k-mers, the whole call: 434, 623, 912,
+// 1821 us; with k_rank_rest alone 433, 667, 1277, 2190; with rounds from the first state
+// alone 492, 593, 924, 1968.
+constexpr uint64_t RANK_DENSE = 1ull << 19;
+__global__ void k_rank_fill(const uint32_t* __restrict__ head, const uint32_t* __restrict__ rank, uint64_t n,
+                            unsigned long long* __restrict__ X, uint32_t* count) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) *count = uint32_t(n);  // the first round takes them all, in order
+  for (uint64_t v = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; v < n; v += uint64_t(gridDim.x) * blockDim.x)
+    if (head[v] != NONE) X[v] = pk(head[v] == uint32_t(v) ? head[v] | HEAD_BIT : head[v], rank[v]);
 }
 
 __global__ void k_head_rank(const unsigned long long* __restrict__ X, uint64_t n,
@@ -4631,19 +4658,31 @@ int contract(Env& e, const uint64_t* d_keys, const uint32_t* succ, const uint32_
   const uint64_t want = (n + 1023) / 1024;
   const unsigned g = unsigned(std::max<uint64_t>(1, std::min<uint64_t>(want, uint64_t(e.sm_count) * std::max(1, occ))));
   uint32_t *bar = cnt + 48, *errp = &e.ctr->err;
-  void* args[] = {&X, &head, &rank, &a0, &a1, &cnt, &rounds, &bar, &errp};
+  uint32_t most = n < RANK_DENSE ? uint32_t(n) : uint32_t(n - n / 4);
+  void* args[] = {&X, &head, &rank, &a0, &a1, &cnt, &rounds, &most, &bar, &errp};
   UC_CK(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(k_rank_rest), dim3(g), dim3(1024), args, 0, e.stream));
-  uint32_t* const hl = reinterpret_cast<uint32_t*>(e.h_io());
-  UC_CK(cudaMemcpyAsync(hl, cnt + rounds, 4, cudaMemcpyDeviceToHost, e.stream));
+  uint32_t* const hl = reinterpret_cast<uint32_t*>(e.h_io());  // the lists' sizes
+  UC_CK(cudaMemcpyAsync(hl, cnt, (rounds + 1) * 4, cudaMemcpyDeviceToHost, e.stream));
   r = e.read_ctr();
   if (r) return r;
+  if (hl[0] > most && !e.h_ctr->err) {
+    const int grid = grid_for(e, n, 256);
+    e.launches += 2 + rounds;
+    k_rank_fill<<<grid, 256, 0, e.stream>>>(head, rank, n, X, cnt);
+    for (uint32_t i = 0; i < rounds; ++i)
+      k_rank_round<<<grid, 256, 0, e.stream>>>(X, i == 0 ? nullptr : (i & 1) ? a1 : a0, cnt + i, (i & 1) ? a0 : a1, cnt + i + 1);
+    k_head_rank<<<grid, 256, 0, e.stream>>>(X, n, head, rank);
+    UC_CK(cudaGetLastError());
+    UC_CK(cudaMemcpyAsync(hl, cnt, (rounds + 1) * 4, cudaMemcpyDeviceToHost, e.stream));
+    UC_CK(cudaStreamSynchronize(e.stream));
+  }
   if (e.h_ctr->err) {
     r = e.check_err(e.h_ctr);
     UC_CK(cudaMemsetAsync(&e.ctr->err, 0, 4, e.stream));
     e.reset();
     return r;
   }
-  const uint32_t hleft = *hl;
+  const uint32_t hleft = hl[rounds];
   const uint32_t* act = (rounds & 1) ? a1 : a0;
   if (hleft) {
     UC_CK(cudaMemsetAsync(seen, 0, n, e.stream));
