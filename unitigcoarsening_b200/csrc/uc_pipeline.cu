@@ -3335,35 +3335,54 @@ __device__ __forceinline__ uint4 ld4(const uint32_t* __restrict__ p, uint64_t v,
 // voff[v]: members of the heads before v.  base[b]: lines (high half) and
 // members (low half) before block b's vertices; base[blocks] the totals.
 // Loads of four words and stores likewise: 87 -> 70 us at 16.3M k-mers.
+// Lines and members share a look-back word, 31 bits each; WIDE (from EMIT_WIDE
+// vertices on): members in st, lines in the words behind it.
+constexpr uint64_t EMIT_WIDE = 0x7FFFFFFFull;
+template <bool WIDE>
 __global__ void __launch_bounds__(256) k_emit_scan(const uint32_t* __restrict__ head, const uint32_t* __restrict__ cnt,
                                                    uint64_t n, uint32_t* __restrict__ voff,
                                                    unsigned long long* __restrict__ base, unsigned long long* st,
                                                    uint32_t* ctl) {
-  __shared__ unsigned long long scan[33], s_base;
-  __shared__ uint32_t s_b;
+  __shared__ unsigned long long scan[33], s_base, s_lines;
+  __shared__ uint32_t s_b, lscan[33];
   if (threadIdx.x == 0) s_b = atomicAdd(ctl, 1u);
   __syncthreads();
   const uint32_t b = s_b;
   const uint64_t v0 = uint64_t(b) * EMIT_TILE + 4u * threadIdx.x;
-  const uint4 h = ld4(head, v0, n, NONE), m = ld4(cnt, v0, n, 0u);
+  // (past the last vertex: no vertex's own id)
+  const uint4 h = ld4(head, v0, n, ~uint32_t(v0)), m = ld4(cnt, v0, n, 0u);
   const uint32_t hd[4] = {h.x, h.y, h.z, h.w}, mem[4] = {m.x, m.y, m.z, m.w};
-  uint32_t c[4];
+  uint32_t c[4], lines = 0;
   unsigned long long sum = 0;
 #pragma unroll
   for (uint32_t q = 0; q < 4; ++q) {
-    c[q] = hd[q] == uint32_t(v0 + q) ? mem[q] + 1u : 0u;  // (ids stay below NONE)
-    sum += c[q] ? (1ull << 31) + c[q] : 0ull;  // (62 bits travel: both below 2^31)
+    c[q] = hd[q] == uint32_t(v0 + q) ? mem[q] + 1u : 0u;
+    if (WIDE) {
+      sum += c[q];
+      lines += c[q] ? 1u : 0u;
+    } else {
+      sum += c[q] ? (1ull << 31) + c[q] : 0ull;  // (62 bits travel: both below 2^31)
+    }
   }
   unsigned long long tot;
+  uint32_t ltot = 0;
   const unsigned long long pre = block_excl_scan(sum, scan, &tot);
+  if (WIDE) block_excl_scan(lines, lscan, &ltot);
   if (threadIdx.x < 32) {
-    if (threadIdx.x == 0) lb_publish(st, b, LB_SUM, tot);
+    if (threadIdx.x == 0) {
+      lb_publish(st, b, LB_SUM, tot);
+      if (WIDE) lb_publish(st + gridDim.x, b, LB_SUM, ltot);
+    }
     __syncwarp();
     const unsigned long long e = lb_exclusive(st, b, tot, ctl + 1);
-    if (threadIdx.x == 0) s_base = e;
+    const unsigned long long l = WIDE ? lb_exclusive(st + gridDim.x, b, ltot, ctl + 1) : 0ull;
+    if (threadIdx.x == 0) {
+      s_base = e;
+      s_lines = l;
+    }
   }
   __syncthreads();
-  const uint32_t p = uint32_t((s_base + pre) & 0x7FFFFFFFull);
+  const uint32_t p = WIDE ? uint32_t(s_base + pre) : uint32_t((s_base + pre) & 0x7FFFFFFFull);
   const uint4 o = make_uint4(p, p + c[0], p + c[0] + c[1], p + c[0] + c[1] + c[2]);
   if (v0 + 4 <= n) {
     *reinterpret_cast<uint4*>(voff + v0) = o;  // (scratch: aligned)
@@ -3372,10 +3391,12 @@ __global__ void __launch_bounds__(256) k_emit_scan(const uint32_t* __restrict__ 
     if (v0 + 1 < n) voff[v0 + 1] = o.y;
     if (v0 + 2 < n) voff[v0 + 2] = o.z;
   }
-  auto split = [](unsigned long long x) { return ((x >> 31) << 32) | (x & 0x7FFFFFFFull); };
+  auto split = [](unsigned long long x, unsigned long long l) {
+    return WIDE ? (l << 32) | (x & 0xFFFFFFFFull) : ((x >> 31) << 32) | (x & 0x7FFFFFFFull);
+  };
   if (threadIdx.x == 0) {
-    base[b] = split(s_base);
-    if (b == gridDim.x - 1) base[b + 1] = split(s_base + tot);
+    base[b] = split(s_base, s_lines);
+    if (b == gridDim.x - 1) base[b + 1] = split(s_base + tot, s_lines + ltot);
   }
 }
 
@@ -3426,7 +3447,7 @@ __global__ void __launch_bounds__(256) k_emit_lines(const uint64_t* __restrict__
   const uint32_t lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
   uint32_t* buf = buf_all[wid];
   const uint64_t t0 = uint64_t(blockIdx.x) * EMIT_TILE, v0 = t0 + 4u * threadIdx.x;
-  const uint4 h = ld4(head, v0, n, NONE);
+  const uint4 h = ld4(head, v0, n, ~uint32_t(v0));
   const uint32_t mask = (h.x == uint32_t(v0) ? 1u : 0u) | (h.y == uint32_t(v0 + 1) ? 2u : 0u) |
                         (h.z == uint32_t(v0 + 2) ? 4u : 0u) | (h.w == uint32_t(v0 + 3) ? 8u : 0u);
   uint32_t nl;
@@ -4718,7 +4739,9 @@ static int emit_over(cudaStream_t s, int sm_count, const uint64_t* keys, const u
   };
   // cleared: the control words (ticket, wait flag, long lines, heads), the
   // look-back words, the member counts
-  char* z = take(256 + tiles * 8);
+  const bool wide = n >= EMIT_WIDE;
+  const uint64_t zero = 256 + tiles * (wide ? 16 : 8);
+  char* z = take(zero);
   uint32_t* ctl = reinterpret_cast<uint32_t*>(z);
   unsigned long long* heads = reinterpret_cast<unsigned long long*>(z + 16);
   unsigned long long* st = reinterpret_cast<unsigned long long*>(z + 256);
@@ -4729,7 +4752,7 @@ static int emit_over(cudaStream_t s, int sm_count, const uint64_t* keys, const u
   char* chars = take(n + 16);
   const uint64_t want = (n + 255) / 256, gcap = uint64_t(sm_count) * 16;
   const int grid = int(std::max<uint64_t>(1, std::min(want, gcap)));
-  int r = ck(cudaMemsetAsync(z, 0, 256 + tiles * 8, s), "cudaMemsetAsync");
+  int r = ck(cudaMemsetAsync(z, 0, zero, s), "cudaMemsetAsync");
   if (r) return r;
   unsigned long long got = 0;
   if (!out) {
@@ -4744,7 +4767,8 @@ static int emit_over(cudaStream_t s, int sm_count, const uint64_t* keys, const u
   if ((r = ck(cudaMemsetAsync(cnt, 0, n * 4, s), "cudaMemsetAsync"))) return r;
   launches += 2;
   k_count_members<<<grid, 256, 0, s>>>(head, n, cnt);
-  k_emit_scan<<<unsigned(tiles), 256, 0, s>>>(head, cnt, n, voff, base, st, ctl);
+  if (wide) k_emit_scan<true><<<unsigned(tiles), 256, 0, s>>>(head, cnt, n, voff, base, st, ctl);
+  else k_emit_scan<false><<<unsigned(tiles), 256, 0, s>>>(head, cnt, n, voff, base, st, ctl);
   if ((r = ck(cudaGetLastError(), "launch"))) return r;
   if ((r = ck(cudaMemcpyAsync(&got, base + tiles, 8, cudaMemcpyDeviceToHost, s), "cudaMemcpyAsync"))) return r;
   uint32_t c[3] = {0, 0, 0};
@@ -4782,7 +4806,7 @@ static int emit_over(cudaStream_t s, int sm_count, const uint64_t* keys, const u
 uint64_t emit_scratch_bytes(uint64_t n) {
   auto al = [](uint64_t b) { return (b + 255) & ~uint64_t(255); };
   const uint64_t tiles = (n + EMIT_TILE - 1) / EMIT_TILE;
-  return al(256 + tiles * 8) + al((tiles + 1) * 8) + 2 * al(n * 4) + al((n / EMIT_HUGE + 1) * 4) + al(n + 16);
+  return al(256 + tiles * (n >= EMIT_WIDE ? 16 : 8)) + al((tiles + 1) * 8) + 2 * al(n * 4) + al((n / EMIT_HUGE + 1) * 4) + al(n + 16);
 }
 
 int emit(Env& e, const uint64_t* d_keys, const uint32_t* succ, const uint32_t* head, const uint32_t* rank,
@@ -4791,7 +4815,7 @@ int emit(Env& e, const uint64_t* d_keys, const uint32_t* succ, const uint32_t* h
   if (k < 2 || k > 63) return e.fail(UC_EINPUT, "k must be in [2, 63]");
   out_bytes = 0;
   if (n == 0) return UC_OK;
-  if (n >= 0x7FFFFFFFull) return e.fail(UC_EINPUT, "too many k-mers for 31-bit ids");
+  if (n > 0xFFFFFFFFull) return e.fail(UC_EINPUT, "too many k-mers for 32-bit ids");
   e.reset();
   int r = e.reserve(1, emit_scratch_bytes(n) + 4096);
   if (r) return r;
@@ -4807,7 +4831,7 @@ int emit_preload(std::string& err) {
   const void* fns[] = {
       reinterpret_cast<const void*>(k_count_members),
       reinterpret_cast<const void*>(k_count_heads),
-      reinterpret_cast<const void*>(k_emit_scan),
+      reinterpret_cast<const void*>(k_emit_scan<false>),
       reinterpret_cast<const void*>(k_emit_chars<1>),
       reinterpret_cast<const void*>(k_emit_chars<2>),
       reinterpret_cast<const void*>(k_emit_lines<1>),
