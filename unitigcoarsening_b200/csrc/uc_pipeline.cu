@@ -121,6 +121,16 @@ static uint32_t pack_pieces(bool fixed, int k) {
 // raw text, codes, two masks (a line's last words reach past the pieces)
 static size_t pack_smem(uint32_t pieces) { return size_t(pieces) * 16 + (size_t(pieces) + 8) * 8; }
 
+// Bit i to bit 2i.
+__device__ __forceinline__ uint64_t even_bits(uint32_t x) {
+  uint64_t y = x;
+  y = (y | (y << 16)) & 0x0000FFFF0000FFFFull;
+  y = (y | (y << 8)) & 0x00FF00FF00FF00FFull;
+  y = (y | (y << 4)) & 0x0F0F0F0F0F0F0F0Full;
+  y = (y | (y << 2)) & 0x3333333333333333ull;
+  return (y | (y << 1)) & 0x5555555555555555ull;
+}
+
 // The piece v of 16 text bytes: codes (of bytes that are ACGT), possible line
 // breaks (nl: a break where the code is 1, which is checked per line) and
 // other bytes (bad), a bit per byte.  Bits 1 and 2 of a letter are free, the
@@ -424,13 +434,12 @@ __global__ void __launch_bounds__(256, NW == 1 && KC ? 6 : 5) k_pack(const JobTa
         lbad |= check_term && (!(nm & term) || after != 1u);
         key.w[NW - 1] &= kmask_hi;
         if ((nm | bm) & chars) {
-          for (Mask m = (nm | bm) & chars; m; m &= m - 1) {
-            const int i = __ffsll((long long)m) - 1;
-            const bool low = NW == 1 || i < 32;
-            const uint64_t at = 3ull << (2 * (i & 31)), w = low ? key.w[0] : key.w[NW - 1];
-            if (((nm >> i) & 1u) && ((w >> (2 * (i & 31))) & 3u) == 1u) lbad = true;  // a line break
-            if (low) key.w[0] &= ~at;
-            else key.w[NW - 1] &= ~at;
+#pragma unroll
+          for (int w = 0; w < NW; ++w) {
+            const uint64_t nl = even_bits(uint32_t((nm & chars) >> (w ? 32 : 0)));
+            const uint64_t any = even_bits(uint32_t(((nm | bm) & chars) >> (w ? 32 : 0)));
+            if (nl & key.w[w] & ~(key.w[w] >> 1)) lbad = true;  // a line break
+            key.w[w] &= ~(3ull * any);
           }
         }
       } else {
