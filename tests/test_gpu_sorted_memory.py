@@ -13,7 +13,7 @@ MIB = 1 << 20
 EBUDGET = "HBM budget"
 
 
-@pytest.mark.parametrize("k", [31, 63])
+@pytest.mark.parametrize("k", [21, 31, 47, 63])
 @pytest.mark.parametrize("warp_capacity", [0, 1])
 def test_scratch_within_budget(comp, k, warp_capacity):
     n = 4_000_000

@@ -90,6 +90,7 @@ __device__ __forceinline__ void count_bin(uint32_t* counts, uint32_t bin) {
 struct LineRecs {
   char* a = nullptr;
   uint64_t cap = 0;  // records that fit at a
+  uint64_t kmers = 0;
   uint32_t* counts = nullptr;
   int bits = 0;
   uint32_t n = 0;

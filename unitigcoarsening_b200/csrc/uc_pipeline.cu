@@ -3614,7 +3614,7 @@ int Env::reserve(int w, size_t bytes) {
   return UC_OK;
 }
 
-int Env::big_scratch(size_t bytes, char*& p, const char* what, size_t beside) {
+int Env::big_scratch(size_t bytes, char*& p, const char* what) {
   if (bytes > big_cap) {
     if (big_buf) {
       cudaStreamSynchronize(stream);
@@ -3622,7 +3622,7 @@ int Env::big_scratch(size_t bytes, char*& p, const char* what, size_t beside) {
     }
     big_buf = nullptr;
     big_cap = 0;
-    if (bytes + beside > budget) return fail(UC_EBUDGET, what);
+    if (bytes > budget) return fail(UC_EBUDGET, what);
     if (dev_malloc(reinterpret_cast<void**>(&big_buf), bytes) != cudaSuccess) {
       cudaGetLastError();
       big_buf = nullptr;
@@ -5278,6 +5278,7 @@ static int compact_jobs(Env& e, uint32_t njobs, const char* const* texts, const 
     // the scatter's region that does not hold the copies
     recs->a = reinterpret_cast<char*>(pkeys) == region1 ? region2 : region1;
     recs->cap = copies;
+    recs->kmers = N;
     // (no more of them than a sixteenth of the lines, or 16)
     recs->counts = reinterpret_cast<uint32_t*>(f.keys);
     recs->bits = rbits;

@@ -82,9 +82,8 @@ struct Env {
   // Make an arena hold `bytes`; only while nothing is taken from it.
   int reserve(int arena, size_t bytes);
   void reset() { ar[0].used = ar[1].used = 0; }
-  // The oversized tiles' scratch, grown to hold `bytes` (not in pool mode),
-  // which with `beside` more have to fit the budget.
-  int big_scratch(size_t bytes, char*& p, const char* what, size_t beside = 0);
+  // The oversized tiles' scratch, grown to hold `bytes` (not in pool mode).
+  int big_scratch(size_t bytes, char*& p, const char* what);
   int read_ctr();
   int check_err(const Counters* h);
 };
@@ -146,8 +145,7 @@ uint64_t output_bound(size_t text_bytes, int k);
 int compact_streamed(Env& e, const char* h_text, size_t bytes, int k, int l, char* h_out, uint64_t cap,
                      uint64_t& out_bytes, uc_stats* st, uint64_t chunk_lines, uint64_t group_copies);
 // The lines of a job in byte order (sorted output): those of out[0, bytes)
-// and of the records in pre, into out (scratch: what else the arenas hold, or
-// big_scratch).
+// and of the records in pre, into out (scratch: what else the arenas hold).
 int sort_lines(Env& e, char* out, uint64_t bytes, int k, const LineRecs& pre);
 // Leading key bits by which that many lines are counted for sort_lines.
 int line_bin_bits(uint64_t lines, int k);

@@ -57,12 +57,14 @@ constexpr uint32_t CUR_STRIDE = 8;
 
 struct LongLine {
   unsigned long long at;   // offset in the text
+  unsigned long long kept; // of the copy of its chars
   unsigned long long len;  // bytes, line break included
   unsigned long long to;   // of a huge line: offset in the sorted text
 };
 
 struct SortCtr {
-  uint32_t nrec, nlong, nhuge, ntiles;
+  uint32_t nrec, nhuge, ntiles, pad;
+  unsigned long long longs;  // long lines (low half), 16-byte units of their copies (high half)
   uint32_t plan_ticket, tile_ticket, fail;
   uint32_t nover;  // oversized bins
 };
@@ -201,8 +203,9 @@ __global__ void __launch_bounds__(256, 5) k_line_recs(const char* __restrict__ o
         tl = u ? ((s1 >> u) | (s2 << (64 - u))) : s1;
       }
       if (is_long) {
-        const uint32_t i = atomicAdd(&sc->nlong, 1u);
-        longs[i] = LongLine{c0 + s - off0, len + 1, 0ull};
+        const unsigned long long v = atomicAdd(&sc->longs, (((len + 16) >> 4) << 32) | 1ull);
+        const uint32_t i = uint32_t(v);
+        longs[i] = LongLine{c0 + s - off0, (v >> 32) << 4, len + 1, 0ull};
         if (len + 1 >= HUGE_LINE) huge[atomicAdd(&sc->nhuge, 1u)] = i;
         r.tail = TAIL_LONG | i;
       } else {
@@ -468,16 +471,16 @@ __global__ void __launch_bounds__(GRP_THREADS, 2) k_line_group(RecArr<RW> in, Re
 __global__ void __launch_bounds__(256) k_line_keep(const char* __restrict__ out, char* __restrict__ keep,
                                                    const LongLine* __restrict__ longs,
                                                    const uint32_t* __restrict__ huge, const SortCtr* sc) {
-  const uint32_t nlong = sc->nlong, nhuge = sc->nhuge;
+  const uint32_t nlong = uint32_t(sc->longs), nhuge = sc->nhuge;
   const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nwarps = (gridDim.x * blockDim.x) >> 5;
   for (uint32_t i = warp; i < nlong; i += nwarps) {
     const LongLine L = longs[i];
-    if (L.len < HUGE_LINE) copy_bytes(keep + L.at, out + L.at, L.len, threadIdx.x & 31u, 32u);
+    if (L.len < HUGE_LINE) copy_bytes(keep + L.kept, out + L.at, L.len, threadIdx.x & 31u, 32u);
   }
   for (uint32_t h = 0; h < nhuge; ++h) {
     const LongLine L = longs[huge[h]];
     for (unsigned long long x = blockIdx.x * HUGE_LINE; x < L.len; x += gridDim.x * HUGE_LINE)
-      copy_bytes(keep + L.at + x, out + L.at + x, min(HUGE_LINE, L.len - x), threadIdx.x, blockDim.x);
+      copy_bytes(keep + L.kept + x, out + L.at + x, min(HUGE_LINE, L.len - x), threadIdx.x, blockDim.x);
   }
 }
 
@@ -542,7 +545,7 @@ __device__ __forceinline__ void store_lines(char* out, uint64_t at, uint32_t r0,
         const unsigned long long n = __shfl_sync(0xFFFFFFFFu, len, q);
         const unsigned long long o = __shfl_sync(0xFFFFFFFFu, inc - len, q);
         char* p = T.dst + o;
-        const unsigned long long src = longs[i].at;
+        const unsigned long long src = longs[i].kept;
         if (n < HUGE_LINE) copy_bytes(p, keep + src, n, lane, 32u);
         else if (lane == 0) longs[i].to = uint64_t(p - out);  // copied by k_huge_lines
       }
@@ -1005,7 +1008,7 @@ __global__ void __launch_bounds__(256) k_huge_lines(char* out, const char* keep,
   for (uint32_t h = 0; h < nhuge; ++h) {
     const LongLine L = longs[huge[h]];
     for (unsigned long long x = blockIdx.x * HUGE_LINE; x < L.len; x += gridDim.x * HUGE_LINE)
-      copy_bytes(out + L.to + x, keep + L.at + x, min(HUGE_LINE, L.len - x), threadIdx.x, blockDim.x);
+      copy_bytes(out + L.to + x, keep + L.kept + x, min(HUGE_LINE, L.len - x), threadIdx.x, blockDim.x);
   }
 }
 
@@ -1057,7 +1060,10 @@ int sort_lines_rw(Env& e, char* out, uint64_t bytes, int k, const LineRecs& pre)
   // (fewer than OVER_MAX bins hold more than lmax / OVER_MAX lines each)
   const uint32_t big = uint32_t(std::max<uint64_t>(OVER_WINS * win, lmax / OVER_MAX));
   const uint64_t nover = lmax / big + 1, nchunk = lmax / OV_CHUNK + nover + 1;  // at most
-  const uint64_t nlongs = bytes / uint64_t(k + TAIL_MAX + 2) + 1, nhuges = bytes / HUGE_LINE + 1;
+  // a long line holds TAIL_MAX + 2 k-mers or more, and k bytes and one per k-mer
+  const uint64_t nlongs = std::min(bytes / uint64_t(k + TAIL_MAX + 2), pre.kmers / (TAIL_MAX + 2)) + 1;
+  const uint64_t kept = std::min(bytes, pre.kmers + nlongs * uint64_t(k)) + nlongs * 16;
+  const uint64_t nhuges = bytes / HUGE_LINE + 1;
   // more tiles than k_line_group counts at once: groups of 2^gsh first
   uint32_t gsh = 0;
   if (ntmax > GRP_BINS)
@@ -1065,66 +1071,50 @@ int sort_lines_rw(Env& e, char* out, uint64_t bytes, int k, const LineRecs& pre)
   // cleared: the counters and the look-back words
   const size_t zero = 256 + (nplan + ntmax) * 8;
   const size_t ovb = OV_PASSES * 4 + (nover * OV_PASSES / (4 - RW) * 4 + nchunk * 8) * 256;
-  // The job's arrays are used up but for the records and their counts, so the
-  // scratch takes what lies around those in both arenas, and device memory of its own
-  // (the oversized tiles' scratch, free by now) only where that is too little.
-  // Sorted output thus fits where the job itself does, but for jobs with more
-  // text lines than half their k-mers and few cross k-mers.
+  // The job's arrays are used up but for the records and their counts, and the
+  // scratch takes what lies around those in both arenas: sorted output fits where
+  // the job does.  (The second records and tails take one of the scatter's regions;
+  // the front arena's 16 or 24 bytes per k-mer hold the rest, 4 bytes per k-mer of
+  // kept chars at most, 1.1 of their index, and 5 per line.)
   struct Room {
     uintptr_t at, end;
   };
   auto addr = [](const void* p) { return reinterpret_cast<uintptr_t>(p); };
   const uintptr_t mid = addr(pre.a) + pre.cap * 16;  // the tails (two key words)
   const uintptr_t last = RW == 3 ? mid + lmax * 8 : addr(pre.a) + lmax * 16;
-  const Room all[4] = {{addr(e.ar[1].base), addr(pre.a)},
-                       {addr(pre.a) + lmax * 16, RW == 3 ? mid : 0},
-                       {last, addr(e.ar[1].base) + e.ar[1].cap},
-                       {addr(pre.counts) + (size_t(4) << bits), addr(e.ar[0].base) + e.ar[0].cap}};
-  char *own = nullptr, *recs, *tails, *keep, *z, *p_longs, *p_cur, *p_gcur, *p_tile, *p_huge, *p_over, *p_item, *p_ov;
-  for (;;) {
-    Room room[4];
-    std::copy(all, all + 4, room);
-    size_t more = 0;
-    auto take = [&](size_t b) {
-      for (Room& r : room) {
-        const uintptr_t at = (r.at + 255) & ~uintptr_t(255);
-        if (at + b > r.end) continue;
-        r.at = at + b;
-        return reinterpret_cast<char*>(at);
-      }
-      char* const p = own + more;
-      more += (b + 255) & ~size_t(255);
-      return p;
-    };
-    keep = take(bytes + 16);
-    recs = take(lmax * 16);
-    tails = RW == 3 ? take(lmax * 8) : nullptr;
-    z = take(zero);
-    p_longs = take(nlongs * sizeof(LongLine));
-    p_cur = take((ntmax + GRP_BINS) * CUR_STRIDE * 4);
-    p_gcur = take(((ntmax >> gsh) + 1 + GRP_BINS) * CUR_STRIDE * 4);
-    p_tile = take((ntmax + 1) * 8);
-    p_huge = take(nhuges * 4);
-    p_over = take(nover * sizeof(OverBin));
-    p_item = take((nover + 1) * 4);
-    p_ov = take(ovb);
-    if (!more || own) break;
-    const int r = e.big_scratch(more, own, "scratch for sorted output", e.ar[0].cap + e.ar[1].cap);
-    if (r) return r;
-  }
-  const RecArr<RW> ra{reinterpret_cast<ulonglong2*>(pre.a), reinterpret_cast<unsigned long long*>(mid)};
-  const RecArr<RW> rb{reinterpret_cast<ulonglong2*>(recs), reinterpret_cast<unsigned long long*>(tails)};
-  uint2* tile = reinterpret_cast<uint2*>(p_tile);
-  uint32_t* cur = reinterpret_cast<uint32_t*>(p_cur);
-  uint32_t* gcur = reinterpret_cast<uint32_t*>(p_gcur);
-  LongLine* longs = reinterpret_cast<LongLine*>(p_longs);
-  uint32_t* huge = reinterpret_cast<uint32_t*>(p_huge);
-  OverBin* over = reinterpret_cast<OverBin*>(p_over);
+  Room room[4] = {{addr(e.ar[1].base), addr(pre.a)},
+                  {addr(pre.a) + lmax * 16, RW == 3 ? mid : 0},
+                  {last, addr(e.ar[1].base) + e.ar[1].cap},
+                  {addr(pre.counts) + (size_t(4) << bits), addr(e.ar[0].base) + e.ar[0].cap}};
+  bool fits = true;
+  auto take = [&](size_t b) -> char* {
+    for (Room& r : room) {
+      const uintptr_t at = (r.at + 255) & ~uintptr_t(255);
+      if (at + b > r.end) continue;
+      r.at = at + b;
+      return reinterpret_cast<char*>(at);
+    }
+    fits = false;
+    return nullptr;
+  };
+  char* recs = take(lmax * 16);
+  char* tails = RW == 3 ? take(lmax * 8) : nullptr;
+  char* keep = take(kept);
+  char* z = take(zero);
+  uint2* tile = reinterpret_cast<uint2*>(take((ntmax + 1) * 8));
+  uint32_t* cur = reinterpret_cast<uint32_t*>(take((ntmax + GRP_BINS) * CUR_STRIDE * 4));
+  uint32_t* gcur = reinterpret_cast<uint32_t*>(take(((ntmax >> gsh) + 1 + GRP_BINS) * CUR_STRIDE * 4));
+  LongLine* longs = reinterpret_cast<LongLine*>(take(nlongs * sizeof(LongLine)));
+  uint32_t* huge = reinterpret_cast<uint32_t*>(take(nhuges * 4));
+  OverBin* over = reinterpret_cast<OverBin*>(take(nover * sizeof(OverBin)));
   OverBins ov{};
   ov.bin = over;
-  ov.item_start = reinterpret_cast<uint32_t*>(p_item);
-  ov.ticket = reinterpret_cast<uint32_t*>(p_ov);
+  ov.item_start = reinterpret_cast<uint32_t*>(take((nover + 1) * 4));
+  ov.ticket = reinterpret_cast<uint32_t*>(take(ovb));
   ov.hist = ov.ticket + OV_PASSES;
+  if (!fits) return e.fail(UC_EBUDGET, "scratch for sorted output");
+  const RecArr<RW> ra{reinterpret_cast<ulonglong2*>(pre.a), reinterpret_cast<unsigned long long*>(mid)};
+  const RecArr<RW> rb{reinterpret_cast<ulonglong2*>(recs), reinterpret_cast<unsigned long long*>(tails)};
   SortCtr* sc = reinterpret_cast<SortCtr*>(z);
   unsigned long long* st_plan = reinterpret_cast<unsigned long long*>(z + 256);
   unsigned long long* st_tile = st_plan + nplan;
