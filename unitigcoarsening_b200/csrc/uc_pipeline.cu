@@ -3572,7 +3572,8 @@ int Env::fail(int code, const std::string& msg) {
 }
 
 cudaError_t Env::dev_malloc(void** p, size_t bytes) {
-  if (faults.fail_alloc_after && --faults.fail_alloc_after == 0) {
+  fault_hit = faults.fail_alloc_after && --faults.fail_alloc_after == 0;
+  if (fault_hit) {
     *p = nullptr;
     return cudaErrorMemoryAllocation;
   }
@@ -3955,7 +3956,9 @@ static uint32_t ceil_log2(uint64_t x) {
   return b;
 }
 
-static Plan plan_buckets(const Env& e, uint64_t nmax, uint32_t njobs, int k, int l) {
+// lean: for a job that does not fit otherwise; l-mers as short as the buckets allow,
+// which make fewer cross k-mers (and larger tiles).
+static Plan plan_buckets(const Env& e, uint64_t nmax, uint32_t njobs, int k, int l, bool lean = false) {
   Plan P{};
   const int nw = (k <= 31) ? 1 : 2;
   uint32_t cap = e.tune.tile_capacity ? e.tune.tile_capacity : 4096;
@@ -3989,7 +3992,7 @@ static Plan plan_buckets(const Env& e, uint64_t nmax, uint32_t njobs, int k, int
   // and 3.32; 257M, k = 31, l = 13 and 14: 9.27 and 8.86 (15: the whole job is
   // as long as at 13).
   int lmin = int((jb + 2 + 1) / 2);
-  while (lmin < std::min(16, k - 1) && 20.0 * std::ldexp(1.0, 2 * lmin) < double(nmax) * double(k - lmin)) ++lmin;
+  while (!lean && lmin < std::min(16, k - 1) && 20.0 * std::ldexp(1.0, 2 * lmin) < double(nmax) * double(k - lmin)) ++lmin;
   int lu = std::max(l, lmin);
   lu = std::min(lu, std::min(16, k - 1));
   // hash slots per 100 copies: 300 for warp tiles (a table of 1024 slots at 218
@@ -5065,7 +5068,8 @@ void batch_footprint(const Env& e, uint32_t njobs, const size_t* bytes, int k, i
 // lines are left as records in the scatter's spare region; out_len counts the
 // text lines alone.
 static int compact_jobs(Env& e, uint32_t njobs, const char* const* texts, const size_t* bytes, int k, int l, char* out,
-                        uint64_t out_cap, uint64_t* out_off, uint64_t* out_len, uc_stats* st, LineRecs* recs) {
+                        uint64_t out_cap, uint64_t* out_off, uint64_t* out_len, uc_stats* st, LineRecs* recs,
+                        bool lean = false) {
   if (k < 2 || k > 63) return e.fail(UC_EINPUT, "k must be in [2, 63]");
   if (l < 1 || l > 16 || l > k - 1) return e.fail(UC_EINPUT, "l must be in [1, min(16, k-1)]");
   if (njobs == 0) return UC_OK;
@@ -5116,7 +5120,7 @@ static int compact_jobs(Env& e, uint32_t njobs, const char* const* texts, const 
   }
   if (N >= 0x7FFFFFFFull) return e.fail(UC_EINPUT, "too many k-mers for 31-bit ids");
   if (ob > out_cap + 15) return e.fail(UC_EINPUT, "output buffer smaller than uc_output_bound");
-  const Plan P = plan_buckets(e, nmax, njobs, k, l);
+  const Plan P = plan_buckets(e, nmax, njobs, k, l, lean);
   r = e.reserve(0, front_bytes(N, nw, P.M, true));
   if (r) return r;
   Front f{};
@@ -5190,7 +5194,6 @@ static int compact_jobs(Env& e, uint32_t njobs, const char* const* texts, const 
     if (e.h_ctr->err & ERR_LAYOUT) return e.fail(UC_EINPUT, "a k-mer line is shorter than k");
     return e.check_err(e.h_ctr);
   }
-  if (e.after_pack) e.after_pack();
   const uint64_t X = copies - N;
   // segment ids: [0, X) the segments that start at a cross k-mer's S-only
   // copy; then each job's head pool (a line's first open segment ends at a
@@ -5222,7 +5225,10 @@ static int compact_jobs(Env& e, uint32_t njobs, const char* const* texts, const 
   // (half of the k-mers start a line at most in canonical input)
   const int rbits = recs ? line_bin_bits(N / 2, k) : 0;
   r = e.reserve(1, back);
+  if (!lean && e.too_large(r) && plan_buckets(e, nmax, njobs, k, l, true).l_used < P.l_used)
+    return compact_jobs(e, njobs, texts, bytes, k, l, out, out_cap, out_off, out_len, st, recs, true);
   if (r) return r;
+  if (e.after_pack) e.after_pack();
   auto T64 = [&](uint64_t c) { return static_cast<unsigned long long*>(e.take(1, c * 8)); };
   auto T32 = [&](uint64_t c) { return static_cast<uint32_t*>(e.take(1, c * 4)); };
   char* region1 = static_cast<char*>(e.take(1, scatter_stage_bytes(copies, nw)));
@@ -5392,7 +5398,7 @@ int compact_batch(Env& e, uint32_t njobs, const char* const* texts, const size_t
 // indices and segment ids 31-bit.  Lines must be k chars + '\n' (the layout
 // the chunks are cut on).  Unsorted output only.
 int compact_streamed(Env& e, const char* h_text, size_t bytes, int k, int l, char* h_out, uint64_t cap,
-                     uint64_t& out_bytes, uc_stats* st, uint64_t chunk_lines, uint64_t group_copies) {
+                     uint64_t& out_bytes, uc_stats* st, uint64_t chunk_lines, uint64_t group_copies, bool lean) {
   out_bytes = 0;
   if (k < 2 || k > 63) return e.fail(UC_EINPUT, "k must be in [2, 63]");
   if (l < 1 || l > 16 || l > k - 1) return e.fail(UC_EINPUT, "l must be in [1, min(16, k-1)]");
@@ -5423,7 +5429,7 @@ int compact_streamed(Env& e, const char* h_text, size_t bytes, int k, int l, cha
   if (!chunk_lines) chunk_lines = 64ull << 20;
   if (!group_copies) group_copies = 256ull << 20;
   chunk_lines = std::min(chunk_lines, n);
-  const Plan P = plan_buckets(e, n, 1, k, l);
+  const Plan P = plan_buckets(e, n, 1, k, l, lean);
   const size_t chunk_text = size_t(chunk_lines * stride + 64);
   int r = e.reserve(0, front_bytes(chunk_lines, nw, P.M, true) + chunk_text + 4096);
   if (r) return r;
@@ -5533,6 +5539,8 @@ int compact_streamed(Env& e, const char* h_text, size_t bytes, int k, int l, cha
   const bool want_hec = e.tune.contract_method == UC_CONTRACT_HEC;
   const uint32_t RH = hec_rounds(e, Sp);
   r = e.reserve(1, back_bytes(e, copies, X, Sp, nw, k, want_hec) + gout + sout + 4096);
+  if (!lean && e.too_large(r) && plan_buckets(e, n, 1, k, l, true).l_used < P.l_used)
+    return compact_streamed(e, h_text, bytes, k, l, h_out, cap, out_bytes, st, chunk_lines, group_copies, true);
   if (r) return r;
   auto T64 = [&](uint64_t c) { return static_cast<unsigned long long*>(e.take(1, c * 8)); };
   auto T32 = [&](uint64_t c) { return static_cast<uint32_t*>(e.take(1, c * 4)); };

@@ -66,9 +66,10 @@ struct Env {
   // whole-job calls (compact_device and the paths built on it) leave the
   // lines in byte order
   bool sorted = false;
-  // called by the fused path once the job is packed (its layout is confirmed)
-  // and ev[1] recorded after the pack kernels: from then on the job's text is no longer read, so
-  // a host pipeline can upload the next job's text into the same buffer
+  // called by the fused path once the job is packed, its layout is confirmed and
+  // its arrays fit, with ev[1] recorded after the pack kernels: from then on the
+  // job's text is no longer read, so a host pipeline can upload the next job's
+  // text into the same buffer
   std::function<void()> after_pack;
   // failure injection (uc_ctx_set_faults); zeros = off
   uc_faults faults{};
@@ -78,6 +79,9 @@ struct Env {
   // Every device allocation of a context goes through here, so that
   // faults.fail_alloc_after can make one fail as out of memory.
   cudaError_t dev_malloc(void** p, size_t bytes);
+  bool fault_hit = false;  // the last one was made to fail
+  // a reserve failed for want of room
+  bool too_large(int r) const { return r == UC_EBUDGET || (r == UC_ENOMEM && !fault_hit); }
   void* take(int arena, size_t bytes);
   // Make an arena hold `bytes`; only while nothing is taken from it.
   int reserve(int arena, size_t bytes);
@@ -143,7 +147,7 @@ uint64_t output_bound(size_t text_bytes, int k);
 // (two passes over the text) and tile groups of about group_copies copies,
 // for jobs whose text and lines exceed the device budget (0 = defaults).
 int compact_streamed(Env& e, const char* h_text, size_t bytes, int k, int l, char* h_out, uint64_t cap,
-                     uint64_t& out_bytes, uc_stats* st, uint64_t chunk_lines, uint64_t group_copies);
+                     uint64_t& out_bytes, uc_stats* st, uint64_t chunk_lines, uint64_t group_copies, bool lean = false);
 // The lines of a job in byte order (sorted output): those of out[0, bytes)
 // and of the records in pre, into out (scratch: what else the arenas hold).
 int sort_lines(Env& e, char* out, uint64_t bytes, int k, const LineRecs& pre);
