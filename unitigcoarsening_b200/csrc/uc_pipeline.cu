@@ -106,7 +106,7 @@ __device__ __forceinline__ uint32_t base_code(uint32_t c) {
 // With FUSE the prefix/suffix minimizer buckets of every key are computed and
 // counted in the same pass (lmin_buckets.h:299-318).
 //
-// Bound by instruction issue (79% at 30 Mbp, k = 31).  256 Mbp, k = 31:
+// Bound by the ALU pipe (half rate: 76% at 30 Mbp, k = 31).  256 Mbp, k = 31:
 // 3.6 ms (8.2 GB of text); 6.3 ms when each thread converted its own line
 // from staged text, 3.8 ms with bits per byte for every piece.
 constexpr int PACK_LINES = 512;
@@ -1533,24 +1533,6 @@ struct WarpGroup {
   static __device__ __forceinline__ uint32_t rank() { return threadIdx.x & 31u; }
   static __device__ __forceinline__ uint32_t size() { return 32u; }
   static __device__ __forceinline__ void sync() { __syncwarp(); }
-  static __device__ __forceinline__ int sync_or(int v) { return __any_sync(0xFFFFFFFFu, v); }
-  // a warp tile's totals fit 32 bits (at most 256 copies)
-  static __device__ __forceinline__ U3 scan3(U3 v, U3* total) {
-    const int lane = threadIdx.x & 31;
-    uint32_t a = uint32_t(v.a), b = uint32_t(v.b), c = uint32_t(v.c);
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t ta = __shfl_up_sync(0xFFFFFFFFu, a, o), tb = __shfl_up_sync(0xFFFFFFFFu, b, o),
-                     tc = __shfl_up_sync(0xFFFFFFFFu, c, o);
-      if (lane >= o) {
-        a += ta;
-        b += tb;
-        c += tc;
-      }
-    }
-    *total = U3{__shfl_sync(0xFFFFFFFFu, a, 31), __shfl_sync(0xFFFFFFFFu, b, 31), __shfl_sync(0xFFFFFFFFu, c, 31)};
-    return U3{a - uint32_t(v.a), b - uint32_t(v.b), c - uint32_t(v.c)};
-  }
   static __device__ __forceinline__ bool reserve(const TileParams& p, uint32_t job, const U3& tot,
                                                  unsigned long long* base) {
     unsigned long long b[3] = {0, 0, 0};
@@ -1594,9 +1576,10 @@ __device__ void jump_rounds(uint32_t c, IT* px, IT* rx, IT* py, IT* ry, IT*& ptr
 // text of 32 segments at a time is spelled into shared memory from those codes
 // and leaves as 16-byte stores.  Against ranking the copies by pointer jumping
 // and storing each copy's char by itself: 64 Mbp, k = 63, the kernel takes
-// 2.36 instead of 3.01 ms; at k = 31 it is as long (8.7 ms at 256 Mbp), with
-// half as many stores.  Segments with more than TAIL_MAX later chars store
-// them byte by byte.
+// 2.36 instead of 3.01 ms; at k = 31 it was as long either way, with half as many
+// stores.  (Now, with longer tables and closed lines as records: 1.77 ms, and 6.4
+// at 256 Mbp, k = 31.)  Segments with more than TAIL_MAX later chars store them
+// byte by byte.
 template <int NW, int KC>
 __device__ __forceinline__ void emit_warp_tile(const TileParams& p, const TileMem<NW, uint16_t>& m, uint64_t beg,
                                                uint32_t c, uint32_t job, unsigned long long& rec_bytes) {
@@ -2788,7 +2771,6 @@ __global__ void k_seg_cycles(Counters* ctr, uint32_t S, const uint32_t* __restri
 // enough.  (2M k-mers, k = 63: 0.40 ms for the call; six launches per round for
 // the 50 rounds of the bound took 1.78, most of them on empty levels.)
 constexpr uint32_t HV_UNSET = 0xFFFFFFFFu, HV_LOCK = 0xFFFFFFFEu, HV_FIN = 0xFFFFFFFDu, HV_CYC = 0xFFFFFFFCu;
-constexpr uint32_t HP_SENT = 0xFFFFFFFBu;  // coarse node not yet given a first member
 
 struct HecPool {
   uint32_t *prv, *nxt, *wt, *hn, *vc, *agg, *loc, *first0;
@@ -2991,7 +2973,7 @@ __device__ __forceinline__ bool hec_round(const HecPool& h, uint32_t r, uint32_t
         atomicOr(err, ERR_CAPACITY);
       } else {
         h.hn[b + j0 + threadIdx.x + q * span] = a;
-        h.prv[a] = HP_SENT;
+        h.prv[a] = NONE;
         h.nxt[a] = NONE;
         h.wt[a] = 0;
         h.first0[a] = NONE;
@@ -4901,13 +4883,7 @@ static uint32_t walk_cap(const Env& e) {
 }
 static uint64_t long_cap(const Env& e, uint64_t X) { return X / walk_cap(e) + 64; }
 
-// The cross-tile stitch over X cross-indexed segments and Hp head-pool ids,
-// into out after each job's closed lines (jd.jout: each job's byte count,
-// closed lines before, all lines after): the line walk, then, for the
-// lines it leaves and for cycles, ranking (pointer jumping, or HEC with
-// pointer jumping when its rounds run out), line lengths at the heads, one
-// reservation per line, the segment copies, and the rare segment cycles.
-// The walk alone: enqueued (counters walked and left zero before).
+// The stitch's line walk alone, enqueued (its counters, walked and left, are zero before).
 static int launch_walk(Env& e, const StitchBufs& b, uint64_t X, uint64_t Hp, int k, const JobDev& jd, char* out,
                        bool guard) {
   ++e.launches;
@@ -4916,6 +4892,12 @@ static int launch_walk(Env& e, const StitchBufs& b, uint64_t X, uint64_t Hp, int
   UC_CK(cudaGetLastError());
   return UC_OK;
 }
+// The cross-tile stitch over X cross-indexed segments and Hp head-pool ids,
+// into out after each job's closed lines (jd.jout: each job's byte count,
+// closed lines before, all lines after): the line walk, then, for the
+// lines it leaves and for cycles, ranking (pointer jumping, or HEC with
+// pointer jumping when its rounds run out), line lengths at the heads, one
+// reservation per line, the segment copies, and the rare segment cycles.
 // walked: the walk is done and its counters are in h_ctr.
 static int run_stitch(Env& e, const StitchBufs& b, uint64_t X, uint64_t Hp, int k, int nw, bool want_hec,
                       uint32_t RH, const JobDev& jd, char* out, uint32_t& rounds, bool walked = false) {

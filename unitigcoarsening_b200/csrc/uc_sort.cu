@@ -16,8 +16,8 @@
 // once.  Lines with more than TAIL_MAX chars after the k-mer keep their chars
 // in a copy of the text and are copied.
 //
-// 256 Mbp, k = 31 (107M lines, 3.6 GB) on a B200: 1.9 + 2.2 + 3.0 ms (records,
-// groups, tiles), where a radix sort of (key, line index) pairs with a gather
+// 256 Mbp, k = 31 (107M lines, 3.6 GB, a fifth of them reaching the sort as text) on a
+// B200: 0.42 + 2.2 + 3.0 ms (records, groups, tiles), where a radix sort of (key, line index) pairs with a gather
 // of the lines (seven passes over pairs or lines) took 28 ms.
 #include <algorithm>
 #include <cstring>
@@ -94,8 +94,9 @@ __device__ __forceinline__ unsigned long long line_bytes_of(uint64_t tail, int k
 // words), lists the chunk's line starts from the bits (two words per thread,
 // one block scan), and makes one line's record per thread.
 // The records come in no particular order: a block reserves the places of its
-// lines with one atomic.  256 Mbp, k = 31: 1.9 ms for 5.3 GB, bound by issue
-// (60%) and barriers; converting each line from staged text instead took 2.3.
+// lines with one atomic.  256 Mbp, k = 31: 0.42 ms for the lines that are not
+// records already; 1.9 ms when it took all of them (5.3 GB), bound by issue (60%)
+// and barriers, where converting each line from staged text took 2.3.
 template <int RW>
 __global__ void __launch_bounds__(256, 5) k_line_recs(const char* __restrict__ out, uint64_t n, int k, int bits,
                                                    RecArr<RW> rec, uint32_t* __restrict__ counts,
@@ -836,9 +837,9 @@ __host__ __device__ constexpr size_t tile_smem(int k) {
 // shared-memory atomics, and each record's final rank is its sub-bin's start
 // plus the smaller records in the sub-bin.  The tile's first byte comes from
 // the look-back over the tiles' byte counts.  Then each warp stores a run of
-// ranks (store_lines).  256 Mbp, k = 31: 3.0 ms for 5.3 GB, issue-bound (about
-// 650 instructions per line, spelling the most of them); 3.5 ms with three
-// blocks per SM instead of four.
+// ranks (store_lines).  256 Mbp, k = 31: 3.0 ms for 5.3 GB, bound by shared memory
+// (67% of L1 throughput) and issue (63%; about 650 instructions per line, spelling
+// the most of them); 3.5 ms with three blocks per SM instead of four.
 template <int RW>
 __global__ void __launch_bounds__(TILE_THREADS, RW == 2 ? 4 : 3) k_line_tiles(RecArr<RW> rec, RecArr<RW> spare,
                                                              const uint2* __restrict__ tile, int bits, char* out, int k,
