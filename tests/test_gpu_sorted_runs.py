@@ -79,6 +79,37 @@ def test_line_lengths_in_a_bin(comp, oracle, k, warp_capacity):
         comp.set_tuning(warp_capacity=0)
 
 
+@pytest.mark.parametrize("k", [31, 63])
+def test_a_hundred_bins(comp, oracle, k):
+    kmers = []
+    for i in range(100):
+        pre = "".join("ACGT"[(i * 41 >> (2 * j)) & 3] for j in range(6)) + "GAT"
+        kmers += [pre + x for x in others(1251 + i, k - len(pre), 700 + i)]
+    check(comp, oracle, kmers + others(500, k, 1), k)
+
+
+@pytest.mark.parametrize("k", [31, 63])
+@pytest.mark.parametrize("bins,n", [(1200, 5200), (3, 1_500_000)])
+def test_millions_of_lines_in_bins(comp, k, bins, n):
+    """Unrelated k-mers, so every line is one of them: the text sorted."""
+    from unitigcoarsening_b200 import synth
+    v = torch.arange(bins * n, device="cuda")
+    w = synth._srl(synth.rand_u64(9, 3, v), 64 - 2 * 31)
+    w = (w & ((1 << 38) - 1)) | ((v // n * 7919 + 3) << 38)
+    if k == 63:
+        w = torch.stack([((w << 2) | (v & 3)) ^ (-(1 << 63)), synth._srl(synth.rand_u64(9, 4, v), 64 - 2 * 31)], 1)
+        w = synth._unique_rows(w)
+    else:
+        w = torch.unique(w)
+    text = synth.format_text(synth.shuffle(w, 1), k)
+    comp.set_sorted_output(True)
+    try:
+        got = comp.compact(text, k, 8)
+    finally:
+        comp.set_sorted_output(False)
+    assert torch.equal(got, synth.kmers_to_lines(w, k).flatten())
+
+
 def test_shared_prefix_is_not_slow(comp):
     """300,000 lines with one prefix among a million others: ordering them costs
     at most as much as the rest of the call does twice over (it costs less than
