@@ -77,8 +77,9 @@ uc_status uc_ctx_sync(uc_ctx *ctx);
 /* Deterministic output: with on != 0, uc_compact_device, uc_compact_host,
  * uc_job_* and uc_compact_file leave the lines in byte order, so equal input
  * gives byte-equal output.  The reference appends lines in an order that
- * varies from run to run (compact.h:7-37); sorting costs one radix sort of
- * the lines by their first k-mer and one copy of the output.  Batches
+ * varies from run to run (compact.h:7-37); here the lines are sorted as
+ * records of their first k-mer and later chars, about a quarter of a call,
+ * without more device memory than the job itself.  Batches
  * (uc_compact_batch) are not reordered. */
 uc_status uc_ctx_set_sorted_output(uc_ctx *ctx, int on);
 uc_status uc_ctx_set_tuning(uc_ctx *ctx, const uc_tuning *t);

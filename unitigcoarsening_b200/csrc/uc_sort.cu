@@ -11,14 +11,15 @@
 //   k_line_tiles   one block per tile: order in shared memory, the tile's
 //                  place in the output by look-back, lines spelled and stored
 // Nothing returns to the host in between, unless a bin holds many tiles' worth
-// of lines (low-complexity k-mers: thousands of lines with the same first chars).
-// Such bins are sorted by the whole grid first (k_over_count, k_over_pass).  The text is read once and written
-// once.  Lines with more than TAIL_MAX chars after the k-mer keep their chars
-// in a copy of the text and are copied.
+// of lines (low-complexity k-mers: thousands of lines with the same first
+// chars).  Such bins are sorted by the whole grid first (k_over_count,
+// k_over_pass).  The text is read once and written once.  Lines with more than
+// TAIL_MAX chars after the k-mer keep their chars in a copy and are copied.
 //
-// 256 Mbp, k = 31 (107M lines, 3.6 GB, a fifth of them reaching the sort as text) on a
-// B200: 0.42 + 2.2 + 3.0 ms (records, groups, tiles), where a radix sort of (key, line index) pairs with a gather
-// of the lines (seven passes over pairs or lines) took 28 ms.
+// 256 Mbp, k = 31 (107M lines, 3.6 GB, a fifth of them reaching the sort as
+// text) on a B200: 0.42 + 2.2 + 3.0 ms (records, groups, tiles), where a radix
+// sort of (key, line index) pairs with a gather of the lines (seven passes over
+// pairs or lines) took 28 ms.
 #include <algorithm>
 #include <cstring>
 #include <utility>
